@@ -538,37 +538,24 @@ int gpw_taskset_create(gpw_plan *plan, const gpw_task *tasks, int64_t ntasks, in
     }
     T->coef_len = coef;
     T->mom_ext_len = mom_ext;
-    // FP64 launch chunks: similar shared-memory needs launch together
-    int64_t k = 0;
-    int smem_limit = 0;
+    // what one CTA holds
+    int smem_limit = 0, sms = 1;
     cudaDeviceGetAttribute(&smem_limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, plan->device);
-    while (k < ntasks) {
-        Chunk c;
-        c.first = (int)k;
-        c.kind = T->h_geom[k].ortho ? 0 : 1;
-        c.smem_bytes = 0;
-        c.smem_ext = 0;
-        int64_t m = k;
-        while (m < ntasks && (T->h_geom[m].ortho ? 0 : 1) == c.kind) {
-            const int need = c.kind == 0 ? smem_ortho_fp64(T->h_geom[m]) : smem_general_fp64(T->h_geom[m]);
-            const int need_ext = c.kind == 0 ? smem_ortho_fp64(T->h_geom[m], 2) : smem_general_fp64(T->h_geom[m], 2);
-            c.smem_ext = std::max(c.smem_ext, std::min(need_ext, smem_limit));
-            if (need > smem_limit) {
-                delete T;
-                return fail(GPW_ERR_UNSUPPORTED, "gpw_taskset_create: a cube is too large for one CTA");
-            }
-            if (m > k && need * 2 < c.smem_bytes && m - k >= 64) break;
-            c.smem_bytes = std::max(c.smem_bytes, need);
-            m++;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, plan->device);
+    for (const PairGeom &g : T->h_geom)
+        if ((g.ortho ? smem_ortho_fp64(g) : smem_general_fp64(g)) > smem_limit) {
+            delete T;
+            return fail(GPW_ERR_UNSUPPORTED, "gpw_taskset_create: a cube is too large for one CTA");
         }
-        c.count = (int)(m - k);
-        T->chunks.push_back(c);
-        k = m;
-    }
+    std::vector<Fp64Item> items;
+    fp64_items(*T, sms, smem_limit, items);
     // general-cell pairs (sorted after the orthorhombic ones) for the float-float kernel
     for (int64_t m = 0; m < ntasks; m++) {
         if (T->h_geom[m].ortho) continue;
-        if (T->gen_count == 0) T->gen_first = (int)m;
+        if (T->gen_count == 0) {
+            T->gen_first = (int)m;
+            T->gen_coef_first = T->h_geom[m].coef_off;
+        }
         T->gen_count++;
         T->gen_smem = std::max(T->gen_smem, smem_general_ff(T->h_geom[m]));
     }
@@ -589,6 +576,9 @@ int gpw_taskset_create(gpw_plan *plan, const gpw_task *tasks, int64_t ntasks, in
     alloc((void **)&T->d_coef, sizeof(double) * (size_t)coef);
     alloc((void **)&T->d_mom, sizeof(double) * (size_t)coef);
     alloc((void **)&T->d_status, sizeof(int));
+    alloc((void **)&T->d_fp64_items, sizeof(Fp64Item) * items.size());
+    if (e == cudaSuccess && !items.empty())
+        e = cudaMemcpy(T->d_fp64_items, items.data(), sizeof(Fp64Item) * items.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && ntasks > 0)
         e = cudaMemcpy(T->d_geom, T->h_geom.data(), sizeof(PairGeom) * (size_t)ntasks, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !table.empty())
@@ -624,6 +614,7 @@ int gpw_taskset_destroy(gpw_taskset *ts) {
     cudaFree(ts->d_geom);
     cudaFree(ts->d_geom_next);
     cudaFree(ts->d_table);
+    cudaFree(ts->d_fp64_items);
     cudaFree(ts->d_coef);
     cudaFree(ts->d_mom);
     cudaFree(ts->d_mom_ext);

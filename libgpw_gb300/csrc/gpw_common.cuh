@@ -110,6 +110,50 @@ GPW_HD int rule_imax(double remk, int jf, double hy, double hx) {
 }
 GPW_HD int fold(int g) { return g <= 0 ? g : 1 - g; }
 
+#if defined(__CUDACC__)
+// Sphere rule with an FP32 fast path.  The FP32 estimate decides unless it lies
+// within its error bound of an integer; then the exact FP64 rule above (the one
+// the host and the oracle use) decides.
+__device__ __forceinline__ int fast_floor_checked(float rem, float r2f, float hinv, bool &unsure) {
+    const float rc = fmaxf(rem, 0.0f);
+    const float rs = rsqrtf(fmaxf(rc, 1e-30f));
+    const float v = __fmul_rn(__fmul_rn(rc, rs), hinv);  // sqrt(rc) / h, relative error < 2^-21
+    const float fl = floorf(v);
+    // error of rem ~ 4 ulp(r2f); of sqrt ~ err/(2 sqrt); plus relative 2^-19
+    const float erem = r2f * 4.8e-7f;
+    const float ev = __fmul_rn(erem * 0.5f, rs) * hinv + v * 2e-6f + 1e-6f;
+    unsure = (v - fl) <= ev || (fl + 1.0f - v) <= ev || rem <= erem;
+    return (int)fl;
+}
+
+// The rule's constants of one pair in both precisions.
+struct SphereRule {
+    double r2, hz, hy, hx;
+    float r2f, hzf, hyf, hyinvf, hxinvf;
+    __device__ SphereRule(double radius, double hx_, double hy_, double hz_)
+        : r2(rmul(radius, radius)), hz(hz_), hy(hy_), hx(hx_), r2f((float)r2), hzf((float)hz_), hyf((float)hy_),
+          hyinvf(1.0f / hyf), hxinvf(1.0f / (float)hx_) {}
+};
+__device__ __noinline__ inline int sphere_jmax_exact(double r2, double hz, double hy, int kf) {
+    return rule_jmax(rule_remk(r2, kf, hz), hy);
+}
+__device__ __noinline__ inline int sphere_imax_exact(double r2, double hz, double hy, double hx, int kf, int jf) {
+    return rule_imax(rule_remk(r2, kf, hz), jf, hy, hx);
+}
+__device__ __forceinline__ int sphere_jmax_fast(const SphereRule &s, int kf) {
+    const float dz = (float)(-kf) * s.hzf;
+    bool unsure;
+    const int j = fast_floor_checked(__fmaf_rn(-dz, dz, s.r2f), s.r2f, s.hyinvf, unsure);
+    return unsure ? sphere_jmax_exact(s.r2, s.hz, s.hy, kf) : j;
+}
+__device__ __forceinline__ int sphere_imax_fast(const SphereRule &s, int kf, int jf) {
+    const float dz = (float)(-kf) * s.hzf, dy = (float)(-jf) * s.hyf;
+    bool unsure;
+    const int i = fast_floor_checked(__fmaf_rn(-dy, dy, __fmaf_rn(-dz, dz, s.r2f)), s.r2f, s.hxinvf, unsure);
+    return unsure ? sphere_imax_exact(s.r2, s.hz, s.hy, s.hx, kf, jf) : i;
+}
+#endif
+
 // Grid index of cube offset g on one axis (grid_base_ref_c.cc:318-351): periodic
 // axes wrap; non-periodic axes address a local window and return -1 outside it.
 GPW_HD int axis_index(int periodic, int cc, int g, int lbc, int lbg, int npts, int ngrid) {
@@ -186,6 +230,11 @@ struct PairGeom {
     double rab[3];
     int ext0[3];       // general: the box extents the task set was planned with
     int pad_;
+};
+
+// One CTA's work in the FP64 launches: planes part, part + nparts, ... of a pair.
+struct Fp64Item {
+    int pair, part, nparts;
 };
 
 // Device status bits (OR-ed by kernels, read by gpw_taskset_check).

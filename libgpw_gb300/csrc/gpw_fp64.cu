@@ -1,50 +1,18 @@
-// Plain FP64 collocate / integrate: one CTA per pair, FP64 everywhere, grid
-// updates by FP64 atomics.  This is the straightforward GPU form of the
+// Plain FP64 collocate / integrate: FP64 everywhere, one CTA per pair or per part
+// of a pair's planes, grid updates by FP64 atomics.  The GPU form of the
 // reference's per-pair loops (grid_collocate_core, grid_base_ref_c.cc:403-508;
 // grid_collocate_general, :593-846) and the denominator the tiled path is
 // measured against.
 #include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cmath>
 
 #include "gpw_coef.cuh"
 #include "gpw_ff.cuh"
 #include "gpw_internal.h"
 
 namespace gpw {
-
-// ---------------------------------------------------------------------------
-// cube lists: sphere rule or explicit (random-access) table
-// table layout at g.table_off: kgmin, then (jgmin, rowstart) per kf, then igmin per row
-__device__ __forceinline__ int cube_jgmin(const PairGeom &g, const LevelDev &lv, const int *table,
-                                          int kf, double r2, double &remk) {
-    if (g.table_off < 0) {
-        remk = rule_remk(r2, kf, lv.dh[2][2]);
-        return -rule_jmax(remk, lv.dh[1][1]);
-    }
-    const int *T = table + g.table_off;
-    remk = 0.0;
-    return T[1 + 2 * (kf - T[0])];
-}
-__device__ __forceinline__ int cube_igmin(const PairGeom &g, const LevelDev &lv, const int *table,
-                                          int kf, int jf, int jgmin, double remk) {
-    if (g.table_off < 0) return -rule_imax(remk, jf, lv.dh[1][1], lv.dh[0][0]);
-    const int *T = table + g.table_off;
-    const int nk = 1 - T[0];
-    return T[1 + 2 * nk + T[2 + 2 * (kf - T[0])] + (jf - jgmin)];
-}
-
-// 1-D tables tab[k][gi] = t^k exp(-zetp t^2), t = (lo+gi)*h - off, k < L  (grid_fill_pol,
-// grid_base_ref_c.cc:355-400; evaluated directly instead of by recurrence)
-__device__ __forceinline__ void fill_table(double *tab, int n, int L, int lo, double h, double off,
-                                           double zetp) {
-    for (int gi = threadIdx.x; gi < n; gi += blockDim.x) {
-        const double t = (double)(lo + gi) * h - off;
-        double e = exp(-zetp * t * t);
-        for (int k = 0; k < L; k++) {
-            tab[k * n + gi] = e;
-            e *= t;
-        }
-    }
-}
 
 // ---------------------------------------------------------------------------
 // pair set-up: packed coefficients c (ortho) or q (general, lattice basis)
@@ -153,148 +121,280 @@ __global__ void k_backtransform(const PairGeom *__restrict__ geoms, const LevelD
 }
 
 // ---------------------------------------------------------------------------
-// orthorhombic collocate, one CTA per pair
-int smem_ortho_fp64(const PairGeom &g, int extra) {
+// Orthorhombic pairs.  An FP64 multiply-add costs 64 float instructions here
+// (two lanes per cycle and SM), so the kernel is laid out to run little else on
+// the FP64 pipe: about L of them per cube point.
+//
+// A CTA (4 warps) takes one item: every nparts-th plane of a pair's cube.  The
+// three 1-D tables are built once per CTA; after that the warps work alone, one
+// plane at a time, with no CTA barrier:
+//   lane = x column (blocks of 32 columns; the last block of 32, 16 or 8, with the
+//   warp's other lanes on the following rows), so that
+//   collocate  T[ly] = sum_lx Cxy[ly][lx] X[lx][x] once per column, in registers,
+//              then rho(y, x) = sum_ly T[ly] Y[ly][y] per point, Y broadcast from
+//              shared memory, one FP64 reduction into the grid;
+//   integrate  T[ly] += V(y, x) Y[ly][y] per point, lane-local: no shuffles per row.
+//              Cxy[ly][lx] = sum_x T[ly][x] X[lx][x] once per plane (spread over the
+//              lanes, T through shared memory), then W[lz][ly][lx] += Cxy Z[lz], the
+//              packed moments spread over the lanes' registers.
+// A row's range comes from the FP32 sphere rule where its error bound allows
+// (sphere_row_fast), one folded row per lane.
+// The form before it (one CTA per pair, three barriers per plane, a shuffle
+// reduction of 11 accumulators per row, launches of similar pairs one after the
+// other) took 21.1 ms to integrate and 6.1 ms to collocate 1000 pairs (l <= 2,
+// 64^3); this one takes 0.49 and 0.46 ms, 58 % and 61 % of the FP64 rate (1.10
+// TFLOP/s in a GEMM) counting L multiply-adds per cube point.
+constexpr int kOrthoWarps = 4;
+
+// the shared memory of orthorhombic item (pair g, 1 of nparts), in bytes
+int smem_ortho_item(const PairGeom &g, int extra, int nparts) {
     const int L = g.lp + 1 + extra;
+    const int nx = g.hi[0] - g.lb[0] + 1, ny = g.hi[1] - g.lb[1] + 1, nz = g.hi[2] - g.lb[2] + 1;
+    const int np = (nz + nparts - 1) / nparts, nc = ncoef(L - 1);
+    return 8 * (nc + L * (nx + ny + np) + kOrthoWarps * (33 * L + nshell(L - 1))) +
+           4 * (nx + ny + nc + kOrthoWarps * (1 - g.lb[1]));
+}
+
+// The cube sizes that the FP64 path accepts: what one CTA held when it kept a
+// whole pair (tables, dense coefficients and one plane's rows) in shared memory.
+int smem_ortho_fp64(const PairGeom &g) {
+    const int L = g.lp + 1;
     const int nx = g.hi[0] - g.lb[0] + 1, ny = g.hi[1] - g.lb[1] + 1, nz = g.hi[2] - g.lb[2] + 1;
     return 8 * (L * L * L + L * (nx + ny + nz) + L * L + ny * L) + 8 * ny;
 }
 
-// kAcc: the row accumulators of the adjoint, L <= kAcc (kNPow for integrate,
-// kNPowB for the backward pass's moments to degree lp + 2: more accumulators cost
-// the plain integrate registers and shuffles)
-template <bool kAdj, int kAcc = kNPow>
-__global__ void __launch_bounds__(256)
-k_ortho_fp64(const PairGeom *__restrict__ geoms, int first, const LevelDev *__restrict__ levels,
-             const int *__restrict__ table, const double *__restrict__ coef, double *__restrict__ mom,
-             GridPtrs grids, int *status, int extra) {
+// kAcc: the registers of T, L <= kAcc (kNPow, or kNPowB for the backward pass's
+// moments to degree lp + 2)
+template <bool kAdj, int kAcc>
+__global__ void __launch_bounds__(32 * kOrthoWarps)
+k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ items, int uparts,
+             const LevelDev *__restrict__ levels, const int *__restrict__ table, const double *__restrict__ coef,
+             double *__restrict__ mom, GridPtrs grids, int *status, int extra) {
     extern __shared__ double sm[];
-    const PairGeom g = geoms[first + blockIdx.x];
+    constexpr int kN2 = (kAcc * (kAcc + 1)) / 2, kM2 = (kN2 + 31) / 32;        // (ly, lx) sums per lane
+    constexpr int kNC = (kAcc * (kAcc + 1) * (kAcc + 2)) / 6, kMC = (kNC + 31) / 32;  // moments per lane
+    const int bid = blockIdx.x;
+    const Fp64Item it = items ? items[bid] : Fp64Item{bid / uparts, bid % uparts, uparts};
+    const PairGeom &g = geoms[it.pair];
     const LevelDev &lv = levels[g.level];
     double *__restrict__ grid = grids.p[g.level];
-    const int lp = g.lp + extra, L = lp + 1;
-    const int64_t mom_off = extra ? g.mom_ext_off : g.coef_off;
-    const int nx = g.hi[0] - g.lb[0] + 1, ny = g.hi[1] - g.lb[1] + 1, nz = g.hi[2] - g.lb[2] + 1;
-    double *C = sm;                // [lz][ly][lx] dense: coefficients, or moments (adjoint)
-    double *Xt = C + L * L * L;    // [k][gi]
-    double *Yt = Xt + L * nx;
-    double *Zt = Yt + L * ny;
-    double *Cxy = Zt + L * nz;     // [ly][lx]
-    double *Cx = Cxy + L * L;      // [row][lx]
-    int *rows = (int *)(Cx + ny * L);  // per row: igmin, j
-    const int tid = threadIdx.x, nthr = blockDim.x;
-    for (int t = tid; t < L * L * L; t += nthr) {
-        const int lx = t % L, ly = (t / L) % L, lz = t / (L * L);
-        C[t] = (!kAdj && lx + ly + lz <= lp) ? coef[g.coef_off + pidx(lp, lz, ly, lx)] : 0.0;
+    const int lp = g.lp + extra, L = lp + 1, nc = ncoef(lp), n2 = nshell(lp);
+    const int lb0 = g.lb[0], lb1 = g.lb[1], kgmin = g.kgmin;
+    const int nx = g.hi[0] - lb0 + 1, ny = g.hi[1] - lb1 + 1;
+    const int tot = 2 - 2 * kgmin;  // planes kgmin .. 1 - kgmin
+    const int np = it.part < tot ? (tot - it.part + it.nparts - 1) / it.nparts : 0;
+    double *C = sm;            // packed coefficients, or the CTA's moments
+    double *Xt = C + nc;       // [lx][x]
+    double *Yt = Xt + L * nx;  // [ly][y]
+    double *Zt = Yt + L * ny;  // [lz][plane of this item]
+    double *wsp = Zt + L * np;
+    int *xidx = reinterpret_cast<int *>(wsp + kOrthoWarps * (33 * L + n2));
+    int *yidx = xidx + nx;
+    int *dec = yidx + ny;      // integrate: packed moment -> lz | (ly, lx) << 8
+    int *rows_all = dec + nc;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double *sT = wsp + warp * (33 * L + n2);  // [ly][lane], rows of 33
+    double *sC = sT + 33 * L;                 // Cxy, packed (ly, lx)
+    int *rows = rows_all + warp * (1 - lb1);  // igmin of the folded rows jf = lb1 .. 0
+    for (int t = tid; t < nx + ny + np; t += 32 * kOrthoWarps) {
+        const int d = t < nx ? 0 : (t < nx + ny ? 1 : 2);
+        const int gi = d == 0 ? t : (d == 1 ? t - nx : t - nx - ny);
+        const int gg = d == 0 ? lb0 + gi : (d == 1 ? lb1 + gi : kgmin + it.part + gi * it.nparts);
+        const int n = d == 0 ? nx : (d == 1 ? ny : np);
+        double *tab = (d == 0 ? Xt : (d == 1 ? Yt : Zt)) + gi;
+        const double u = (double)gg * lv.dh[d][d] - g.off[d];
+        double e = exp(-g.zetp * u * u);
+        for (int k = 0; k < L; k++) {
+            tab[k * n] = e;
+            e *= u;
+        }
+        if (d < 2)
+            (d == 0 ? xidx : yidx)[gi] =
+                axis_index(lv.periodic[d], g.cc[d], gg, g.lb[d], lv.lb_grid[d], lv.npts[d], lv.ngrid[d]);
     }
-    fill_table(Xt, nx, L, g.lb[0], lv.dh[0][0], g.off[0], g.zetp);
-    fill_table(Yt, ny, L, g.lb[1], lv.dh[1][1], g.off[1], g.zetp);
-    fill_table(Zt, nz, L, g.lb[2], lv.dh[2][2], g.off[2], g.zetp);
-    __syncthreads();
-    const double r2 = rmul(g.radius, g.radius);
-    const int lane = tid & 31, warp = tid >> 5, nwarp = nthr >> 5;
-    for (int kg = g.kgmin; kg <= 1 - g.kgmin; kg++) {
-        const int kf = fold(kg);
-        const int k = axis_index(lv.periodic[2], g.cc[2], kg, g.lb[2], lv.lb_grid[2], lv.npts[2],
-                                 lv.ngrid[2]);
-        if (k < 0) {
-            if (tid == 0) atomicOr(status, kStatOutOfWindow);
+    for (int t = tid; t < nc; t += 32 * kOrthoWarps) {
+        if (!kAdj) {
+            C[t] = coef[g.coef_off + t];
             continue;
         }
-        double remk;
-        const int jgmin = cube_jgmin(g, lv, table, kf, r2, remk);
-        const int nrows = 2 - 2 * jgmin;
-        const double *Zk = Zt + (kg - g.lb[2]);
+        C[t] = 0.0;
+        int lz = 0, ly = 0, r = t;
+        while (r >= nshell(lp - lz)) r -= nshell(lp - lz++);
+        while (r > lp - lz - ly) r -= lp - lz - ly++ + 1;
+        dec[t] = lz | ((ly * L - (ly * (ly - 1)) / 2 + r) << 8);
+    }
+    // this lane's (ly, lx) entries: with n2 <= 16 of them, np2 = 2^lg lanes share one
+    int lg = 0;
+    if (kAdj)
+        while ((n2 << (lg + 1)) <= 32) lg++;
+    int oly[kM2], olx[kM2];
+#pragma unroll
+    for (int m = 0; m < kM2; m++) {
+        const int o = (lane >> lg) + 32 * m;
+        int ly = 0, r = o;
+        while (ly < L && r > lp - ly) r -= lp - ly++ + 1;
+        oly[m] = o < n2 ? ly : -1;
+        olx[m] = r;
+    }
+    double W[kAdj ? kMC : 1];
+#pragma unroll
+    for (int m = 0; m < (kAdj ? kMC : 1); m++) W[m] = 0.0;
+    const SphereRule rule(g.radius, lv.dh[0][0], lv.dh[1][1], lv.dh[2][2]);
+    const int *T0 = g.table_off >= 0 ? table + g.table_off : nullptr;
+    const int gn0 = lv.ngrid[0], gn1 = lv.ngrid[1];
+    __syncthreads();
+    for (int pl = warp; pl < np; pl += kOrthoWarps) {
+        const int kg = kgmin + it.part + pl * it.nparts, kf = fold(kg);
+        const int k = axis_index(lv.periodic[2], g.cc[2], kg, g.lb[2], lv.lb_grid[2], lv.npts[2], lv.ngrid[2]);
+        if (k < 0) {
+            if (lane == 0) atomicOr(status, kStatOutOfWindow);
+            continue;
+        }
+        // folded rows jgmin .. 0 of the plane and the plane's widest x range
+        const int jgmin = T0 ? T0[1 + 2 * (kf - T0[0])] : -sphere_jmax_fast(rule, kf);
+        const int *Tr = T0 ? T0 + 1 + 2 * (1 - T0[0]) + T0[2 + 2 * (kf - T0[0])] : nullptr;
+        int wide = 1;
+        __syncwarp();
+        for (int jf = jgmin + lane; jf <= 0; jf += 32) {
+            const int ig = Tr ? Tr[jf - jgmin] : -sphere_imax_fast(rule, kf, jf);
+            rows[jf - lb1] = ig;
+            wide = min(wide, ig);
+        }
+        wide = __reduce_min_sync(0xffffffffu, wide);
+        const double *Zk = Zt + pl;
         if (!kAdj) {
-            // Cxy[ly][lx] = sum_lz C[lz][ly][lx] Z[lz]
-            for (int t = tid; t < L * L; t += nthr) {
-                const int lx = t % L, ly = t / L;
-                double s = 0.0;
-                for (int lz = 0; lz <= lp - lx - ly; lz++) s += C[(lz * L + ly) * L + lx] * Zk[lz * nz];
-                Cxy[t] = s;
-            }
-            __syncthreads();
-        }
-        for (int t = tid; t < nrows * L; t += nthr) {
-            const int row = t / L, lx = t % L;
-            const int jg = jgmin + row;
-            if (!kAdj) {
-                double s = 0.0;
-                for (int ly = 0; ly <= lp - lx; ly++) s += Cxy[ly * L + lx] * Yt[ly * ny + (jg - g.lb[1])];
-                Cx[t] = s;
-            }
-            if (lx == 0) {
-                rows[2 * row] = cube_igmin(g, lv, table, kf, fold(jg), jgmin, remk);
-                rows[2 * row + 1] = axis_index(lv.periodic[1], g.cc[1], jg, g.lb[1], lv.lb_grid[1],
-                                               lv.npts[1], lv.ngrid[1]);
-            }
-        }
-        __syncthreads();
-        for (int row = warp; row < nrows; row += nwarp) {
-            const int igmin = rows[2 * row], j = rows[2 * row + 1];
-            if (j < 0) {
-                if (lane == 0) atomicOr(status, kStatOutOfWindow);
-                continue;
-            }
-            const int64_t rowbase = ((int64_t)k * lv.ngrid[1] + j) * lv.ngrid[0];
-            double acc[kAcc];
 #pragma unroll
-            for (int lx = 0; lx < kAcc; lx++) acc[lx] = 0.0;
-            for (int ig = igmin + lane; ig <= 1 - igmin; ig += 32) {
-                const int i = axis_index(lv.periodic[0], g.cc[0], ig, g.lb[0], lv.lb_grid[0],
-                                         lv.npts[0], lv.ngrid[0]);
-                if (i < 0) {
-                    atomicOr(status, kStatOutOfWindow);
-                    continue;
+            for (int m = 0; m < kM2; m++) {
+                if (oly[m] < 0) continue;
+                const int ly = oly[m], lx = olx[m];
+                double s = 0.0;
+                int base = 0;  // packed index of (lz, 0, 0)
+                for (int lz = 0; lz <= lp - lx - ly; lz++) {
+                    const int q = lp - lz;
+                    s += C[base + ly * (q + 1) - (ly * (ly - 1)) / 2 + lx] * Zk[lz * np];
+                    base += nshell(q);
                 }
-                const double *Xi = Xt + (ig - g.lb[0]);
-                if (!kAdj) {
-                    double v = 0.0;
-                    for (int lx = 0; lx < L; lx++) v += Cx[row * L + lx] * Xi[lx * nx];
-                    atomicAdd(grid + rowbase + i, v);
-                } else {
-                    const double v = grid[rowbase + i];
+                sC[lane + 32 * m] = s;
+            }
+        }
+        __syncwarp();
+        double cxy[kAdj ? kM2 : 1];
 #pragma unroll
-                    for (int lx = 0; lx < kAcc; lx++)
-                        if (lx < L) acc[lx] += v * Xi[lx * nx];
+        for (int m = 0; m < (kAdj ? kM2 : 1); m++) cxy[m] = 0.0;
+        const int nrow = 2 - 2 * jgmin, xend = 1 - wide;
+        for (int c0 = wide; c0 <= xend;) {
+            const int left = xend - c0 + 1;
+            const int lw = left > 16 ? 5 : (left > 8 ? 4 : 3);  // log2 of the block's columns
+            const int grp = lane >> lw, ng = 32 >> lw;          // the lane's row group
+            const int ig = c0 + (lane & ((1 << lw) - 1)), xc = min(ig - lb0, nx - 1);
+            const bool in = ig <= xend;
+            const int igf = fold(ig), xi = xidx[xc];
+            double T[kAcc];
+            if (!kAdj) {
+                const double *c = sC;
+#pragma unroll
+                for (int ly = 0; ly < kAcc; ly++) {
+                    if (ly >= L) break;
+                    double s = 0.0;
+                    for (int lx = 0; lx < L - ly; lx++) s += c[lx] * Xt[lx * nx + xc];
+                    c += L - ly;
+                    T[ly] = s;
+                }
+            } else {
+#pragma unroll
+                for (int ly = 0; ly < kAcc; ly++) T[ly] = 0.0;
+            }
+            constexpr int kU = kAdj ? 4 : 2;  // rows in flight per lane
+            for (int r0 = grp; r0 - grp < nrow; r0 += kU * ng) {
+                bool act[kU];
+                int jy[kU];
+                int64_t at[kU];
+                bool any = false;
+#pragma unroll
+                for (int u = 0; u < kU; u++) {
+                    const int r = r0 + u * ng, jg = jgmin + min(r, nrow - 1);
+                    jy[u] = jg - lb1;
+                    act[u] = in && r < nrow && igf >= rows[fold(jg) - lb1];
+                    const int yi = yidx[jy[u]];
+                    if (act[u] && (xi < 0 || yi < 0)) {
+                        atomicOr(status, kStatOutOfWindow);
+                        act[u] = false;
+                    }
+                    at[u] = ((int64_t)k * gn1 + yi) * gn0 + xi;
+                    any = any || act[u];
+                }
+                if (!__any_sync(0xffffffffu, any)) continue;
+                double v[kU];
+#pragma unroll
+                for (int u = 0; u < kU; u++) v[u] = kAdj && act[u] ? grid[at[u]] : 0.0;
+#pragma unroll
+                for (int ly = 0; ly < kAcc; ly++) {
+                    if (ly >= L) break;
+#pragma unroll
+                    for (int u = 0; u < kU; u++) {
+                        const double y = Yt[ly * ny + jy[u]];
+                        if (kAdj) T[ly] = fma(v[u], y, T[ly]);
+                        else v[u] = fma(T[ly], y, v[u]);
+                    }
+                }
+                if (!kAdj) {
+#pragma unroll
+                    for (int u = 0; u < kU; u++)
+                        if (act[u]) atomicAdd(grid + at[u], v[u]);
                 }
             }
             if (kAdj) {
-                // warp-shuffle reduction of the row moments
 #pragma unroll
-                for (int lx = 0; lx < kAcc; lx++) {
-                    double v = acc[lx];
-                    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                    acc[lx] = v;
+                for (int ly = 0; ly < kAcc; ly++)
+                    if (ly < L) sT[ly * 33 + lane] = T[ly];
+                __syncwarp();
+                const int wm = (1 << lw) - 1, cx = c0 - lb0;
+#pragma unroll
+                for (int m = 0; m < kM2; m++) {
+                    if (oly[m] < 0) continue;
+                    const double *t = sT + oly[m] * 33, *x = Xt + olx[m] * nx;
+                    double s = cxy[m];
+                    for (int i = lane & ((1 << lg) - 1); i < 32; i += 1 << lg)
+                        s = fma(t[i], x[min(cx + (i & wm), nx - 1)], s);
+                    cxy[m] = s;
                 }
-                if (lane == 0)
-                    for (int lx = 0; lx < L; lx++) Cx[row * L + lx] = acc[lx];
+                __syncwarp();
             }
+            c0 += 1 << lw;
         }
-        __syncthreads();
         if (kAdj) {
-            // Cxy[ly][lx] = sum_rows Cx[row][lx] Y[ly][jg];  C[lz][ly][lx] += Cxy * Z[lz]
-            for (int t = tid; t < L * L; t += nthr) {
-                const int lx = t % L, ly = t / L;
-                if (lx + ly > lp) continue;
-                double s = 0.0;
-                for (int row = 0; row < nrows; row++)
-                    if (rows[2 * row + 1] >= 0) s += Cx[row * L + lx] * Yt[ly * ny + (jgmin + row - g.lb[1])];
-                for (int lz = 0; lz <= lp - lx - ly; lz++) C[(lz * L + ly) * L + lx] += s * Zk[lz * nz];
+            for (int o = 1; o < (1 << lg); o <<= 1) cxy[0] += __shfl_xor_sync(0xffffffffu, cxy[0], o);
+#pragma unroll
+            for (int m = 0; m < kM2; m++)
+                if (oly[m] >= 0) sC[(lane >> lg) + 32 * m] = cxy[m];
+            __syncwarp();
+#pragma unroll
+            for (int m = 0; m < kMC; m++) {
+                const int t = lane + 32 * m;
+                if (t < nc) W[m] = fma(sC[dec[t] >> 8], Zk[(dec[t] & 255) * np], W[m]);
             }
-            __syncthreads();
         }
     }
     if (kAdj) {
-        for (int t = tid; t < L * L * L; t += nthr) {
-            const int lx = t % L, ly = (t / L) % L, lz = t / (L * L);
-            if (lx + ly + lz <= lp) mom[mom_off + pidx(lp, lz, ly, lx)] = C[t];
+        for (int w = 0; w < kOrthoWarps; w++) {
+            if (warp == w) {
+#pragma unroll
+                for (int m = 0; m < kMC; m++)
+                    if (lane + 32 * m < nc) C[lane + 32 * m] += W[m];
+            }
+            __syncthreads();
+        }
+        double *out = mom + (extra ? g.mom_ext_off : g.coef_off);
+        for (int t = tid; t < nc; t += 32 * kOrthoWarps) {
+            if (it.nparts == 1) out[t] = C[t];
+            else atomicAdd(out + t, C[t]);  // several items of one pair (zeroed before the launch)
         }
     }
 }
 
 // ---------------------------------------------------------------------------
-// general cell, one CTA per pair (row bounds: general_row, gpw_common.cuh)
+// general cell, one CTA per item (every nparts-th plane of a pair's index box; row
+// bounds: general_row, gpw_common.cuh)
 // (one row of margin: a geometry update moves a box's extent by at most one)
 int smem_general_fp64(const PairGeom &g, int extra) {
     const int L = g.lp + 1 + extra;
@@ -304,11 +404,13 @@ int smem_general_fp64(const PairGeom &g, int extra) {
 
 template <bool kAdj>
 __global__ void __launch_bounds__(256)
-k_general_fp64(const PairGeom *__restrict__ geoms, int first, const LevelDev *__restrict__ levels,
+k_general_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ items, int uparts,
+             const LevelDev *__restrict__ levels,
                const double *__restrict__ coef, double *__restrict__ mom, GridPtrs grids,
                int *status, int extra) {
     extern __shared__ double sm[];
-    const PairGeom g = geoms[first + blockIdx.x];
+    const Fp64Item it = items ? items[blockIdx.x] : Fp64Item{(int)blockIdx.x / uparts, (int)blockIdx.x % uparts, uparts};
+    const PairGeom g = geoms[it.pair];
     const LevelDev &lv = levels[g.level];
     double *__restrict__ grid = grids.p[g.level];
     const int lp = g.lp + extra, L = lp + 1;
@@ -327,7 +429,7 @@ k_general_fp64(const PairGeom *__restrict__ geoms, int first, const LevelDev *__
     __syncthreads();
     int off[3];
     for (int d = 0; d < 3; d++) off[d] = imod(g.cc[d] + lv.lb_grid[d], lv.npts[d]);
-    for (int kk = g.cc[2]; kk <= g.hi[2]; kk++) {
+    for (int kk = g.cc[2] + it.part; kk <= g.hi[2]; kk += it.nparts) {
         const double dk = rsub((double)kk, g.off[2]);
         const int kidx = lv.periodic[2] ? imod(kk, lv.npts[2]) : kk - g.cc[2] + off[2];
         if (kidx < 0 || kidx >= lv.ngrid[2]) {
@@ -446,7 +548,10 @@ k_general_fp64(const PairGeom *__restrict__ geoms, int first, const LevelDev *__
     if (kAdj) {
         for (int t = tid; t < L * L * L; t += nthr) {
             const int i = t % L, j = (t / L) % L, k = t / (L * L);
-            if (i + j + k <= lp) mom[mom_off + pidx(lp, k, j, i)] = Q[t];
+            if (i + j + k > lp) continue;
+            double *out = mom + mom_off + pidx(lp, k, j, i);
+            if (it.nparts == 1) *out = Q[t];
+            else atomicAdd(out, Q[t]);
         }
     }
 }
@@ -469,10 +574,12 @@ __device__ __forceinline__ ff ff_shfl_xor(ff v, int o) {
 
 template <bool kAdj>
 __global__ void __launch_bounds__(256)
-k_general_ff(const PairGeom *__restrict__ geoms, int first, const LevelDev *__restrict__ levels,
+k_general_ff(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ items, int uparts,
+             const LevelDev *__restrict__ levels,
              const double *__restrict__ coef, double *__restrict__ mom, GridPtrs grids, int *status) {
     extern __shared__ double smd[];
-    const PairGeom g = geoms[first + blockIdx.x];
+    const Fp64Item it = items ? items[blockIdx.x] : Fp64Item{(int)blockIdx.x / uparts, (int)blockIdx.x % uparts, uparts};
+    const PairGeom g = geoms[it.pair];
     const LevelDev &lv = levels[g.level];
     double *__restrict__ grid = grids.p[g.level];
     const int lp = g.lp, L = lp + 1;
@@ -498,7 +605,7 @@ k_general_ff(const PairGeom *__restrict__ geoms, int first, const LevelDev *__re
     __syncthreads();
     int off[3];
     for (int d = 0; d < 3; d++) off[d] = imod(g.cc[d] + lv.lb_grid[d], lv.npts[d]);
-    for (int kk = g.cc[2]; kk <= g.hi[2]; kk++) {
+    for (int kk = g.cc[2] + it.part; kk <= g.hi[2]; kk += it.nparts) {
         const double dk = rsub((double)kk, g.off[2]);
         const int kidx = lv.periodic[2] ? imod(kk, lv.npts[2]) : kk - g.cc[2] + off[2];
         if (kidx < 0 || kidx >= lv.ngrid[2]) {
@@ -618,7 +725,11 @@ k_general_ff(const PairGeom *__restrict__ geoms, int first, const LevelDev *__re
     if (kAdj) {
         for (int t = tid; t < L * L * L; t += nthr) {
             const int i = t % L, j = (t / L) % L, k = t / (L * L);
-            if (i + j + k <= lp) mom[g.coef_off + pidx(lp, k, j, i)] = (double)Q[t].hi + (double)Q[t].lo;
+            if (i + j + k > lp) continue;
+            double *out = mom + g.coef_off + pidx(lp, k, j, i);
+            const double v = (double)Q[t].hi + (double)Q[t].lo;
+            if (it.nparts == 1) *out = v;
+            else atomicAdd(out, v);
         }
     }
 }
@@ -636,7 +747,7 @@ static cudaError_t set_smem(const void *fn, int bytes) {
 // so that launches (and CUDA graph capture) need no attribute calls.
 cudaError_t fp64_kernel_attributes(int smem_max) {
     const void *fns[] = {(const void *)k_prep, (const void *)k_backtransform,
-                         (const void *)k_ortho_fp64<false>, (const void *)k_ortho_fp64<true>,
+                         (const void *)k_ortho_fp64<false, kNPow>, (const void *)k_ortho_fp64<true, kNPow>,
                          (const void *)k_ortho_fp64<true, kNPowB>,
                          (const void *)k_general_fp64<false>, (const void *)k_general_fp64<true>,
                          (const void *)k_general_ff<false>, (const void *)k_general_ff<true>};
@@ -656,36 +767,76 @@ cudaError_t launch_prep(const TaskSet &ts, const double *d_pab, cudaStream_t s) 
     return cudaGetLastError();
 }
 
-static cudaError_t launch_fp64_impl(const TaskSet &ts, const GridPtrs &g, bool adj, int kind, int extra,
-                                    double *mom, cudaStream_t s) {
-    for (const Chunk &c0 : ts.chunks) {
-        Chunk c = c0;
-        if (extra) c.smem_bytes = c0.smem_ext;
-        if (c.count == 0 || (kind >= 0 && c.kind != kind)) continue;
-        cudaError_t e;
-        ProfScope prof(ts, s);
-        if (c.kind == 0) {
-            if (adj && extra)
-                k_ortho_fp64<true, kNPowB><<<c.count, 256, c.smem_bytes, s>>>(ts.d_geom, c.first, ts.plan->d_levels,
-                                                                             ts.d_table, ts.d_coef, mom, g,
-                                                                             ts.d_status, extra);
-            else if (adj)
-                k_ortho_fp64<true><<<c.count, 256, c.smem_bytes, s>>>(ts.d_geom, c.first, ts.plan->d_levels,
-                                                                     ts.d_table, ts.d_coef, mom, g,
-                                                                     ts.d_status, 0);
-            else
-                k_ortho_fp64<false><<<c.count, 256, c.smem_bytes, s>>>(ts.d_geom, c.first, ts.plan->d_levels,
-                                                                      ts.d_table, ts.d_coef, mom, g,
-                                                                      ts.d_status, 0);
+// The items of the FP64 launches and of the float-float general-cell kernel (1500
+// pairs of a general cell, 128^3, collocate + integrate: one CTA per pair 38.1 ms,
+// most of it the tail of the largest boxes; items 10.7 ms).  A pair is divided into parts (interleaved planes, so
+// that parts cost alike) where it holds more than 1/kWaves of an even per-CTA share
+// of all cube points, down to one plane per warp; the largest pairs come first
+// (the sorted order).  The number of planes is not needed exactly: a geometry
+// update may move a general box's extent by one.
+void fp64_items(TaskSet &ts, int sms, int smem_limit, std::vector<Fp64Item> &items) {
+    constexpr int kWaves = 8, kCtas = 4;
+    constexpr double kLeast = 16384.0;  // points x powers: below this a part is mostly tables and set-up
+    double total = 0.0;
+    for (const PairGeom &g : ts.h_geom) total += (double)g.cost * (g.lp + 1);
+    const double target = std::max(kLeast, total / ((double)sms * kCtas * kWaves));
+    ts.fp64_ortho = ts.fp64_general = 0;
+    ts.fp64_smem = ts.fp64_smem_ext = ts.fp64_smem_gen = ts.fp64_smem_gen_ext = 0;
+    ts.fp64_split = false;
+    for (int64_t k = 0; k < (int64_t)ts.h_geom.size(); k++) {
+        const PairGeom &g = ts.h_geom[k];
+        const int planes = g.ortho ? 2 - 2 * g.kgmin : g.ext0[2];
+        const int most = std::max(1, (planes + kOrthoWarps - 1) / kOrthoWarps);
+        int parts = (int)std::min<double>(most, std::ceil((double)g.cost * (g.lp + 1) / target));
+        parts = std::max(parts, 1);
+        if (g.ortho) {
+            while (parts < planes && smem_ortho_item(g, 2, parts) > smem_limit) parts++;
+            ts.fp64_smem = std::max(ts.fp64_smem, smem_ortho_item(g, 0, parts));
+            ts.fp64_smem_ext = std::max(ts.fp64_smem_ext, smem_ortho_item(g, 2, parts));
+            ts.fp64_ortho += parts;
         } else {
-            if (adj)
-                k_general_fp64<true><<<c.count, 256, c.smem_bytes, s>>>(ts.d_geom, c.first, ts.plan->d_levels,
-                                                                       ts.d_coef, mom, g, ts.d_status, extra);
-            else
-                k_general_fp64<false><<<c.count, 256, c.smem_bytes, s>>>(ts.d_geom, c.first, ts.plan->d_levels,
-                                                                        ts.d_coef, mom, g, ts.d_status, 0);
+            ts.fp64_smem_gen = std::max(ts.fp64_smem_gen, smem_general_fp64(g));
+            ts.fp64_smem_gen_ext = std::max(ts.fp64_smem_gen_ext, std::min(smem_general_fp64(g, 2), smem_limit));
+            ts.fp64_general += parts;
         }
-        e = cudaGetLastError();
+        ts.fp64_split = ts.fp64_split || parts > 1;
+        for (int p = 0; p < parts; p++) items.push_back(Fp64Item{(int)k, p, parts});
+    }
+}
+
+static cudaError_t launch_fp64_impl(const TaskSet &ts, const GridPtrs &g, bool adj, int extra, double *mom,
+                                    cudaStream_t s) {
+    const Plan &P = *ts.plan;
+    if (adj && ts.fp64_split) {  // several items add to one pair's moments
+        const cudaError_t e = cudaMemsetAsync(mom, 0, sizeof(double) * (extra ? ts.mom_ext_len : ts.coef_len), s);
+        if (e != cudaSuccess) return e;
+    }
+    if (ts.fp64_ortho > 0) {
+        ProfScope prof(ts, s);
+        const unsigned n = (unsigned)ts.fp64_ortho;
+        if (adj && extra)
+            k_ortho_fp64<true, kNPowB><<<n, 32 * kOrthoWarps, ts.fp64_smem_ext, s>>>(
+                ts.d_geom, ts.d_fp64_items, 1, P.d_levels, ts.d_table, ts.d_coef, mom, g, ts.d_status, extra);
+        else if (adj)
+            k_ortho_fp64<true, kNPow><<<n, 32 * kOrthoWarps, ts.fp64_smem, s>>>(
+                ts.d_geom, ts.d_fp64_items, 1, P.d_levels, ts.d_table, ts.d_coef, mom, g, ts.d_status, 0);
+        else
+            k_ortho_fp64<false, kNPow><<<n, 32 * kOrthoWarps, ts.fp64_smem, s>>>(
+                ts.d_geom, ts.d_fp64_items, 1, P.d_levels, ts.d_table, ts.d_coef, mom, g, ts.d_status, 0);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    if (ts.fp64_general > 0) {
+        ProfScope prof(ts, s);
+        const unsigned n = (unsigned)ts.fp64_general;
+        const Fp64Item *items = ts.d_fp64_items + ts.fp64_ortho;
+        if (adj)
+            k_general_fp64<true><<<n, 256, extra ? ts.fp64_smem_gen_ext : ts.fp64_smem_gen, s>>>(
+                ts.d_geom, items, 1, P.d_levels, ts.d_coef, mom, g, ts.d_status, extra);
+        else
+            k_general_fp64<false><<<n, 256, ts.fp64_smem_gen, s>>>(ts.d_geom, items, 1, P.d_levels, ts.d_coef, mom, g,
+                                                                  ts.d_status, 0);
+        const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -698,29 +849,33 @@ int smem_general_ff(const PairGeom &g) {
     return 8 * (L * L * L + L * L + 2 * ny * L + 3 * ny) + 12 * ny;
 }
 
-// one launch over all general-cell pairs (contiguous in the sorted order)
+// one launch over the items of all general-cell pairs
 cudaError_t launch_general_ff(const TaskSet &ts, const GridPtrs &g, bool adj, cudaStream_t s) {
     if (ts.gen_count == 0) return cudaSuccess;
+    if (adj && ts.fp64_split) {  // several items add to one pair's moments
+        const int64_t c0 = ts.gen_coef_first;
+        const cudaError_t e = cudaMemsetAsync(ts.d_mom + c0, 0, sizeof(double) * (ts.coef_len - c0), s);
+        if (e != cudaSuccess) return e;
+    }
     ProfScope prof(ts, s);
+    const unsigned n = (unsigned)ts.fp64_general;
+    const Fp64Item *items = ts.d_fp64_items + ts.fp64_ortho;
     if (adj)
-        k_general_ff<true><<<ts.gen_count, 256, ts.gen_smem, s>>>(ts.d_geom, ts.gen_first, ts.plan->d_levels,
-                                                                 ts.d_coef, ts.d_mom, g, ts.d_status);
+        k_general_ff<true><<<n, 256, ts.gen_smem, s>>>(ts.d_geom, items, 1, ts.plan->d_levels, ts.d_coef, ts.d_mom, g,
+                                                      ts.d_status);
     else
-        k_general_ff<false><<<ts.gen_count, 256, ts.gen_smem, s>>>(ts.d_geom, ts.gen_first, ts.plan->d_levels,
-                                                                  ts.d_coef, ts.d_mom, g, ts.d_status);
+        k_general_ff<false><<<n, 256, ts.gen_smem, s>>>(ts.d_geom, items, 1, ts.plan->d_levels, ts.d_coef, ts.d_mom, g,
+                                                       ts.d_status);
     return cudaGetLastError();
 }
 
-cudaError_t launch_fp64_kind(const TaskSet &ts, const GridPtrs &g, bool adj, int kind, cudaStream_t s) {
-    return launch_fp64_impl(ts, g, adj, kind, 0, ts.d_mom, s);
-}
-
 cudaError_t launch_moments_fp64(const TaskSet &ts, const GridPtrs &g, int extra, double *out, cudaStream_t s) {
-    return launch_fp64_impl(ts, g, true, -1, extra, out, s);
+    return launch_fp64_impl(ts, g, true, extra, out, s);
 }
 
+// n pairs without a task set: every pair in uparts parts
 cudaError_t launch_pairs_fp64(const PairGeom *d_geoms, const LevelDev *d_levels, const double *d_tmat,
-                              double *d_coef, int *d_status, int n, int tau, int max_A, int max_B,
+                              double *d_coef, int *d_status, int n, int uparts, int tau, int max_A, int max_B,
                               int smem_coll, const double *d_pab, double *d_grid, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     k_prep<<<(unsigned)n, 128, smem_prep(max_A, max_B), s>>>(d_geoms, d_levels, d_tmat, tau, d_pab, d_coef);
@@ -728,9 +883,15 @@ cudaError_t launch_pairs_fp64(const PairGeom *d_geoms, const LevelDev *d_levels,
     if (e != cudaSuccess) return e;
     GridPtrs g;
     for (int l = 0; l < GPW_MAX_LEVELS; l++) g.p[l] = d_grid;
-    k_ortho_fp64<false><<<(unsigned)n, 256, smem_coll, s>>>(d_geoms, 0, d_levels, nullptr, d_coef, nullptr, g,
-                                                          d_status, 0);
+    k_ortho_fp64<false, kNPow><<<(unsigned)(n * uparts), 32 * kOrthoWarps, smem_coll, s>>>(
+        d_geoms, nullptr, uparts, d_levels, nullptr, d_coef, nullptr, g, d_status, 0);
     return cudaGetLastError();
+}
+
+// one plane per warp (orthorhombic), four planes per CTA (general cell)
+int fp64_single_parts(const PairGeom &g) {
+    const int planes = g.ortho ? 2 - 2 * g.kgmin : g.ext0[2];
+    return std::max(1, (planes + kOrthoWarps - 1) / kOrthoWarps);
 }
 
 // One pair from raw device pointers, orthorhombic (with its cube list in d_table
@@ -743,21 +904,22 @@ cudaError_t launch_one_fp64(const PairGeom &g, const PairGeom *d_geom, const Lev
     if (e != cudaSuccess) return e;
     GridPtrs gp;
     for (int l = 0; l < GPW_MAX_LEVELS; l++) gp.p[l] = d_grid;
+    const int parts = fp64_single_parts(g);
     if (g.ortho)
-        k_ortho_fp64<false><<<1, 256, smem_ortho_fp64(g), s>>>(d_geom, 0, d_levels, d_table, d_coef, nullptr, gp,
-                                                             d_status, 0);
+        k_ortho_fp64<false, kNPow><<<(unsigned)parts, 32 * kOrthoWarps, smem_ortho_item(g, 0, parts), s>>>(
+            d_geom, nullptr, parts, d_levels, d_table, d_coef, nullptr, gp, d_status, 0);
     else
-        k_general_fp64<false><<<1, 256, smem_general_fp64(g), s>>>(d_geom, 0, d_levels, d_coef, nullptr, gp,
-                                                                  d_status, 0);
+        k_general_fp64<false><<<(unsigned)parts, 256, smem_general_fp64(g), s>>>(d_geom, nullptr, parts, d_levels,
+                                                                               d_coef, nullptr, gp, d_status, 0);
     return cudaGetLastError();
 }
 
 cudaError_t launch_collocate_fp64(const TaskSet &ts, const GridPtrs &g, cudaStream_t s) {
-    return launch_fp64_kind(ts, g, false, -1, s);
+    return launch_fp64_impl(ts, g, false, 0, ts.d_mom, s);
 }
 
 cudaError_t launch_integrate_fp64(const TaskSet &ts, const GridPtrs &g, cudaStream_t s) {
-    return launch_fp64_kind(ts, g, true, -1, s);
+    return launch_fp64_impl(ts, g, true, 0, ts.d_mom, s);
 }
 
 cudaError_t launch_backtransform(const TaskSet &ts, const double *d_mom, double *d_hab,

@@ -14,14 +14,6 @@ struct GridPtrs {
     double *p[GPW_MAX_LEVELS];
 };
 
-// A contiguous run of sorted tasks launched together (same kind, similar size).
-struct Chunk {
-    int first, count;
-    int smem_bytes;
-    int smem_ext;  // with two extra powers (backward moments)
-    int kind;      // 0 ortho, 1 general
-};
-
 struct Plan {
     int device = 0;
     int nlevels = 0;
@@ -53,7 +45,13 @@ struct TaskSet {
     int64_t mom_ext_len = 0;
     double *d_mom_ext = nullptr;   // backward: moments up to degree lp + 2
     int *d_status = nullptr;
-    std::vector<Chunk> chunks;     // FP64 launches
+    // FP64 launches: items of the orthorhombic pairs, then of the general-cell pairs
+    Fp64Item *d_fp64_items = nullptr;
+    int64_t fp64_ortho = 0, fp64_general = 0;
+    int fp64_smem = 0, fp64_smem_ext = 0;          // shared memory (ext: with two extra powers)
+    int fp64_smem_gen = 0, fp64_smem_gen_ext = 0;
+    bool fp64_split = false;       // some pair is divided into several items
+    int64_t gen_coef_first = 0;    // general-cell pairs: first coefficient
     MixedState *mixed = nullptr;
     int tile_lz[GPW_MAX_LEVELS];   // tiled path: log2 of the tile's z extent per level
     int gen_first = 0, gen_count = 0, gen_smem = 0;  // general-cell pairs (float-float kernel)
@@ -91,11 +89,12 @@ struct ProfScope {
 cudaError_t launch_prep(const TaskSet &ts, const double *d_pab, cudaStream_t s);
 cudaError_t launch_collocate_fp64(const TaskSet &ts, const GridPtrs &g, cudaStream_t s);
 cudaError_t launch_integrate_fp64(const TaskSet &ts, const GridPtrs &g, cudaStream_t s);
-// kind: 0 orthorhombic chunks, 1 general-cell chunks, -1 all
-cudaError_t launch_fp64_kind(const TaskSet &ts, const GridPtrs &g, bool adj, int kind, cudaStream_t s);
 cudaError_t launch_backtransform(const TaskSet &ts, const double *d_mom, double *d_hab,
                                  cudaStream_t s);
-int smem_ortho_fp64(const PairGeom &g, int extra = 0);
+void fp64_items(TaskSet &ts, int sms, int smem_limit, std::vector<Fp64Item> &items);
+int smem_ortho_fp64(const PairGeom &g);
+int smem_ortho_item(const PairGeom &g, int extra, int nparts);
+int fp64_single_parts(const PairGeom &g);
 int smem_general_fp64(const PairGeom &g, int extra = 0);
 // moments <V | t^k...> up to degree lp + extra into out (offsets coef_off, or mom_ext_off when extra > 0)
 cudaError_t launch_moments_fp64(const TaskSet &ts, const GridPtrs &g, int extra, double *out, cudaStream_t s);
@@ -126,7 +125,7 @@ void set_last_error(const std::string &msg);
 
 // gpw_fp64.cu: set-up + orthorhombic collocate of n pairs from raw device pointers
 cudaError_t launch_pairs_fp64(const PairGeom *d_geoms, const LevelDev *d_levels, const double *d_tmat,
-                              double *d_coef, int *d_status, int n, int tau, int max_A, int max_B,
+                              double *d_coef, int *d_status, int n, int uparts, int tau, int max_A, int max_B,
                               int smem_coll, const double *d_pab, double *d_grid, cudaStream_t s);
 
 // gpw_fp64.cu: one pair (the drop-in entry): set-up + collocation from raw device pointers

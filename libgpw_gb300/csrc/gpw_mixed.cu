@@ -160,21 +160,7 @@ struct MixedState {
 
 
 // ---------------------------------------------------------------------------
-// Sphere rule with an FP32 fast path.  The FP32 estimate decides unless it lies
-// within its error bound of an integer; then the exact FP64 rule (the one the
-// host and the oracle use) decides.
-__device__ __forceinline__ int fast_floor_checked(float rem, float r2f, float hinv, bool &unsure) {
-    const float rc = fmaxf(rem, 0.0f);
-    const float rs = rsqrtf(fmaxf(rc, 1e-30f));
-    const float v = __fmul_rn(__fmul_rn(rc, rs), hinv);  // sqrt(rc) / h, relative error < 2^-21
-    const float fl = floorf(v);
-    // error of rem ~ 4 ulp(r2f); of sqrt ~ err/(2 sqrt); plus relative 2^-19
-    const float erem = r2f * 4.8e-7f;
-    const float ev = __fmul_rn(erem * 0.5f, rs) * hinv + v * 2e-6f + 1e-6f;
-    unsure = (v - fl) <= ev || (fl + 1.0f - v) <= ev || rem <= erem;
-    return (int)fl;
-}
-
+// Sphere rule (FP32 with an error bound, fast_floor_checked in gpw_common.cuh).
 // the exact FP64 rule, out of line: taken only where the FP32 estimate is unsure
 __device__ __noinline__ int rule_jmax_exact(const TPair &p, int kf) { return rule_jmax(rule_remk(p.r2, kf, p.hz), p.hy); }
 __device__ __noinline__ int rule_imax_exact(const TPair &p, int kf, int jf) {

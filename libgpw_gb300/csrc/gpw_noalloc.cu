@@ -84,7 +84,7 @@ extern "C" int gpw_collocate_noalloc(const gpw_grid_desc *level, const gpw_task 
     if (ntasks == 0) return GPW_SUCCESS;
     // host geometry, checked exactly as gpw_taskset_create checks it
     std::vector<PairGeom> geo((size_t)ntasks);
-    int max_A = 0, max_B = 0, smem_coll = 0;
+    int max_A = 0, max_B = 0, smem_cube = 0, parts = 1;
     int64_t coef = 0;
     for (int i = 0; i < ntasks; i++) {
         if (tasks[i].level != 0 || tasks[i].sphere_offset >= 0) {
@@ -97,7 +97,8 @@ extern "C" int gpw_collocate_noalloc(const gpw_grid_desc *level, const gpw_task 
         coef += ncoef(geo[i].lp);
         max_A = std::max(max_A, geo[i].la_max);
         max_B = std::max(max_B, geo[i].lb_max);
-        smem_coll = std::max(smem_coll, smem_ortho_fp64(geo[i]));
+        smem_cube = std::max(smem_cube, smem_ortho_fp64(geo[i]));
+        parts = std::max(parts, fp64_single_parts(geo[i]));
     }
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) {
@@ -106,10 +107,15 @@ extern "C" int gpw_collocate_noalloc(const gpw_grid_desc *level, const gpw_task 
     }
     int smem_limit = 0;
     cudaDeviceGetAttribute(&smem_limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (smem_coll > smem_limit || smem_prep(max_A, max_B) > smem_limit) {
+    if (smem_cube > smem_limit || smem_prep(max_A, max_B) > smem_limit) {
         set_last_error("gpw_collocate_noalloc: a cube is too large for one CTA");
         return GPW_ERR_UNSUPPORTED;
     }
+    // few pairs: divide each one so that the launch has about four CTAs per SM
+    int sms = 1, smem_coll = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    parts = std::max(1, std::min(parts, 4 * sms / ntasks));
+    for (int i = 0; i < ntasks; i++) smem_coll = std::max(smem_coll, smem_ortho_item(geo[i], 0, parts));
     unsigned char *base = nullptr;
     st = scratch_address(dev, &base);
     if (st) return st;
@@ -129,7 +135,7 @@ extern "C" int gpw_collocate_noalloc(const gpw_grid_desc *level, const gpw_task 
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(d_geom, geo.data(), sizeof(PairGeom) * ntasks, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
-        e = launch_pairs_fp64(d_geom, d_level, nullptr, d_coef, d_status, ntasks, compute_tau ? 1 : 0, max_A, max_B,
+        e = launch_pairs_fp64(d_geom, d_level, nullptr, d_coef, d_status, ntasks, parts, compute_tau ? 1 : 0, max_A, max_B,
                               smem_coll, d_pab, d_grid, s);
     // the kernels' error bits, read into a stack variable (a copy, no allocation)
     int flags = 0;
