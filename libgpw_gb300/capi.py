@@ -219,7 +219,7 @@ class TaskSet:
         return ms.value, nc.value, nk.value
 
     def bins(self) -> tuple:
-        """(tile, pair) items and work units of the tiled path (gpw_taskset_bins)."""
+        """(tile, pair image) items and work units of the tiled path (gpw_taskset_bins)."""
         a, b = C.c_int64(), C.c_int64()
         check(lib().gpw_taskset_bins(self.handle, C.byref(a), C.byref(b)), "gpw_taskset_bins")
         return a.value, b.value

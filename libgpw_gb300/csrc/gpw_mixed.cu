@@ -72,8 +72,15 @@ struct TileDesc {
     int level;
     int t[3];  // tile indices
     int lz;    // log2 TZ (TY = MROWS >> lz)
-    int split; // the tile's pairs are divided among several work units: flush with atomics
+    int flags; // kUnitSplit, kUnitOver
 };
+
+// the tile's pairs are divided among several work units: flush with atomics
+constexpr int kUnitSplit = 1;
+// some cube has more than kMaxImages images over a tile axis: reported when the unit
+// runs (once per unit: a check per item, an atomic in the item loop, cost collocate
+// 7 % more instructions, since no level data then stays in registers across it)
+constexpr int kUnitOver = 2;
 
 // tile extents of a tile descriptor
 struct TileShape {
@@ -110,7 +117,7 @@ struct GenLevel {
 constexpr int kHdr16 = (int)((sizeof(TPair) + 15) / 16);
 constexpr int kCoef16Max = (NCOEF_MAX * (int)sizeof(float2) + 15) / 16;
 
-// the current periodic image of a pair over the tile
+// one periodic image of a pair over the tile
 struct ImgState {
     ff tc;              // collocate: x of the re-expansion column minus xp
     int o[3];           // cube offset of the tile origin
@@ -119,13 +126,15 @@ struct ImgState {
     int sb;             // collocate: x-variable scale 2^sb of the slices (balancing)
 };
 
-// Per (tile, pair) item, computed once per task set: the images of the pair's
-// cube over the tile (counts per axis packed as n0 | n1 << 8 | n2 << 16) and the
-// state of the first image.  Items with more than one image (small periodic
-// cells) derive the others in the kernel.
+// Per (tile, pair image) item, computed once per task set: the image's state.  A
+// cube that reaches a tile through several periodic images (small cells) has one
+// item per image, each kept only if its own sphere reaches the tile.  (Before, one
+// item that the kernels looped over, every combination of the axes' images a full
+// pass: 1000 pairs, l <= 2, in a 10-bohr cell, 64^3, took 0.94 ms to collocate; with
+// items per image and shorter units 0.36 ms.)
 struct alignas(16) ItemImg {
     ImgState im;
-    int nimg;
+    int pad_;
 };
 static_assert(sizeof(ItemImg) == 48, "ItemImg is three 16-byte chunks");
 
@@ -136,8 +145,8 @@ struct MixedState {
     uint4 *d_blob = nullptr;       // pair blobs of the orthorhombic tasks (sorted order)
     int64_t *d_blob_off = nullptr; // per task: blob offset in 16-byte chunks
     int64_t *d_start = nullptr;    // per work unit: first item, end
-    uint64_t *d_items = nullptr;   // per (tile, pair): blob offset << 16 | chunks
-    ItemImg *d_iimg = nullptr;     // per (tile, pair): images
+    uint64_t *d_items = nullptr;   // per (tile, pair image): blob offset << 16 | chunks
+    ItemImg *d_iimg = nullptr;     // per item: its image
     int *d_queue = nullptr;      // [0]: collocate, [1]: integrate (orthorhombic tiles), [2], [3]: general tiles
     GenLevel *d_glv = nullptr;   // per level (general levels only meaningful)
     int northo = 0;              // ortho tasks come first in sorted order
@@ -309,8 +318,8 @@ struct MixedArgs {
     const LevelDev *levels;
     const TileDesc *tiles;
     const int64_t *start;
-    const uint64_t *items;    // per (tile, pair): blob offset in 16-byte chunks << 16 | chunks to copy
-    const ItemImg *iimg;      // per (tile, pair): images
+    const uint64_t *items;    // per (tile, pair image): blob offset in 16-byte chunks << 16 | chunks to copy
+    const ItemImg *iimg;      // per item: its image
     const int *table;
     const GenLevel *glv;  // general levels: FP32 steps, cosines
     double *mom;  // integrate: per-pair moments
@@ -340,13 +349,10 @@ struct alignas(16) PairHdr {
 
 // shared state of both tiled kernels
 struct TileCommon {
-    ItemImg ii[2];  // images over this tile of the current pair and of the one being fetched
-    ImgState im;    // images after the first of a multi-image item
+    ItemImg ii[2];  // the image of the current item and of the one being fetched
     ff Y[kNPow][kMaxTY + 1];  // rows padded: lanes reading different rows hit different banks
     ff Z[kNPow][kMaxTZ + 1];
     int tile;
-    int img[3][kMaxImages];
-    int nimg[3];
     uint64_t mbar;
     uint32_t tmem;
     int abort;
@@ -466,32 +472,12 @@ __device__ __forceinline__ void fetch_pair(uint4 *dst, ItemImg &ii, const MixedA
     cp_async_commit();
 }
 
-// images of one axis: cube offsets o such that the tile [tT, tT+ext) maps onto [lb, hi]
-__device__ void axis_images(const LevelDev &lv, int d, int tt, int T, const TPair &p, int *img, int &n, int *status) {
-    n = 0;
-    const int N = lv.ngrid[d];
-    const int ext = min(T, N - tt * T);
-    if (lv.periodic[d]) {
-        const int np = lv.npts[d];
-        const int base = tt * T - p.cc[d];
-        const int num = p.lb[d] - base - ext + 1;
-        const int kmin = (num >= 0 ? num / np : -((-num + np - 1) / np)) - 1;
-        for (int k = kmin;; k++) {
-            const int o = k * np + base;
-            if (o > p.hi[d]) break;
-            if (o + ext - 1 >= p.lb[d]) {
-                if (n == kMaxImages) {
-                    atomicOr(status, kStatTooManyImages);
-                    break;
-                }
-                img[n++] = o;
-            }
-        }
-    } else {
-        const int b = imod(p.cc[d] + p.lb[d] + lv.lb_grid[d], lv.npts[d]) - p.lb[d];
-        const int o = tt * T - b;
-        if (o <= p.hi[d] && o + ext - 1 >= p.lb[d]) img[n++] = o;
-    }
+// the number of images of one axis: cube offsets o such that the tile [o, o + ext) meets [lb, hi]
+__device__ int axis_image_count(const LevelDev &lv, int d, int tt, int T, const TPair &p) {
+    if (!lv.periodic[d]) return 1;
+    const int N = lv.npts[d], ext = min(T, lv.ngrid[d] - tt * T), base = tt * T - p.cc[d];
+    auto floor_div = [](int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); };
+    return floor_div(p.hi[d] - base, N) - floor_div(p.lb[d] - base - ext, N);
 }
 
 __device__ __forceinline__ void set_image_x(const TPair &p, ImgState &q, int ox, int ext_x) {
@@ -518,28 +504,6 @@ __device__ __forceinline__ void set_image_x(const TPair &p, ImgState &q, int ox,
     const int e = ((__float_as_int(ext) >> 23) & 0xff) - 126;  // ext = f 2^e, f in [0.5, 1)
     q.sb = ext >= 1.1754944e-38f ? min(max(e, -10), 10) : 0;
 }
-__device__ __forceinline__ void set_image(const TPair &p, ImgState &q, int ox, int oy, int oz, int ext_x) {
-    q.o[1] = oy;
-    q.o[2] = oz;
-    set_image_x(p, q, ox, ext_x);
-}
-
-// Threads 0-2 derive the periodic images of one axis each and set the first
-// image; the caller's next barrier publishes them.
-__device__ __forceinline__ void pair_images(TileCommon &sm, const TPair &p, const LevelDev &lv, const TileDesc &td,
-                                            int ext_x, int *status) {
-    const int tid = threadIdx.x;
-    if (tid < 3) {
-        const TileShape sh(td.lz);
-        const int T = tid == 0 ? TX : (tid == 1 ? sh.TY : sh.TZ);
-        axis_images(lv, tid, td.t[tid], T, p, sm.img[tid], sm.nimg[tid], status);
-        if (sm.nimg[tid] > 0) {
-            if (tid == 0) set_image_x(p, sm.im, sm.img[0][0], ext_x);
-            else sm.im.o[tid] = sm.img[tid][0];
-        }
-    }
-}
-
 // tab[k][i] = u^k exp(-zetp t^2), t = g h - off, g = o + i, and u = t or, for x
 // with recentre, u = (i - ic) h / 2^sb (the balanced offset from the
 // re-expansion column); zero outside the cube box, outside the valid tile extent
@@ -551,27 +515,22 @@ __device__ __forceinline__ void pair_images(TileCommon &sm, const TPair &p, cons
 // float-float exponential, its largest inlined function: collocate is limited by
 // instruction fetch, and this alone took it from 995 to 926 ms per launch on the
 // 1M-pair workload.
+struct TileExt {
+    int x, y, z;  // the tile's points inside the grid, per axis
+};
 struct TabEntry {
     ff t, e;    // t = g h - off and exp(-zetp t^2) (zero outside)
     int d, i;   // axis and tile-local index
     bool in;    // inside the cube box and the tile's valid extent
 };
-__device__ __forceinline__ TabEntry tab_entry(const TPair &p, const ImgState &q, const LevelDev &lv,
-                                              const TileDesc &td, const TileShape &sh, int warp, int ent) {
+__device__ __forceinline__ TabEntry tab_entry(const TPair &p, const ImgState &q, const TileExt &ext,
+                                              const TileShape &sh, int warp, int ent) {
     TabEntry r;
-    int T;
-    if (warp == 0) {
-        r.d = 0;
-        r.i = ent;
-        T = TX;
-    } else {
-        const bool isy = ent < sh.TY;
-        r.d = isy ? 1 : 2;
-        r.i = isy ? ent : ent - sh.TY;
-        T = isy ? sh.TY : sh.TZ;
-    }
+    const bool isy = ent < sh.TY;
+    r.d = warp == 0 ? 0 : (isy ? 1 : 2);
+    r.i = warp == 0 || isy ? ent : ent - sh.TY;
     const int g = q.o[r.d] + r.i;
-    r.in = r.i < min(T, lv.ngrid[r.d] - td.t[r.d] * T) && g >= p.lb[r.d] && g <= p.hi[r.d];
+    r.in = r.i < (warp == 0 ? ext.x : (isy ? ext.y : ext.z)) && g >= p.lb[r.d] && g <= p.hi[r.d];
     r.t = ff_add(ff_mul_f(p.h[r.d], (float)g), ff{-p.off[r.d].hi, -p.off[r.d].lo});
     r.e = r.in ? ff_exp(ff_mul(ff_mul(r.t, r.t), ff{-p.zetp.hi, -p.zetp.lo})) : ff{0.0f, 0.0f};
     return r;
@@ -858,22 +817,6 @@ __device__ __forceinline__ void first_pair(TileCommon &cm, Buf *pb, const MixedA
     if (it0 + 1 < it1) nxt = A.items[it0 + 1];
 }
 
-// images of the current item: 1 for the common case (state precomputed in ii);
-// for more, threads 0-2 derive them here (one extra barrier, out of line)
-__device__ __noinline__ void item_images_multi(TileCommon &cm, const TPair &P, const LevelDev &lv,
-                                               const TileDesc &td, int ext_x, int *status) {
-    pair_images(cm, P, lv, td, ext_x, status);
-    __syncthreads();
-}
-__device__ __forceinline__ int item_images(TileCommon &cm, const ItemImg &ii, const TPair &P, const LevelDev &lv,
-                                           const TileDesc &td, int ext_x, int *status) {
-    const int np = ii.nimg;
-    const int nimg = (np & 0xff) * ((np >> 8) & 0xff) * ((np >> 16) & 0xff);
-    if (nimg > 1) item_images_multi(cm, P, lv, td, ext_x, status);
-    return nimg;
-}
-
-
 // Stage 1 of collocate: Cxy[z][(b,a)] = sum_g c'[g][b][a] Z[g][z]; one output per
 // thread (16 consecutive threads share (b, a)), two partial sums over even and
 // odd g; the packed index of (g, b, a) is zs[g] - b g + k0.
@@ -977,6 +920,7 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
         const int tile = cm.tile;
         if (tile >= A.ntiles || cm.abort) break;
         const TileDesc td = A.tiles[tile];
+        if (tid == 0 && (td.flags & kUnitOver)) atomicOr(A.status, kStatTooManyImages);
         const LevelDev &lv = A.levels[td.level];
         const TileShape sh(td.lz);
         const int TY = sh.TY, TZ = sh.TZ, z = m >> sh.ly, y = m & (TY - 1);
@@ -988,8 +932,9 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
         float *acc_lo = sm.acc_lo[m];
 #pragma unroll
         for (int x = 0; x < TX; x++) acc_hi[x] = acc_lo[x] = 0.0f;
-        const int ext_z = min(TZ, lv.ngrid[2] - td.t[2] * TZ), ext_y = min(TY, lv.ngrid[1] - td.t[1] * TY);
-        const int ext_x = min(TX, lv.ngrid[0] - td.t[0] * TX);
+        const TileExt ext = {min(TX, lv.ngrid[0] - td.t[0] * TX), min(TY, lv.ngrid[1] - td.t[1] * TY),
+                             min(TZ, lv.ngrid[2] - td.t[2] * TZ)};
+        const bool row_ok = z < ext.z && y < ext.y;
         const int64_t it0 = A.start[2 * tile], it1 = A.start[2 * tile + 1];
         uint64_t nxt = 0;
         first_pair(cm, sm.pb, A, it0, it1, nxt, true);
@@ -998,24 +943,14 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
             const PairBuf &pb = sm.pb[cur];
             const TPair &P = pb.p;
             const int L = P.L, lp = P.lp;
-            const int nimg = item_images(cm, cm.ii[cur], P, lv, td, ext_x, A.status);
-            const ImgState &Q = nimg == 1 ? cm.ii[cur].im : cm.im;
-            for (int im = 0; im < nimg && !cm.abort; im++) {
-                if (im > 0) {
-                    if (tid == 0) {
-                        const int ix = im % cm.nimg[0], iy = (im / cm.nimg[0]) % cm.nimg[1],
-                                  iz = im / (cm.nimg[0] * cm.nimg[1]);
-                        set_image(P, cm.im, cm.img[0][ix], cm.img[1][iy], cm.img[2][iz], ext_x);
-                    }
-                    __syncthreads();
-                }
-                if (Q.gx0 > Q.gx1) continue;  // uniform: no x overlap
+            const ImgState &Q = cm.ii[cur].im;
+            {
                 // warp 0: X column (lane x) and its B slices, scaled by 2^(SLB - fx); warp 1:
                 // Y and Z tables; warps 2-3: re-expansion of the coefficients
                 if (warp < 2) {
 #pragma unroll 1
                     for (int ent = tid & 31; ent < (warp == 0 ? TX : TY + TZ); ent += 32) {
-                        const TabEntry te = tab_entry(P, Q, lv, td, sh, warp, ent);
+                        const TabEntry te = tab_entry(P, Q, ext, sh, warp, ent);
                         if (warp == 0) {
                             ff xv[kNPow];
                             x_powers(P, Q, te, ent, true, xv);
@@ -1043,10 +978,10 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                 // stage 2 (this thread's row, all a at once) + culling + A slices
                 int x0, x1;
                 if constexpr (kGeneral)
-                    general_row_range(lv, A.glv[td.level], P, Q, Q.o[2] + z, Q.o[1] + y, z < ext_z && y < ext_y, x0,
+                    general_row_range(lv, A.glv[td.level], P, Q, Q.o[2] + z, Q.o[1] + y, row_ok, x0,
                                       x1);
                 else
-                    row_range(P, Q, A.table, Q.o[2] + z, Q.o[1] + y, z < ext_z && y < ext_y, x0, x1);
+                    row_range(P, Q, A.table, Q.o[2] + z, Q.o[1] + y, row_ok, x0, x1);
                 const int em = stage2_row(sm, cm, L, lp, Q.sb, z, y, x0 <= x1, max(L, cm.kmax), m);
                 // stage 3 on the tensor cores: D_s = sum_{i+j=s} A_i B_j^T
                 tc::fence_async_smem();
@@ -1152,7 +1087,7 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
         cp_async_wait_all();
         if (cm.abort) break;
         // flush: grid += tile sum (FP64)
-        if (z < ext_z && y < ext_y) {
+        if (row_ok) {
             double *grid = A.grids.p[td.level];
             const int64_t row = ((int64_t)(td.t[2] * TZ + z) * lv.ngrid[1] + (td.t[1] * TY + y)) * lv.ngrid[0] +
                                 td.t[0] * TX;
@@ -1162,9 +1097,9 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
                     const int x = 8 * c + i;
-                    if (x >= ext_x) continue;
+                    if (x >= ext.x) continue;
                     const double v = (double)acc_hi[i] + (double)acc_lo[x];
-                    if (td.split) atomicAdd(grid + row + x, v);  // other work units add to the same tile
+                    if (td.flags & kUnitSplit) atomicAdd(grid + row + x, v);  // other work units add to the same tile
                     else grid[row + x] += v;
                 }
 #pragma unroll
@@ -1207,23 +1142,25 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
         const int tile = cm.tile;
         if (tile >= A.ntiles || cm.abort) break;
         const TileDesc td = A.tiles[tile];
+        if (tid == 0 && (td.flags & kUnitOver)) atomicOr(A.status, kStatTooManyImages);
         const LevelDev &lv = A.levels[td.level];
         const TileShape sh(td.lz);
         const int TY = sh.TY, TZ = sh.TZ, z = m >> sh.ly, y = m & (TY - 1);
-        const int ext_z = min(TZ, lv.ngrid[2] - td.t[2] * TZ), ext_y = min(TY, lv.ngrid[1] - td.t[1] * TY);
-        const int ext_x = min(TX, lv.ngrid[0] - td.t[0] * TX);
+        const TileExt ext = {min(TX, lv.ngrid[0] - td.t[0] * TX), min(TY, lv.ngrid[1] - td.t[1] * TY),
+                             min(TZ, lv.ngrid[2] - td.t[2] * TZ)};
+        const bool row_ok = z < ext.z && y < ext.y;
         // this thread's V row, sliced once per tile (row exponent vm)
         int vm;
         {
             const double *grid = A.grids.p[td.level];
-            const bool ok = z < ext_z && y < ext_y;
+            const bool ok = row_ok;
             const int64_t row = ((int64_t)(td.t[2] * TZ + z) * lv.ngrid[1] + (td.t[1] * TY + y)) * lv.ngrid[0] +
                                 td.t[0] * TX;
             // compact loops (once per tile): the row maximum, then 16-byte chunks of 8 x
             float mx = 0.0f;
 #pragma unroll 1
             for (int x = 0; x < TX; x++) {
-                const ff v = (ok && x < ext_x) ? ff_from_double(grid[row + x]) : ff{0.0f, 0.0f};
+                const ff v = (ok && x < ext.x) ? ff_from_double(grid[row + x]) : ff{0.0f, 0.0f};
                 if constexpr (kGeneral) sm.Vff[x][m] = v;
                 mx = fmaxf(mx, fabsf(v.hi));
             }
@@ -1235,8 +1172,8 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     const int x = 8 * c + 2 * i;
-                    const ff v0 = (ok && x < ext_x) ? ff_from_double(grid[row + x]) : ff{0.0f, 0.0f};
-                    const ff v1 = (ok && x + 1 < ext_x) ? ff_from_double(grid[row + x + 1]) : ff{0.0f, 0.0f};
+                    const ff v0 = (ok && x < ext.x) ? ff_from_double(grid[row + x]) : ff{0.0f, 0.0f};
+                    const ff v1 = (ok && x + 1 < ext.x) ? ff_from_double(grid[row + x + 1]) : ff{0.0f, 0.0f};
                     float s0[NSL], s1[NSL];
                     slice_scaled(v0, sc, s0);
                     slice_scaled(v1, sc, s1);
@@ -1262,26 +1199,16 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
             const int L = P.L, lp = P.lp;
             const int npair = (L * (L + 1)) / 2;
             const int64_t moff = P.coef_off;
-            const int nimg = item_images(cm, cm.ii[cur], P, lv, td, ext_x, A.status);
-            const ImgState &Q = nimg == 1 ? cm.ii[cur].im : cm.im;
-            for (int im = 0; im < nimg && !cm.abort; im++) {
-                if (im > 0) {
-                    if (tid == 0) {
-                        const int ix = im % cm.nimg[0], iy = (im / cm.nimg[0]) % cm.nimg[1],
-                                  iz = im / (cm.nimg[0] * cm.nimg[1]);
-                        set_image(P, cm.im, cm.img[0][ix], cm.img[1][iy], cm.img[2][iz], ext_x);
-                    }
-                    __syncthreads();
-                }
-                if (Q.gx0 > Q.gx1) continue;
+            const ImgState &Q = cm.ii[cur].im;
+            {
                 {
                     // every thread: its row's cube x range, for the A operand of warps 2-3
                     int x0, x1;
                     if constexpr (kGeneral)
-                        general_row_range(lv, A.glv[td.level], P, Q, Q.o[2] + z, Q.o[1] + y, z < ext_z && y < ext_y,
+                        general_row_range(lv, A.glv[td.level], P, Q, Q.o[2] + z, Q.o[1] + y, row_ok,
                                           x0, x1);
                     else
-                        row_range(P, Q, A.table, Q.o[2] + z, Q.o[1] + y, z < ext_z && y < ext_y, x0, x1);
+                        row_range(P, Q, A.table, Q.o[2] + z, Q.o[1] + y, row_ok, x0, x1);
                     const bool empty = x0 > x1;  // otherwise both lie in [0, TX)
                     sm.rx0[m] = (signed char)(empty ? 1 : x0);
                     sm.rx1[m] = (signed char)(empty ? 0 : x1);
@@ -1294,7 +1221,7 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                     // collocate, integrate is not limited by instruction fetch: warps 0 and 1
                     // keep separate table code.
                     ff xv[kNPow];
-                    x_powers(P, Q, tab_entry(P, Q, lv, td, sh, 0, tid), tid, false, xv);
+                    x_powers(P, Q, tab_entry(P, Q, ext, sh, 0, tid), tid, false, xv);
 #pragma unroll
                     for (int a = 0; a < kNPow; a++) {
                         if (a >= L) break;
@@ -1316,7 +1243,7 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                     if constexpr (!kGeneral) bar_arrive1(NTHR);
                     if (tid - 32 <= kNPow) sm.zs[tid - 32] = tid - 32 <= lp + 1 ? row_start(lp, tid - 32, 0) : 0;
 #pragma unroll 1
-                    for (int ent = tid - 32; ent < TY + TZ; ent += 32) yz_fill(cm, P, tab_entry(P, Q, lv, td, sh, 1, ent));
+                    for (int ent = tid - 32; ent < TY + TZ; ent += 32) yz_fill(cm, P, tab_entry(P, Q, ext, sh, 1, ent));
                 } else if constexpr (!kGeneral) {
                     bar_sync1(NTHR);
                     // A operand: V slices of rows u and u + 64 (the CTA's slot) masked to the rows' cube ranges,
@@ -1513,26 +1440,25 @@ __global__ void k_coef_to_blob(const double *__restrict__ c, uint4 *blob, const 
     }
 }
 
-// the images of every (tile, pair) item, once per task set; one block per tile
-__global__ void k_item_images(const TileDesc *__restrict__ tiles, const int64_t *__restrict__ start,
+// the image state of every item from its offsets (left in im.o by the binning),
+// once per task set; one block per work unit
+__global__ void k_item_images(TileDesc *tiles, const int64_t *__restrict__ start,
                               const uint64_t *__restrict__ items, const uint4 *__restrict__ blob,
-                              const LevelDev *__restrict__ levels, ItemImg *out, int ntiles, int *status) {
+                              const LevelDev *__restrict__ levels, ItemImg *out, int ntiles) {
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const TileDesc td = tiles[tile];
         const LevelDev &lv = levels[td.level];
+        const TileShape sh(td.lz);
         const int ext_x = min(TX, lv.ngrid[0] - td.t[0] * TX);
         for (int64_t it = start[2 * tile] + threadIdx.x; it < start[2 * tile + 1]; it += blockDim.x) {
             const TPair &p = *reinterpret_cast<const TPair *>(blob + (items[it] >> 16));
-            int img[3][kMaxImages], n[3];
-            axis_images(lv, 0, td.t[0], TX, p, img[0], n[0], status);
-            const TileShape sh(td.lz);
-            axis_images(lv, 1, td.t[1], sh.TY, p, img[1], n[1], status);
-            axis_images(lv, 2, td.t[2], sh.TZ, p, img[2], n[2], status);
-            ItemImg r;
-            memset(&r, 0, sizeof r);
-            r.nimg = n[0] | (n[1] << 8) | (n[2] << 16);
-            if (n[0] > 0 && n[1] > 0 && n[2] > 0) set_image(p, r.im, img[0][0], img[1][0], img[2][0], ext_x);
+            ItemImg r = out[it];
+            set_image_x(p, r.im, r.im.o[0], ext_x);
             out[it] = r;
+            if (axis_image_count(lv, 0, td.t[0], TX, p) > kMaxImages ||
+                axis_image_count(lv, 1, td.t[1], sh.TY, p) > kMaxImages ||
+                axis_image_count(lv, 2, td.t[2], sh.TZ, p) > kMaxImages)
+                atomicOr(&tiles[tile].flags, kUnitOver);
         }
     }
 }
@@ -1541,6 +1467,7 @@ __global__ void k_item_images(const TileDesc *__restrict__ tiles, const int64_t 
 // Binning on the device: the (tile, pair) items of every binned pair.
 struct BinLevel {
     double G[3][3];     // metric of the lattice steps, G_ab = v_a . v_b (general cells)
+    double plane[3];    // |r|^2 >= plane[a] d_a^2 whatever the other two (1 / (G^-1)_aa)
     int first;          // index of the level's first tile
     int nt[3];          // tiles per axis
     int lz;             // log2 of the tile z extent
@@ -1599,97 +1526,55 @@ __device__ double box_min_q(const double (&G)[3][3], const double (&lo)[3], cons
 }
 
 // One axis of a pair's cube (cube offsets lb..hi around cc, as grid_base_ref_c.cc:318-351
-// maps them) cut into runs of consecutive grid indices inside one tile.
+// maps them) cut into runs of consecutive grid indices inside one tile.  The runs
+// into one tile are the cube's periodic images over it, one item each.  Run r is the
+// (t0 + r)-th tile counted through the wraps of a periodic axis.
 struct AxisRuns {
-    int lb, hi, cc, T, N, npts, periodic, lbg;
-    bool dedupe;  // the cube spans so much of a periodic axis that two runs may hit one tile
-    __device__ void init(const LevelDev &lv, int d, int cc_, int lb_, int hi_, int T_) {
-        lb = lb_; hi = hi_; cc = cc_; T = T_;
-        N = lv.ngrid[d]; npts = lv.npts[d]; periodic = lv.periodic[d]; lbg = lv.lb_grid[d];
-        dedupe = periodic && (hi - lb + 1) + T > N;
-    }
-    // the run starting at offset gg: its tile and its offsets g0..g1; gg moves
-    // past the run; false: outside the window
-    __device__ bool next(int &gg, int &t, int &g0, int &g1) const {
-        const int w = periodic ? imod(cc + gg, npts) : gg + imod(cc + lb + lbg, npts) - lb;
-        if (w < 0 || w >= N) {
-            gg++;
-            return false;
+    int lb, hi, T, N, nt, o0, t0, n;  // o0: cube offset of tile 0's origin (first wrap); n runs
+    __device__ void init(const LevelDev &lv, int d, int cc, int lb_, int hi_, int T_, int nt_) {
+        lb = lb_; hi = hi_; T = T_; nt = nt_; N = lv.ngrid[d];
+        int w = lv.periodic[d] ? imod(cc + lb, lv.npts[d]) : imod(cc + lb + lv.lb_grid[d], lv.npts[d]);
+        o0 = lb - w;
+        if (!lv.periodic[d]) {  // points outside the window belong to no tile
+            lb = max(lb, o0);
+            hi = min(hi, o0 + N - 1);
+            w = lb - o0;
         }
-        t = w / T;
-        const int len = min(T - (w - t * T), N - w);
-        g0 = gg;
-        g1 = min(gg + len - 1, hi);
-        gg += len;
-        return true;
+        t0 = w / T;
+        const int we = hi - o0, k = we / N;
+        n = hi < lb ? 0 : k * nt + (we - k * N) / T - t0 + 1;
     }
-    // calls fn(tile, g0, g1) once per tile the axis touches; where several runs
-    // reach one tile, only the first reports it, with the hull of their offsets
-    template <class Fn>
-    __device__ void each_range(Fn &&fn) const {
-        for (int gg = lb; gg <= hi;) {
-            const int gs = gg;
-            int t, g0, g1;
-            if (!next(gg, t, g0, g1)) continue;
-            if (dedupe) {
-                bool seen = false;
-                for (int g2 = lb; g2 < gs && !seen;) {
-                    int t2, a2, b2;
-                    if (next(g2, t2, a2, b2) && t2 == t) seen = true;
-                }
-                if (seen) continue;
-                for (int g2 = gg; g2 <= hi;) {
-                    int t2, a2, b2;
-                    if (next(g2, t2, a2, b2) && t2 == t) {
-                        g0 = min(g0, a2);
-                        g1 = max(g1, b2);
-                    }
-                }
-            }
-            fn(t, g0, g1);
-        }
-    }
-    // calls fn(tile, fmin) once per tile the axis touches, fmin the smallest folded
-    // offset |f| (f = g <= 0 ? -g : g - 1) over the runs into the tile
-    template <class Fn>
-    __device__ void each(Fn &&fn) const {
-        for (int gg = lb; gg <= hi;) {
-            const int gs = gg;
-            int t, g0, g1;
-            if (!next(gg, t, g0, g1)) continue;
-            auto fold = [](int a, int b) { return (a <= 1 && b >= 0) ? 0 : (b < 0 ? -b : a - 1); };
-            int f = fold(g0, g1);
-            if (dedupe) {  // only the first run into a tile reports it, with the minimum over all runs
-                bool seen = false;
-                for (int g2 = lb; g2 < gs && !seen;) {
-                    int t2, a2, b2;
-                    if (next(g2, t2, a2, b2) && t2 == t) seen = true;
-                }
-                if (seen) continue;
-                for (int g2 = gg; g2 <= hi;) {
-                    int t2, a2, b2;
-                    if (next(g2, t2, a2, b2) && t2 == t) f = min(f, fold(a2, b2));
-                }
-            }
-            fn(t, f);
-        }
+    // run r: its tile, its offsets g0..g1 and the cube offset o of the tile's origin
+    __device__ __forceinline__ void get(int r, int &t, int &g0, int &g1, int &o) const {
+        const int q = t0 + r, k = q < nt ? 0 : q / nt;
+        t = q - k * nt;
+        o = o0 + t * T + k * N;
+        g0 = max(lb, o);
+        g1 = min(hi, o + min(T, N - t * T) - 1);
     }
 };
+// the smallest folded offset |f| (f = g <= 0 ? -g : g - 1) of a run
+__device__ __forceinline__ int run_fold(int a, int b) { return (a <= 1 && b >= 0) ? 0 : (b < 0 ? -b : a - 1); }
 
-// Pass 0: items per tile (count).  Pass 1: item words into the tile's slots
-// (cursor).  A pair visits a tile only if some cube point of the tile can be
-// inside its sphere (with a margin): orthorhombic, the folded distance of the
-// tile's nearest offsets <= radius; general cell, the least |r - rp|^2 over the
-// lattice-index box of the tile's offsets (box_min_q) <= radius^2, tested per z
-// run, then per (z, y) runs, then per tile.  Explicit cube lists are not culled.
+// Pass 0: items per tile (count).  Pass 1: item words and image offsets into the
+// tile's slots (cursor).  A pair's image visits a tile only if some cube point of
+// the image in the tile can be inside its sphere (with a margin): orthorhombic, the
+// folded distance of the runs' nearest offsets <= radius; general cell, the least
+// |r - rp|^2 over the lattice-index box of the runs (box_min_q) <= radius^2, tested
+// per axis, then per item.  Explicit cube lists are not culled.
 // kGen: the general-cell pairs [k0, k1) (the culling's box minimum needs registers
 // and stack that would slow the orthorhombic launch, kGen = false).
+// 2^lper threads share a pair, each on its own (z, y) runs: the largest cubes have
+// hundreds of them, and few pairs alone would leave the chip idle (8000 general-cell
+// pairs, one thread each, took 0.4 s to bin).
 template <bool kGen>
-__global__ void k_bin_pairs(const PairGeom *__restrict__ geoms, int64_t k0, int64_t k1,
+__global__ void k_bin_pairs(const PairGeom *__restrict__ geoms, int64_t k0, int64_t k1, int lper,
                             const LevelDev *__restrict__ levels, const BinLevel *__restrict__ bl,
                             const int64_t *__restrict__ off16, const int *__restrict__ len16, int pass, int *count,
-                            unsigned long long *cursor, uint64_t *items) {
-    for (int64_t k = k0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < k1; k += (int64_t)gridDim.x * blockDim.x) {
+                            unsigned long long *cursor, uint64_t *items, ItemImg *iimg) {
+    const int mask = (1 << lper) - 1;
+    for (int64_t k = k0 + ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> lper); k < k1;
+         k += ((int64_t)gridDim.x * blockDim.x) >> lper) {
         const PairGeom &g = geoms[k];
         const LevelDev &lv = levels[g.level];
         const BinLevel B = bl[g.level];
@@ -1700,72 +1585,96 @@ __global__ void k_bin_pairs(const PairGeom *__restrict__ geoms, int64_t k0, int6
             hi[d] = g.ortho ? g.hi[d] : g.hi[d] - g.cc[d];
         }
         AxisRuns ax, ay, az;
-        ax.init(lv, 0, g.cc[0], lb[0], hi[0], TX);
-        ay.init(lv, 1, g.cc[1], lb[1], hi[1], sh.TY);
-        az.init(lv, 2, g.cc[2], lb[2], hi[2], sh.TZ);
+        ax.init(lv, 0, g.cc[0], lb[0], hi[0], TX, B.nt[0]);
+        ay.init(lv, 1, g.cc[1], lb[1], hi[1], sh.TY, B.nt[1]);
+        az.init(lv, 2, g.cc[2], lb[2], hi[2], sh.TZ, B.nt[2]);
+        int tx, ty, tz, x0, x1, y0, y1, z0, z1, ox, oy, oz;
         const double r2 = g.radius * g.radius * (1.0 + 1e-9) + 1e-12;
         const double hx = lv.dh[0][0], hy = lv.dh[1][1], hz = lv.dh[2][2];
         const bool table = g.table_off >= 0;
         const uint64_t word = ((uint64_t)off16[k] << 16) | (uint64_t)len16[k];
-        auto emit = [&](int tz, int ty, int tx) {
+        auto emit = [&]() {
             const int tile = B.first + (tz * B.nt[1] + ty) * B.nt[0] + tx;
-            if (pass == 0) atomicAdd(count + tile, 1);
-            else items[atomicAdd(cursor + tile, 1ull)] = word;
+            if (pass == 0) {
+                atomicAdd(count + tile, 1);
+                return;
+            }
+            const unsigned long long at = atomicAdd(cursor + tile, 1ull);
+            items[at] = word;
+            iimg[at].im.o[0] = ox;
+            iimg[at].im.o[1] = oy;
+            iimg[at].im.o[2] = oz;
         };
         if constexpr (kGen) {
             // lattice-index offsets from the product centre: d_a = cc_a + gg - gp_a
             const double c[3] = {g.off[0] - g.cc[0], g.off[1] - g.cc[1], g.off[2] - g.cc[2]};
             const double rg = g.radius * g.radius * (1.0 + 1e-6) + 1e-12;
-            double lo[3] = {-HUGE_VAL, -HUGE_VAL, 0.0}, up[3] = {HUGE_VAL, HUGE_VAL, 0.0};
-            az.each_range([&](int tz, int z0, int z1) {
-                lo[2] = z0 - c[2];
-                up[2] = z1 - c[2];
-                lo[1] = lo[0] = -HUGE_VAL;
-                up[1] = up[0] = HUGE_VAL;
-                if (box_min_q(B.G, lo, up) > rg) return;
-                ay.each_range([&](int ty, int y0, int y1) {
-                    lo[1] = y0 - c[1];
-                    up[1] = y1 - c[1];
-                    lo[0] = -HUGE_VAL;
-                    up[0] = HUGE_VAL;
-                    if (box_min_q(B.G, lo, up) > rg) return;
-                    ax.each_range([&](int tx, int x0, int x1) {
-                        lo[0] = x0 - c[0];
-                        up[0] = x1 - c[0];
-                        if (box_min_q(B.G, lo, up) > rg) return;
-                        emit(tz, ty, tx);
-                    });
-                });
-            });
+            double lo[3], up[3];
+            auto set = [&](int a, int g0, int g1) {  // false: the run's slab lies outside the sphere
+                lo[a] = g0 - c[a];
+                up[a] = g1 - c[a];
+                const double d = lo[a] > 0.0 ? lo[a] : (up[a] < 0.0 ? up[a] : 0.0);
+                return B.plane[a] * d * d <= rg;
+            };
+            auto meets = [&]() {  // the box's least |r|^2 <= rg: its point nearest in indices is an upper bound
+                double p[3], q = 0.0;
+                for (int a = 0; a < 3; a++) p[a] = fmin(fmax(0.0, lo[a]), up[a]);
+                for (int a = 0; a < 3; a++)
+                    for (int b = 0; b < 3; b++) q += p[a] * B.G[a][b] * p[b];
+                return q <= rg || box_min_q(B.G, lo, up) <= rg;
+            };
+            for (int zy = threadIdx.x & mask; zy < az.n * ay.n; zy += mask + 1) {
+                const int rz = zy / ay.n;
+                az.get(rz, tz, z0, z1, oz);
+                ay.get(zy - rz * ay.n, ty, y0, y1, oy);
+                if (!set(2, z0, z1) || !set(1, y0, y1)) continue;
+                for (int rx = 0; rx < ax.n; rx++) {
+                    ax.get(rx, tx, x0, x1, ox);
+                    if (set(0, x0, x1) && meets()) emit();
+                }
+            }
         } else {
-        az.each([&](int tz, int fz) {
-            const double dz = fz * hz;
-            if (!table && dz * dz > r2) return;
-            ay.each([&](int ty, int fy) {
-                const double dy = fy * hy;
-                if (!table && dz * dz + dy * dy > r2) return;
-                ax.each([&](int tx, int fx) {
-                    const double dx = fx * hx;
-                    if (!table && dz * dz + dy * dy + dx * dx > r2) return;
-                    emit(tz, ty, tx);
-                });
-            });
-        });
+            for (int zy = threadIdx.x & mask; zy < az.n * ay.n; zy += mask + 1) {
+                const int rz = zy / ay.n;
+                az.get(rz, tz, z0, z1, oz);
+                ay.get(zy - rz * ay.n, ty, y0, y1, oy);
+                const double dz = run_fold(z0, z1) * hz, dy = run_fold(y0, y1) * hy;
+                if (!table && dz * dz + dy * dy > r2) continue;
+                for (int rx = 0; rx < ax.n; rx++) {
+                    ax.get(rx, tx, x0, x1, ox);
+                    const double dx = run_fold(x0, x1) * hx;
+                    if (table || dz * dz + dy * dy + dx * dx <= r2) emit();
+                }
+            }
         }
     }
 }
 
 // both kinds of pairs of a task set (orthorhombic first in the sorted order)
 static cudaError_t bin_pairs(const TaskSet &ts, const MixedState &M, int pass, int *count,
-                             unsigned long long *cursor, uint64_t *items) {
+                             unsigned long long *cursor, uint64_t *items, ItemImg *iimg) {
     const Plan &P = *ts.plan;
-    auto blocks = [](int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 127) / 128, 8192)); };
-    if (M.northo > 0)
-        k_bin_pairs<false><<<blocks(M.northo), 128>>>(ts.d_geom, 0, M.northo, P.d_levels, M.d_bl, M.d_blob_off,
-                                                      M.d_blob_len, pass, count, cursor, items);
-    if (M.nbin > M.northo)
-        k_bin_pairs<true><<<blocks(M.nbin - M.northo), 128>>>(ts.d_geom, M.northo, M.nbin, P.d_levels, M.d_bl,
-                                                              M.d_blob_off, M.d_blob_len, pass, count, cursor, items);
+    auto blocks = [](int64_t threads) {
+        return (unsigned)std::max<int64_t>(1, std::min<int64_t>((threads + 127) / 128, 8192));
+    };
+    // about 2^18 threads (the chip's 152 SMs hold 1.2 waves of them) or one per pair
+    auto share = [](int64_t n) {
+        int l = 0;
+        while (l < 5 && (n << l) < (1 << 18)) l++;
+        return l;
+    };
+    if (M.northo > 0) {
+        const int l = share(M.northo);
+        k_bin_pairs<false><<<blocks((int64_t)M.northo << l), 128>>>(ts.d_geom, 0, M.northo, l, P.d_levels, M.d_bl,
+                                                                  M.d_blob_off, M.d_blob_len, pass, count, cursor,
+                                                                  items, iimg);
+    }
+    if (M.nbin > M.northo) {
+        const int l = share(M.nbin - M.northo);
+        k_bin_pairs<true><<<blocks((M.nbin - M.northo) << l), 128>>>(ts.d_geom, M.northo, M.nbin, l, P.d_levels,
+                                                                   M.d_bl, M.d_blob_off, M.d_blob_len, pass, count,
+                                                                   cursor, items, iimg);
+    }
     return cudaGetLastError();
 }
 
@@ -1928,6 +1837,14 @@ int mixed_build(TaskSet &ts, std::string &err) {
         for (int a = 0; a < 3; a++)
             for (int b = 0; b < 3; b++)
                 blv[l].G[a][b] = lv.dh[a][0] * lv.dh[b][0] + lv.dh[a][1] * lv.dh[b][1] + lv.dh[a][2] * lv.dh[b][2];
+        const double(&G)[3][3] = blv[l].G;
+        const double det = G[0][0] * (G[1][1] * G[2][2] - G[1][2] * G[1][2]) -
+                           G[0][1] * (G[0][1] * G[2][2] - G[1][2] * G[0][2]) +
+                           G[0][2] * (G[0][1] * G[1][2] - G[1][1] * G[0][2]);
+        for (int a = 0; a < 3; a++) {
+            const int b = (a + 1) % 3, c = (a + 2) % 3;
+            blv[l].plane[a] = det / (G[b][b] * G[c][c] - G[b][c] * G[b][c]);
+        }
     }
     const int ntiles = (int)tiles.size();
     // blob layout: per task the record, then its coefficients
@@ -1949,7 +1866,7 @@ int mixed_build(TaskSet &ts, std::string &err) {
     alloc((void **)&M->d_bl, sizeof(BinLevel) * blv.size());
     alloc((void **)&M->d_count, sizeof(int) * (size_t)std::max(ntiles, 1));
     alloc((void **)&M->d_cursor, sizeof(unsigned long long) * (size_t)std::max(ntiles, 1));
-    alloc((void **)&M->d_queue, sizeof(int) * 5);  // [4]: status sink of the set-up kernels
+    alloc((void **)&M->d_queue, sizeof(int) * 4);
     alloc((void **)&M->d_glv, sizeof(GenLevel) * glv.size());
     if (e == cudaSuccess) e = cudaMemset(M->d_blob, 0, sizeof(uint4) * (size_t)std::max<int64_t>(nchunks, 1));
     if (e == cudaSuccess)
@@ -1959,7 +1876,7 @@ int mixed_build(TaskSet &ts, std::string &err) {
     if (e == cudaSuccess) e = cudaMemcpy(M->d_bl, blv.data(), sizeof(BinLevel) * blv.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
         e = cudaMemcpy(M->d_glv, glv.data(), sizeof(GenLevel) * glv.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(M->d_queue, 0, sizeof(int) * 5);
+    if (e == cudaSuccess) e = cudaMemset(M->d_queue, 0, sizeof(int) * 4);
     if (e != cudaSuccess) {
         err = std::string("mixed_build: ") + cudaGetErrorString(e);
         return GPW_ERR_CUDA;
@@ -2026,7 +1943,7 @@ int mixed_rebin(TaskSet &ts, std::string &err) {
         if ((e = cudaGetLastError()) != cudaSuccess) return fail(e);
     }
     if ((e = cudaMemset(M->d_count, 0, sizeof(int) * (size_t)std::max(ntiles, 1))) != cudaSuccess) return fail(e);
-    if (nbin > 0 && (e = bin_pairs(ts, *M, 0, M->d_count, nullptr, nullptr)) != cudaSuccess) return fail(e);
+    if (nbin > 0 && (e = bin_pairs(ts, *M, 0, M->d_count, nullptr, nullptr, nullptr)) != cudaSuccess) return fail(e);
     std::vector<int> count((size_t)std::max(ntiles, 1), 0);
     if ((e = cudaMemcpy(count.data(), M->d_count, sizeof(int) * count.size(), cudaMemcpyDeviceToHost)) != cudaSuccess)
         return fail(e);
@@ -2038,13 +1955,17 @@ int mixed_rebin(TaskSet &ts, std::string &err) {
     while (nto < ntiles && P.lv[M->h_tiles[nto].level].ortho) nto++;
     // Work units for the persistent queue: a tile with more items than ~1/64 of
     // an even share per SM is divided into units of consecutive items (their
-    // flushes add with FP64 atomics).  Within each group (orthorhombic, general)
-    // units run by decreasing work class (item counts within a factor 2^(1/4)
-    // share a class), and within a class in the tiles' raster order: the tiles in
-    // flight at one time then form a compact slab of the grid, so a pair's record,
-    // coefficients and moments stay in L2 between the neighbouring tiles that use
-    // them, while the short units still come last.
-    const int64_t target = std::max<int64_t>(64, (nitems + 64LL * M->sms - 1) / std::max(1, 64 * M->sms));
+    // flushes add with FP64 atomics), and where that leaves fewer than about four
+    // units per resident CTA, than 1/16 of it, down to 16 items (1000 pairs, 64^3:
+    // 359 units of up to 64 items for 608 CTAs, 2203 of up to 16).  Within each group
+    // (orthorhombic, general) units run by decreasing work class (item counts within a
+    // factor 2^(1/4) share a class), and within a class in the tiles' raster order: the
+    // tiles in flight at one time then form a compact slab of the grid, so a pair's
+    // record, coefficients and moments stay in L2 between the neighbouring tiles that
+    // use them, while the short units still come last.
+    const int64_t sms = std::max(1, M->sms);
+    const int64_t target = std::max((nitems + 64 * sms - 1) / (64 * sms),
+                                    std::min<int64_t>(64, std::max<int64_t>(16, nitems / (16 * sms))));
     struct Unit {
         int tile;
         int64_t it0, it1;
@@ -2071,7 +1992,7 @@ int mixed_rebin(TaskSet &ts, std::string &err) {
     std::vector<int64_t> ubounds(2 * (size_t)std::max(nunits, 1), 0);  // per unit: first item, end
     for (int u = 0; u < nunits; u++) {
         tiles_sorted[u] = M->h_tiles[units[u].tile];
-        tiles_sorted[u].split = units[u].split ? 1 : 0;
+        tiles_sorted[u].flags = units[u].split ? kUnitSplit : 0;
         ubounds[2 * u] = units[u].it0;
         ubounds[2 * u + 1] = units[u].it1;
     }
@@ -2109,12 +2030,12 @@ int mixed_rebin(TaskSet &ts, std::string &err) {
     if ((e = cudaMemcpy(M->d_cursor, cur.data(), sizeof(unsigned long long) * cur.size(), cudaMemcpyHostToDevice)) !=
         cudaSuccess)
         return fail(e);
-    if (nbin > 0 && (e = bin_pairs(ts, *M, 1, nullptr, M->d_cursor, M->d_items)) != cudaSuccess) return fail(e);
+    if (nbin > 0 && (e = bin_pairs(ts, *M, 1, nullptr, M->d_cursor, M->d_items, M->d_iimg)) != cudaSuccess) return fail(e);
     if (nitems) {
-        // image overflows are reported by the tiled kernels when they run (a plain
+        // (image overflows are reported by the tiled kernels when they run: a plain
         // FP64 call on this task set must not see them)
         k_item_images<<<std::max(1, std::min(nunits, 8192)), 128>>>(M->d_tiles, M->d_start, M->d_items, M->d_blob,
-                                                                    P.d_levels, M->d_iimg, nunits, M->d_queue + 4);
+                                                                    P.d_levels, M->d_iimg, nunits);
         if ((e = cudaGetLastError()) != cudaSuccess) return fail(e);
     }
     if ((e = cudaDeviceSynchronize()) != cudaSuccess) return fail(e);
