@@ -170,26 +170,23 @@ struct MixedState {
 
 // ---------------------------------------------------------------------------
 // Sphere rule (FP32 with an error bound, fast_floor_checked in gpw_common.cuh).
-// the exact FP64 rule, out of line: taken only where the FP32 estimate is unsure
-__device__ __noinline__ int rule_jmax_exact(const TPair &p, int kf) { return rule_jmax(rule_remk(p.r2, kf, p.hz), p.hy); }
-__device__ __noinline__ int rule_imax_exact(const TPair &p, int kf, int jf) {
-    return rule_imax(rule_remk(p.r2, kf, p.hz), jf, p.hy, p.hx);
+// the exact FP64 rule, out of line: taken only where the FP32 estimate is unsure;
+// the row's imax, or -1 for a row outside the cube
+__device__ __noinline__ int rule_row_exact(const TPair &p, int kf, int jf) {
+    const double remk = rule_remk(p.r2, kf, p.hz);
+    return jf < -rule_jmax(remk, p.hy) ? -1 : rule_imax(remk, jf, p.hy, p.hx);
 }
 
-__device__ __forceinline__ int row_jmax(const TPair &p, int kf) {
-    const float dz = (float)(-kf) * p.hzf;
-    bool unsure;
-    int j = fast_floor_checked(__fmaf_rn(-dz, dz, p.r2f), p.r2f, p.hyinvf, unsure);
-    if (unsure) j = rule_jmax_exact(p, kf);
-    return j;
-}
-
+// imax of the folded row (kf, jf), negative outside the cube.  The row lies in the
+// cube when (jf hy)^2 <= r^2 - (kf hz)^2: the sign of the remainder decides it, away
+// from zero by more than its error bound.
 __device__ __forceinline__ int row_imax(const TPair &p, int kf, int jf) {
     const float dz = (float)(-kf) * p.hzf, dy = (float)(-jf) * p.hyf;
+    const float rem = __fmaf_rn(-dy, dy, __fmaf_rn(-dz, dz, p.r2f));
+    if (rem < p.r2f * -4.8e-7f) return -1;
     bool unsure;
-    int i = fast_floor_checked(__fmaf_rn(-dy, dy, __fmaf_rn(-dz, dz, p.r2f)), p.r2f, p.hxinvf, unsure);
-    if (unsure) i = rule_imax_exact(p, kf, jf);
-    return i;
+    const int i = fast_floor_checked(rem, p.r2f, p.hxinvf, unsure);
+    return unsure ? rule_row_exact(p, kf, jf) : i;
 }
 
 // Row (z, y) of the tile: cube-local x range [x0, x1] (empty if x0 > x1).
@@ -200,15 +197,14 @@ __device__ __forceinline__ void row_range(const TPair &p, const ImgState &q, con
     if (!ext_ok || gz < p.lb[2] || gz > p.hi[2] || gy < p.lb[1] || gy > p.hi[1]) return;
     const int kf = fold(gz), jf = fold(gy);
     if (kf < p.kgmin) return;
-    int jmin, imin;
+    int imin;
     if (p.table_off < 0) {
-        const int jmax = row_jmax(p, kf);
-        if (jf < -jmax) return;
         imin = -row_imax(p, kf, jf);
+        if (imin > 0) return;
     } else {
         const int *T = table + p.table_off;
         const int kidx = kf - T[0];
-        jmin = T[1 + 2 * kidx];
+        const int jmin = T[1 + 2 * kidx];
         if (jf < jmin) return;
         imin = T[1 + 2 * (1 - T[0]) + T[2 + 2 * kidx] + (jf - jmin)];
     }
@@ -299,17 +295,22 @@ __device__ __forceinline__ float pow2i(int k) { return __int_as_float((127 + k) 
 __device__ __forceinline__ int exp_of(float m) {
     return m >= 7.888609052210118e-31f ? ((__float_as_int(m) >> 23) & 0xff) - 126 : kZeroExp;
 }
-// the NSL fixed-point slices of v * scale, scale = 2^(SLB - e)
-__device__ __forceinline__ void slice_scaled(ff v, float scale, float *sl) {
-    const float hi = __fmul_rn(v.hi, scale), lo = __fmul_rn(v.lo, scale);
-    sl[0] = rintf(hi);
-    float r = __fadd_rn(__fsub_rn(hi, sl[0]), lo);
+// the NSL fixed-point slices of two values v * scale, scale = 2^(SLB - e)
+__device__ __forceinline__ void slice_scaled2(ff2 v, float2 scale, float2 *sl) {
+    const float2 hi = f2_mul(v.hi, scale), lo = f2_mul(v.lo, scale);
+    sl[0] = f2_rint(hi);
+    float2 r = f2_add(f2_sub(hi, sl[0]), lo);
 #pragma unroll
     for (int i = 1; i < NSL; i++) {
-        r = __fmul_rn(r, 1024.0f);
-        sl[i] = rintf(r);
-        r = __fsub_rn(r, sl[i]);
+        r = f2_mul(r, f2(1024.0f));
+        sl[i] = f2_rint(r);
+        r = f2_sub(r, sl[i]);
     }
+}
+// two slices (integers of at most 2^SLB) as packed halves
+__device__ __forceinline__ uint32_t pack_halves(float2 s) {
+    const __half2 h2 = __floats2half2_rn(s.x, s.y);
+    return *reinterpret_cast<const uint32_t *>(&h2);
 }
 
 struct MixedArgs {
@@ -351,7 +352,7 @@ struct alignas(16) PairHdr {
 struct TileCommon {
     ItemImg ii[2];  // the image of the current item and of the one being fetched
     ff Y[kNPow][kMaxTY + 1];  // rows padded: lanes reading different rows hit different banks
-    ff Z[kNPow][kMaxTZ + 1];
+    alignas(8) float Zh[kNPow][kMaxTZ], Zl[kNPow][kMaxTZ];
     int tile;
     uint64_t mbar;
     uint32_t tmem;
@@ -359,17 +360,26 @@ struct TileCommon {
     int kmax;  // collocate: K slots of A written by the previous pair (zeroed up to here)
 };
 
+// Cxy rows b (L - b values of a) padded to an even length: start of row b
+__host__ __device__ constexpr int cxy_pad_row(int L, int b) {
+    int q = 0;
+    for (int i = 0; i < b; i++) q += (L - i + 1) & ~1;
+    return q;
+}
+constexpr int kNPair = (kNPow + 1) / 2;                     // pairs of a
+constexpr int kCxyRow = cxy_pad_row(kNPow, kNPow) / 2;      // 16-byte entries of one z
+
 struct alignas(128) SmemColl {
     __half A[NSL][MROWS * KP];  // Cx slices, M=128 x K=16
     __half B[NSL][TX * KP];     // X slices, N=32 x K=16
     ff rc[NCOEF_MAX];           // coefficients re-expanded around the tile's column ic
-    ff Cxy[kMaxTZColl][NPAIR_MAX];  // stage 1 output
-    ff cxy_pad_[4];             // stage-2 reads up to 3 entries past a row
+    float4 Cxy[kMaxTZColl][kCxyRow];  // stage 1 output, pairs of a: {hi, hi, lo, lo}
     PairBuf pb[2];              // the current pair and the one being fetched
-    float acc_lo[MROWS][TX + 1];  // low parts of the tile sums (row m belongs to thread m; padded rows)
+    alignas(16) float acc_lo[MROWS][TX + 4];  // low parts of the tile sums (row m belongs to thread m; padded rows)
     float bin[kNPow][kNPow];    // binomials C(a', a) of the re-expansion
     alignas(16) float cs[TX];   // 2^fx per column (0 for an empty column)
     unsigned char qb[kNPow][NPAIR_MAX + 2];  // qb[L-1][pair_index(L, b, a)] = b
+    unsigned char qpad[kNPow][2 * kCxyRow];  // qpad[L-1][padded index of (b, a)] = b | a << 4
     int zs[kNPow + 1];          // zs[g]: packed index of (g, 0, 0) for the current pair's lp
     TileCommon c;
 };
@@ -537,45 +547,36 @@ __device__ __forceinline__ TabEntry tab_entry(const TPair &p, const ImgState &q,
 }
 // warp 1: one y or z entry into shared memory
 __device__ __forceinline__ void yz_fill(TileCommon &sm, const TPair &p, const TabEntry &te) {
-    ff *col = te.d == 1 ? &sm.Y[0][te.i] : &sm.Z[0][te.i];
-    const int stride = te.d == 1 ? kMaxTY + 1 : kMaxTZ + 1;
+    // Y as float-float entries, Z as separate high and low parts (read in pairs of z)
+    float *hi = te.d == 1 ? &sm.Y[0][te.i].hi : &sm.Zh[0][te.i], *lo = te.d == 1 ? hi + 1 : &sm.Zl[0][te.i];
+    const int stride = te.d == 1 ? 2 * (kMaxTY + 1) : kMaxTZ;
     const int L = te.in ? p.L : 0;
     ff e = te.e;
 #pragma unroll 1
     for (int k = 0; k < L; k++) {
-        col[k * stride] = e;
+        hi[k * stride] = e.hi;
+        lo[k * stride] = e.lo;
         e = ff_mul(e, te.t);
     }
 #pragma unroll 1
-    for (int k = L; k < kNPow; k++) col[k * stride] = ff{0.0f, 0.0f};
+    for (int k = L; k < kNPow; k++) hi[k * stride] = lo[k * stride] = 0.0f;
 }
-// warp 0: the x column of entry x in registers, xv[k] for k < kNPow
+// warp 0: the x column of entry x in registers, xv[i] the powers 2 i and 2 i + 1: of u
+// (collocate: recentre) or of t (integrate); each step multiplies a pair by u^2.
 __device__ __forceinline__ void x_powers(const TPair &p, const ImgState &q, const TabEntry &te, int x, bool recentre,
-                                         ff *xv) {
+                                         ff2 *xv) {
 #pragma unroll
-    for (int k = 0; k < kNPow; k++) xv[k] = ff{0.0f, 0.0f};
+    for (int i = 0; i < kNPair; i++) xv[i] = ff2{f2(0.0f), f2(0.0f)};
     if (!te.in) return;
-    if (recentre) {  // collocate: one chain (its code size matters more than this latency)
-        ff e = te.e;
-        const ff u = ff_mul_f(p.h[0], ldexpf((float)(x - q.ic), -q.sb));
+    const ff u = recentre ? ff_mul_f(p.h[0], ldexpf((float)(x - q.ic), -q.sb)) : te.t;
+    const ff2 u2 = ff2_dup(ff_mul(u, u));
+    ff2 e = ff2_pair(te.e, ff_mul(te.e, u));
 #pragma unroll
-        for (int k = 0; k < kNPow; k++) {
-            if (k >= p.L) break;
-            xv[k] = e;
-            e = ff_mul(e, u);
-        }
-        return;
-    }
-    // integrate: even and odd powers of t as two independent chains in t^2
-    const ff u2 = ff_mul(te.t, te.t);
-    ff e0 = te.e, e1 = ff_mul(te.e, te.t);
-#pragma unroll
-    for (int k = 0; k < kNPow; k += 2) {
-        if (k >= p.L) break;
-        xv[k] = e0;
-        if (k + 1 < kNPow && k + 1 < p.L) xv[k + 1] = e1;
-        e0 = ff_mul(e0, u2);
-        e1 = ff_mul(e1, u2);
+    for (int i = 0; i < kNPair; i++) {
+        if (2 * i >= p.L) break;
+        xv[i] = e;
+        if (2 * i + 1 >= p.L) xv[i].hi.y = xv[i].lo.y = 0.0f;
+        e = ff2_mul(e, u2);
     }
 }
 
@@ -599,8 +600,9 @@ __constant__ float c_binom[kNPow][kNPow] = {
 // One item (g, b, a) per thread of [t0, t0 + nt): Horner in tc over a' = amax .. a
 // with the binomials from shared memory (bin[a'][a] = C(a', a)).  zs[g] is the
 // packed index of (g, 0, 0) and qb[q][r] the b of row-in-slab r of a slab with
-// q = lp - g, so that decoding t needs no arithmetic series.
-__device__ void recentre_x(const PairBuf &pb, ff tc, ff *out, const float (*bin)[kNPow], const int *zs,
+// q = lp - g, so that decoding t needs no arithmetic series.  The row coefficients'
+// balancing factor 2^(a sb) is applied here, once per coefficient.
+__device__ void recentre_x(const PairBuf &pb, ff tc, int sb, ff *out, const float (*bin)[kNPow], const int *zs,
                            const unsigned char (*qb)[NPAIR_MAX + 2], int t0, int nt) {
     const int lp = pb.p.lp;
     const int nc = ncoef(lp);
@@ -617,7 +619,8 @@ __device__ void recentre_x(const PairBuf &pb, ff tc, ff *out, const float (*bin)
             const float2 c = pb.coef[base + ap];
             s = ff_fma(s, tc, ff_mul_f(ff{c.x, c.y}, bin[ap][a]));
         }
-        out[t] = s;
+        const float bal = pow2i(a * sb);  // balancing of the x powers (exact)
+        out[t] = ff{__fmul_rn(s.hi, bal), __fmul_rn(s.lo, bal)};
     }
 }
 
@@ -637,21 +640,21 @@ __device__ __forceinline__ uint4 chunk_mask(uint32_t b) {
     return m;
 }
 
-// The NSL slices of one K = 16 operand row (v[k] for k < kNPow, zero beyond),
-// scaled by sc, as 16-byte chunks of 8 K values in the UMMA layout (planes of
-// plane_halves halves); K groups at or beyond kw are left as they are, and those
-// at or beyond nval (v[k] == 0 for k >= nval) are written as zeros directly.
-__device__ __forceinline__ void slice_row16(const ff *vin, float sc, int kw, int nval, __half *plane0,
+// The NSL slices of one K = 16 operand row (v[i]: the values 2 i and 2 i + 1, zero
+// beyond kNPow), scaled by sc, as 16-byte chunks of 8 K values in the UMMA layout
+// (planes of plane_halves halves); K groups at or beyond kw are left as they are, and
+// those at or beyond nval (only zeros there) are written as zeros directly.
+__device__ __forceinline__ void slice_row16(const ff2 *vin, float sc, int kw, int nval, __half *plane0,
                                             int plane_halves, int row) {
     // one compact loop body for both K groups: the second group's values are moved down
-    ff v[8];
+    ff2 v[4];
 #pragma unroll
-    for (int k = 0; k < 8; k++) v[k] = vin[k];
+    for (int i = 0; i < 4; i++) v[i] = vin[i];
 #pragma unroll 1
     for (int kg = 0; kg < KP / 8; kg++) {
         if (8 * kg >= kw) break;
+        const int o16 = (row >> 3) * 16 + kg * 8 + (row & 7);  // umma_off(row, 8 kg) / 16
         if (8 * kg >= nval) {  // only zeros left: rewrite the stale slots without slicing
-            const int o16 = (row >> 3) * 16 + kg * 8 + (row & 7);
 #pragma unroll
             for (int q = 0; q < NSL; q++) reinterpret_cast<uint4 *>(plane0 + q * plane_halves)[o16] = make_uint4(0, 0, 0, 0);
             continue;
@@ -659,21 +662,16 @@ __device__ __forceinline__ void slice_row16(const ff *vin, float sc, int kw, int
         uint32_t w[NSL][4];
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            float s0[NSL], s1[NSL];
-            slice_scaled(v[2 * i], sc, s0);
-            slice_scaled(v[2 * i + 1], sc, s1);
+            float2 sl[NSL];
+            slice_scaled2(v[i], f2(sc), sl);
 #pragma unroll
-            for (int q = 0; q < NSL; q++) {
-                const __half2 h2 = __floats2half2_rn(s0[q], s1[q]);
-                w[q][i] = *reinterpret_cast<const uint32_t *>(&h2);
-            }
+            for (int q = 0; q < NSL; q++) w[q][i] = pack_halves(sl[q]);
         }
-        const int o16 = (row >> 3) * 16 + kg * 8 + (row & 7);  // umma_off(row, 8 kg) / 16
 #pragma unroll
         for (int q = 0; q < NSL; q++)
             reinterpret_cast<uint4 *>(plane0 + q * plane_halves)[o16] = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
 #pragma unroll
-        for (int k = 0; k < 8; k++) v[k] = 8 + k < kNPow ? vin[8 + k < kNPow ? 8 + k : 0] : ff{0.0f, 0.0f};
+        for (int i = 0; i < 4; i++) v[i] = 4 + i < kNPair ? vin[4 + i < kNPair ? 4 + i : 0] : ff2{f2(0.0f), f2(0.0f)};
     }
 }
 
@@ -743,14 +741,10 @@ __device__ __forceinline__ void general_a_row(Smem &sm, const GenLevel &G, const
                 v2[h] = in ? ff_mul(sm.Vff[x][r], e) : ff{0.0f, 0.0f};
                 if (in) e = ff_mul(e, q);
             }
-            float s0[NSL], s1[NSL];
-            slice_scaled(v2[0], sc, s0);
-            slice_scaled(v2[1], sc, s1);
+            float2 sl[NSL];
+            slice_scaled2(ff2_pair(v2[0], v2[1]), f2(sc), sl);
 #pragma unroll
-            for (int qq = 0; qq < NSL; qq++) {
-                const __half2 h2 = __floats2half2_rn(s0[qq], s1[qq]);
-                w[qq][i] = *reinterpret_cast<const uint32_t *>(&h2);
-            }
+            for (int qq = 0; qq < NSL; qq++) w[qq][i] = pack_halves(sl[qq]);
         }
         const int o16 = (r >> 3) * 16 + (c & 1) * 8 + (r & 7);
 #pragma unroll
@@ -777,37 +771,43 @@ __device__ __forceinline__ void tc_setup(TileCommon &c, uint32_t ncols) {
 }
 
 __device__ __forceinline__ void tc_teardown(TileCommon &c, uint32_t ncols, uint32_t phase) {
-    if (c.abort) tc::mbar_wait_bounded(&c.mbar, phase, 1u << 22);  // let an MMA in flight finish
+    if (c.abort) tc::mbar_wait_bounded(&c.mbar, phase ^ 1u, 1u << 22);  // let an MMA in flight finish
     cp_async_wait_all();
     tc::fence_before_sync();
     __syncthreads();
     if (threadIdx.x < 32) tc::tmem_dealloc(c.tmem, ncols);
 }
 
-// waits for the MMAs of the current item; false (and abort flagged) on timeout
-__device__ __forceinline__ bool tc_wait(TileCommon &c, uint32_t phase, int *status) {
+// Waits for the MMAs of the current item.  On a timeout the abort flag is set; the
+// thread goes on to the item's last barrier, after which every thread sees the flag
+// and leaves (a barrier here would only carry the flag: each thread waits by itself).
+__device__ __forceinline__ void tc_wait(TileCommon &c, uint32_t phase, int *status) {
     if (!tc::mbar_wait_bounded(&c.mbar, phase, 1u << 24)) {
         atomicOr(status, kStatTimeout);
         c.abort = 1;
     }
-    __syncthreads();
     tc::fence_after_sync();
-    return !c.abort;
 }
 
-// The pair loop of a tile: item it + 1 is copied while item it is processed.
-// Returns the buffer slot of item it once it is visible to all threads.
+// The pair loop of a tile: item it + 1 is copied while item it is processed.  Item
+// it is visible to all threads and every thread is done with the other slot:
+// first_pair and end_item end with a barrier.
 template <class Buf>
 __device__ __forceinline__ int next_pair(TileCommon &cm, Buf *pb, const MixedArgs &A, int64_t it, int64_t it0,
                                          int64_t it1, uint64_t &nxt, bool with_coef) {
     const int cur = (int)((it - it0) & 1);
-    cp_async_wait_all();
-    __syncthreads();  // item it visible; every thread is done with the other slot
     if (it + 1 < it1) {
         fetch_pair(pb[cur ^ 1].hdr_, cm.ii[cur ^ 1], A, it + 1, nxt, with_coef);
         if (it + 2 < it1) nxt = A.items[it + 2];
     }
     return cur;
+}
+// the last barrier of an item: its TMEM columns and shared memory may be reused, the
+// next item's copies are visible
+__device__ __forceinline__ void end_item() {
+    cp_async_wait_all();
+    tc::fence_before_sync();
+    __syncthreads();
 }
 
 template <class Buf>
@@ -815,67 +815,71 @@ __device__ __forceinline__ void first_pair(TileCommon &cm, Buf *pb, const MixedA
                                            uint64_t &nxt, bool with_coef) {
     if (it0 < it1) fetch_pair(pb[0].hdr_, cm.ii[0], A, it0, A.items[it0], with_coef);
     if (it0 + 1 < it1) nxt = A.items[it0 + 1];
+    cp_async_wait_all();
+    __syncthreads();
 }
 
-// Stage 1 of collocate: Cxy[z][(b,a)] = sum_g c'[g][b][a] Z[g][z]; one output per
-// thread (16 consecutive threads share (b, a)), two partial sums over even and
-// odd g; the packed index of (g, b, a) is zs[g] - b g + k0.
+// Stage 1 of collocate: Cxy[z][(b,a)] = sum_g c'[g][b][a] Z[g][z]; one (b, a) and two
+// z per thread (packed float-float), two partial sums over even and odd g; the
+// packed index of (g, b, a) is zs[g] - b g + k0.  Rows b of Cxy are padded to an even
+// number of a (the padding gets zeros), so that stage 2 reads its pairs of a as
+// 16-byte entries {hi(a), hi(a+1), lo(a), lo(a+1)}.
 __device__ __forceinline__ void stage1_cxy(SmemColl &sm, int L, int lp, const TileShape &sh) {
     const TileCommon &cm = sm.c;
-    const int npair = (L * (L + 1)) / 2;
-    const unsigned char *qbL = sm.qb[L - 1];
-    for (int t = threadIdx.x; t < sh.TZ * npair; t += NTHR) {
-        const int zz = t & (sh.TZ - 1), q = t >> sh.lz;
-        const int b = qbL[q];
-        const int a = q - (b * L - (b * (b - 1)) / 2), n = lp - a - b;
-        const int k0 = b * (lp + 1) - (b * (b - 1)) / 2 + a;
-        ff s0 = {0.0f, 0.0f}, s1 = {0.0f, 0.0f};
+    const int npad = 2 * (L >> 1) * ((L >> 1) + 1) + (L & 1) * (L + 1);  // cxy_pad_row(L, L)
+    const unsigned char *qp = sm.qpad[L - 1];
+    for (int t = threadIdx.x; t < (npad << (sh.lz - 1)); t += NTHR) {
+        const int zz = 2 * (t & ((sh.TZ >> 1) - 1)), q = t >> (sh.lz - 1);
+        const int b = qp[q] & 15, a = qp[q] >> 4, n = lp - a - b;
+        const ff *c = sm.rc + (b * (lp + 1) - (b * (b - 1)) / 2 + a);
+        ff2 s0 = {f2(0.0f), f2(0.0f)}, s1 = s0;
+        auto zpair = [&](int g) {
+            return ff2{*reinterpret_cast<const float2 *>(&cm.Zh[g][zz]), *reinterpret_cast<const float2 *>(&cm.Zl[g][zz])};
+        };
         int g = 0, bg = 0;
 #pragma unroll 1
         for (; g + 1 <= n; g += 2, bg += 2 * b) {
-            s0 = ff_fma(sm.rc[sm.zs[g] - bg + k0], cm.Z[g][zz], s0);
-            s1 = ff_fma(sm.rc[sm.zs[g + 1] - bg - b + k0], cm.Z[g + 1][zz], s1);
+            s0 = ff2_fma(zpair(g), ff2_dup(c[sm.zs[g] - bg]), s0);
+            s1 = ff2_fma(zpair(g + 1), ff2_dup(c[sm.zs[g + 1] - bg - b]), s1);
         }
-        if (g <= n) s0 = ff_fma(sm.rc[sm.zs[g] - bg + k0], cm.Z[g][zz], s0);
-        sm.Cxy[zz][q] = ff_add(s0, s1);
+        if (g <= n) s0 = ff2_fma(zpair(g), ff2_dup(c[sm.zs[g] - bg]), s0);
+        s0 = ff2_add(s0, s1);
+        float *o = reinterpret_cast<float *>(&sm.Cxy[zz][q >> 1]) + (q & 1);
+        o[0] = s0.hi.x;
+        o[2] = s0.lo.x;
+        o += 4 * kCxyRow;
+        o[0] = s0.hi.y;
+        o[2] = s0.lo.y;
     }
 }
 
-// Stage 2 of collocate for this thread's row (z, y), all a at once, then the
-// row's A slices (K slots below kw rewritten); returns the row exponent.  a in
-// pairs (a0, a0 + 1; unrolled, uniform exit at lp), b inner (runtime bound
-// lp - a0): only the products that exist, two independent float-float sums, each
-// renormalised once at the end.
-__device__ __forceinline__ int stage2_row(SmemColl &sm, const TileCommon &cm, int L, int lp, int sb, int z, int y,
-                                          bool live, int kw, int m) {
-    ff cx[kNPow];
+// Stage 2 of collocate for this thread's row (z, y): Cx[a] = sum_b Cxy[z][b][a] Y[b][y],
+// two a per instruction, then the row's A slices (K slots below kw rewritten);
+// returns the row exponent.  b outer, the pairs of a unrolled inside (uniform exit at
+// the row's end), so that Y is read once per b; each sum renormalised once at the end.
+__device__ __forceinline__ int stage2_row(SmemColl &sm, const TileCommon &cm, int L, int lp, int z, int y, bool live,
+                                          int kw, int m) {
+    ff2 cx[kNPair];
 #pragma unroll
-    for (int a = 0; a < kNPow; a++) cx[a] = ff{0.0f, 0.0f};
+    for (int i = 0; i < kNPair; i++) cx[i] = ff2{f2(0.0f), f2(0.0f)};
     float mx = 0.0f;
     if (live) {
-        const ff *crow = sm.Cxy[z];
-#pragma unroll
-        for (int a0 = 0; a0 < kNPow; a0 += 2) {
-            if (a0 > lp) break;
-            ff s0 = {0.0f, 0.0f}, s1 = {0.0f, 0.0f};
-            const int nb = lp - a0;
-            int q = a0;  // pair_index(L, b, a0); (b, a0 + 1) is q + 1
+        const float4 *crow = sm.Cxy[z];
 #pragma unroll 1
-            for (int b = 0; b <= nb; b++) {
-                const ff yb = cm.Y[b][y];
-                ff_acc_lazy(s0, crow[q], yb);
-                if (b < nb) ff_acc_lazy(s1, crow[q + 1], yb);  // a0 + 1 + b <= lp
-                q += L - b;
+        for (int b = 0; b <= lp; b++) {
+            const ff2 yb = ff2_dup(cm.Y[b][y]);
+#pragma unroll
+            for (int i = 0; i < kNPair; i++) {
+                if (2 * i > lp - b) break;
+                const float4 c = crow[i];
+                ff2_acc_lazy(cx[i], ff2{make_float2(c.x, c.y), make_float2(c.z, c.w)}, yb);
             }
-            cx[a0] = fast_two_sum(s0.hi, s0.lo);
-            if (a0 + 1 < kNPow) cx[a0 + 1] = fast_two_sum(s1.hi, s1.lo);
+            crow += (L - b + 1) >> 1;
         }
 #pragma unroll
-        for (int a = 0; a < kNPow; a++) {
-            const float bal = pow2i(a * sb);  // balancing of the x powers (exact)
-            cx[a].hi = __fmul_rn(cx[a].hi, bal);
-            cx[a].lo = __fmul_rn(cx[a].lo, bal);
-            mx = fmaxf(mx, fabsf(cx[a].hi));  // entries a > lp are zero
+        for (int i = 0; i < kNPair; i++) {
+            cx[i] = fast_two_sum2(cx[i].hi, cx[i].lo);
+            mx = fmaxf(mx, fmaxf(fabsf(cx[i].hi.x), fabsf(cx[i].hi.y)));  // entries a > lp are zero
         }
     }
     const int em = exp_of(mx);
@@ -914,6 +918,12 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
         while (b < Lq && r >= Lq - b) r -= Lq - b++;
         sm.qb[Lq - 1][q] = (unsigned char)min(b, kNPow - 1);
     }
+    for (int t = tid; t < kNPow * 2 * kCxyRow; t += NTHR) {
+        const int Lq = t / (2 * kCxyRow) + 1, q = t % (2 * kCxyRow);
+        int b = 0, r = q;
+        while (b < Lq && r >= ((Lq - b + 1) & ~1)) r -= (Lq - b++ + 1) & ~1;
+        sm.qpad[Lq - 1][q] = (unsigned char)(min(b, kNPow - 1) | (r & 15) << 4);
+    }
     for (;;) {
         if (tid == 0) cm.tile = atomicAdd(A.queue, 1);
         __syncthreads();
@@ -928,10 +938,12 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
             if (tid == 0) atomicOr(A.status, kStatBadTile);
             continue;
         }
-        float acc_hi[TX];  // the low parts live in shared memory (registers for 4 CTAs per SM)
+        float2 acc_hi[TX / 2];  // pairs of x; the low parts live in shared memory (registers for 4 CTAs per SM)
         float *acc_lo = sm.acc_lo[m];
 #pragma unroll
-        for (int x = 0; x < TX; x++) acc_hi[x] = acc_lo[x] = 0.0f;
+        for (int x = 0; x < TX; x++) acc_lo[x] = 0.0f;
+#pragma unroll
+        for (int x = 0; x < TX / 2; x++) acc_hi[x] = f2(0.0f);
         const TileExt ext = {min(TX, lv.ngrid[0] - td.t[0] * TX), min(TY, lv.ngrid[1] - td.t[1] * TY),
                              min(TZ, lv.ngrid[2] - td.t[2] * TZ)};
         const bool row_ok = z < ext.z && y < ext.y;
@@ -952,11 +964,12 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                     for (int ent = tid & 31; ent < (warp == 0 ? TX : TY + TZ); ent += 32) {
                         const TabEntry te = tab_entry(P, Q, ext, sh, warp, ent);
                         if (warp == 0) {
-                            ff xv[kNPow];
+                            ff2 xv[kNPair];
                             x_powers(P, Q, te, ent, true, xv);
                             float mx = 0.0f;
 #pragma unroll
-                            for (int k = 0; k < kNPow; k++) mx = fmaxf(mx, fabsf(xv[k].hi));
+                            for (int i = 0; i < kNPair; i++)
+                                mx = fmaxf(mx, fmaxf(fabsf(xv[i].hi.x), fabsf(xv[i].hi.y)));
                             const int e = exp_of(mx);
                             sm.cs[tid] = e == kZeroExp ? 0.0f : pow2i(e);
                             const float sc = e == kZeroExp ? 0.0f : pow2i(SLB - e);
@@ -970,7 +983,7 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                     // slab starts zs[g] = packed index of (g, 0, 0), then the re-expansion
                     if (tid - 64 <= kNPow) sm.zs[tid - 64] = tid - 64 <= lp + 1 ? row_start(lp, tid - 64, 0) : 0;
                     asm volatile("bar.sync 2, 64;" ::: "memory");
-                    recentre_x(pb, Q.tc, sm.rc, sm.bin, sm.zs, sm.qb, 64, NTHR - 64);
+                    recentre_x(pb, Q.tc, Q.sb, sm.rc, sm.bin, sm.zs, sm.qb, 64, NTHR - 64);
                 }
                 __syncthreads();
                 stage1_cxy(sm, L, lp, sh);
@@ -982,7 +995,7 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                                       x1);
                 else
                     row_range(P, Q, A.table, Q.o[2] + z, Q.o[1] + y, row_ok, x0, x1);
-                const int em = stage2_row(sm, cm, L, lp, Q.sb, z, y, x0 <= x1, max(L, cm.kmax), m);
+                const int em = stage2_row(sm, cm, L, lp, z, y, x0 <= x1, max(L, cm.kmax), m);
                 // stage 3 on the tensor cores: D_s = sum_{i+j=s} A_i B_j^T
                 tc::fence_async_smem();
                 tc::fence_before_sync();
@@ -1002,9 +1015,8 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                         for (int i = 0; i <= sd; i++) tc::mma_f16(cm.tmem + 32 * sd, ad[i], bd[sd - i], idesc, i > 0);
                     tc::mma_commit(&cm.mbar);
                 }
-                const bool ok = tc_wait(cm, phase, A.status);
+                tc_wait(cm, phase, A.status);
                 phase ^= 1u;
-                if (!ok) break;
                 if (tid == 0) cm.kmax = L;  // read again only after the next barrier
                 // cross factor of the general cell along this row: E0 at x0, ratio q
                 ff ecur = {1.0f, 0.0f}, eq = {1.0f, 0.0f};
@@ -1033,58 +1045,67 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                                 uint32_t r2[8], r3[8], r4[8], r5[8];
                                 const float4 csa = reinterpret_cast<const float4 *>(sm.cs)[2 * c];
                                 const float4 csb = reinterpret_cast<const float4 *>(sm.cs)[2 * c + 1];
-                                const float csv[8] = {csa.x, csa.y, csa.z, csa.w, csb.x, csb.y, csb.z, csb.w};
+                                const float2 csv[4] = {{csa.x, csa.y}, {csa.z, csa.w}, {csb.x, csb.y}, {csb.z, csb.w}};
                                 tc::tmem_ld8(tbase + 8 * c, r2);
                                 tc::tmem_ld8(tbase + 32 + 8 * c, r3);
                                 tc::tmem_ld8(tbase + 64 + 8 * c, r4);
                                 tc::tmem_ld8(tbase + 96 + 8 * c, r5);
+                                float4 *const lop = reinterpret_cast<float4 *>(acc_lo) + 2 * c;
+                                const float4 loa = lop[0], lob = lop[1];
+                                float2 lov[4] = {{loa.x, loa.y}, {loa.z, loa.w}, {lob.x, lob.y}, {lob.z, lob.w}};
                                 tc::tmem_wait_ld32(r2, r3, r4, r5);
 #pragma unroll
-                                for (int i = 0; i < 8; i++) {
-                                    const int x = 8 * c + i;
-                                    const bool in = (mc >> i) & 1u;  // straight-line code: selects, no branches
+                                for (int i = 0; i < 4; i++) {  // two x per instruction, selects instead of branches
+                                    const bool in0 = (mc >> (2 * i)) & 1u, in1 = (mc >> (2 * i + 1)) & 1u;
+                                    auto two = [&](const uint32_t *r) {
+                                        return make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+                                    };
                                     // value = scl * (D2 + D3 2^-10 + D4 2^-20 + D5 2^-30) as hi + lo with
                                     // lo the exact remainder (fast two-sum), then an exact two-sum into
                                     // acc_hi: acc_lo then only gathers rounding errors and remainders,
                                     // so it stays ~2^-24 below acc_hi however many pairs a point sees
-                                    const float d2 = __uint_as_float(r2[i]);
-                                    const float corr = __fmaf_rn(__uint_as_float(r5[i]), 9.313225746154785e-10f,
-                                                       __fmaf_rn(__uint_as_float(r4[i]), 9.5367431640625e-07f,
-                                                                 __fmul_rn(__uint_as_float(r3[i]), 0.0009765625f)));
-                                    float scl = __fmul_rn(rs, csv[i]);
-                                    const float h0 = __fadd_rn(d2, corr);
-                                    float hi = __fmul_rn(h0, scl);
-                                    float rem = __fsub_rn(corr, __fsub_rn(h0, d2));  // lo = rem scl exactly
+                                    const float2 d2 = two(r2);
+                                    const float2 corr =
+                                        f2_fma(two(r5), f2(9.313225746154785e-10f),
+                                               f2_fma(two(r4), f2(9.5367431640625e-07f), f2_mul(two(r3), f2(0.0009765625f))));
+                                    float2 scl = f2_mul(f2(rs), csv[i]);
+                                    const float2 h0 = f2_add(d2, corr);
+                                    float2 hi = f2_mul(h0, scl);
+                                    float2 rem = f2_sub(corr, f2_sub(h0, d2));  // lo = rem scl exactly
                                     if constexpr (kGeneral) {
+                                        const int x = 8 * c + 2 * i;
                                         if (x > x0) ecur = ff_mul(ecur, eq);  // E(x) on the row's cube points
-                                        const ff v = ff_mul(ff{hi, __fmul_rn(rem, scl)}, ecur);
-                                        hi = v.hi;
-                                        rem = v.lo;
-                                        scl = 1.0f;
+                                        const ff v = ff_mul(ff{hi.x, __fmul_rn(rem.x, scl.x)}, ecur);
+                                        if (x + 1 > x0) ecur = ff_mul(ecur, eq);
+                                        const ff w = ff_mul(ff{hi.y, __fmul_rn(rem.y, scl.y)}, ecur);
+                                        hi = make_float2(v.hi, w.hi);
+                                        rem = make_float2(v.lo, w.lo);
+                                        scl = f2(1.0f);
                                     }
-                                    float &ah = acc_hi[8 * hh + i];
-                                    const float sv = __fadd_rn(ah, hi);
-                                    const float bb = __fsub_rn(sv, ah);
-                                    const float err = __fadd_rn(__fsub_rn(ah, __fsub_rn(sv, bb)), __fsub_rn(hi, bb));
-                                    if (in) acc_lo[x] = __fadd_rn(acc_lo[x], __fmaf_rn(rem, scl, err));
-                                    ah = in ? sv : ah;
+                                    float2 &ah = acc_hi[4 * hh + i];
+                                    const float2 sv = f2_add(ah, hi);
+                                    const float2 bb = f2_sub(sv, ah);
+                                    const float2 err = f2_add(f2_sub(ah, f2_sub(sv, bb)), f2_sub(hi, bb));
+                                    const float2 lo = f2_add(lov[i], f2_fma(rem, scl, err));
+                                    ah = make_float2(in0 ? sv.x : ah.x, in1 ? sv.y : ah.y);
+                                    lov[i] = make_float2(in0 ? lo.x : lov[i].x, in1 ? lo.y : lov[i].y);
                                 }
+                                lop[0] = make_float4(lov[0].x, lov[0].y, lov[1].x, lov[1].y);
+                                lop[1] = make_float4(lov[2].x, lov[2].y, lov[3].x, lov[3].y);
                             }
                         }
-                        float tr[8 * kCh];
+                        float2 tr[4 * kCh];
 #pragma unroll
-                        for (int i = 0; i < 8 * kCh; i++) tr[i] = acc_hi[i];
+                        for (int i = 0; i < 4 * kCh; i++) tr[i] = acc_hi[i];
 #pragma unroll
-                        for (int i = 0; i < TX - 8 * kCh; i++) acc_hi[i] = acc_hi[i + 8 * kCh];
+                        for (int i = 0; i < TX / 2 - 4 * kCh; i++) acc_hi[i] = acc_hi[i + 4 * kCh];
 #pragma unroll
-                        for (int i = 0; i < 8 * kCh; i++) acc_hi[TX - 8 * kCh + i] = tr[i];
+                        for (int i = 0; i < 4 * kCh; i++) acc_hi[TX / 2 - 4 * kCh + i] = tr[i];
                     }
                 }
-                tc::fence_before_sync();
-                __syncthreads();
+                end_item();
             }
         }
-        cp_async_wait_all();
         if (cm.abort) break;
         // flush: grid += tile sum (FP64)
         if (row_ok) {
@@ -1098,12 +1119,12 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                 for (int i = 0; i < 8; i++) {
                     const int x = 8 * c + i;
                     if (x >= ext.x) continue;
-                    const double v = (double)acc_hi[i] + (double)acc_lo[x];
+                    const double v = (double)(i & 1 ? acc_hi[i / 2].y : acc_hi[i / 2].x) + (double)acc_lo[x];
                     if (td.flags & kUnitSplit) atomicAdd(grid + row + x, v);  // other work units add to the same tile
                     else grid[row + x] += v;
                 }
 #pragma unroll
-                for (int i = 0; i < TX - 8; i++) acc_hi[i] = acc_hi[i + 8];
+                for (int i = 0; i < TX / 2 - 4; i++) acc_hi[i] = acc_hi[i + 4];
             }
         }
         __syncthreads();
@@ -1174,14 +1195,10 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                     const int x = 8 * c + 2 * i;
                     const ff v0 = (ok && x < ext.x) ? ff_from_double(grid[row + x]) : ff{0.0f, 0.0f};
                     const ff v1 = (ok && x + 1 < ext.x) ? ff_from_double(grid[row + x + 1]) : ff{0.0f, 0.0f};
-                    float s0[NSL], s1[NSL];
-                    slice_scaled(v0, sc, s0);
-                    slice_scaled(v1, sc, s1);
+                    float2 sl[NSL];
+                    slice_scaled2(ff2_pair(v0, v1), f2(sc), sl);
 #pragma unroll
-                    for (int q = 0; q < NSL; q++) {
-                        const __half2 h2 = __floats2half2_rn(s0[q], s1[q]);
-                        w[q][i] = *reinterpret_cast<const uint32_t *>(&h2);
-                    }
+                    for (int q = 0; q < NSL; q++) w[q][i] = pack_halves(sl[q]);
                 }
                 const int o16 = (m >> 3) * 16 + (c & 1) * 8 + (m & 7);  // umma_off / 16
 #pragma unroll
@@ -1220,24 +1237,32 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                     // are left as they are (their output columns are not read).  Unlike
                     // collocate, integrate is not limited by instruction fetch: warps 0 and 1
                     // keep separate table code.
-                    ff xv[kNPow];
+                    ff2 xv[kNPair];
                     x_powers(P, Q, tab_entry(P, Q, ext, sh, 0, tid), tid, false, xv);
 #pragma unroll
-                    for (int a = 0; a < kNPow; a++) {
+                    for (int a = 0; a < kNPow; a += 2) {  // in pairs; xv[a] = 0 for a >= L
                         if (a >= L) break;
                         // per-alpha maximum over x: one warp reduction (the bit patterns of
                         // non-negative floats order as their values)
-                        const float mxb =
-                            __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(xv[a].hi))));
-                        const int e = exp_of(mxb);
-                        if (tid == a) sm.gexp[a] = e;
-                        const float sc = e == kZeroExp ? 0.0f : pow2i(SLB - e);
-                        float sl[NSL];
-                        slice_scaled(xv[a], sc, sl);
+                        float sc[2];
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            const float mxb =
+                                __uint_as_float(__reduce_max_sync(
+                                    0xffffffffu, __float_as_uint(fabsf(h ? xv[a / 2].hi.y : xv[a / 2].hi.x))));
+                            const int e = exp_of(mxb);
+                            if (tid == a + h) sm.gexp[a + h] = e;
+                            sc[h] = e == kZeroExp ? 0.0f : pow2i(SLB - e);
+                        }
+                        float2 sl[NSL];
+                        slice_scaled2(xv[a / 2], make_float2(sc[0], sc[1]), sl);
                         unsigned char *const bp = sm.B + (tid >> 4) * kBHalf + b_off(a, tid & 15);
 #pragma unroll
-                        for (int q = 0; q < NSL; q++)
-                            *reinterpret_cast<__half *>(bp + q * kBPlane) = __float2half_rn(sl[q]);
+                        for (int q = 0; q < NSL; q++) {
+                            const uint32_t w = pack_halves(sl[q]);
+                            *reinterpret_cast<uint16_t *>(bp + q * kBPlane) = (uint16_t)w;
+                            *reinterpret_cast<uint16_t *>(bp + q * kBPlane + 16) = (uint16_t)(w >> 16);
+                        }
                     }
                 } else if (warp == 1) {
                     if constexpr (!kGeneral) bar_arrive1(NTHR);
@@ -1308,9 +1333,8 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                     }
                     tc::mma_commit(&cm.mbar);
                 }
-                const bool ok = tc_wait(cm, phase, A.status);
+                tc_wait(cm, phase, A.status);
                 phase ^= 1u;
-                if (!ok) break;
                 const bool live = sm.rx0[m] <= sm.rx1[m];
                 ff *const srow = sm.st.S + s_index(m, sh.ly);
 #pragma unroll 1
@@ -1378,8 +1402,8 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                     const int pi = pair_index(L, b, a);
 #pragma unroll 2
                     for (int zz = 0; zz < TZ; zz += 2) {
-                        ff_acc_lazy(s0, sm.st.T[zz][pi], cm.Z[g][zz]);
-                        ff_acc_lazy(s1, sm.st.T[zz + 1][pi], cm.Z[g][zz + 1]);
+                        ff_acc_lazy(s0, sm.st.T[zz][pi], ff{cm.Zh[g][zz], cm.Zl[g][zz]});
+                        ff_acc_lazy(s1, sm.st.T[zz + 1][pi], ff{cm.Zh[g][zz + 1], cm.Zl[g][zz + 1]});
                     }
                     const ff s = ff_add(s0, s1);
                     if (s.hi != 0.0f) {
@@ -1393,10 +1417,9 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                         atomicAdd(A.mom + moff + t, val);
                     }
                 }
-                __syncthreads();
+                end_item();
             }
         }
-        cp_async_wait_all();
         if (cm.abort) break;
     }
     tc_teardown(cm, kCols, phase);
