@@ -119,24 +119,29 @@ __device__ __forceinline__ ff2 ff2_add(ff2 a, ff2 b) {
     const ff2 s = two_sum2(a.hi, b.hi);
     return fast_two_sum2(s.hi, f2_add(s.lo, f2_add(a.lo, b.lo)));
 }
-// the leading product and its error terms: a b = p - n, n formed with the sign
-// turned (one negated operand, which stays in registers where b is reused)
-__device__ __forceinline__ ff2 ff2_prodn(ff2 a, ff2 b) {
-    const float2 p = f2_mul(a.hi, b.hi), n = f2_neg(b.hi);
-    float2 e = f2_fma(a.hi, n, p);
-    e = f2_fma(a.hi, f2_neg(b.lo), e);
-    e = f2_fma(a.lo, n, e);
-    return {p, e};
+// A factor with its negatives at hand: the product's error needs a b and -(a b), and a
+// table that many products read keeps both signs instead of turning one each time.
+struct ff2n {
+    float2 hi, nhi, nlo;  // b.hi, -b.hi, -b.lo
+};
+__device__ __forceinline__ ff2n ff2n_dup(ff a) { return {f2(a.hi), f2(-a.hi), f2(-a.lo)}; }
+// the leading product and its error terms: a b = p - n
+__device__ __forceinline__ ff2 ff2_prodn(ff2 a, ff2n b) {
+    const float2 p = f2_mul(a.hi, b.hi);
+    float2 n = f2_fma(a.hi, b.nhi, p);
+    n = f2_fma(a.hi, b.nlo, n);
+    n = f2_fma(a.lo, b.nhi, n);
+    return {p, n};
 }
-__device__ __forceinline__ ff2 ff2_mul(ff2 a, ff2 b) {
+__device__ __forceinline__ ff2 ff2_mul(ff2 a, ff2n b) {
     const ff2 q = ff2_prodn(a, b);
     return fast_two_sum2(q.hi, f2_neg(q.lo));
 }
-__device__ __forceinline__ ff2 ff2_fma(ff2 a, ff2 b, ff2 c) {
+__device__ __forceinline__ ff2 ff2_fma(ff2 a, ff2n b, ff2 c) {
     const ff2 q = ff2_prodn(a, b), s = two_sum2(q.hi, c.hi);
     return fast_two_sum2(s.hi, f2_add(s.lo, f2_sub(c.lo, q.lo)));
 }
-__device__ __forceinline__ void ff2_acc_lazy(ff2 &s, ff2 a, ff2 b) {
+__device__ __forceinline__ void ff2_acc_lazy(ff2 &s, ff2 a, ff2n b) {
     const ff2 q = ff2_prodn(a, b), t = two_sum2(s.hi, q.hi);
     s.hi = t.hi;
     s.lo = f2_add(s.lo, f2_sub(t.lo, q.lo));

@@ -351,8 +351,8 @@ struct alignas(16) PairHdr {
 // shared state of both tiled kernels
 struct TileCommon {
     ItemImg ii[2];  // the image of the current item and of the one being fetched
-    ff Y[kNPow][kMaxTY + 1];  // rows padded: lanes reading different rows hit different banks
-    alignas(8) float Zh[kNPow][kMaxTZ], Zl[kNPow][kMaxTZ];
+    // the z table for packed products of two or four z: high parts, and both parts negated
+    alignas(16) float Zh[kNPow][kMaxTZ], Znh[kNPow][kMaxTZ], Znl[kNPow][kMaxTZ];
     int tile;
     uint64_t mbar;
     uint32_t tmem;
@@ -375,6 +375,7 @@ struct alignas(128) SmemColl {
     ff rc[NCOEF_MAX];           // coefficients re-expanded around the tile's column ic
     float4 Cxy[kMaxTZColl][kCxyRow];  // stage 1 output, pairs of a: {hi, hi, lo, lo}
     PairBuf pb[2];              // the current pair and the one being fetched
+    ff Y[kNPow][kMaxTY + 1];  // rows padded: lanes reading different rows hit different banks
     alignas(16) float acc_lo[MROWS][TX + 4];  // low parts of the tile sums (row m belongs to thread m; padded rows)
     float bin[kNPow][kNPow];    // binomials C(a', a) of the re-expansion
     alignas(16) float cs[TX];   // 2^fx per column (0 for an empty column)
@@ -386,29 +387,25 @@ struct alignas(128) SmemColl {
 
 static_assert(4 * (sizeof(SmemColl) + 1024) <= 228 * 1024, "4 collocate CTAs per SM");
 
-// The V slices of the tile an orthorhombic integrate CTA works on (the A
-// operand's layout, both K halves, all slices): 32 KB in a per-CTA global slot
-// that stays in L1/L2 while the tile's items are processed.  Kept out of shared
-// memory, they leave room for 4 CTAs per SM.  General cells keep V as
-// float-float in shared memory (the rows are rescaled per image).
+// The V slices of the tile an orthorhombic integrate CTA works on stand in its A
+// operand; each pair zeroes what lies outside its rows' ranges, and restores it
+// afterwards from a copy of the slices (the A operand's layout, both K halves) in a
+// 32 KB per-CTA global slot that stays in L2.  General cells keep V as float-float in
+// shared memory (the rows are rescaled per image) and build A anew each time, so their
+// S and T may lie in A once the MMAs have read it.
 constexpr int kVSlot16 = 2 * NSL * MROWS * KP / 8;
-template <bool kGeneral>
-struct IntVTile {};
-template <>
-struct IntVTile<true> {
-    ff Vff[TX][MROWS];  // general cell: this tile's V (x-major: lanes read consecutive rows)
-};
 
-// Integrate's S[(z,y)][alpha] rows hold KP + 1 values (row stores by thread
-// (z,y) spread over the banks), and the block of rows of z starts 8 ceil(z/2)
-// values later still: the rows of z = 2w and 2w + 1, which the lanes of stage 2T
-// read side by side at the same alpha (16 x 34 words apart, one bank otherwise),
-// then lie 16 banks apart, and no block runs into the next.  T rows hold NPAIR_T
-// values (2 NPAIR_T = 16 mod 32 words) for the same reason.
-constexpr int kSRow = KP + 1;
-constexpr int NPAIR_T = NPAIR_MAX + (24 - NPAIR_MAX % 16) % 16;
-static_assert((2 * NPAIR_T) % 32 == 16, "T rows of adjacent z 16 banks apart");
-__device__ __forceinline__ int s_index(int row, int ly) { return row * kSRow + 8 * (((row >> ly) + 1) >> 1); }
+// Integrate's tables and sums for packed products of four y or z (16-byte loads):
+// Y[b][y] in three planes; S[alpha][(z,y)] and T[(b,a)][z] in two, rows of S padded so
+// that the lanes' different alpha fall into different banks.
+constexpr int kYRow = kMaxTY + 4;
+constexpr int kSRow = MROWS + 4;
+struct IntSums {
+    alignas(16) float Sh[kNPow][kSRow], Sl[kNPow][kSRow];
+};
+struct IntTsum {
+    alignas(16) float Th[NPAIR_MAX][kMaxTZ], Tl[NPAIR_MAX][kMaxTZ];
+};
 
 // Integrate's B operand (N = 16 alpha x K = 16 x per half, per slice): core
 // matrices 160 bytes apart along K and 288 along N, the second K half 64 bytes
@@ -422,26 +419,48 @@ __host__ __device__ constexpr int b_off(int row, int k) {    // bytes within a p
     return (row >> 3) * kBSbo + (k >> 3) * kBLbo + (row & 7) * 16 + (k & 7) * 2;
 }
 static_assert(b_off(15, 15) + 2 <= kBPlane && kBPlane % 16 == 0 && kBHalf % 16 == 0, "B planes");
+static_assert(kBPlane == 2 * kBSbo, "the planes follow one another along N");
 
-template <bool kGeneral>
-struct alignas(128) SmemInt : IntVTile<kGeneral> {
-    union {
-        __half A[2][NSL][MROWS * KP];  // masked V slices, K halves x in [0,16) and [16,32)
-        struct {                       // after the MMAs have read A:
-            ff S[MROWS * kSRow + 8 * (kMaxTZ / 2)];  //   S[(z,y)][alpha] at s_index((z,y)) + alpha
-            ff T[kMaxTZ][NPAIR_T];     //   stage-2 output T[z][(b,a)]
-        } st;
-    };
-    alignas(16) unsigned char B[2 * kBHalf];  // X' slices: plane (h, q) at h kBHalf + q kBPlane
-    int vmr[MROWS];  // general cell: each row's exponent of V E in the current image
-    int gexp[KP];
-    signed char rx0[MROWS], rx1[MROWS];  // each row's cube x range in the current image
+struct IntCommon {
+    alignas(16) float Yh[kNPow][kYRow], Ynl[kNPow][kYRow];
+    alignas(8) float gsc[KP];                // 2^(g - SLB), g the alpha row's exponent (0: an empty row)
     unsigned char qb[kNPow][NPAIR_MAX + 2];  // qb[L-1][pair_index(L, b, a)] = b
     int zs[kNPow + 1];                       // zs[g]: packed index of (g, 0, 0) for the current pair's lp
-    PairHdr pb[2];                       // the current pair's record and the one being fetched
+    PairHdr pb[2];                           // the current pair's record and the one being fetched
     TileCommon c;
 };
-static_assert(sizeof(((SmemInt<false> *)0)->st) <= sizeof(((SmemInt<false> *)0)->A), "S and T fit in A");
+template <bool kGeneral>
+struct alignas(128) SmemInt : IntCommon {
+    alignas(16) float Ynh[kNPow][kYRow];
+    uint32_t mask[MROWS];          // each row's points inside the current item's range
+    __half A[2][NSL][MROWS * KP];  // masked V slices, K halves x in [0,16) and [16,32)
+    IntSums st;
+    union {
+        alignas(16) unsigned char B[2 * kBHalf];  // X' slices: plane (h, q) at h kBHalf + q kBPlane
+        IntTsum tt;                               // after the MMAs have read B
+    };
+};
+template <>  // (without the plane of -Y: three CTAs per SM)
+struct alignas(128) SmemInt<true> : IntCommon {
+    union {
+        __half A[2][NSL][MROWS * KP];
+        IntSums st;  // after the MMAs have read A
+    };
+    union {
+        alignas(16) unsigned char B[2 * kBHalf];
+        IntTsum tt;
+    };
+    ff Vff[TX][MROWS];  // this tile's V (x-major: lanes read consecutive rows)
+};
+static_assert(sizeof(IntTsum) <= 2 * kBHalf, "T fits in B");
+static_assert(3 * (sizeof(SmemInt<true>) + 1024) <= 228 * 1024, "3 general-cell integrate CTAs per SM");
+// planes of the y table: none (collocate: float-float entries), high and negated low, and -Y.hi
+template <class Smem>
+constexpr int kYPlanes = 3;
+template <>
+constexpr int kYPlanes<SmemColl> = 0;
+template <>
+constexpr int kYPlanes<SmemInt<true>> = 2;
 // dynamic shared memory of the orthorhombic integrate CTAs: at least 46 KB, so
 // that no fifth CTA (for which TMEM has no columns left) is placed on an SM
 constexpr size_t kSmemIntOrtho = sizeof(SmemInt<false>) > 46 * 1024 ? sizeof(SmemInt<false>) : 46 * 1024;
@@ -545,21 +564,39 @@ __device__ __forceinline__ TabEntry tab_entry(const TPair &p, const ImgState &q,
     r.e = r.in ? ff_exp(ff_mul(ff_mul(r.t, r.t), ff{-p.zetp.hi, -p.zetp.lo})) : ff{0.0f, 0.0f};
     return r;
 }
-// warp 1: one y or z entry into shared memory
-__device__ __forceinline__ void yz_fill(TileCommon &sm, const TPair &p, const TabEntry &te) {
-    // Y as float-float entries, Z as separate high and low parts (read in pairs of z)
-    float *hi = te.d == 1 ? &sm.Y[0][te.i].hi : &sm.Zh[0][te.i], *lo = te.d == 1 ? hi + 1 : &sm.Zl[0][te.i];
-    const int stride = te.d == 1 ? 2 * (kMaxTY + 1) : kMaxTZ;
+// warp 1: one y or z entry's powers: Y as float-float entries (collocate) or, as Z, in
+// three planes (high parts, both parts negated) for packed products
+template <class Smem>
+__device__ __forceinline__ void yz_fill(Smem &sm, const TPair &p, const TabEntry &te) {
+    constexpr int kY = kYPlanes<Smem>;
+    const bool isy = te.d == 1;
     const int L = te.in ? p.L : 0;
     ff e = te.e;
+    if constexpr (kY == 0) {
+        float *hi = isy ? &sm.Y[0][te.i].hi : &sm.c.Zh[0][te.i], *lo = isy ? hi + 1 : &sm.c.Znl[0][te.i];
+        const int stride = isy ? 2 * (kMaxTY + 1) : kMaxTZ;
+        float *nhi = &sm.c.Znh[0][te.i];
+        const float sg = isy ? 1.0f : -1.0f;
 #pragma unroll 1
-    for (int k = 0; k < L; k++) {
-        hi[k * stride] = e.hi;
-        lo[k * stride] = e.lo;
-        e = ff_mul(e, te.t);
+        for (int k = 0; k < kNPow; k++) {
+            hi[k * stride] = k < L ? e.hi : 0.0f;
+            lo[k * stride] = k < L ? sg * e.lo : 0.0f;
+            if (!isy) nhi[k * stride] = k < L ? -e.hi : 0.0f;
+            e = ff_mul(e, te.t);
+        }
+    } else {
+        float *hi = isy ? &sm.Yh[0][te.i] : &sm.c.Zh[0][te.i];
+        float *nlo = isy ? &sm.Ynl[0][te.i] : &sm.c.Znl[0][te.i], *nhi = &sm.c.Znh[0][te.i];
+        if constexpr (kY == 3) nhi = isy ? &sm.Ynh[0][te.i] : nhi;
+        const int stride = isy ? kYRow : kMaxTZ;
+#pragma unroll 1
+        for (int k = 0; k < p.L; k++) {
+            hi[k * stride] = k < L ? e.hi : 0.0f;
+            if (kY == 3 || !isy) nhi[k * stride] = k < L ? -e.hi : 0.0f;
+            nlo[k * stride] = k < L ? -e.lo : 0.0f;
+            e = ff_mul(e, te.t);
+        }
     }
-#pragma unroll 1
-    for (int k = L; k < kNPow; k++) hi[k * stride] = lo[k * stride] = 0.0f;
 }
 // warp 0: the x column of entry x in registers, xv[i] the powers 2 i and 2 i + 1: of u
 // (collocate: recentre) or of t (integrate); each step multiplies a pair by u^2.
@@ -569,7 +606,7 @@ __device__ __forceinline__ void x_powers(const TPair &p, const ImgState &q, cons
     for (int i = 0; i < kNPair; i++) xv[i] = ff2{f2(0.0f), f2(0.0f)};
     if (!te.in) return;
     const ff u = recentre ? ff_mul_f(p.h[0], ldexpf((float)(x - q.ic), -q.sb)) : te.t;
-    const ff2 u2 = ff2_dup(ff_mul(u, u));
+    const ff2n u2 = ff2n_dup(ff_mul(u, u));
     ff2 e = ff2_pair(te.e, ff_mul(te.e, u));
 #pragma unroll
     for (int i = 0; i < kNPair; i++) {
@@ -695,23 +732,11 @@ __device__ __forceinline__ void cross_factor_row(const GenLevel &G, const TPair 
 }
 
 // General cell, integrate: the A operand row r = the slices of V(x) E(x) over the
-// row's cube points (zero elsewhere), with the row's own exponent (vmr[r]).
+// row's cube points [x0, x1] (zero elsewhere), with the row's own exponent (returned).
 template <class Smem>
-__device__ __forceinline__ void general_a_row(Smem &sm, const GenLevel &G, const TPair &P, const ImgState &Q,
-                                              const TileShape &sh, int r, bool &zero_row) {
-    const int x0 = sm.rx0[r], x1 = sm.rx1[r];
-    if (x0 > x1) {
-        sm.vmr[r] = kZeroExp;
-        if (zero_row) return;
-        zero_row = true;
-#pragma unroll
-        for (int v = 0; v < TX / 8; v++)
-#pragma unroll
-            for (int q = 0; q < NSL; q++)
-                reinterpret_cast<uint4 *>(sm.A[v >> 1][q])[(r >> 3) * 16 + (v & 1) * 8 + (r & 7)] = make_uint4(0, 0, 0, 0);
-        return;
-    }
-    zero_row = false;
+__device__ __forceinline__ int general_a_row(Smem &sm, const GenLevel &G, const TPair &P, const ImgState &Q,
+                                             const TileShape &sh, int r, int x0, int x1) {
+    if (x0 > x1) return kZeroExp;  // the row's products are not read
     ff e0, q;
     cross_factor_row(G, P, Q, r >> sh.ly, r & (sh.TY - 1), x0, e0, q);
     // pass 1: the row maximum of |V E|
@@ -724,7 +749,6 @@ __device__ __forceinline__ void general_a_row(Smem &sm, const GenLevel &G, const
         }
     }
     const int vmx = exp_of(mx);
-    sm.vmr[r] = vmx;
     const float sc = vmx == kZeroExp ? 0.0f : pow2i(SLB - vmx);
     // pass 2: slices, 16-byte chunks of 8 x
     ff e = e0;
@@ -751,6 +775,42 @@ __device__ __forceinline__ void general_a_row(Smem &sm, const GenLevel &G, const
         for (int qq = 0; qq < NSL; qq++)
             reinterpret_cast<uint4 *>(sm.A[c >> 1][qq])[o16] = make_uint4(w[qq][0], w[qq][1], w[qq][2], w[qq][3]);
     }
+    return vmx;
+}
+
+// Orthorhombic integrate: bits of the row's mask M (bit x: point x inside the pair's
+// range) to its A row, chunk by chunk of 8 x: chunks not wholly inside are masked in
+// place.  A row with no point inside stays as it is: its products are not read.
+template <class Smem>
+__device__ __forceinline__ void mask_a_row(Smem &sm, int r, uint32_t M) {
+    if (M == 0u) return;
+#pragma unroll 1
+    for (int v = 0; v < TX / 8; v++) {
+        const uint32_t mb = (M >> (8 * v)) & 0xFFu;
+        if (mb == 0xFFu) continue;
+        const uint4 mk = chunk_mask(mb);
+        uint4 *a = reinterpret_cast<uint4 *>(sm.A[v >> 1][0]) + (r >> 3) * 16 + (v & 1) * 8 + (r & 7);
+        uint4 t[NSL];
+#pragma unroll
+        for (int q = 0; q < NSL; q++) t[q] = a[q * (MROWS * KP / 8)];
+#pragma unroll
+        for (int q = 0; q < NSL; q++)
+            a[q * (MROWS * KP / 8)] = make_uint4(t[q].x & mk.x, t[q].y & mk.y, t[q].z & mk.z, t[q].w & mk.w);
+    }
+}
+// copies the masked chunks of row r back from the CTA's slot (asynchronously: waited
+// for at the item's end)
+template <class Smem>
+__device__ __forceinline__ void restore_a_row(Smem &sm, const uint4 *vslot, int r, uint32_t M) {
+#pragma unroll 1
+    for (int v = 0; v < TX / 8 && M != 0u; v++) {
+        if (((M >> (8 * v)) & 0xFFu) == 0xFFu) continue;
+        const int o16 = (r >> 3) * 16 + (v & 1) * 8 + (r & 7);
+#pragma unroll
+        for (int q = 0; q < NSL; q++)
+            cp_async16(reinterpret_cast<uint4 *>(sm.A[v >> 1][q]) + o16, vslot + ((v >> 1) * NSL + q) * (MROWS * KP / 8) + o16);
+    }
+    cp_async_commit();
 }
 
 // TMEM set-up shared by both kernels: warp 0 allocates, thread 0 inits the mbarrier
@@ -834,15 +894,16 @@ __device__ __forceinline__ void stage1_cxy(SmemColl &sm, int L, int lp, const Ti
         const ff *c = sm.rc + (b * (lp + 1) - (b * (b - 1)) / 2 + a);
         ff2 s0 = {f2(0.0f), f2(0.0f)}, s1 = s0;
         auto zpair = [&](int g) {
-            return ff2{*reinterpret_cast<const float2 *>(&cm.Zh[g][zz]), *reinterpret_cast<const float2 *>(&cm.Zl[g][zz])};
+            return ff2n{*reinterpret_cast<const float2 *>(&cm.Zh[g][zz]), *reinterpret_cast<const float2 *>(&cm.Znh[g][zz]),
+                        *reinterpret_cast<const float2 *>(&cm.Znl[g][zz])};
         };
         int g = 0, bg = 0;
 #pragma unroll 1
         for (; g + 1 <= n; g += 2, bg += 2 * b) {
-            s0 = ff2_fma(zpair(g), ff2_dup(c[sm.zs[g] - bg]), s0);
-            s1 = ff2_fma(zpair(g + 1), ff2_dup(c[sm.zs[g + 1] - bg - b]), s1);
+            s0 = ff2_fma(ff2_dup(c[sm.zs[g] - bg]), zpair(g), s0);
+            s1 = ff2_fma(ff2_dup(c[sm.zs[g + 1] - bg - b]), zpair(g + 1), s1);
         }
-        if (g <= n) s0 = ff2_fma(zpair(g), ff2_dup(c[sm.zs[g] - bg]), s0);
+        if (g <= n) s0 = ff2_fma(ff2_dup(c[sm.zs[g] - bg]), zpair(g), s0);
         s0 = ff2_add(s0, s1);
         float *o = reinterpret_cast<float *>(&sm.Cxy[zz][q >> 1]) + (q & 1);
         o[0] = s0.hi.x;
@@ -867,7 +928,7 @@ __device__ __forceinline__ int stage2_row(SmemColl &sm, const TileCommon &cm, in
         const float4 *crow = sm.Cxy[z];
 #pragma unroll 1
         for (int b = 0; b <= lp; b++) {
-            const ff2 yb = ff2_dup(cm.Y[b][y]);
+            const ff2n yb = ff2n_dup(sm.Y[b][y]);
 #pragma unroll
             for (int i = 0; i < kNPair; i++) {
                 if (2 * i > lp - b) break;
@@ -908,7 +969,6 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
     constexpr uint32_t kCols = 128;  // diagonals D2..D5: 32 columns each
     tc_setup(cm, kCols);
     const uint32_t tbase = cm.tmem + ((uint32_t)(warp * 32) << 16);
-    const uint32_t idesc = tc::idesc_f16_f32(MROWS, TX);
     uint32_t phase = 0;
     for (int t = tid; t < kNPow * kNPow; t += NTHR) sm.bin[t / kNPow][t % kNPow] = c_binom[t / kNPow][t % kNPow];
     // qb[L-1][pair_index(L, b, a)] = b: the (b, a) of a pair index without a search per use
@@ -976,7 +1036,7 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                             // K slots beyond L may hold an earlier pair's slices: rewritten as zeros
                             slice_row16(xv, sc, max(L, cm.kmax), L, sm.B[0], TX * KP, tid);
                         } else {
-                            yz_fill(cm, P, te);
+                            yz_fill(sm, P, te);
                         }
                     }
                 } else {
@@ -1002,17 +1062,14 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                 __syncthreads();
                 if (tid == 0) {
                     tc::fence_after_sync();
-                    uint64_t ad[NSL], bd[NSL];
+                    // diagonal s = i + j into TMEM columns [32 s, 32 s + 32): the planes of B lie
+                    // one after the other along N, so A_i times B_0 .. B_{3-i} is one MMA of
+                    // N = 32 (4 - i) whose columns start at 32 i (4 MMAs instead of 10)
+                    const uint64_t ad = tc::desc_kmajor(sm.A[0], 128, 256), bd = tc::desc_kmajor(sm.B[0], 128, 256);
 #pragma unroll
-                    for (int q = 0; q < NSL; q++) {
-                        ad[q] = tc::desc_kmajor(sm.A[q], 128, 256);
-                        bd[q] = tc::desc_kmajor(sm.B[q], 128, 256);
-                    }
-                    // diagonal s = i + j into TMEM columns [32 s, 32 s + 32)
-#pragma unroll
-                    for (int sd = 0; sd < NSL; sd++)
-#pragma unroll
-                        for (int i = 0; i <= sd; i++) tc::mma_f16(cm.tmem + 32 * sd, ad[i], bd[sd - i], idesc, i > 0);
+                    for (int i = 0; i < NSL; i++)
+                        tc::mma_f16(cm.tmem + 32 * i, ad + (uint64_t)(i * (int)sizeof(sm.A[0]) >> 4), bd,
+                                    tc::idesc_f16_f32(MROWS, TX * (NSL - i)), i > 0);
                     tc::mma_commit(&cm.mbar);
                 }
                 tc_wait(cm, phase, A.status);
@@ -1132,6 +1189,14 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
     tc_teardown(cm, kCols, phase);
 }
 
+// s += four products a b, the even and the odd ones in the two halves of s
+__device__ __forceinline__ void acc_four(ff2 &s, float4 ah, float4 al, float4 bh, float4 bnh, float4 bnl) {
+    ff2_acc_lazy(s, ff2{make_float2(ah.x, ah.y), make_float2(al.x, al.y)},
+                 ff2n{make_float2(bh.x, bh.y), make_float2(bnh.x, bnh.y), make_float2(bnl.x, bnl.y)});
+    ff2_acc_lazy(s, ff2{make_float2(ah.z, ah.w), make_float2(al.z, al.w)},
+                 ff2n{make_float2(bh.z, bh.w), make_float2(bnh.z, bnh.w), make_float2(bnl.z, bnl.w)});
+}
+
 // kGeneral: tiles of general-cell levels; the A operand holds the slices of
 // V(x) E(x) (E the cross factor of the Gaussian along the row), one row per
 // thread, with its own exponent per row and image.
@@ -1146,7 +1211,6 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
     constexpr uint32_t kCols = 128;  // D2 (two K halves), D3, D4, D5: 16 columns each
     tc_setup(cm, kCols);
     const uint32_t tbase = cm.tmem + ((uint32_t)(warp * 32) << 16);
-    const uint32_t idesc = tc::idesc_f16_f32(MROWS, KP);
     uint32_t phase = 0;
     for (int t = tid; t < kNPow * (NPAIR_MAX + 2); t += NTHR) {
         const int Lq = t / (NPAIR_MAX + 2) + 1, q = t % (NPAIR_MAX + 2);
@@ -1170,18 +1234,17 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
         const TileExt ext = {min(TX, lv.ngrid[0] - td.t[0] * TX), min(TY, lv.ngrid[1] - td.t[1] * TY),
                              min(TZ, lv.ngrid[2] - td.t[2] * TZ)};
         const bool row_ok = z < ext.z && y < ext.y;
-        // this thread's V row, sliced once per tile (row exponent vm)
+        // this thread's V row, sliced once per tile (row exponent vm), into A and the slot
         int vm;
         {
             const double *grid = A.grids.p[td.level];
-            const bool ok = row_ok;
             const int64_t row = ((int64_t)(td.t[2] * TZ + z) * lv.ngrid[1] + (td.t[1] * TY + y)) * lv.ngrid[0] +
                                 td.t[0] * TX;
             // compact loops (once per tile): the row maximum, then 16-byte chunks of 8 x
             float mx = 0.0f;
 #pragma unroll 1
             for (int x = 0; x < TX; x++) {
-                const ff v = (ok && x < ext.x) ? ff_from_double(grid[row + x]) : ff{0.0f, 0.0f};
+                const ff v = (row_ok && x < ext.x) ? ff_from_double(grid[row + x]) : ff{0.0f, 0.0f};
                 if constexpr (kGeneral) sm.Vff[x][m] = v;
                 mx = fmaxf(mx, fabsf(v.hi));
             }
@@ -1193,8 +1256,8 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     const int x = 8 * c + 2 * i;
-                    const ff v0 = (ok && x < ext.x) ? ff_from_double(grid[row + x]) : ff{0.0f, 0.0f};
-                    const ff v1 = (ok && x + 1 < ext.x) ? ff_from_double(grid[row + x + 1]) : ff{0.0f, 0.0f};
+                    const ff v0 = (row_ok && x < ext.x) ? ff_from_double(grid[row + x]) : ff{0.0f, 0.0f};
+                    const ff v1 = (row_ok && x + 1 < ext.x) ? ff_from_double(grid[row + x + 1]) : ff{0.0f, 0.0f};
                     float2 sl[NSL];
                     slice_scaled2(ff2_pair(v0, v1), f2(sc), sl);
 #pragma unroll
@@ -1202,11 +1265,14 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                 }
                 const int o16 = (m >> 3) * 16 + (c & 1) * 8 + (m & 7);  // umma_off / 16
 #pragma unroll
-                for (int q = 0; q < NSL; q++)
-                    vslot[((c >> 1) * NSL + q) * (MROWS * KP / 8) + o16] = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
+                for (int q = 0; q < NSL; q++) {
+                    const uint4 val = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
+                    vslot[((c >> 1) * NSL + q) * (MROWS * KP / 8) + o16] = val;
+                    reinterpret_cast<uint4 *>(sm.A[c >> 1][q])[o16] = val;
+                }
             }
+            if constexpr (!kGeneral) __threadfence();  // the slot's rows are read back by cp.async
         }
-        bool zero_row[2] = {false, false};  // A rows u, u + 64 hold zeros (warps 2-3)
         const int64_t it0 = A.start[2 * tile], it1 = A.start[2 * tile + 1];
         uint64_t nxt = 0;
         first_pair(cm, sm.pb, A, it0, it1, nxt, false);
@@ -1218,22 +1284,24 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
             const int64_t moff = P.coef_off;
             const ImgState &Q = cm.ii[cur].im;
             {
-                {
-                    // every thread: its row's cube x range, for the A operand of warps 2-3
-                    int x0, x1;
-                    if constexpr (kGeneral)
-                        general_row_range(lv, A.glv[td.level], P, Q, Q.o[2] + z, Q.o[1] + y, row_ok,
-                                          x0, x1);
-                    else
-                        row_range(P, Q, A.table, Q.o[2] + z, Q.o[1] + y, row_ok, x0, x1);
-                    const bool empty = x0 > x1;  // otherwise both lie in [0, TX)
-                    sm.rx0[m] = (signed char)(empty ? 1 : x0);
-                    sm.rx1[m] = (signed char)(empty ? 0 : x1);
+                // every thread: its row's cube x range, applied to its A row
+                int x0, x1;
+                if constexpr (kGeneral)
+                    general_row_range(lv, A.glv[td.level], P, Q, Q.o[2] + z, Q.o[1] + y, row_ok, x0, x1);
+                else
+                    row_range(P, Q, A.table, Q.o[2] + z, Q.o[1] + y, row_ok, x0, x1);
+                int vrow = vm;
+                uint32_t M = 0;
+                if constexpr (kGeneral) {
+                    vrow = general_a_row(sm, A.glv[td.level], P, Q, sh, m, x0, x1);
+                } else {  // (a row of zeros needs no mask)
+                    M = vm == kZeroExp ? ~0u : (x0 > x1 ? 0u : (uint32_t)(((2ull << x1) - 1ull) & ~((1ull << x0) - 1ull)));
+                    sm.mask[m] = M;
                 }
                 if (warp == 0) {
                     if constexpr (!kGeneral) bar_arrive1(NTHR);
                     // X column (lane x) in registers, then B: row alpha = X[alpha][x] over x,
-                    // scaled by 2^(SLB - gexp[alpha]) (maximum over the warp); rows alpha >= L
+                    // scaled by 2^(SLB - g[alpha]) (maximum over the warp); rows alpha >= L
                     // are left as they are (their output columns are not read).  Unlike
                     // collocate, integrate is not limited by instruction fetch: warps 0 and 1
                     // keep separate table code.
@@ -1251,7 +1319,7 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                                 __uint_as_float(__reduce_max_sync(
                                     0xffffffffu, __float_as_uint(fabsf(h ? xv[a / 2].hi.y : xv[a / 2].hi.x))));
                             const int e = exp_of(mxb);
-                            if (tid == a + h) sm.gexp[a + h] = e;
+                            if (tid == a + h) sm.gsc[a + h] = e == kZeroExp ? 0.0f : pow2i(e - SLB);
                             sc[h] = e == kZeroExp ? 0.0f : pow2i(SLB - e);
                         }
                         float2 sl[NSL];
@@ -1268,75 +1336,39 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                     if constexpr (!kGeneral) bar_arrive1(NTHR);
                     if (tid - 32 <= kNPow) sm.zs[tid - 32] = tid - 32 <= lp + 1 ? row_start(lp, tid - 32, 0) : 0;
 #pragma unroll 1
-                    for (int ent = tid - 32; ent < TY + TZ; ent += 32) yz_fill(cm, P, tab_entry(P, Q, ext, sh, 1, ent));
+                    for (int ent = tid - 32; ent < TY + TZ; ent += 32) yz_fill(sm, P, tab_entry(P, Q, ext, sh, 1, ent));
                 } else if constexpr (!kGeneral) {
-                    bar_sync1(NTHR);
-                    // A operand: V slices of rows u and u + 64 (the CTA's slot) masked to the rows' cube ranges,
-                    // 16-byte chunks (8 x of one K half); rows already zero stay untouched
-                    const int u = tid - 64;
-#pragma unroll 1
-                    for (int rr = 0; rr < 2; rr++) {
-                        const int r = u + 64 * rr;
-                        const int x0 = sm.rx0[r], x1 = sm.rx1[r];
-                        const uint32_t M =
-                            x0 > x1 ? 0u : (uint32_t)(((2ull << x1) - 1ull) & ~((1ull << x0) - 1ull));  // bits x0..x1
-                        if (M == 0u && zero_row[rr]) continue;
-                        zero_row[rr] = M == 0u;
-                        // all loads of the row first (from the slot): latencies overlap; chunks of 8
-                        // x outside the row's range are not loaded (they are stored as zeros)
-                        uint4 val[TX / 8][NSL];
-#pragma unroll
-                        for (int v = 0; v < TX / 8; v++)
-#pragma unroll
-                            for (int q = 0; q < NSL; q++)
-                                val[v][q] = ((M >> (8 * v)) & 0xFFu)
-                                                ? vslot[((v >> 1) * NSL + q) * (MROWS * KP / 8) + (r >> 3) * 16 +
-                                                        (v & 1) * 8 + (r & 7)]
-                                                : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-                        for (int v = 0; v < TX / 8; v++) {
-                            const uint4 mk = chunk_mask(M >> (8 * v));
-                            const int o16 = (r >> 3) * 16 + (v & 1) * 8 + (r & 7);  // umma_off / 16
-#pragma unroll
-                            for (int q = 0; q < NSL; q++)
-                                reinterpret_cast<uint4 *>(sm.A[v >> 1][q])[o16] =
-                                    make_uint4(val[v][q].x & mk.x, val[v][q].y & mk.y, val[v][q].z & mk.z,
-                                               val[v][q].w & mk.w);
-                        }
-                    }
+                    bar_sync1(NTHR);  // every row's mask
+                    mask_a_row(sm, tid - 64, sm.mask[tid - 64]);
+                    mask_a_row(sm, tid, sm.mask[tid]);
                 }
-                if constexpr (kGeneral) general_a_row(sm, A.glv[td.level], P, Q, sh, m, zero_row[0]);
                 tc::fence_async_smem();
                 tc::fence_before_sync();
                 __syncthreads();
                 if (tid == 0) {
                     tc::fence_after_sync();
-                    uint64_t a_[2][NSL], b_[2][NSL];
-                    for (int h = 0; h < 2; h++)
-                        for (int q = 0; q < NSL; q++) {
-                            a_[h][q] = tc::desc_kmajor(sm.A[h][q], 128, 256);
-                            b_[h][q] = tc::desc_kmajor(sm.B + h * kBHalf + q * kBPlane, kBLbo, kBSbo);
-                        }
-                    // D2 per K half (exact: 16 products each); diagonals 3.. over both halves
-                    tc::mma_f16(cm.tmem + 0, a_[0][0], b_[0][0], idesc, 0);
-                    tc::mma_f16(cm.tmem + 16, a_[1][0], b_[1][0], idesc, 0);
+                    // as in collocate, A_i of K half h times the planes B_0 .. B_{3-i} in one MMA
+                    // of N = 16 (4 - i), diagonal s into columns [16 + 16 s, 32 + 16 s); D2 of the
+                    // second half apart, in columns [0, 16) (exact: 16 products each): 9 MMAs
+                    // instead of 20
+                    const uint64_t ad = tc::desc_kmajor(sm.A[0][0], 128, 256), bd = tc::desc_kmajor(sm.B, kBLbo, kBSbo);
+                    constexpr uint64_t kA = sizeof(sm.A[0][0]) >> 4, kB1 = kBHalf >> 4, kBP = kBPlane >> 4;
 #pragma unroll
-                    for (int sd = 1; sd < NSL; sd++) {
-                        int first = 1;
+                    for (int i = 0; i < NSL; i++)
+                        tc::mma_f16(cm.tmem + 16 + 16 * i, ad + kA * i, bd, tc::idesc_f16_f32(MROWS, KP * (NSL - i)), i > 0);
+                    tc::mma_f16(cm.tmem, ad + kA * NSL, bd + kB1, tc::idesc_f16_f32(MROWS, KP), 0);
+                    tc::mma_f16(cm.tmem + 32, ad + kA * NSL, bd + kB1 + kBP, tc::idesc_f16_f32(MROWS, KP * (NSL - 1)), 1);
 #pragma unroll
-                        for (int i = 0; i <= sd; i++)
-#pragma unroll
-                            for (int h = 0; h < 2; h++) {
-                                tc::mma_f16(cm.tmem + 16 + 16 * sd, a_[h][i], b_[h][sd - i], idesc, first ? 0u : 1u);
-                                first = 0;
-                            }
-                    }
+                    for (int i = 1; i < NSL; i++)
+                        tc::mma_f16(cm.tmem + 16 + 16 * i, ad + kA * (NSL + i), bd + kB1,
+                                    tc::idesc_f16_f32(MROWS, KP * (NSL - i)), 1);
                     tc::mma_commit(&cm.mbar);
                 }
                 tc_wait(cm, phase, A.status);
                 phase ^= 1u;
-                const bool live = sm.rx0[m] <= sm.rx1[m];
-                ff *const srow = sm.st.S + s_index(m, sh.ly);
+                if constexpr (!kGeneral) restore_a_row(sm, vslot, m, M);
+                const bool live = x0 <= x1;  // other rows give zeros
+                const float2 rsc = f2(vrow != kZeroExp ? pow2i(vrow - SLB) : 0.0f);  // 2^(row exponent - SLB)
 #pragma unroll 1
                 for (int c = 0; c < KP / 8; c++) {
                     if (8 * c >= L) break;  // uniform: S columns alpha >= L are not read
@@ -1345,33 +1377,39 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                     tc::tmem_ld8(tbase + 16 + 8 * c, rb);
                     tc::tmem_ld8(tbase + 32 + 8 * c, r3);
                     tc::tmem_ld8(tbase + 48 + 8 * c, r4);
-                    tc::tmem_wait_ld32(ra, rb, r3, r4);
                     tc::tmem_ld8(tbase + 64 + 8 * c, r5);
-                    tc::tmem_wait_ld8(r5);
+                    tc::tmem_wait_ld32(ra, rb, r3, r4);
+                    tc::tmem_wait_ld8(r5);  // (one wait covers all loads; the second only orders r5's use)
 #pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        const int a = 8 * c + i;
-                        ff s = {0.0f, 0.0f};
-                        if (a < L && live) {
-                            const ff d2 = two_sum(__uint_as_float(ra[i]), __uint_as_float(rb[i]));
-                            ff t = two_sum(d2.hi, __fmul_rn(__uint_as_float(r3[i]), 0.0009765625f));
-                            t.lo = __fadd_rn(t.lo, __fmaf_rn(__uint_as_float(r4[i]), 9.5367431640625e-07f,
-                                                             __fmaf_rn(__uint_as_float(r5[i]), 9.313225746154785e-10f, d2.lo)));
-                            t = fast_two_sum(t.hi, t.lo);
-                            const int vrow = kGeneral ? sm.vmr[m] : vm;
-                            const int E = vrow + sm.gexp[a] - 2 * SLB;
-                            if (E >= -126 && vrow != kZeroExp && sm.gexp[a] != kZeroExp) {
-                                const float scl = pow2i(min(E, 127));
-                                s = {__fmul_rn(t.hi, scl), __fmul_rn(t.lo, scl)};
-                            }
+                    for (int i = 0; i < 4; i++) {  // two alpha per instruction
+                        if (8 * c + 2 * i >= kNPow) break;
+                        auto two = [&](const uint32_t *r) {
+                            return make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+                        };
+                        const ff2 d2 = two_sum2(two(ra), two(rb));
+                        ff2 t = two_sum2(d2.hi, f2_mul(two(r3), f2(0.0009765625f)));
+                        t.lo = f2_add(t.lo, f2_fma(two(r4), f2(9.5367431640625e-07f),
+                                                   f2_fma(two(r5), f2(9.313225746154785e-10f), d2.lo)));
+                        t = fast_two_sum2(t.hi, t.lo);
+                        const float2 g = *reinterpret_cast<const float2 *>(&sm.gsc[8 * c + 2 * i]);
+                        const float2 sp = f2_mul(rsc, g);
+                        const float2 scl = make_float2(fminf(sp.x, 1.7014118e38f), fminf(sp.y, 1.7014118e38f));
+                        float2 sh2 = f2_mul(t.hi, scl), sl2 = f2_mul(t.lo, scl);
+                        if (!live) sh2 = sl2 = f2(0.0f);
+                        const int a = 8 * c + 2 * i;
+                        sm.st.Sh[a][m] = sh2.x;
+                        sm.st.Sl[a][m] = sl2.x;
+                        if (a + 1 < kNPow) {
+                            sm.st.Sh[a + 1][m] = sh2.y;
+                            sm.st.Sl[a + 1][m] = sl2.y;
                         }
-                        srow[a] = s;
                     }
                 }
                 tc::fence_before_sync();
                 __syncwarp();
                 // stage 2 transposed: T[z][(b,a)] = sum_y S[(z,y)][a] Y[b][y], by the warp whose
-                // rows have this z (a warp barrier after the readout suffices)
+                // rows have this z (a warp barrier after the readout suffices); two partial
+                // sums, over even and odd y, as one packed sum
                 const int lzw = 5 - sh.ly;  // log2 of the z values per warp
                 const int zbase = (warp * 32) >> sh.ly;
                 const unsigned char *qbL = sm.qb[L - 1];
@@ -1379,14 +1417,22 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                     const int zz = zbase + (t & ((1 << lzw) - 1));
                     const int q = t >> lzw, b = qbL[q];  // q = pair_index(L, b, a)
                     const int a = q - (b * L - (b * (b - 1)) / 2);
-                    ff s0 = {0.0f, 0.0f}, s1 = {0.0f, 0.0f};
-                    const ff *sz = sm.st.S + s_index(zz * TY, sh.ly) + a;  // rows (zz, y) at sz[y * kSRow]
-#pragma unroll 2
-                    for (int yy = 0; yy < TY; yy += 2) {
-                        ff_acc_lazy(s0, sz[yy * kSRow], cm.Y[b][yy]);
-                        ff_acc_lazy(s1, sz[(yy + 1) * kSRow], cm.Y[b][yy + 1]);
+                    const float4 *ph = reinterpret_cast<const float4 *>(&sm.st.Sh[a][zz * TY]);
+                    const float4 *pl = reinterpret_cast<const float4 *>(&sm.st.Sl[a][zz * TY]);
+                    const float4 *yh = reinterpret_cast<const float4 *>(sm.Yh[b]);
+                    const float4 *ynh = yh;
+                    if constexpr (!kGeneral) ynh = reinterpret_cast<const float4 *>(sm.Ynh[b]);
+                    const float4 *ynl = reinterpret_cast<const float4 *>(sm.Ynl[b]);
+                    ff2 s = {f2(0.0f), f2(0.0f)};
+#pragma unroll 4
+                    for (int y4 = 0; y4 < TY / 4; y4++) {
+                        float4 nh = ynh[y4];
+                        if constexpr (kGeneral) nh = make_float4(-nh.x, -nh.y, -nh.z, -nh.w);
+                        acc_four(s, ph[y4], pl[y4], yh[y4], nh, ynl[y4]);
                     }
-                    sm.st.T[zz][q] = ff_add(s0, s1);
+                    const ff r = ff_add(ff{s.hi.x, s.lo.x}, ff{s.hi.y, s.lo.y});
+                    sm.tt.Th[q][zz] = r.hi;
+                    sm.tt.Tl[q][zz] = r.lo;
                 }
                 __syncthreads();
                 // stage 1 transposed: W[g][b][a] += sum_z T[z][(b,a)] Z[g][z]
@@ -1398,14 +1444,16 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                     const int qn = lp - g, r = t - sm.zs[g];
                     const int b = sm.qb[qn][r];
                     const int a = r - (b * (qn + 1) - (b * (b - 1)) / 2);
-                    ff s0 = {0.0f, 0.0f}, s1 = {0.0f, 0.0f};
                     const int pi = pair_index(L, b, a);
-#pragma unroll 2
-                    for (int zz = 0; zz < TZ; zz += 2) {
-                        ff_acc_lazy(s0, sm.st.T[zz][pi], ff{cm.Zh[g][zz], cm.Zl[g][zz]});
-                        ff_acc_lazy(s1, sm.st.T[zz + 1][pi], ff{cm.Zh[g][zz + 1], cm.Zl[g][zz + 1]});
-                    }
-                    const ff s = ff_add(s0, s1);
+                    ff2 s2 = {f2(0.0f), f2(0.0f)};
+#pragma unroll 1
+                    for (int z4 = 0; z4 < TZ; z4 += 4)
+                        acc_four(s2, *reinterpret_cast<const float4 *>(&sm.tt.Th[pi][z4]),
+                                 *reinterpret_cast<const float4 *>(&sm.tt.Tl[pi][z4]),
+                                 *reinterpret_cast<const float4 *>(&cm.Zh[g][z4]),
+                                 *reinterpret_cast<const float4 *>(&cm.Znh[g][z4]),
+                                 *reinterpret_cast<const float4 *>(&cm.Znl[g][z4]));
+                    const ff s = ff_add(ff{s2.hi.x, s2.lo.x}, ff{s2.hi.y, s2.lo.y});
                     if (s.hi != 0.0f) {
                         double val = (double)s.hi + (double)s.lo;
                         if constexpr (kGeneral) {
