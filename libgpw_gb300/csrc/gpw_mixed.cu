@@ -1240,13 +1240,20 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
             const double *grid = A.grids.p[td.level];
             const int64_t row = ((int64_t)(td.t[2] * TZ + z) * lv.ngrid[1] + (td.t[1] * TY + y)) * lv.ngrid[0] +
                                 td.t[0] * TX;
-            // compact loops (once per tile): the row maximum, then 16-byte chunks of 8 x
+            // compact loops (once per unit): the row maximum, then 16-byte chunks of 8 x; 8
+            // loads in flight (one at a time, their latency was a tenth of a 16-item unit)
             float mx = 0.0f;
 #pragma unroll 1
-            for (int x = 0; x < TX; x++) {
-                const ff v = (row_ok && x < ext.x) ? ff_from_double(grid[row + x]) : ff{0.0f, 0.0f};
-                if constexpr (kGeneral) sm.Vff[x][m] = v;
-                mx = fmaxf(mx, fabsf(v.hi));
+            for (int x8 = 0; x8 < TX; x8 += 8) {
+                double v8[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) v8[i] = (row_ok && x8 + i < ext.x) ? grid[row + x8 + i] : 0.0;
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const ff v = ff_from_double(v8[i]);
+                    if constexpr (kGeneral) sm.Vff[x8 + i][m] = v;
+                    mx = fmaxf(mx, fabsf(v.hi));
+                }
             }
             vm = exp_of(mx);
             const float sc = vm == kZeroExp ? 0.0f : pow2i(SLB - vm);
@@ -2027,8 +2034,9 @@ int mixed_rebin(TaskSet &ts, std::string &err) {
     // Work units for the persistent queue: a tile with more items than ~1/64 of
     // an even share per SM is divided into units of consecutive items (their
     // flushes add with FP64 atomics), and where that leaves fewer than about four
-    // units per resident CTA, than 1/16 of it, down to 16 items (1000 pairs, 64^3:
-    // 359 units of up to 64 items for 608 CTAs, 2203 of up to 16).  Within each group
+    // units per resident CTA, than 1/16 of it, down to 32 items (1000 pairs, 64^3, with
+    // its 34,733 items in units of up to 16, 24, 32: integrate 354, 351, 323 us,
+    // collocate 292, 298, 298).  Within each group
     // (orthorhombic, general) units run by decreasing work class (item counts within a
     // factor 2^(1/4) share a class), and within a class in the tiles' raster order: the
     // tiles in flight at one time then form a compact slab of the grid, so a pair's
@@ -2036,7 +2044,7 @@ int mixed_rebin(TaskSet &ts, std::string &err) {
     // use them, while the short units still come last.
     const int64_t sms = std::max(1, M->sms);
     const int64_t target = std::max((nitems + 64 * sms - 1) / (64 * sms),
-                                    std::min<int64_t>(64, std::max<int64_t>(16, nitems / (16 * sms))));
+                                    std::min<int64_t>(64, std::max<int64_t>(32, nitems / (16 * sms))));
     struct Unit {
         int tile;
         int64_t it0, it1;
