@@ -24,31 +24,42 @@ namespace gpw {
 constexpr int kBI = kMaxL + 4;          // components up to l_max + 1 (local block) + 2
 constexpr int kBK = 2 * kBI - 1;
 
+constexpr int kBWarps = 12;  // 3 axes x (centre a, centre b) x 2 halves of the local block
+
 struct BwdSmem {
     double al[3][kBI][kBI][kBK];
     double W[(kNPowB * (kNPowB + 1) * (kNPowB + 2)) / 6];  // moments up to degree lp + 2
-    double red[8][4];
+    short row[kNPowB][kNPowB];                             // packed index of (lz, ly, 0)
+    double red[8][kBWarps];
 };
 
-__device__ __forceinline__ double pair_integral(const BwdSmem &s, int lpe, const int a[3], const int b[3]) {
+__device__ __forceinline__ double pair_integral(const BwdSmem &s, const int a[3], const int b[3]) {
+    const double *ax = s.al[0][a[0]][b[0]];
     double acc = 0.0;
     for (int lz = 0; lz <= a[2] + b[2]; lz++) {
-        const double az = s.al[2][a[2]][b[2]][lz];
+        double accz = 0.0;
         for (int ly = 0; ly <= a[1] + b[1]; ly++) {
-            const double ayz = az * s.al[1][a[1]][b[1]][ly];
-            for (int lx = 0; lx <= a[0] + b[0]; lx++)
-                acc += ayz * s.al[0][a[0]][b[0]][lx] * s.W[pidx(lpe, lz, ly, lx)];
+            const double *W = s.W + s.row[lz][ly];
+            double accy = 0.0;
+            for (int lx = 0; lx <= a[0] + b[0]; lx++) accy += ax[lx] * W[lx];
+            accz += s.al[1][a[1]][b[1]][ly] * accy;
         }
+        acc += s.al[2][a[2]][b[2]][lz] * accz;
     }
     return acc;
 }
 
-__global__ void __launch_bounds__(128)
+// One CTA per pair.  The pair integrals are dependent FP64 chains, so they are spread
+// over 12 warps: a warp takes one axis d, one centre and every second element of the
+// local block, up to three integrals per element (a +- e_d, a + 2 e_d).  (Four warps
+// with an element's 18 integrals to a thread and the packed index searched in the inner
+// loop: 459 us for 2000 pairs, l <= 2.)
+__global__ void __launch_bounds__(32 * kBWarps)
 k_backward_epilogue(const PairGeom *__restrict__ geoms, const LevelDev *__restrict__ levels,
                     const double *__restrict__ tmat, const double *__restrict__ mom_ext, int func,
                     const double *__restrict__ pab, double *dra, double *drb, double *dza, double *dzb) {
     __shared__ BwdSmem s;
-    const PairGeom g = geoms[blockIdx.x];
+    const PairGeom &g = geoms[blockIdx.x];
     const int tid = threadIdx.x;
     const int lpe = g.lp + 2;
     const int ia = g.la_max + 2, jb = g.lb_max + 2;  // local shells (after the function's shift)
@@ -57,23 +68,22 @@ k_backward_epilogue(const PairGeom *__restrict__ geoms, const LevelDev *__restri
         const int j = t % (jb + 1), i = (t / (jb + 1)) % (ia + 1), ax = t / ((jb + 1) * (ia + 1));
         const double pa = g.rp[ax] - g.ra[ax], pb = g.rp[ax] - g.rb[ax];
         double *out = s.al[ax][i][j];
-        for (int k = 0; k < kBK; k++) out[k] = 0.0;
-        double ci = 1.0;
-        for (int k1 = 0; k1 <= i; k1++) {
-            double pai = 1.0;
-            for (int e = 0; e < i - k1; e++) pai *= pa;
-            double cj = 1.0;
-            for (int k2 = 0; k2 <= j; k2++) {
-                double pbj = 1.0;
-                for (int e = 0; e < j - k2; e++) pbj *= pb;
-                out[k1 + k2] += ci * pai * cj * pbj;
-                cj = cj * (double)(j - k2) / (double)(k2 + 1);
-            }
-            ci = ci * (double)(i - k1) / (double)(k1 + 1);
+        // one multiplication by (u + pa) or (u + pb) at a time, as fill_alpha
+        out[0] = 1.0;
+        for (int k = 1; k < kBK; k++) out[k] = 0.0;
+        for (int m = 0; m < i + j; m++) {
+            const double c = m < i ? pa : pb;
+            out[m + 1] = out[m];
+            for (int k = m; k >= 1; k--) out[k] = fma(c, out[k], out[k - 1]);
+            out[0] *= c;
         }
     }
     // Cartesian moments (general cells: transpose of the lattice transform)
     const int nc = ncoef(lpe);
+    for (int t = tid; t < kNPowB * kNPowB; t += blockDim.x) {
+        const int lz = t / kNPowB, ly = t - lz * kNPowB;
+        s.row[lz][ly] = (short)(lz + ly <= lpe ? pidx(lpe, lz, ly, 0) : 0);
+    }
     const double *Wsrc = mom_ext + g.mom_ext_off;
     for (int t = tid; t < nc; t += blockDim.x) {
         if (g.ortho) {
@@ -102,59 +112,53 @@ k_backward_epilogue(const PairGeom *__restrict__ geoms, const LevelDev *__restri
         s.W[t] = acc;
     }
     __syncthreads();
-    double grad[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // dRa[3], dRb[3], dza, dzb
-    const int na = ncoset(g.la_max), nb = ncoset(g.lb_max);
-    for (int t = tid; t < na * nb; t += blockDim.x) {
-        const int jco = t / na, ico = t % na;
-        int a[3], b[3];
-        coset_decode(ico, a[0], a[1], a[2]);
-        coset_decode(jco, b[0], b[1], b[2]);
-        double dPa, dPb;  // dP'/dzeta, dP'/dzetb of the local element
-        const double P = local_entry(g, func, pab, a, b, &dPa, &dPb);
-        if (P == 0.0 && dPa == 0.0 && dPb == 0.0) continue;
-        if (dPa != 0.0 || dPb != 0.0) {
-            const double I0 = pair_integral(s, lpe, a, b);
-            grad[6] += dPa * I0;
-            grad[7] += dPb * I0;
+    const int lane = tid & 31, warp = tid >> 5;
+    const int d = warp % 3, side = (warp / 3) % 2, half = warp / 6;
+    double gc = 0.0, gz[2] = {0.0, 0.0};  // this centre's derivative along d; dza, dzb
+    const int a0 = ncoset(g.la_min - 1), b0 = ncoset(g.lb_min - 1);  // the local block's shells
+    const int na = ncoset(g.la_max) - a0, nb = ncoset(g.lb_max) - b0;
+    for (int t = 2 * lane + half; t < na * nb; t += 64) {
+        const int jco = b0 + t / na, ico = a0 + t % na;
+        int c[2][3];
+        coset_decode(ico, c[0][0], c[0][1], c[0][2]);
+        coset_decode(jco, c[1][0], c[1][1], c[1][2]);
+        double dP[2];  // dP'/dzeta, dP'/dzetb of the local element
+        const double P = local_entry(g, func, pab, c[0], c[1], &dP[0], &dP[1]);
+        if (d == 0 && side == 0 && (dP[0] != 0.0 || dP[1] != 0.0)) {
+            const double I0 = pair_integral(s, c[0], c[1]);
+            gz[0] += dP[0] * I0;
+            gz[1] += dP[1] * I0;
         }
         if (P == 0.0) continue;
-        for (int d = 0; d < 3; d++) {
-            int a2[3] = {a[0], a[1], a[2]}, b2[3] = {b[0], b[1], b[2]};
-            // centre a
-            a2[d] = a[d] + 1;
-            double v = 2.0 * g.zeta * pair_integral(s, lpe, a2, b);
-            if (a[d] > 0) {
-                a2[d] = a[d] - 1;
-                v -= a[d] * pair_integral(s, lpe, a2, b);
-            }
-            grad[d] += P * v;
-            a2[d] = a[d] + 2;
-            grad[6] -= P * pair_integral(s, lpe, a2, b);
-            a2[d] = a[d];
-            // centre b
-            b2[d] = b[d] + 1;
-            v = 2.0 * g.zetb * pair_integral(s, lpe, a, b2);
-            if (b[d] > 0) {
-                b2[d] = b[d] - 1;
-                v -= b[d] * pair_integral(s, lpe, a, b2);
-            }
-            grad[3 + d] += P * v;
-            b2[d] = b[d] + 2;
-            grad[7] -= P * pair_integral(s, lpe, a, b2);
+        const int l = c[side][d];
+        const double zeta = side == 0 ? g.zeta : g.zetb;
+        c[side][d] = l + 1;
+        double v = 2.0 * zeta * pair_integral(s, c[0], c[1]);
+        if (l > 0) {
+            c[side][d] = l - 1;
+            v -= l * pair_integral(s, c[0], c[1]);
         }
+        gc += P * v;
+        c[side][d] = l + 2;
+        const double q = P * pair_integral(s, c[0], c[1]);
+        gz[0] -= side == 0 ? q : 0.0;
+        gz[1] -= side == 0 ? 0.0 : q;
     }
-    // block reduction of the eight gradients
-    const int lane = tid & 31, warp = tid >> 5;
+    // block reduction: the warps' three sums, then the eight gradients
+    double r3[3] = {gc, gz[0], gz[1]};
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-        double v = grad[k];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) s.red[k][warp] = v;
+    for (int k = 0; k < 3; k++) {
+        for (int o = 16; o > 0; o >>= 1) r3[k] += __shfl_xor_sync(0xffffffffu, r3[k], o);
+        if (lane == 0) s.red[k][warp] = r3[k];
     }
     __syncthreads();
     if (tid < 8) {
         double v = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) v += s.red[tid][w];
+        if (tid < 6) {  // dRa, dRb: the two halves of (axis, centre)
+            v = s.red[0][tid] + s.red[0][tid + 6];
+        } else {
+            for (int w = 0; w < kBWarps; w++) v += s.red[tid - 5][w];
+        }
         v *= g.prefactor;
         const int64_t t = g.task;
         if (tid < 3) {
@@ -169,15 +173,18 @@ k_backward_epilogue(const PairGeom *__restrict__ geoms, const LevelDev *__restri
     }
 }
 
+// orthorhombic moments go to degree lp + 2 <= kMaxLpB; general cells map them through
+// the lattice transform, which is built to degree kMaxLp
+bool backward_supported(const TaskSet &ts) {
+    for (int64_t k = ts.gen_first; k < ts.gen_first + ts.gen_count; k++)
+        if (ts.h_geom[k].lp + 2 > kMaxLp) return false;
+    return ts.max_lp + 2 <= kMaxLpB;
+}
+
 cudaError_t launch_backward(const TaskSet &ts, const double *d_pab, const GridPtrs &g, double *d_hab,
                             double *d_dra, double *d_drb, double *d_dza, double *d_dzb, cudaStream_t s) {
-    (void)d_hab;
     if (ts.ntasks == 0) return cudaSuccess;
-    // orthorhombic moments go to degree lp + 2 <= kMaxLpB; general cells map them
-    // through the lattice transform, which is built to degree kMaxLp
-    for (int64_t k = ts.gen_first; k < ts.gen_first + ts.gen_count; k++)
-        if (ts.h_geom[k].lp + 2 > kMaxLp) return cudaErrorNotSupported;
-    if (ts.max_lp + 2 > kMaxLpB) return cudaErrorNotSupported;
+    if (!backward_supported(ts)) return cudaErrorNotSupported;
     TaskSet &mts = const_cast<TaskSet &>(ts);
     if (!mts.d_mom_ext) {
         cudaError_t e = cudaMalloc(&mts.d_mom_ext, sizeof(double) * std::max<int64_t>(ts.mom_ext_len, 1));
@@ -185,8 +192,10 @@ cudaError_t launch_backward(const TaskSet &ts, const double *d_pab, const GridPt
     }
     cudaError_t e = launch_moments_fp64(ts, g, 2, mts.d_mom_ext, s);
     if (e != cudaSuccess) return e;
+    // the matrix elements come from the same moments (those to degree lp)
+    if (d_hab && (e = launch_backtransform(ts, mts.d_mom_ext, 2, d_hab, s)) != cudaSuccess) return e;
     ts.n_kernels++;
-    k_backward_epilogue<<<(unsigned)ts.ntasks, 128, 0, s>>>(ts.d_geom, ts.plan->d_levels, ts.plan->d_tmat,
+    k_backward_epilogue<<<(unsigned)ts.ntasks, 32 * kBWarps, 0, s>>>(ts.d_geom, ts.plan->d_levels, ts.plan->d_tmat,
                                                            mts.d_mom_ext, ts.tau, d_pab, d_dra, d_drb, d_dza,
                                                            d_dzb);
     return cudaGetLastError();

@@ -659,7 +659,7 @@ int gpw_integrate(gpw_taskset *ts, int precision, double *const *d_grids, double
     } else {
         return fail(GPW_ERR_INVALID_ARG, "gpw_integrate: unknown precision");
     }
-    GPW_CUDA(launch_backtransform(*ts, ts->d_mom, d_hab, s));
+    GPW_CUDA(launch_backtransform(*ts, ts->d_mom, 0, d_hab, s));
     return GPW_SUCCESS;
 }
 
@@ -668,11 +668,12 @@ int gpw_backward(gpw_taskset *ts, const double *d_pab, double *const *d_grids, d
     if (!ts || !d_grids || (ts->ntasks > 0 && !d_pab)) return fail(GPW_ERR_INVALID_ARG, "gpw_backward: null argument");
     cudaStream_t s = (cudaStream_t)stream;
     GridPtrs g = grid_ptrs(*ts->plan, d_grids);
-    if (d_hab) {
+    const bool grads = d_dra || d_drb || d_dzeta || d_dzetb;
+    if (d_hab && !(grads && backward_supported(*ts))) {
         int st = gpw_integrate(ts, GPW_PREC_FP64, d_grids, d_hab, stream);
         if (st) return st;
     }
-    if (d_dra || d_drb || d_dzeta || d_dzetb) {
+    if (grads) {
         cudaError_t e = launch_backward(*ts, d_pab, g, d_hab, d_dra, d_drb, d_dzeta, d_dzetb, s);
         if (e == cudaErrorNotSupported) return fail(GPW_ERR_UNSUPPORTED, "gpw_backward: not available");
         if (e != cudaSuccess) return cuda_fail(e, "gpw_backward");

@@ -263,11 +263,12 @@ __device__ inline void forward_coef(CoefWs &w, const PairGeom &g, double *out) {
 // the derivative functions)
 constexpr int kNcoLocal = ((kMaxL + 2) * (kMaxL + 3) * (kMaxL + 4)) / 6;
 
-// Adjoint: given moments W (packed like c), accumulate into hab.  Only the
+// Adjoint: given moments W (packed like c, or to a higher degree lpw), accumulate
+// into hab.  Only the
 // entries the next stage reads are formed: X^T reads T1[(lya,lza)][(lyb,lzb)][lx]
 // for lx <= lxa + lxb <= (A-lya-lza) + (B-lyb-lzb), so Y^T reads T2[lza][lzb][ly][lx]
 // only for lx + ly <= (A-lza) + (B-lzb).
-__device__ inline void adjoint_coef(CoefWs &w, const PairGeom &g, int func, const double *W,
+__device__ inline void adjoint_coef(CoefWs &w, const PairGeom &g, int func, const double *W, int lpw,
                                     double *hab) {
     const CoefDims &d = w.d;
     const int L = d.L, lp = g.lp;
@@ -287,7 +288,7 @@ __device__ inline void adjoint_coef(CoefWs &w, const PairGeom &g, int func, cons
         if (lx + ly > d.A + d.B - lza - lzb) continue;
         double s = 0.0;
         for (int lz = 0; lz <= lza + lzb && lz + ly + lx <= lp; lz++)
-            s += w.AL(2, lza, lzb, lz) * W[pidx(lp, lz, ly, lx)];
+            s += w.AL(2, lza, lzb, lz) * W[pidx(lpw, lz, ly, lx)];
         w.T2[t] = s;
     }
     __syncthreads();

@@ -73,17 +73,19 @@ int smem_prep(int A, int B) {
 }
 
 // ---------------------------------------------------------------------------
-// integrate back-transform: moments -> hab
+// integrate back-transform: moments -> hab.  extra: the moments go to degree lp + extra
+// (the backward pass's; those beyond lp are not read).
 __global__ void k_backtransform(const PairGeom *__restrict__ geoms, const LevelDev *__restrict__ levels,
                                 const double *__restrict__ tmat, int tau,
-                                const double *__restrict__ mom, double *__restrict__ hab) {
+                                const double *__restrict__ mom, int extra, double *__restrict__ hab) {
     extern __shared__ double sm[];
     const PairGeom &g = geoms[blockIdx.x];  // read in place (L1), not copied per thread
     CoefWs w;
     w.carve(sm, g.la_max, g.lb_max);
     fill_alpha(w, g);
     const int nc = ncoef(g.lp);
-    const double *W = mom + g.coef_off;
+    const double *W = mom + (extra ? g.mom_ext_off : g.coef_off);
+    int lpw = g.lp + extra;
     double *Wc = w.end();
     if (!g.ortho) {
         // Wc[lz][ly][lx] = sum over same-degree (k,j,i) of T[(k,j,i)][(lz,ly,lx)] * Wq[k][j][i]
@@ -110,14 +112,15 @@ __global__ void k_backtransform(const PairGeom *__restrict__ geoms, const LevelD
             for (int k = 0; k <= n; k++)
                 for (int j = 0; j <= n - k; j++) {
                     const int i = n - k - j;
-                    s += Tm[(int64_t)pidx(kMaxLp, k, j, i) * NT + col] * W[pidx(g.lp, k, j, i)];
+                    s += Tm[(int64_t)pidx(kMaxLp, k, j, i) * NT + col] * W[pidx(lpw, k, j, i)];
                 }
             Wc[t] = s;
         }
         W = Wc;
+        lpw = g.lp;
     }
     __syncthreads();
-    adjoint_coef(w, g, tau, W, hab);
+    adjoint_coef(w, g, tau, W, lpw, hab);
 }
 
 // ---------------------------------------------------------------------------
@@ -922,13 +925,13 @@ cudaError_t launch_integrate_fp64(const TaskSet &ts, const GridPtrs &g, cudaStre
     return launch_fp64_impl(ts, g, true, 0, ts.d_mom, s);
 }
 
-cudaError_t launch_backtransform(const TaskSet &ts, const double *d_mom, double *d_hab,
+cudaError_t launch_backtransform(const TaskSet &ts, const double *d_mom, int extra, double *d_hab,
                                  cudaStream_t s) {
     if (ts.ntasks == 0) return cudaSuccess;
     const int smem = smem_prep(ts.max_A, ts.max_B);
     ts.n_kernels++;
     k_backtransform<<<(unsigned)ts.ntasks, 128, smem, s>>>(ts.d_geom, ts.plan->d_levels,
-                                                           ts.plan->d_tmat, ts.tau, d_mom, d_hab);
+                                                           ts.plan->d_tmat, ts.tau, d_mom, extra, d_hab);
     return cudaGetLastError();
 }
 

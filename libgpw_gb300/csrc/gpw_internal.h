@@ -89,7 +89,7 @@ struct ProfScope {
 cudaError_t launch_prep(const TaskSet &ts, const double *d_pab, cudaStream_t s);
 cudaError_t launch_collocate_fp64(const TaskSet &ts, const GridPtrs &g, cudaStream_t s);
 cudaError_t launch_integrate_fp64(const TaskSet &ts, const GridPtrs &g, cudaStream_t s);
-cudaError_t launch_backtransform(const TaskSet &ts, const double *d_mom, double *d_hab,
+cudaError_t launch_backtransform(const TaskSet &ts, const double *d_mom, int extra, double *d_hab,
                                  cudaStream_t s);
 void fp64_items(TaskSet &ts, int sms, int smem_limit, std::vector<Fp64Item> &items);
 int smem_ortho_fp64(const PairGeom &g);
@@ -137,7 +137,8 @@ cudaError_t launch_one_fp64(const PairGeom &g, const PairGeom *d_geom, const Lev
 int tc_selftest(int64_t *mismatches, std::string &err);
 int ffexp_selftest(int64_t n, double *err_normal, double *err_low, std::string &err);
 
-// gpw_backward.cu
+// gpw_backward.cu: gradients and, when d_hab is given, the matrix elements
+bool backward_supported(const TaskSet &ts);
 cudaError_t launch_backward(const TaskSet &ts, const double *d_pab, const GridPtrs &g,
                             double *d_hab, double *d_dra, double *d_drb, double *d_dza,
                             double *d_dzb, cudaStream_t s);
