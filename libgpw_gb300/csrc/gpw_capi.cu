@@ -550,6 +550,7 @@ int gpw_taskset_create(gpw_plan *plan, const gpw_task *tasks, int64_t ntasks, in
     std::vector<Fp64Item> items;
     fp64_items(*T, sms, smem_limit, items);
     // general-cell pairs (sorted after the orthorhombic ones) for the float-float kernel
+    int gen_limit = 0;
     for (int64_t m = 0; m < ntasks; m++) {
         if (T->h_geom[m].ortho) continue;
         if (T->gen_count == 0) {
@@ -558,8 +559,9 @@ int gpw_taskset_create(gpw_plan *plan, const gpw_task *tasks, int64_t ntasks, in
         }
         T->gen_count++;
         T->gen_smem = std::max(T->gen_smem, smem_general_ff(T->h_geom[m]));
+        gen_limit = std::max(gen_limit, smem_general_ff_limit(T->h_geom[m]));
     }
-    if (T->gen_smem > smem_limit) {
+    if (std::max(T->gen_smem, gen_limit) > smem_limit) {
         delete T;
         return fail(GPW_ERR_UNSUPPORTED, "gpw_taskset_create: a general-cell cube is too large for one CTA");
     }

@@ -184,6 +184,57 @@ GPW_HD bool general_row(const double dh[3][3], const double gp[3], double dj, do
     return true;
 }
 
+#if defined(__CUDACC__)
+// general_row with an FP32 fast path in box-relative units i' = i - cc0 with a running
+// error bound; the exact FP64 rule decides where a root lies within its bound of an
+// integer or the discriminant within its bound of zero.
+struct GeneralRow32 {
+    float dh[3][3];   // lattice steps
+    float a, inv2a;   // |v0|^2 and 1 / (2 |v0|^2)
+};
+__device__ __forceinline__ bool general_row_fast32(const GeneralRow32 &G, float gi, float gj, float gk, float dj,
+                                                   float dk, float r2, int cc0, int &ismin, int &ismax, bool &unsure) {
+    const float eps = 1.2e-7f;  // 2^-23, with room
+    float b = 0.0f, c = 0.0f, eb = 0.0f, ec = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        // v_i = dk dh2_i + dj dh1_i - gi dh0_i (box-relative), with its error bound
+        const float v = __fsub_rn(__fadd_rn(__fmul_rn(G.dh[2][i], dk), __fmul_rn(G.dh[1][i], dj)),
+                                  __fmul_rn(gi, G.dh[0][i]));
+        const float ev = eps * (fabsf(G.dh[2][i]) * (2.0f * fabsf(dk) + fabsf(gk)) +
+                                fabsf(G.dh[1][i]) * (2.0f * fabsf(dj) + fabsf(gj)) +
+                                2.0f * fabsf(gi * G.dh[0][i]) + 2.0f * fabsf(v));
+        b = __fadd_rn(b, __fmul_rn(2.0f * v, G.dh[0][i]));
+        c = __fadd_rn(c, __fmul_rn(v, v));
+        eb += 2.0f * ev * fabsf(G.dh[0][i]) + 2.0f * eps * fabsf(b);
+        ec += (2.0f * fabsf(v) + ev) * ev + 2.0f * eps * c;
+    }
+    // d = b^2 - 4a(c - r^2): propagated input errors, the representation errors of
+    // a and r^2, and the rounding of each operation
+    const float a = G.a;
+    const float cr = __fsub_rn(c, r2);
+    const float d = __fsub_rn(__fmul_rn(b, b), __fmul_rn(4.0f * a, cr));
+    const float ed = 2.0f * fabsf(b) * eb + eb * eb + eps * b * b +
+                     4.0f * a * (ec + eps * r2 + 2.5f * eps * fabsf(cr)) + eps * fabsf(d);
+    unsure = fabsf(d) <= 1.5f * ed;
+    if (!unsure && d < 0.0f) return false;  // surely empty
+    if (!unsure) {
+        const float sd = sqrtf(d);
+        const float esd = 1.8f * ed / sd + eps * sd;  // d > 1.5 ed: sqrt(d - ed) >= sd / sqrt(3)
+        const float lo = __fmul_rn(__fsub_rn(-b, sd), G.inv2a), hi = __fmul_rn(__fadd_rn(-b, sd), G.inv2a);
+        const float er = 1.25f * ((eb + esd + eps * (fabsf(b) + sd)) * G.inv2a + 1.5f * eps * (fabsf(lo) + fabsf(hi))) +
+                         1e-6f;
+        unsure = fabsf(lo - rintf(lo)) <= er || fabsf(hi - rintf(hi)) <= er;
+        ismin = cc0 + (int)ceilf(lo);
+        ismax = cc0 + (int)floorf(hi);
+    }
+    return true;
+}
+__device__ __noinline__ inline bool general_row_exact64(const double dh[3][3], const double gp[3], double dj, double dk,
+                                                        double radius, int &ismin, int &ismax) {
+    return general_row(dh, gp, dj, dk, radius, ismin, ismax);
+}
+#endif
 
 // ---------------------------------------------------------------------------
 // Per-level constants on the device.

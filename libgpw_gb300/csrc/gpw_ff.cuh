@@ -16,6 +16,36 @@ struct alignas(8) ff {
 
 __device__ __forceinline__ ff ff_make(float a) { return {a, 0.0f}; }
 
+// The same split on the integer pipe (a conversion costs as much as an FP64 multiply-add
+// here, 17 cycles a warp and SM): the 23 leading mantissa bits rounded to nearest, then
+// the signed 29-bit rest.  Values whose low part would leave the normal range of float
+// (below 2^-70, zero among them; above 2^126; infinities, NaN) take ff_from_double.
+__device__ __forceinline__ ff ff_from_double_bits(double d) {
+    const int hw = __double2hiint(d);
+    const unsigned lw = (unsigned)__double2loint(d);
+    const int e = (hw >> 20) & 0x7ff;  // biased by 1023
+    if ((unsigned)(e - (1023 - 70)) > 196u) return {__double2float_rn(d), __double2float_rn(d - (double)__double2float_rn(d))};
+    const int up = (int)(lw >> 28) & 1;                   // the rest is half a unit or more
+    const int rest = (int)(lw & 0x1fffffffu) - (up << 29);
+    const int fb = ((e - 896) << 23 | (hw & 0xfffff) << 3 | (int)(lw >> 29)) + up;
+    const float sg = __int_as_float((hw & 0x80000000) | (e - 1023 - 52 + 127) << 23);  // +- 2^(e - 52)
+    return {__int_as_float((hw & 0x80000000) | fb), __fmul_rn((float)rest, sg)};
+}
+// hi + lo (|lo| <= ulp(hi) / 2) as a double, rounded to nearest (ties to even of the low
+// part's scale), on the integer pipe; hi below 2^-70 or beyond float's range takes the
+// FP64 addition.
+__device__ __forceinline__ double ff_to_double_bits(ff a) {
+    const int h = __float_as_int(a.hi), e = (h >> 23) & 0xff;  // biased by 127
+    if ((unsigned)(e - (127 - 70)) > 196u) return (double)a.hi + (double)a.lo;
+    // the low part in units of hi's 2^-52, away from hi's sign: |r| <= 2^28; one binade
+    // down where hi is a power of two and the low part takes away from it
+    const float u = __int_as_float((h & 0x80000000) | (52 + 127 - (e - 127)) << 23);  // +- 2^(52 - e)
+    float r = __fmul_rn(a.lo, u);
+    if ((h & 0x7fffff) == 0 && r < 0.0f) r = __fadd_rn(r, r);
+    const long long bits = ((long long)(e - 127 + 1023) << 52 | (long long)(h & 0x7fffff) << 29) + (long long)__float2int_rn(r);
+    return __hiloint2double((int)(bits >> 32) | (h & 0x80000000), (int)bits);
+}
+
 __device__ __forceinline__ ff ff_from_double(double d) {
     const float h = __double2float_rn(d);
     return {h, __double2float_rn(d - (double)h)};
@@ -147,6 +177,10 @@ __device__ __forceinline__ void ff2_acc_lazy(ff2 &s, ff2 a, ff2n b) {
     s.lo = f2_add(s.lo, f2_sub(t.lo, q.lo));
 }
 
+__device__ __forceinline__ ff2n ff2n_of(ff2 b) {
+    return {b.hi, f2_mul(b.hi, f2(-1.0f)), f2_mul(b.lo, f2(-1.0f))};
+}
+
 // 2^(j/32), j = 0..31, as float-float (hi = the float nearest, lo = the rest)
 __constant__ float2 c_exp2_32[32] = {
     {1.0f, 0.0f},
@@ -208,6 +242,32 @@ __device__ __forceinline__ ff ff_exp(ff a) {
     const int m = k >> 5, m1 = m >> 1, m2 = m - m1;
     const float s1 = __int_as_float((127 + m1) << 23), s2 = __int_as_float((127 + m2) << 23);
     return {__fmul_rn(__fmul_rn(p.hi, s1), s2), __fmul_rn(__fmul_rn(p.lo, s1), s2)};
+}
+
+// Two exponentials at once, ff_exp operation by operation.  tab: c_exp2_32 in shared
+// memory (the lanes' indices differ: a constant-bank read would be replayed per value).
+__device__ __forceinline__ ff2 ff2_exp(ff2 a, const float2 *tab) {
+    const float2 ah = make_float2(fmaxf(a.hi.x, -104.0f), fmaxf(a.hi.y, -104.0f));
+    const float2 km = f2_add(f2_mul(ah, f2(46.16624069213867f)), f2(12582912.0f));  // 1.5 * 2^23 + k
+    const float2 nk = f2_sub(f2(12582912.0f), km);                                  // -k
+    const int k0 = __float_as_int(km.x) - 0x4b400000, k1 = __float_as_int(km.y) - 0x4b400000;
+    ff2 r = two_sum2(f2_fma(nk, f2(0.02166748046875f), ah), a.lo);
+    const ff2n c = ff2n_dup(ff{-6.631076303165173e-06f, 5.14560928046269e-14f});
+    const float2 cp = f2_mul(nk, c.hi);
+    const float2 cn = f2_fma(nk, c.nlo, f2_fma(nk, c.nhi, cp));  // the product's error terms, negated
+    r = ff2_add(r, fast_two_sum2(cp, f2_mul(cn, f2(-1.0f))));
+    const float2 q = r.hi;
+    const float2 t = f2_mul(q, f2_fma(q, f2_fma(q, f2(0.008333333767950535f), f2(0.0416666679084301f)), f2(0.1666666716337204f)));
+    const ff2 h = fast_two_sum2(f2(0.5f), t);
+    const ff2n rn = ff2n_of(r);
+    ff2 p = ff2_add(ff2_add(ff2{f2(1.0f), f2(0.0f)}, r), ff2_mul(h, ff2n_of(ff2_mul(r, rn))));
+    const float2 t0 = tab[k0 & 31], t1 = tab[k1 & 31];
+    p = ff2_mul(p, ff2n_of(ff2{make_float2(t0.x, t1.x), make_float2(t0.y, t1.y)}));
+    auto pw = [](int m) { return __int_as_float((127 + m) << 23); };
+    const int m0 = k0 >> 5, m1 = k1 >> 5, u0 = m0 >> 1, u1 = m1 >> 1;
+    const float2 s1 = make_float2(a.hi.x < -103.0f ? 0.0f : pw(u0), a.hi.y < -103.0f ? 0.0f : pw(u1));
+    const float2 s2 = make_float2(pw(m0 - u0), pw(m1 - u1));
+    return {f2_mul(f2_mul(p.hi, s1), s2), f2_mul(f2_mul(p.lo, s1), s2)};
 }
 
 }  // namespace gpw

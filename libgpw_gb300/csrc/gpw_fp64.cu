@@ -145,8 +145,8 @@ __global__ void k_backtransform(const PairGeom *__restrict__ geoms, const LevelD
 // The form before it (one CTA per pair, three barriers per plane, a shuffle
 // reduction of 11 accumulators per row, launches of similar pairs one after the
 // other) took 21.1 ms to integrate and 6.1 ms to collocate 1000 pairs (l <= 2,
-// 64^3); this one takes 0.49 and 0.46 ms, 58 % and 61 % of the FP64 rate (1.10
-// TFLOP/s in a GEMM) counting L multiply-adds per cube point.
+// 64^3); this one takes 0.46 and 0.46 ms, 62 % of the FP64 rate (1.10 TFLOP/s in a
+// GEMM) counting L multiply-adds per cube point.
 constexpr int kOrthoWarps = 4;
 
 // the shared memory of orthorhombic item (pair g, 1 of nparts), in bytes
@@ -164,6 +164,14 @@ int smem_ortho_fp64(const PairGeom &g) {
     const int L = g.lp + 1;
     const int nx = g.hi[0] - g.lb[0] + 1, ny = g.hi[1] - g.lb[1] + 1, nz = g.hi[2] - g.lb[2] + 1;
     return 8 * (L * L * L + L * (nx + ny + nz) + L * L + ny * L) + 8 * ny;
+}
+
+// the item's next plane, taken warp by warp (planes differ in size: the middle ones hold
+// most of a sphere's points)
+__device__ __forceinline__ int next_plane(int *counter) {
+    int p = 0;
+    if ((threadIdx.x & 31) == 0) p = atomicAdd(counter, 1);
+    return __shfl_sync(0xffffffffu, p, 0);
 }
 
 // kAcc: the registers of T, L <= kAcc (kNPow, or kNPowB for the backward pass's
@@ -243,10 +251,14 @@ k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
 #pragma unroll
     for (int m = 0; m < (kAdj ? kMC : 1); m++) W[m] = 0.0;
     const SphereRule rule(g.radius, lv.dh[0][0], lv.dh[1][1], lv.dh[2][2]);
+    __shared__ int s_next;
+    if (tid == 0) s_next = 0;
     const int *T0 = g.table_off >= 0 ? table + g.table_off : nullptr;
     const int gn0 = lv.ngrid[0], gn1 = lv.ngrid[1];
     __syncthreads();
-    for (int pl = warp; pl < np; pl += kOrthoWarps) {
+    // integrate's CTAs end with a sum over the warps: planes taken as warps come free (485
+    // -> 455 us on the workload above; collocate, whose warps end alone, loses 1 %)
+    for (int pl = kAdj ? next_plane(&s_next) : warp; pl < np; pl = kAdj ? next_plane(&s_next) : pl + kOrthoWarps) {
         const int kg = kgmin + it.part + pl * it.nparts, kf = fold(kg);
         const int k = axis_index(lv.periodic[2], g.cc[2], kg, g.lb[2], lv.lb_grid[2], lv.npts[2], lv.ngrid[2]);
         if (k < 0) {
@@ -561,178 +573,312 @@ k_general_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ 
 
 
 // ---------------------------------------------------------------------------
-// General cell in float-float (the mixed path): the structure of k_general_fp64
-// -- one CTA per pair, the lattice-basis polynomial contracted over k, then j,
-// per row of the index box, the row's i-range from the reference's quadratic
-// (FP64, general_row, so the point set is the reference's) -- with every
-// per-point operation in float-float instead of FP64 (GB300 runs FP64 at ~1/64
-// of its FP32 rate):
-//   r^2(di) = G00 di^2 + A1 di + A0 per row (metric G = dh dh^T; A1, A0 per row
-//   in FP64, split to float-float), exp(-zetp r^2) by ff_exp, the polynomial in
-//   di by Horner; collocate adds hi + lo to the grid with FP64 atomics,
-//   integrate reduces V exp(..) di^n over each row with warp shuffles.
+// General cell in float-float (the mixed path).  The value at a point of the index
+// box is P(di, dj, dk) exp(-zetp r^2), r^2 = G00 di^2 + A1 di + A0 along a row (metric
+// G = dh dh^T; A1, A0 per row in FP64, split to float-float); the row's i-range is the
+// reference's quadratic (general_row_checked), so the point set is the reference's.
+//
+// As k_ortho_fp64: a CTA (4 warps) takes an item, a warp a plane, 64 rows at a time, a
+// lane a column i (blocks of 32, 16 or 8 columns):
+//   collocate  T[j] = sum_i Qjk[j][i] di^i once per column, then Horner in dj per point;
+//   integrate  T[j] += V E dj^j per point, lane-local; then over the columns and dk once
+//              per 64 rows and plane (T through shared memory).
+// Two rows share each instruction (packed float-float), and what meets FP64 (the grid's
+// values) is converted on the integer pipe: the FP64 pipe takes 17 cycles per
+// instruction, conversions included.  (One warp per row, points one at a time, shuffle
+// reductions per row and conversions on the FP64 pipe: 6.84 ms to integrate and 3.86 ms
+// to collocate 1500 pairs, l <= 4, 128^3; this form 4.20 and 3.66 ms.)  128 registers
+// for four CTAs per SM: with 232 (two CTAs) 5.52 and 4.53 ms, the chains being long.
+constexpr int kGenRows = 64;  // rows of a plane in hand
+
+// a warp's working set (floats): row data, Qjk; integrate: T of the block's columns
+__host__ __device__ constexpr int general_ff_warp_bytes(int L) {
+    return kGenRows * (4 * 4 + 3 * 4) + 8 * nshell(L - 1) + 8 * 33 * L;
+}
+// its static part in front (per CTA): coefficients or moments, per-row powers base and
+// grid row, the decode table
+static int general_ff_cta_bytes(const PairGeom &g) {
+    const int ny = g.hi[1] - g.cc[1] + 2;  // one row of margin: a geometry update moves a box's extent by at most one
+    return 8 * ncoef(g.lp) + 4 * ncoef(g.lp) + 16 * (ny + 2) + 16 + 256;
+}
+
+__device__ __forceinline__ float2 ld2(const float *p) { return *reinterpret_cast<const float2 *>(p); }
+
 __device__ __forceinline__ ff ff_shfl_xor(ff v, int o) {
     return {__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
 }
 
 template <bool kAdj>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(32 * kOrthoWarps, 4)
 k_general_ff(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ items, int uparts,
-             const LevelDev *__restrict__ levels,
-             const double *__restrict__ coef, double *__restrict__ mom, GridPtrs grids, int *status) {
+             const LevelDev *__restrict__ levels, const double *__restrict__ coef, double *__restrict__ mom,
+             GridPtrs grids, int *status) {
     extern __shared__ double smd[];
+    constexpr int kM2 = (kNPow * (kNPow + 1) / 2 + 31) / 32, kMC = ((kMaxLp + 1) * (kMaxLp + 2) * (kMaxLp + 3) / 6 + 31) / 32;
     const Fp64Item it = items ? items[blockIdx.x] : Fp64Item{(int)blockIdx.x / uparts, (int)blockIdx.x % uparts, uparts};
-    const PairGeom g = geoms[it.pair];
+    const PairGeom &g = geoms[it.pair];
     const LevelDev &lv = levels[g.level];
     double *__restrict__ grid = grids.p[g.level];
-    const int lp = g.lp, L = lp + 1;
-    const int ny = g.hi[1] - g.cc[1] + 1;
-    ff *Q = reinterpret_cast<ff *>(smd);  // [k][j][i] dense
-    ff *Qjk = Q + L * L * L;              // [j][i]
-    ff *Qj = Qjk + L * L;                 // [row][i]
-    ff *rc = Qj + ny * L;                 // per row: a1, a0, d0 (r^2 along the row, first di)
-    ff *powj = rc + 3 * ny;               // integrate: per row dj^j, j <= lp
-    int *rows = reinterpret_cast<int *>(powj + ny * L);  // ismin, ismax, jidx
-    const int tid = threadIdx.x, nthr = blockDim.x;
-    const int lane = tid & 31, warp = tid >> 5, nwarp = nthr >> 5;
-    for (int t = tid; t < L * L * L; t += nthr) {
-        const int i = t % L, j = (t / L) % L, k = t / (L * L);
-        Q[t] = (!kAdj && i + j + k <= lp) ? ff_from_double(coef[g.coef_off + pidx(lp, k, j, i)]) : ff{0.0f, 0.0f};
-    }
-    // metric of the lattice steps
-    double G[3][3];
-    for (int a = 0; a < 3; a++)
-        for (int b = 0; b < 3; b++) G[a][b] = lv.dh[a][0] * lv.dh[b][0] + lv.dh[a][1] * lv.dh[b][1] + lv.dh[a][2] * lv.dh[b][2];
-    const ff g00 = ff_from_double(G[0][0]);
-    const ff mz = ff_from_double(-g.zetp);
-    __syncthreads();
+    const int lp = g.lp, L = lp + 1, nc = ncoef(lp), n2 = nshell(lp);
+    const int cc0 = g.cc[0], cc1 = g.cc[1], cc2 = g.cc[2];
+    const int ny = g.hi[1] - cc1 + 1, ny2 = (ny + 1) & ~1;  // rows come in pairs
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // shared memory: per CTA, then per warp
+    ff *Q = reinterpret_cast<ff *>(smd);              // packed (k, j, i): coefficients, or the CTA's moments
+    float2 *exptab = reinterpret_cast<float2 *>(Q + nc);
+    float *djh = reinterpret_cast<float *>(exptab + 32), *djn = djh + ny2, *djl = djn + ny2;  // dj, -dj.hi, -dj.lo
+    int *jrow = reinterpret_cast<int *>(djl + ny2);   // grid row of the box row, -1 outside the window
+    int *dec = jrow + ny2;                            // packed (k, j, i) -> k | (j, i) << 8
+    float *wbase = reinterpret_cast<float *>(dec + ((nc + 1) & ~1));
+    float *ws = wbase + warp * (general_ff_warp_bytes(L) / 4);
+    float *a1h = ws, *a1l = a1h + kGenRows, *a0h = a1l + kGenRows, *a0l = a0h + kGenRows;
+    int *i0 = reinterpret_cast<int *>(a0l + kGenRows), *i1 = i0 + kGenRows;
+    ff *sC = reinterpret_cast<ff *>(i1 + 2 * kGenRows);  // Qjk, packed (j, i)
+    ff *sT = sC + n2;                                    // [j][lane], rows of 33
+    __shared__ int s_next;
+    if (tid == 0) s_next = 0;
+    if (tid < 32) exptab[tid] = c_exp2_32[tid];
     int off[3];
     for (int d = 0; d < 3; d++) off[d] = imod(g.cc[d] + lv.lb_grid[d], lv.npts[d]);
-    for (int kk = g.cc[2] + it.part; kk <= g.hi[2]; kk += it.nparts) {
+    for (int r = tid; r < ny2; r += 32 * kOrthoWarps) {
+        const ff dj = ff_from_double(rsub((double)(cc1 + r), g.off[1]));
+        djh[r] = dj.hi;
+        djn[r] = -dj.hi;
+        djl[r] = -dj.lo;
+        const int j = lv.periodic[1] ? imod(cc1 + r, lv.npts[1]) : r + off[1];
+        jrow[r] = j < lv.ngrid[1] ? j : -1;
+    }
+    for (int t = tid; t < nc; t += 32 * kOrthoWarps) {
+        Q[t] = kAdj ? ff{0.0f, 0.0f} : ff_from_double(coef[g.coef_off + t]);
+        int k = 0, j = 0, r = t;
+        while (r >= nshell(lp - k)) r -= nshell(lp - k++);
+        while (r > lp - k - j) r -= lp - k - j++ + 1;
+        dec[t] = k | ((j * L - (j * (j - 1)) / 2 + r) << 8);
+    }
+    // this lane's (j, i) entries of Qjk; with n2 <= 16 of them, 2^lg lanes share one
+    int lg = 0;
+    if (kAdj)
+        while ((n2 << (lg + 1)) <= 32) lg++;
+    int oj[kM2], oi[kM2];
+#pragma unroll
+    for (int m = 0; m < kM2; m++) {
+        const int o = (lane >> lg) + 32 * m;
+        int j = 0, r = o;
+        while (j < L && r > lp - j) r -= lp - j++ + 1;
+        oj[m] = o < n2 ? j : -1;
+        oi[m] = r;
+    }
+    ff W[kAdj ? kMC : 1];
+#pragma unroll
+    for (int m = 0; m < (kAdj ? kMC : 1); m++) W[m] = ff{0.0f, 0.0f};
+    // metric of the lattice steps
+    auto met = [&](int a, int b) { return lv.dh[a][0] * lv.dh[b][0] + lv.dh[a][1] * lv.dh[b][1] + lv.dh[a][2] * lv.dh[b][2]; };
+    const double G01 = met(0, 1), G02 = met(0, 2), G11 = met(1, 1), G12 = met(1, 2), G22 = met(2, 2);
+    const ff g00 = ff_from_double(met(0, 0));
+    GeneralRow32 R32;
+    for (int a = 0; a < 3; a++)
+        for (int b = 0; b < 3; b++) R32.dh[a][b] = (float)lv.dh[a][b];
+    R32.a = (float)met(0, 0);
+    R32.inv2a = (float)(0.5 / met(0, 0));
+    const float gi = (float)(g.off[0] - (double)cc0), gj = (float)(g.off[1] - (double)cc1), gk = (float)(g.off[2] - (double)cc2);
+    const float r2f = (float)(g.radius * g.radius);
+    const ff2n mz = ff2n_dup(ff_from_double(-g.zetp));
+    const int gn0 = lv.ngrid[0], gn1 = lv.ngrid[1], np0 = lv.npts[0], per0 = lv.periodic[0];
+    __syncthreads();
+    for (;;) {
+        const int kk = cc2 + it.part + next_plane(&s_next) * it.nparts;
+        if (kk > g.hi[2]) break;
         const double dk = rsub((double)kk, g.off[2]);
-        const int kidx = lv.periodic[2] ? imod(kk, lv.npts[2]) : kk - g.cc[2] + off[2];
+        const int kidx = lv.periodic[2] ? imod(kk, lv.npts[2]) : kk - cc2 + off[2];
         if (kidx < 0 || kidx >= lv.ngrid[2]) {
-            if (tid == 0) atomicOr(status, kStatOutOfWindow);
+            if (lane == 0) atomicOr(status, kStatOutOfWindow);
             continue;
         }
         const ff dkf = ff_from_double(dk);
-        if (!kAdj) {
-            for (int t = tid; t < L * L; t += nthr) {
-                const int i = t % L, j = t / L;
-                ff s = {0.0f, 0.0f};
-                for (int k = lp - i - j; k >= 0; k--) s = ff_fma(s, dkf, Q[(k * L + j) * L + i]);
-                Qjk[t] = s;
-            }
-            __syncthreads();
-        }
-        // rows: the reference's i-range (FP64 quadratic), one row per lane
-        for (int row = tid; row < ny; row += nthr) {
-            const int jj = g.cc[1] + row;
-            const double dj = rsub((double)jj, g.off[1]);
-            int ismin = 0, ismax = -1;
-            if (!general_row(lv.dh, g.off, dj, dk, g.radius, ismin, ismax)) { ismin = 0; ismax = -1; }
-            rows[3 * row] = ismin;
-            rows[3 * row + 1] = ismax;
-            rows[3 * row + 2] = lv.periodic[1] ? imod(jj, lv.npts[1]) : jj - g.cc[1] + off[1];
-            // r^2 = G00 di^2 + A1 di + A0 along the row; di = (ismin - off0) + n
-            rc[3 * row] = ff_from_double(2.0 * (G[0][1] * dj + G[0][2] * dk));
-            rc[3 * row + 1] = ff_from_double(G[1][1] * dj * dj + 2.0 * G[1][2] * dj * dk + G[2][2] * dk * dk);
-            rc[3 * row + 2] = ff_from_double((double)ismin - g.off[0]);
-            if (kAdj) {
-                const ff djf = ff_from_double(dj);
-                ff p = {1.0f, 0.0f};
-                for (int j = 0; j <= lp; j++) {
-                    powj[row * L + j] = p;
-                    p = ff_mul(p, djf);
-                }
-            }
-        }
-        if (!kAdj) {
-            for (int t = tid; t < ny * L; t += nthr) {
-                const int row = t / L, i = t % L;
-                const ff djf = ff_from_double(rsub((double)(g.cc[1] + row), g.off[1]));
-                ff s = {0.0f, 0.0f};
-                for (int j = lp - i; j >= 0; j--) s = ff_fma(s, djf, Qjk[j * L + i]);
-                Qj[t] = s;
-            }
-        }
-        __syncthreads();
-        for (int row = warp; row < ny; row += nwarp) {
-            const int ismin = rows[3 * row], ismax = rows[3 * row + 1], jidx = rows[3 * row + 2];
-            if (ismax < ismin) continue;
-            if (jidx < 0 || jidx >= lv.ngrid[1]) {
-                if (lane == 0) atomicOr(status, kStatOutOfWindow);
-                continue;
-            }
-            const ff a1 = rc[3 * row], a0 = rc[3 * row + 1], d0 = rc[3 * row + 2];
-            const int64_t rowbase = ((int64_t)kidx * lv.ngrid[1] + jidx) * lv.ngrid[0];
-            ff acc[kNPow];
+        const float dkc = (float)(kk - cc2) - gk;
+        __syncwarp();
+        if (!kAdj) {  // Qjk[j][i] = sum_k Q[k][j][i] dk^k (Horner)
 #pragma unroll
-            for (int n = 0; n < kNPow; n++) acc[n] = ff{0.0f, 0.0f};
-            for (int ii = ismin + lane; ii <= ismax; ii += 32) {
-                const int iidx = lv.periodic[0] ? imod(ii, lv.npts[0]) : ii - g.cc[0] + off[0];
-                if (iidx < 0 || iidx >= lv.ngrid[0]) {
-                    atomicOr(status, kStatOutOfWindow);
-                    continue;
+            for (int m = 0; m < kM2; m++) {
+                if (oj[m] < 0) continue;
+                const int j = oj[m], i = oi[m], top = lp - i - j;
+                int base = nc;  // packed index of (k + 1, 0, 0)
+                for (int k = lp; k > top; k--) base -= nshell(lp - k);
+                ff s = {0.0f, 0.0f};
+                for (int k = top; k >= 0; k--) {
+                    const int q = lp - k;
+                    base -= nshell(q);
+                    s = ff_fma(s, dkf, Q[base + j * (q + 1) - (j * (j - 1)) / 2 + i]);
                 }
-                const ff di = ff_add(d0, ff{(float)(ii - ismin), 0.0f});
-                const ff r2 = ff_fma(ff_fma(g00, di, a1), di, a0);
-                const ff e = ff_exp(ff_mul(r2, mz));
-                if (!kAdj) {
-                    ff s = Qj[row * L + lp];
-                    for (int n = lp - 1; n >= 0; n--) s = ff_fma(s, di, Qj[row * L + n]);
-                    const ff v = ff_mul(s, e);
-                    atomicAdd(grid + rowbase + iidx, (double)v.hi + (double)v.lo);
-                } else {
-                    ff p = ff_mul(ff_from_double(grid[rowbase + iidx]), e);
+                sC[lane + 32 * m] = s;
+            }
+        }
+        ff cji[kAdj ? kM2 : 1];
 #pragma unroll
-                    for (int n = 0; n < kNPow; n++) {  // L is uniform over the CTA
-                        if (n >= L) break;
-                        acc[n] = ff_add(acc[n], p);
-                        p = ff_mul(p, di);
+        for (int m = 0; m < (kAdj ? kM2 : 1); m++) cji[m] = ff{0.0f, 0.0f};
+        for (int r0 = 0; r0 < ny; r0 += kGenRows) {
+            const int nr = min(kGenRows, ny - r0);
+            __syncwarp();
+            int imin = INT32_MAX, imax = INT32_MIN;
+            for (int r = lane; r < ((nr + 1) & ~1); r += 32) {
+                int ismin = 1, ismax = 0;
+                if (r < nr) {
+                    const int jj = cc1 + r0 + r;
+                    bool unsure;
+                    bool some = general_row_fast32(R32, gi, gj, gk, (float)(r0 + r) - gj, dkc, r2f, cc0, ismin, ismax,
+                                                   unsure);
+                    if (unsure)
+                        some = general_row_exact64(lv.dh, g.off, rsub((double)jj, g.off[1]), dk, g.radius, ismin, ismax);
+                    if (!some || ismin > ismax) {
+                        ismin = 1;
+                        ismax = 0;
+                    } else if (jrow[r0 + r] < 0) {
+                        atomicOr(status, kStatOutOfWindow);
+                        ismin = 1;
+                        ismax = 0;
+                    } else {  // (rows without points need no constants)
+                        const double dj = rsub((double)jj, g.off[1]);
+                        imin = min(imin, ismin);
+                        imax = max(imax, ismax);
+                        const ff a1 = ff_from_double_bits(2.0 * (G01 * dj + G02 * dk));
+                        const ff a0 = ff_from_double_bits(G11 * dj * dj + 2.0 * G12 * dj * dk + G22 * dk * dk);
+                        a1h[r] = a1.hi;
+                        a1l[r] = a1.lo;
+                        a0h[r] = a0.hi;
+                        a0l[r] = a0.lo;
                     }
                 }
+                i0[r] = ismin;
+                i1[r] = ismax;
             }
-            if (kAdj) {
+            imin = __reduce_min_sync(0xffffffffu, imin);
+            imax = __reduce_max_sync(0xffffffffu, imax);
+            __syncwarp();
+            for (int c0 = imin; c0 <= imax;) {
+                const int left = imax - c0 + 1, lw = left > 16 ? 5 : (left > 8 ? 4 : 3);
+                const int grp = lane >> lw, ng = 32 >> lw;
+                const int ii = c0 + (lane & ((1 << lw) - 1));
+                const int iidx = per0 ? imod(ii, np0) : ii - cc0 + off[0];
+                const bool iok = iidx >= 0 && iidx < gn0;
+                const ff di = ff_from_double(rsub((double)ii, g.off[0]));
+                const ff2n din = ff2n_dup(di);
+                const ff2 gd = ff2_dup(ff_mul(g00, di));
+                ff2 T[kNPow];  // collocate: the column's value twice; integrate: sums over even and odd rows
 #pragma unroll
-                for (int n = 0; n < kNPow; n++) {
-                    if (n >= L) break;
-                    ff v = acc[n];
-                    for (int o = 16; o > 0; o >>= 1) v = ff_add(v, ff_shfl_xor(v, o));
-                    acc[n] = v;
+                for (int j = 0; j < kNPow; j++) T[j] = ff2{f2(0.0f), f2(0.0f)};
+                if (!kAdj) {
+                    const ff *c = sC;
+#pragma unroll
+                    for (int j = 0; j < kNPow; j++) {
+                        if (j >= L) break;
+                        ff s = c[lp - j];
+                        for (int i = lp - j - 1; i >= 0; i--) s = ff_fma(s, di, c[i]);
+                        c += L - j;
+                        T[j] = ff2_dup(s);
+                    }
                 }
-                if (lane == 0)
-                    for (int n = 0; n < L; n++) Qj[row * L + n] = acc[n];
+                for (int rp = grp; 2 * (rp - grp) < nr; rp += ng) {  // row pairs
+                    const int r = min(2 * rp, (nr - 1) & ~1);
+                    const int2 lo2 = *reinterpret_cast<const int2 *>(i0 + r), hi2 = *reinterpret_cast<const int2 *>(i1 + r);
+                    const bool mine = 2 * rp < nr;
+                    bool act0 = mine && ii >= lo2.x && ii <= hi2.x, act1 = mine && ii >= lo2.y && ii <= hi2.y;
+                    if ((act0 || act1) && !iok) {
+                        atomicOr(status, kStatOutOfWindow);
+                        act0 = act1 = false;
+                    }
+                    if (!__any_sync(0xffffffffu, act0 || act1)) continue;
+                    const int2 jr = *reinterpret_cast<const int2 *>(jrow + r0 + r);
+                    double *const p0 = grid + ((int64_t)kidx * gn1 + jr.x) * gn0 + iidx;
+                    double *const p1 = grid + ((int64_t)kidx * gn1 + jr.y) * gn0 + iidx;
+                    double v0 = 1.0, v1 = 1.0;  // (zero would take the split's slow path)
+                    if (kAdj) {
+                        if (act0) v0 = __ldg(p0);
+                        if (act1) v1 = __ldg(p1);
+                    }
+                    const ff2 t = ff2_add(gd, ff2{ld2(a1h + r), ld2(a1l + r)});
+                    const ff2 r2 = ff2_fma(t, din, ff2{ld2(a0h + r), ld2(a0l + r)});
+                    const ff2 e = ff2_exp(ff2_mul(r2, mz), exptab);
+                    const ff2n dj = {ld2(djh + r0 + r), ld2(djn + r0 + r), ld2(djl + r0 + r)};
+                    if (!kAdj) {
+                        ff2 s = {f2(0.0f), f2(0.0f)};
+#pragma unroll
+                        for (int j = kNPow - 1; j >= 0; j--) {
+                            if (j >= L) continue;
+                            s = j == L - 1 ? T[j] : ff2_fma(s, dj, T[j]);
+                        }
+                        const ff2 v = ff2_mul(s, ff2n_of(e));
+                        if (act0) atomicAdd(p0, ff_to_double_bits(ff{v.hi.x, v.lo.x}));
+                        if (act1) atomicAdd(p1, ff_to_double_bits(ff{v.hi.y, v.lo.y}));
+                    } else {
+                        ff2 w = ff2_mul(ff2_pair(ff_from_double_bits(v0), ff_from_double_bits(v1)), ff2n_of(e));
+                        if (!act0) w.hi.x = w.lo.x = 0.0f;
+                        if (!act1) w.hi.y = w.lo.y = 0.0f;
+#pragma unroll
+                        for (int j = 0; j < kNPow; j++) {
+                            if (j >= L) break;
+                            T[j] = ff2_add(T[j], w);
+                            w = ff2_mul(w, dj);
+                        }
+                    }
+                }
+                if (kAdj) {  // cji[j][i] += sum over the block's lanes of T[j] di^i
+                    for (int i = 0; i < L; i++) {  // one power of di at a time (T di^i for j <= lp - i)
+                        __syncwarp();
+#pragma unroll
+                        for (int j = 0; j < kNPow; j++) {
+                            if (j > lp - i) break;
+                            const ff v = i == 0 ? ff_add(ff{T[j].hi.x, T[j].lo.x}, ff{T[j].hi.y, T[j].lo.y})
+                                                : ff_mul(ff{T[j].hi.x, T[j].lo.x}, di);
+                            T[j].hi.x = v.hi;
+                            T[j].lo.x = v.lo;
+                            sT[j * 33 + lane] = v;
+                        }
+                        __syncwarp();
+#pragma unroll
+                        for (int m = 0; m < kM2; m++) {
+                            if (oj[m] < 0 || oi[m] != i) continue;
+                            ff s = cji[m];
+                            for (int l = lane & ((1 << lg) - 1); l < 32; l += 1 << lg) s = ff_add(s, sT[oj[m] * 33 + l]);
+                            cji[m] = s;
+                        }
+                    }
+                    __syncwarp();
+                }
+                c0 += 1 << lw;
             }
         }
-        __syncthreads();
-        if (kAdj) {
-            // Qjk[j][i] = sum_rows Qj[row][i] dj^j;  Q[k][j][i] += Qjk[j][i] dk^k
-            for (int t = tid; t < L * L; t += nthr) {
-                const int i = t % L, j = t / L;
-                if (i + j > lp) continue;
-                ff s = {0.0f, 0.0f};
-                for (int row = 0; row < ny; row++) {
-                    if (rows[3 * row + 1] < rows[3 * row]) continue;
-                    s = ff_fma(Qj[row * L + i], powj[row * L + j], s);
-                }
-                ff p = {1.0f, 0.0f};
-                for (int k = 0; k <= lp - i - j; k++) {
-                    Q[(k * L + j) * L + i] = ff_fma(s, p, Q[(k * L + j) * L + i]);
-                    p = ff_mul(p, dkf);
-                }
+        if (kAdj) {  // W[k][j][i] += Qjk[j][i] dk^k
+            for (int o = 1; o < (1 << lg); o <<= 1) cji[0] = ff_add(cji[0], ff_shfl_xor(cji[0], o));
+            __syncwarp();
+#pragma unroll
+            for (int m = 0; m < kM2; m++)
+                if (oj[m] >= 0) sC[(lane >> lg) + 32 * m] = cji[m];
+            __syncwarp();
+#pragma unroll
+            for (int m = 0; m < kMC; m++) {
+                const int t = lane + 32 * m;
+                if (t >= nc) continue;
+                const int k = dec[t] & 255;
+                ff dp = {1.0f, 0.0f};
+                for (int e = 0; e < k; e++) dp = ff_mul(dp, dkf);
+                W[m] = ff_fma(sC[dec[t] >> 8], dp, W[m]);
             }
-            __syncthreads();
         }
     }
     if (kAdj) {
-        for (int t = tid; t < L * L * L; t += nthr) {
-            const int i = t % L, j = (t / L) % L, k = t / (L * L);
-            if (i + j + k > lp) continue;
-            double *out = mom + g.coef_off + pidx(lp, k, j, i);
+        for (int w = 0; w < kOrthoWarps; w++) {
+            if (warp == w) {
+#pragma unroll
+                for (int m = 0; m < kMC; m++)
+                    if (lane + 32 * m < nc) Q[lane + 32 * m] = ff_add(Q[lane + 32 * m], W[m]);
+            }
+            __syncthreads();
+        }
+        double *out = mom + g.coef_off;
+        for (int t = tid; t < nc; t += 32 * kOrthoWarps) {
             const double v = (double)Q[t].hi + (double)Q[t].lo;
-            if (it.nparts == 1) *out = v;
-            else atomicAdd(out, v);
+            if (it.nparts == 1) out[t] = v;
+            else atomicAdd(out + t, v);
         }
     }
 }
@@ -771,8 +917,8 @@ cudaError_t launch_prep(const TaskSet &ts, const double *d_pab, cudaStream_t s) 
 }
 
 // The items of the FP64 launches and of the float-float general-cell kernel (1500
-// pairs of a general cell, 128^3, collocate + integrate: one CTA per pair 38.1 ms,
-// most of it the tail of the largest boxes; items 10.7 ms).  A pair is divided into parts (interleaved planes, so
+// pairs of a general cell, 128^3, collocate + integrate: one CTA per pair 38.1 ms, most
+// of it the tail of the largest boxes; with items and the same kernel 10.7 ms).  A pair is divided into parts (interleaved planes, so
 // that parts cost alike) where it holds more than 1/kWaves of an even per-CTA share
 // of all cube points, down to one plane per warp; the largest pairs come first
 // (the sorted order).  The number of planes is not needed exactly: a geometry
@@ -847,8 +993,13 @@ static cudaError_t launch_fp64_impl(const TaskSet &ts, const GridPtrs &g, bool a
 
 // general-cell pairs of a mixed call: the float-float kernel
 int smem_general_ff(const PairGeom &g) {
+    return general_ff_cta_bytes(g) + kOrthoWarps * general_ff_warp_bytes(g.lp + 1);
+}
+// the boxes that the float-float path accepts: what one CTA held when it kept all rows
+// of a plane in shared memory
+int smem_general_ff_limit(const PairGeom &g) {
     const int L = g.lp + 1;
-    const int ny = g.hi[1] - g.cc[1] + 2;  // one row of margin, as smem_general_fp64
+    const int ny = g.hi[1] - g.cc[1] + 2;
     return 8 * (L * L * L + L * L + 2 * ny * L + 3 * ny) + 12 * ny;
 }
 
@@ -864,10 +1015,10 @@ cudaError_t launch_general_ff(const TaskSet &ts, const GridPtrs &g, bool adj, cu
     const unsigned n = (unsigned)ts.fp64_general;
     const Fp64Item *items = ts.d_fp64_items + ts.fp64_ortho;
     if (adj)
-        k_general_ff<true><<<n, 256, ts.gen_smem, s>>>(ts.d_geom, items, 1, ts.plan->d_levels, ts.d_coef, ts.d_mom, g,
+        k_general_ff<true><<<n, 32 * kOrthoWarps, ts.gen_smem, s>>>(ts.d_geom, items, 1, ts.plan->d_levels, ts.d_coef, ts.d_mom, g,
                                                       ts.d_status);
     else
-        k_general_ff<false><<<n, 256, ts.gen_smem, s>>>(ts.d_geom, items, 1, ts.plan->d_levels, ts.d_coef, ts.d_mom, g,
+        k_general_ff<false><<<n, 32 * kOrthoWarps, ts.gen_smem, s>>>(ts.d_geom, items, 1, ts.plan->d_levels, ts.d_coef, ts.d_mom, g,
                                                        ts.d_status);
     return cudaGetLastError();
 }

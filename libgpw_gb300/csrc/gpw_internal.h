@@ -116,6 +116,7 @@ void mixed_free(TaskSet &ts);
 cudaError_t launch_collocate_mixed(const TaskSet &ts, const GridPtrs &g, cudaStream_t s);
 cudaError_t launch_general_ff(const TaskSet &ts, const GridPtrs &g, bool adj, cudaStream_t s);
 int smem_general_ff(const PairGeom &g);
+int smem_general_ff_limit(const PairGeom &g);
 cudaError_t launch_integrate_mixed(const TaskSet &ts, const GridPtrs &g, cudaStream_t s);
 
 // gpw_capi.cu (host helpers)

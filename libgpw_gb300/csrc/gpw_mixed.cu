@@ -108,8 +108,7 @@ struct TPair {
 // General-cell level constants of the tiled path: FP32 lattice steps for the row
 // rule, and the cosines between the steps (cross terms of the Gaussian).
 struct GenLevel {
-    float dh[3][3];
-    float a, inv2a;     // |v0|^2 and 1 / (2 |v0|^2)
+    GeneralRow32 row;
     ff c01, c02, c12;   // cos(v0, v1), cos(v0, v2), cos(v1, v2)
 };
 // A pair's blob: the record padded to kHdr16 16-byte chunks, then its
@@ -214,57 +213,17 @@ __device__ __forceinline__ void row_range(const TPair &p, const ImgState &q, con
 }
 
 // General cell: the row (jj, kk) of the index box holds the points i with
-// |i v0 + w|^2 <= r^2 (the reference's quadratic, grid_base_ref_c.cc:781-807).
-// FP32 estimate in box-relative units i' = i - cc0 with a running error bound;
-// the exact FP64 rule (general_row, gpw_common.cuh) decides where a root lies
-// within its bound of an integer or the discriminant within its bound of zero.
-__device__ __noinline__ bool general_row_exact(const LevelDev &lv, const TPair &p, int jj, int kk, int &ismin,
-                                               int &ismax) {
-    const double dj = rsub((double)jj, p.gp[1]), dk = rsub((double)kk, p.gp[2]);
-    return general_row(lv.dh, p.gp, dj, dk, p.radius, ismin, ismax);
-}
-
+// |i v0 + w|^2 <= r^2 (the reference's quadratic, grid_base_ref_c.cc:781-807; FP32 with
+// an error bound, general_row_fast32 in gpw_common.cuh).
 __device__ __forceinline__ bool general_row_fast(const LevelDev &lv, const GenLevel &G, const TPair &p, int jj,
                                                  int kk, int &ismin, int &ismax) {
-    const float eps = 1.2e-7f;  // 2^-23, with room
-    const float gj = (float)(p.gp[1] - (double)p.cc[1]), gk = (float)(p.gp[2] - (double)p.cc[2]);
     const float gi = (float)(p.gp[0] - (double)p.cc[0]);
-    const float dj = (float)(jj - p.cc[1]) - gj, dk = (float)(kk - p.cc[2]) - gk;
-    float b = 0.0f, c = 0.0f, eb = 0.0f, ec = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        // v_i = dk dh2_i + dj dh1_i - gi dh0_i (box-relative), with its error bound
-        const float v = __fsub_rn(__fadd_rn(__fmul_rn(G.dh[2][i], dk), __fmul_rn(G.dh[1][i], dj)),
-                                  __fmul_rn(gi, G.dh[0][i]));
-        const float ev = eps * (fabsf(G.dh[2][i]) * (2.0f * fabsf(dk) + fabsf(gk)) +
-                                fabsf(G.dh[1][i]) * (2.0f * fabsf(dj) + fabsf(gj)) +
-                                2.0f * fabsf(gi * G.dh[0][i]) + 2.0f * fabsf(v));
-        b = __fadd_rn(b, __fmul_rn(2.0f * v, G.dh[0][i]));
-        c = __fadd_rn(c, __fmul_rn(v, v));
-        eb += 2.0f * ev * fabsf(G.dh[0][i]) + 2.0f * eps * fabsf(b);
-        ec += (2.0f * fabsf(v) + ev) * ev + 2.0f * eps * c;
-    }
-    // d = b^2 - 4a(c - r^2): propagated input errors, the representation errors of
-    // a and r^2, and the rounding of each operation
-    const float a = G.a, r2 = p.r2f;
-    const float cr = __fsub_rn(c, r2);
-    const float d = __fsub_rn(__fmul_rn(b, b), __fmul_rn(4.0f * a, cr));
-    const float ed = 2.0f * fabsf(b) * eb + eb * eb + eps * b * b +
-                     4.0f * a * (ec + eps * r2 + 2.5f * eps * fabsf(cr)) + eps * fabsf(d);
-    bool unsure = fabsf(d) <= 1.5f * ed;
-    if (!unsure && d < 0.0f) return false;  // surely empty
-    if (!unsure) {
-        const float sd = sqrtf(d);
-        const float esd = 1.8f * ed / sd + eps * sd;  // d > 1.5 ed: sqrt(d - ed) >= sd / sqrt(3)
-        const float lo = __fmul_rn(__fsub_rn(-b, sd), G.inv2a), hi = __fmul_rn(__fadd_rn(-b, sd), G.inv2a);
-        const float er = 1.25f * ((eb + esd + eps * (fabsf(b) + sd)) * G.inv2a + 1.5f * eps * (fabsf(lo) + fabsf(hi))) +
-                         1e-6f;
-        unsure = fabsf(lo - rintf(lo)) <= er || fabsf(hi - rintf(hi)) <= er;
-        ismin = p.cc[0] + (int)ceilf(lo);
-        ismax = p.cc[0] + (int)floorf(hi);
-    }
-    if (unsure) return general_row_exact(lv, p, jj, kk, ismin, ismax);
-    return true;
+    const float gj = (float)(p.gp[1] - (double)p.cc[1]), gk = (float)(p.gp[2] - (double)p.cc[2]);
+    bool unsure;
+    const bool some = general_row_fast32(G.row, gi, gj, gk, (float)(jj - p.cc[1]) - gj, (float)(kk - p.cc[2]) - gk,
+                                         p.r2f, p.cc[0], ismin, ismax, unsure);
+    if (!unsure) return some;
+    return general_row_exact64(lv.dh, p.gp, rsub((double)jj, p.gp[1]), rsub((double)kk, p.gp[2]), p.radius, ismin, ismax);
 }
 
 // Row (z, y) of the tile for a general-cell pair: tile-local x range [x0, x1].
@@ -1856,9 +1815,9 @@ int mixed_build(TaskSet &ts, std::string &err) {
         if (!(m1 > 0.0 && m2 > 0.0 && m3 > 0.0)) gen_ok = false;
         GenLevel &q = glv[l];
         for (int a = 0; a < 3; a++)
-            for (int b = 0; b < 3; b++) q.dh[a][b] = (float)lv.dh[a][b];
-        q.a = (float)G[0][0];
-        q.inv2a = (float)(0.5 / G[0][0]);
+            for (int b = 0; b < 3; b++) q.row.dh[a][b] = (float)lv.dh[a][b];
+        q.row.a = (float)G[0][0];
+        q.row.inv2a = (float)(0.5 / G[0][0]);
         auto sp = [](double d) {
             const float hi = (float)d;
             return ff{hi, (float)(d - (double)hi)};
