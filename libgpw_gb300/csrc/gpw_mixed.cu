@@ -1045,12 +1045,14 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                     // bits x0..x1 of the row: the points of this pair's sphere on the row
                     const uint32_t rmask =
                         x0 > x1 ? 0u : (uint32_t)(((2ull << x1) - 1ull) & ~((1ull << x0) - 1ull));
-                    // kCh chunks of 8 x per iteration (a compact loop body: instruction fetch
-                    // is a stall of this kernel); acc_hi[0 .. 8 kCh) always holds the current
+                    // kCh chunks of 8 x per iteration; acc_hi[0 .. 8 kCh) always holds the current
                     // chunks' sums, rotated by 8 kCh after each iteration (TX / (8 kCh)
-                    // rotations restore the order).  Two chunks halve the register moves of
-                    // the rotation; the general-cell body, longer by the cross factor, keeps one.
-                    constexpr int kCh = kGeneral ? 1 : 2;
+                    // rotations restore the order).  All four chunks in line need no
+                    // rotation, and with packed arithmetic the code still fits the
+                    // instruction cache: 73.2, 71.5 and 66.8 ms with 1, 2 and 4 chunks (100k
+                    // pairs, 256^3).  The general-cell body, longer by the cross factor, keeps
+                    // one chunk: 7.36, 7.95 and 8.72 ms (8000 pairs, 128^3).
+                    constexpr int kCh = kGeneral ? 1 : 4;
 #pragma unroll 1
                     for (int c2 = 0; c2 < TX / (8 * kCh); c2++) {
 #pragma unroll
