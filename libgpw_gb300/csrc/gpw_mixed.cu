@@ -163,7 +163,8 @@ struct MixedState {
     int *d_blob_len = nullptr;      // per binned pair: chunks of its blob
     int *d_count = nullptr;         // per tile: items
     unsigned long long *d_cursor = nullptr;  // per tile: next item slot (fill pass)
-    int64_t cap_items = 0, cap_units = 0;    // capacities of d_items / d_iimg and d_tiles / d_start
+    unsigned char *d_units = nullptr;        // d_cursor, d_start and d_tiles, one after the other
+    int64_t cap_items = 0, cap_units = 0;    // capacities of d_items / d_iimg, and of d_units in bytes
 };
 
 
@@ -1904,7 +1905,6 @@ int mixed_build(TaskSet &ts, std::string &err) {
     alloc((void **)&M->d_blob_len, sizeof(int) * len16.size());
     alloc((void **)&M->d_bl, sizeof(BinLevel) * blv.size());
     alloc((void **)&M->d_count, sizeof(int) * (size_t)std::max(ntiles, 1));
-    alloc((void **)&M->d_cursor, sizeof(unsigned long long) * (size_t)std::max(ntiles, 1));
     alloc((void **)&M->d_queue, sizeof(int) * 4);
     alloc((void **)&M->d_glv, sizeof(GenLevel) * glv.size());
     if (e == cudaSuccess) e = cudaMemset(M->d_blob, 0, sizeof(uint4) * (size_t)std::max<int64_t>(nchunks, 1));
@@ -2006,35 +2006,38 @@ int mixed_rebin(TaskSet &ts, std::string &err) {
     const int64_t sms = std::max(1, M->sms);
     const int64_t target = std::max((nitems + 64 * sms - 1) / (64 * sms),
                                     std::min<int64_t>(64, std::max<int64_t>(32, nitems / (16 * sms))));
-    struct Unit {
-        int tile;
-        int64_t it0, it1;
-        bool split;
-    };
-    std::vector<Unit> units;
+    // counting sort by (group, class, tile): a tile's units differ by at most one item
+    // and take the class of the smaller
+    std::vector<int> cls((size_t)std::max(ntiles, 1)), nu((size_t)std::max(ntiles, 1), 0);
+    constexpr int kClasses = 4 * 64;
+    std::vector<int> first(2 * kClasses + 1, 0);  // per group and class, the largest class first
+    int nunits = 0, nuo = 0;
     for (int t = 0; t < ntiles; t++) {
-        const int64_t n = count[t];
-        if (n == 0) continue;
-        const int64_t nu = (n + target - 1) / target;
-        for (int64_t u = 0; u < nu; u++)
-            units.push_back(Unit{t, start[t] + n * u / nu, start[t] + n * (u + 1) / nu, nu > 1});
+        if (count[t] == 0) continue;
+        nu[t] = (int)((count[t] + target - 1) / target);
+        const int c = (int)std::floor(4.0 * std::log2((double)(count[t] / nu[t])));
+        cls[t] = (t < nto ? 0 : kClasses) + kClasses - 1 - c;
+        first[cls[t] + 1] += nu[t];
+        nunits += nu[t];
+        if (t < nto) nuo += nu[t];
     }
-    auto work_class = [](const Unit &u) { return (int)std::floor(4.0 * std::log2((double)(u.it1 - u.it0))); };
-    std::stable_sort(units.begin(), units.end(), [&](const Unit &a, const Unit &b) {
-        const bool ga = a.tile >= nto, gb = b.tile >= nto;
-        if (ga != gb) return !ga;
-        return work_class(a) > work_class(b);
-    });
-    const int nunits = (int)units.size();
-    int nuo = 0;
-    while (nuo < nunits && units[nuo].tile < nto) nuo++;
-    std::vector<TileDesc> tiles_sorted(std::max(nunits, 1));
-    std::vector<int64_t> ubounds(2 * (size_t)std::max(nunits, 1), 0);  // per unit: first item, end
-    for (int u = 0; u < nunits; u++) {
-        tiles_sorted[u] = M->h_tiles[units[u].tile];
-        tiles_sorted[u].flags = units[u].split ? kUnitSplit : 0;
-        ubounds[2 * u] = units[u].it0;
-        ubounds[2 * u + 1] = units[u].it1;
+    for (int c = 0; c < 2 * kClasses; c++) first[c + 1] += first[c];
+    // one image of everything the device needs: slots per tile, bounds per unit, tiles
+    const size_t nslot = (size_t)std::max(ntiles, 1), nun = (size_t)std::max(nunits, 1);
+    std::vector<unsigned char> image(8 * nslot + 16 * nun + sizeof(TileDesc) * nun);
+    int64_t *slots = reinterpret_cast<int64_t *>(image.data()), *ubounds = slots + nslot;
+    TileDesc *tiles_sorted = reinterpret_cast<TileDesc *>(ubounds + 2 * nun);
+    for (int t = 0; t < ntiles; t++) {
+        slots[t] = start[t];
+        if (count[t] == 0) continue;
+        const int64_t n = count[t];
+        for (int64_t u = 0; u < nu[t]; u++) {
+            const int at = first[cls[t]]++;
+            tiles_sorted[at] = M->h_tiles[t];
+            tiles_sorted[at].flags = nu[t] > 1 ? kUnitSplit : 0;
+            ubounds[2 * at] = start[t] + n * u / nu[t];
+            ubounds[2 * at + 1] = start[t] + n * (u + 1) / nu[t];
+        }
     }
     // storage for the items and units (kept when large enough)
     if (nitems > M->cap_items || !M->d_items) {
@@ -2048,28 +2051,18 @@ int mixed_rebin(TaskSet &ts, std::string &err) {
         if ((e = cudaMalloc(&M->d_iimg, sizeof(ItemImg) * cap)) != cudaSuccess) return fail(e);
         M->cap_items = cap;
     }
-    if (nunits > M->cap_units || !M->d_tiles) {
-        cudaFree(M->d_tiles);
-        cudaFree(M->d_start);
-        M->d_tiles = nullptr;
-        M->d_start = nullptr;
+    if ((int64_t)image.size() > M->cap_units || !M->d_units) {
+        cudaFree(M->d_units);
+        M->d_units = nullptr;
         M->cap_units = 0;
-        const int64_t cap = std::max<int64_t>(nunits + nunits / 16, 1);
-        if ((e = cudaMalloc(&M->d_tiles, sizeof(TileDesc) * cap)) != cudaSuccess) return fail(e);
-        if ((e = cudaMalloc(&M->d_start, sizeof(int64_t) * 2 * cap)) != cudaSuccess) return fail(e);
+        const int64_t cap = (int64_t)image.size() + image.size() / 16;
+        if ((e = cudaMalloc(&M->d_units, cap)) != cudaSuccess) return fail(e);
         M->cap_units = cap;
     }
-    if (nunits && (e = cudaMemcpy(M->d_tiles, tiles_sorted.data(), sizeof(TileDesc) * nunits,
-                                  cudaMemcpyHostToDevice)) != cudaSuccess)
-        return fail(e);
-    if ((e = cudaMemcpy(M->d_start, ubounds.data(), sizeof(int64_t) * ubounds.size(), cudaMemcpyHostToDevice)) !=
-        cudaSuccess)
-        return fail(e);
-    std::vector<unsigned long long> cur((size_t)std::max(ntiles, 1), 0ull);
-    for (int t = 0; t < ntiles; t++) cur[t] = (unsigned long long)start[t];
-    if ((e = cudaMemcpy(M->d_cursor, cur.data(), sizeof(unsigned long long) * cur.size(), cudaMemcpyHostToDevice)) !=
-        cudaSuccess)
-        return fail(e);
+    M->d_cursor = reinterpret_cast<unsigned long long *>(M->d_units);
+    M->d_start = reinterpret_cast<int64_t *>(M->d_units) + nslot;
+    M->d_tiles = reinterpret_cast<TileDesc *>(M->d_start + 2 * nun);
+    if ((e = cudaMemcpy(M->d_units, image.data(), image.size(), cudaMemcpyHostToDevice)) != cudaSuccess) return fail(e);
     if (nbin > 0 && (e = bin_pairs(ts, *M, 1, nullptr, M->d_cursor, M->d_items, M->d_iimg)) != cudaSuccess) return fail(e);
     if (nitems) {
         // (image overflows are reported by the tiled kernels when they run: a plain
@@ -2093,10 +2086,9 @@ int64_t mixed_units(const TaskSet &ts) { return ts.mixed ? ts.mixed->ntiles : 0;
 void mixed_free(TaskSet &ts) {
     MixedState *M = ts.mixed;
     if (!M) return;
-    cudaFree(M->d_tiles);
+    cudaFree(M->d_units);
     cudaFree(M->d_blob);
     cudaFree(M->d_blob_off);
-    cudaFree(M->d_start);
     cudaFree(M->d_items);
     cudaFree(M->d_iimg);
     cudaFree(M->d_queue);
@@ -2105,7 +2097,6 @@ void mixed_free(TaskSet &ts) {
     cudaFree(M->d_bl);
     cudaFree(M->d_blob_len);
     cudaFree(M->d_count);
-    cudaFree(M->d_cursor);
     delete M;
     ts.mixed = nullptr;
 }
