@@ -341,7 +341,6 @@ struct alignas(128) SmemColl {
     alignas(16) float cs[TX];   // 2^fx per column (0 for an empty column)
     unsigned char qb[kNPow][NPAIR_MAX + 2];  // qb[L-1][pair_index(L, b, a)] = b
     unsigned char qpad[kNPow][2 * kCxyRow];  // qpad[L-1][padded index of (b, a)] = b | a << 4
-    int zs[kNPow + 1];          // zs[g]: packed index of (g, 0, 0) for the current pair's lp
     TileCommon c;
 };
 
@@ -593,6 +592,14 @@ __constant__ float c_binom[kNPow][kNPow] = {
     {1, 8, 28, 56, 70, 56, 28, 8, 1},
     {1, 9, 36, 84, 126, 126, 84, 36, 9, 1},
     {1, 10, 45, 120, 210, 252, 210, 120, 45, 10, 1}};
+
+// c_zs[lp][g]: packed index of (g, 0, 0)
+#define GPW_ZS(lp) {ZS_(lp, 0), ZS_(lp, 1), ZS_(lp, 2), ZS_(lp, 3), ZS_(lp, 4), ZS_(lp, 5), ZS_(lp, 6), ZS_(lp, 7), ZS_(lp, 8), ZS_(lp, 9), ZS_(lp, 10), ZS_(lp, 11)}
+#define ZS_(lp, g) ((g) > (lp) + 1 ? 0 : (((lp) + 1) * ((lp) + 2) * ((lp) + 3) - ((lp) + 1 - (g)) * ((lp) + 2 - (g)) * ((lp) + 3 - (g))) / 6)
+__constant__ int c_zs[kNPow][kNPow + 1] = {GPW_ZS(0), GPW_ZS(1), GPW_ZS(2), GPW_ZS(3), GPW_ZS(4), GPW_ZS(5),
+                                           GPW_ZS(6), GPW_ZS(7), GPW_ZS(8), GPW_ZS(9), GPW_ZS(10)};
+#undef ZS_
+#undef GPW_ZS
 
 // One item (g, b, a) per thread of [t0, t0 + nt): Horner in tc over a' = amax .. a
 // with the binomials from shared memory (bin[a'][a] = C(a', a)).  zs[g] is the
@@ -846,9 +853,10 @@ __device__ __forceinline__ void first_pair(TileCommon &cm, Buf *pb, const MixedA
 // 16-byte entries {hi(a), hi(a+1), lo(a), lo(a+1)}.
 __device__ __forceinline__ void stage1_cxy(SmemColl &sm, int L, int lp, const TileShape &sh) {
     const TileCommon &cm = sm.c;
+    const int *zs = c_zs[lp];
     const int npad = 2 * (L >> 1) * ((L >> 1) + 1) + (L & 1) * (L + 1);  // cxy_pad_row(L, L)
     const unsigned char *qp = sm.qpad[L - 1];
-    for (int t = threadIdx.x; t < (npad << (sh.lz - 1)); t += NTHR) {
+    for (int t = (int)threadIdx.x - 32; t < (npad << (sh.lz - 1)); t += NTHR - 32) {
         const int zz = 2 * (t & ((sh.TZ >> 1) - 1)), q = t >> (sh.lz - 1);
         const int b = qp[q] & 15, a = qp[q] >> 4, n = lp - a - b;
         const ff *c = sm.rc + (b * (lp + 1) - (b * (b - 1)) / 2 + a);
@@ -860,10 +868,10 @@ __device__ __forceinline__ void stage1_cxy(SmemColl &sm, int L, int lp, const Ti
         int g = 0, bg = 0;
 #pragma unroll 1
         for (; g + 1 <= n; g += 2, bg += 2 * b) {
-            s0 = ff2_fma(ff2_dup(c[sm.zs[g] - bg]), zpair(g), s0);
-            s1 = ff2_fma(ff2_dup(c[sm.zs[g + 1] - bg - b]), zpair(g + 1), s1);
+            s0 = ff2_fma(ff2_dup(c[zs[g] - bg]), zpair(g), s0);
+            s1 = ff2_fma(ff2_dup(c[zs[g + 1] - bg - b]), zpair(g + 1), s1);
         }
-        if (g <= n) s0 = ff2_fma(ff2_dup(c[sm.zs[g] - bg]), zpair(g), s0);
+        if (g <= n) s0 = ff2_fma(ff2_dup(c[zs[g] - bg]), zpair(g), s0);
         s0 = ff2_add(s0, s1);
         float *o = reinterpret_cast<float *>(&sm.Cxy[zz][q >> 1]) + (q & 1);
         o[0] = s0.hi.x;
@@ -953,7 +961,9 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
         if (tid == 0 && (td.flags & kUnitOver)) atomicOr(A.status, kStatTooManyImages);
         const LevelDev &lv = A.levels[td.level];
         const TileShape sh(td.lz);
-        const int TY = sh.TY, TZ = sh.TZ, z = m >> sh.ly, y = m & (TY - 1);
+        const int TY = sh.TY, TZ = sh.TZ;
+        // a warp's 32 rows: 8 y x 4 z, so that more warps (and chunks) lie wholly outside a sphere
+        const int wy = TY >> 3, y = (warp & (wy - 1)) * 8 + (m & 7), z = (warp / wy) * 4 + ((m >> 3) & 3);
         if (TZ > kMaxTZColl) {  // shapes are validated on the host; never taken
             if (tid == 0) atomicOr(A.status, kStatBadTile);
             continue;
@@ -1000,13 +1010,14 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                         }
                     }
                 } else {
-                    // slab starts zs[g] = packed index of (g, 0, 0), then the re-expansion
-                    if (tid - 64 <= kNPow) sm.zs[tid - 64] = tid - 64 <= lp + 1 ? row_start(lp, tid - 64, 0) : 0;
-                    asm volatile("bar.sync 2, 64;" ::: "memory");
-                    recentre_x(pb, Q.tc, Q.sb, sm.rc, sm.bin, sm.zs, sm.qb, 64, NTHR - 64);
+                    recentre_x(pb, Q.tc, Q.sb, sm.rc, sm.bin, c_zs[lp], sm.qb, 64, NTHR - 64);
                 }
-                __syncthreads();
-                stage1_cxy(sm, L, lp, sh);
+                // stage 1 needs the z table and the re-expansion, not the x slices: warps 1-3
+                // go on to it while warp 0 still slices
+                if (warp > 0) {
+                    asm volatile("bar.sync 2, 96;" ::: "memory");
+                    stage1_cxy(sm, L, lp, sh);
+                }
                 __syncthreads();
                 // stage 2 (this thread's row, all a at once) + culling + A slices
                 int x0, x1;
