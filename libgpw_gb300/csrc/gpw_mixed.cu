@@ -384,14 +384,14 @@ struct IntCommon {
     alignas(16) float Yh[kNPow][kYRow], Ynl[kNPow][kYRow];
     alignas(8) float gsc[KP];                // 2^(g - SLB), g the alpha row's exponent (0: an empty row)
     unsigned char qb[kNPow][NPAIR_MAX + 2];  // qb[L-1][pair_index(L, b, a)] = b
-    int zs[kNPow + 1];                       // zs[g]: packed index of (g, 0, 0) for the current pair's lp
     PairHdr pb[2];                           // the current pair's record and the one being fetched
     TileCommon c;
 };
 template <bool kGeneral>
 struct alignas(128) SmemInt : IntCommon {
     alignas(16) float Ynh[kNPow][kYRow];
-    uint32_t mask[MROWS];          // each row's points inside the current item's range
+    uint32_t mask[MROWS];          // each row's points inside the item's range
+    uint8_t todo[MROWS];           // the chunks of its A row to be masked to them
     __half A[2][NSL][MROWS * KP];  // masked V slices, K halves x in [0,16) and [16,32)
     IntSums st;
     union {
@@ -679,10 +679,6 @@ __device__ __forceinline__ void slice_row16(const ff2 *vin, float sc, int kw, in
     }
 }
 
-// named barrier 1 between producer warps (arrive) and consumer warps (sync)
-__device__ __forceinline__ void bar_arrive1(int n) { asm volatile("bar.arrive 1, %0;" ::"r"(n) : "memory"); }
-__device__ __forceinline__ void bar_sync1(int n) { asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory"); }
-
 // General cell: the cross factor along row (z, y) of the current image, E(x) =
 // exp(alpha + beta t0(x)) with beta = -2 zetp (c01 t1 + c02 t2), alpha = -2 zetp
 // c12 t1 t2: returns E(x0) and q = E(x + 1) / E(x).
@@ -745,17 +741,14 @@ __device__ __forceinline__ int general_a_row(Smem &sm, const GenLevel &G, const 
     return vmx;
 }
 
-// Orthorhombic integrate: bits of the row's mask M (bit x: point x inside the pair's
-// range) to its A row, chunk by chunk of 8 x: chunks not wholly inside are masked in
-// place.  A row with no point inside stays as it is: its products are not read.
+// Orthorhombic integrate: the A row r to the points of M (bit x) in its chunks of 8 x
+// that hold more than those (bits of todo).
 template <class Smem>
-__device__ __forceinline__ void mask_a_row(Smem &sm, int r, uint32_t M) {
-    if (M == 0u) return;
-#pragma unroll 1
+__device__ __forceinline__ void mask_a_row(Smem &sm, int r, uint32_t M, uint32_t todo) {
+#pragma unroll
     for (int v = 0; v < TX / 8; v++) {
-        const uint32_t mb = (M >> (8 * v)) & 0xFFu;
-        if (mb == 0xFFu) continue;
-        const uint4 mk = chunk_mask(mb);
+        if (!((todo >> v) & 1u)) continue;
+        const uint4 mk = chunk_mask((M >> (8 * v)) & 0xFFu);
         uint4 *a = reinterpret_cast<uint4 *>(sm.A[v >> 1][0]) + (r >> 3) * 16 + (v & 1) * 8 + (r & 7);
         uint4 t[NSL];
 #pragma unroll
@@ -765,19 +758,41 @@ __device__ __forceinline__ void mask_a_row(Smem &sm, int r, uint32_t M) {
             a[q * (MROWS * KP / 8)] = make_uint4(t[q].x & mk.x, t[q].y & mk.y, t[q].z & mk.z, t[q].w & mk.w);
     }
 }
-// copies the masked chunks of row r back from the CTA's slot (asynchronously: waited
-// for at the item's end)
+// Copies from the CTA's slot the chunks of row r in which the next item (mask M) needs
+// points that the row no longer holds (asynchronously: waited for at the item's end);
+// returns what the row then holds.
 template <class Smem>
-__device__ __forceinline__ void restore_a_row(Smem &sm, const uint4 *vslot, int r, uint32_t M) {
-#pragma unroll 1
-    for (int v = 0; v < TX / 8 && M != 0u; v++) {
-        if (((M >> (8 * v)) & 0xFFu) == 0xFFu) continue;
-        const int o16 = (r >> 3) * 16 + (v & 1) * 8 + (r & 7);
+__device__ __forceinline__ uint32_t restore_a_row(Smem &sm, const uint4 *vslot, int r, uint32_t M, uint32_t have) {
+    // chunk v of slice q lies a constant away from the row's first chunk, in both copies
+    const uint32_t dst = tc::smem_addr(sm.A) + 16 * ((r >> 3) * 16 + (r & 7));
+    const uint4 *src = vslot + (r >> 3) * 16 + (r & 7);
+    const uint32_t lack = M & ~have;
+    if (lack != 0u) {
 #pragma unroll
-        for (int q = 0; q < NSL; q++)
-            cp_async16(reinterpret_cast<uint4 *>(sm.A[v >> 1][q]) + o16, vslot + ((v >> 1) * NSL + q) * (MROWS * KP / 8) + o16);
+        for (int v = 0; v < TX / 8; v++) {
+            if (((lack >> (8 * v)) & 0xFFu) == 0u) continue;
+            have |= 0xFFu << (8 * v);
+#pragma unroll
+            for (int q = 0; q < NSL; q++) {
+                const int o = ((v >> 1) * NSL + q) * (MROWS * KP / 8) + (v & 1) * 8;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * o), "l"(src + o) : "memory");
+            }
+        }
     }
     cp_async_commit();
+    return have;
+}
+// the chunks (bits 0..3) of a row holding the points `have` that an item with the points M
+// masks; none in a row without points: its products are not read
+__device__ __forceinline__ uint8_t chunks_to_mask(uint32_t M, uint32_t have) {
+    const uint32_t d = __vcmpne4(M, have) & 0x08040201u;  // a byte per chunk
+    return M == 0u ? 0 : (uint8_t)((d | d >> 8 | d >> 16 | d >> 24) & 15u);
+}
+// bits x0..x1 of a row's cube range in the item (P, Q)
+__device__ __forceinline__ uint32_t row_mask(const TPair &P, const ImgState &Q, const int *table, int z, int y, bool ok) {
+    int x0, x1;
+    row_range(P, Q, table, Q.o[2] + z, Q.o[1] + y, ok, x0, x1);
+    return x0 > x1 ? 0u : (uint32_t)(((2ull << x1) - 1ull) & ~((1ull << x0) - 1ull));
 }
 
 // TMEM set-up shared by both kernels: warp 0 allocates, thread 0 inits the mbarrier
@@ -1162,6 +1177,26 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
     tc_teardown(cm, kCols, phase);
 }
 
+// The (g, b, a) of packed index t of degree lp as g | b << 4 | a << 8 | pair_index << 16,
+// for all lp: read through L1 (a search of the slab starts in shared memory took up to
+// lp dependent loads, on the path that ends every item).
+constexpr int d_decode_at(int lp) { return lp * (lp + 1) * (lp + 2) * (lp + 3) / 24; }
+struct Decode {
+    uint32_t e[d_decode_at(kMaxLp + 1)];
+};
+constexpr Decode make_decode() {
+    Decode d{};
+    for (int lp = 0; lp <= kMaxLp; lp++) {
+        int t = d_decode_at(lp);
+        for (int g = 0; g <= lp; g++)
+            for (int b = 0; b <= lp - g; b++)
+                for (int a = 0; a <= lp - g - b; a++)
+                    d.e[t++] = (uint32_t)(g | b << 4 | a << 8 | (b * (lp + 1) - (b * (b - 1)) / 2 + a) << 16);
+    }
+    return d;
+}
+__device__ const Decode d_decode = make_decode();
+
 // s += four products a b, the even and the odd ones in the two halves of s
 __device__ __forceinline__ void acc_four(ff2 &s, float4 ah, float4 al, float4 bh, float4 bnh, float4 bnl) {
     ff2_acc_lazy(s, ff2{make_float2(ah.x, ah.y), make_float2(al.x, al.y)},
@@ -1256,6 +1291,13 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
         const int64_t it0 = A.start[2 * tile], it1 = A.start[2 * tile + 1];
         uint64_t nxt = 0;
         first_pair(cm, sm.pb, A, it0, it1, nxt, false);
+        uint32_t M = 0, have = ~0u;  // this row's points in the current item, and those its A row holds
+        if constexpr (!kGeneral) {
+            if (it0 < it1) M = row_mask(sm.pb[0].p, cm.ii[0].im, A.table, z, y, row_ok);
+            sm.mask[m] = M;
+            sm.todo[m] = chunks_to_mask(M, have);
+            __syncthreads();
+        }
         for (int64_t it = it0; it < it1 && !cm.abort; it++) {
             const int cur = next_pair(cm, sm.pb, A, it, it0, it1, nxt, false);
             const TPair &P = sm.pb[cur].p;
@@ -1264,22 +1306,12 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
             const int64_t moff = P.coef_off;
             const ImgState &Q = cm.ii[cur].im;
             {
-                // every thread: its row's cube x range, applied to its A row
-                int x0, x1;
-                if constexpr (kGeneral)
+                int x0 = 1, x1 = 0, vrow = vm;
+                if constexpr (kGeneral) {  // every thread: its row's cube x range and its A row
                     general_row_range(lv, A.glv[td.level], P, Q, Q.o[2] + z, Q.o[1] + y, row_ok, x0, x1);
-                else
-                    row_range(P, Q, A.table, Q.o[2] + z, Q.o[1] + y, row_ok, x0, x1);
-                int vrow = vm;
-                uint32_t M = 0;
-                if constexpr (kGeneral) {
                     vrow = general_a_row(sm, A.glv[td.level], P, Q, sh, m, x0, x1);
-                } else {  // (a row of zeros needs no mask)
-                    M = vm == kZeroExp ? ~0u : (x0 > x1 ? 0u : (uint32_t)(((2ull << x1) - 1ull) & ~((1ull << x0) - 1ull)));
-                    sm.mask[m] = M;
                 }
                 if (warp == 0) {
-                    if constexpr (!kGeneral) bar_arrive1(NTHR);
                     // X column (lane x) in registers, then B: row alpha = X[alpha][x] over x,
                     // scaled by 2^(SLB - g[alpha]) (maximum over the warp); rows alpha >= L
                     // are left as they are (their output columns are not read).  Unlike
@@ -1313,15 +1345,13 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                         }
                     }
                 } else if (warp == 1) {
-                    if constexpr (!kGeneral) bar_arrive1(NTHR);
-                    if (tid - 32 <= kNPow) sm.zs[tid - 32] = tid - 32 <= lp + 1 ? row_start(lp, tid - 32, 0) : 0;
 #pragma unroll 1
                     for (int ent = tid - 32; ent < TY + TZ; ent += 32) yz_fill(sm, P, tab_entry(P, Q, ext, sh, 1, ent));
                 } else if constexpr (!kGeneral) {
-                    bar_sync1(NTHR);  // every row's mask
-                    mask_a_row(sm, tid - 64, sm.mask[tid - 64]);
-                    mask_a_row(sm, tid, sm.mask[tid]);
+                    mask_a_row(sm, tid - 64, sm.mask[tid - 64], sm.todo[tid - 64]);
+                    mask_a_row(sm, tid, sm.mask[tid], sm.todo[tid]);
                 }
+                cp_async_wait_all();  // the next item's record, read after this barrier
                 tc::fence_async_smem();
                 tc::fence_before_sync();
                 __syncthreads();
@@ -1346,8 +1376,18 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                 }
                 tc_wait(cm, phase, A.status);
                 phase ^= 1u;
-                if constexpr (!kGeneral) restore_a_row(sm, vslot, m, M);
-                const bool live = x0 <= x1;  // other rows give zeros
+                const bool live = kGeneral ? x0 <= x1 : M != 0u;  // other rows give zeros
+                if constexpr (!kGeneral) {
+                    // the next item's range of this row, and what A lacks of it
+                    if (M != 0u) have = M;
+                    M = 0u;
+                    if (it + 1 < it1) {
+                        M = row_mask(sm.pb[cur ^ 1].p, cm.ii[cur ^ 1].im, A.table, z, y, row_ok);
+                        have = restore_a_row(sm, vslot, m, M, have);
+                        sm.mask[m] = M;
+                        sm.todo[m] = chunks_to_mask(M, have);
+                    }
+                }
                 const float2 rsc = f2(vrow != kZeroExp ? pow2i(vrow - SLB) : 0.0f);  // 2^(row exponent - SLB)
 #pragma unroll 1
                 for (int c = 0; c < KP / 8; c++) {
@@ -1362,7 +1402,7 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                     tc::tmem_wait_ld8(r5);  // (one wait covers all loads; the second only orders r5's use)
 #pragma unroll
                     for (int i = 0; i < 4; i++) {  // two alpha per instruction
-                        if (8 * c + 2 * i >= kNPow) break;
+                        if (8 * c + 2 * i >= L) break;  // (L <= kNPow)
                         auto two = [&](const uint32_t *r) {
                             return make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
                         };
@@ -1418,13 +1458,9 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                 // stage 1 transposed: W[g][b][a] += sum_z T[z][(b,a)] Z[g][z]
                 const int nc = ncoef(lp);
                 for (int t = tid; t < nc; t += NTHR) {
-                    // (g, b, a) of packed index t: slab g by the slab starts, b by the pair table
-                    int g = 0;
-                    while (g < lp && sm.zs[g + 1] <= t) g++;
-                    const int qn = lp - g, r = t - sm.zs[g];
-                    const int b = sm.qb[qn][r];
-                    const int a = r - (b * (qn + 1) - (b * (b - 1)) / 2);
-                    const int pi = pair_index(L, b, a);
+                    const uint32_t de = __ldg(&d_decode.e[d_decode_at(lp) + t]);  // (g, b, a) of packed index t
+                    const int g = de & 15, pi = de >> 16;
+                    [[maybe_unused]] const int b = (de >> 4) & 15, a = (de >> 8) & 15;
                     ff2 s2 = {f2(0.0f), f2(0.0f)};
 #pragma unroll 1
                     for (int z4 = 0; z4 < TZ; z4 += 4)
@@ -1435,7 +1471,7 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                                  *reinterpret_cast<const float4 *>(&cm.Znl[g][z4]));
                     const ff s = ff_add(ff{s2.hi.x, s2.lo.x}, ff{s2.hi.y, s2.lo.y});
                     if (s.hi != 0.0f) {
-                        double val = (double)s.hi + (double)s.lo;
+                        double val = ff_to_double_bits(s);
                         if constexpr (kGeneral) {
                             // moments in powers of t_d = d_d |v_d| -> lattice-index powers d_d
                             for (int e = 0; e < a; e++) val *= P.hx;
