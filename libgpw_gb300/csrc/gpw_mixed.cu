@@ -339,7 +339,6 @@ struct alignas(128) SmemColl {
     alignas(16) float acc_lo[MROWS][TX + 4];  // low parts of the tile sums (row m belongs to thread m; padded rows)
     float bin[kNPow][kNPow];    // binomials C(a', a) of the re-expansion
     alignas(16) float cs[TX];   // 2^fx per column (0 for an empty column)
-    unsigned char qb[kNPow][NPAIR_MAX + 2];  // qb[L-1][pair_index(L, b, a)] = b
     unsigned char qpad[kNPow][2 * kCxyRow];  // qpad[L-1][padded index of (b, a)] = b | a << 4
     TileCommon c;
 };
@@ -601,21 +600,36 @@ __constant__ int c_zs[kNPow][kNPow + 1] = {GPW_ZS(0), GPW_ZS(1), GPW_ZS(2), GPW_
 #undef ZS_
 #undef GPW_ZS
 
+// The (g, b, a) of packed index t of degree lp as g | b << 4 | a << 8 | pair_index << 16,
+// for all lp: read through L1 (a search of the slab starts in shared memory took up to
+// lp dependent loads; integrate's last stage, which ends every item: 59.6 -> 56.5 ms
+// with the table and with the moments joined to doubles on the integer pipe).
+constexpr int d_decode_at(int lp) { return lp * (lp + 1) * (lp + 2) * (lp + 3) / 24; }
+struct Decode {
+    uint32_t e[d_decode_at(kMaxLp + 1)];
+};
+constexpr Decode make_decode() {
+    Decode d{};
+    for (int lp = 0; lp <= kMaxLp; lp++) {
+        int t = d_decode_at(lp);
+        for (int g = 0; g <= lp; g++)
+            for (int b = 0; b <= lp - g; b++)
+                for (int a = 0; a <= lp - g - b; a++)
+                    d.e[t++] = (uint32_t)(g | b << 4 | a << 8 | (b * (lp + 1) - (b * (b - 1)) / 2 + a) << 16);
+    }
+    return d;
+}
+__device__ const Decode d_decode = make_decode();
+
 // One item (g, b, a) per thread of [t0, t0 + nt): Horner in tc over a' = amax .. a
-// with the binomials from shared memory (bin[a'][a] = C(a', a)).  zs[g] is the
-// packed index of (g, 0, 0) and qb[q][r] the b of row-in-slab r of a slab with
-// q = lp - g, so that decoding t needs no arithmetic series.  The row coefficients'
+// with the binomials from shared memory (bin[a'][a] = C(a', a)).  The row coefficients'
 // balancing factor 2^(a sb) is applied here, once per coefficient.
-__device__ void recentre_x(const PairBuf &pb, ff tc, int sb, ff *out, const float (*bin)[kNPow], const int *zs,
-                           const unsigned char (*qb)[NPAIR_MAX + 2], int t0, int nt) {
+__device__ void recentre_x(const PairBuf &pb, ff tc, int sb, ff *out, const float (*bin)[kNPow], int t0, int nt) {
     const int lp = pb.p.lp;
     const int nc = ncoef(lp);
     for (int t = (int)threadIdx.x - t0; t < nc; t += nt) {
-        int g = 0;
-        while (g < lp && zs[g + 1] <= t) g++;
-        const int qn = lp - g, r = t - zs[g];
-        const int b = qb[qn][r];
-        const int a = r - (b * (qn + 1) - (b * (b - 1)) / 2), amax = lp - g - b;
+        const uint32_t de = __ldg(&d_decode.e[d_decode_at(lp) + t]);
+        const int g = de & 15, b = (de >> 4) & 15, a = (de >> 8) & 15, amax = lp - g - b;
         const int base = t - a;  // packed index of (g, b, 0)
         ff s = {0.0f, 0.0f};
 #pragma unroll 1
@@ -954,13 +968,6 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
     const uint32_t tbase = cm.tmem + ((uint32_t)(warp * 32) << 16);
     uint32_t phase = 0;
     for (int t = tid; t < kNPow * kNPow; t += NTHR) sm.bin[t / kNPow][t % kNPow] = c_binom[t / kNPow][t % kNPow];
-    // qb[L-1][pair_index(L, b, a)] = b: the (b, a) of a pair index without a search per use
-    for (int t = tid; t < kNPow * (NPAIR_MAX + 2); t += NTHR) {
-        const int Lq = t / (NPAIR_MAX + 2) + 1, q = t % (NPAIR_MAX + 2);
-        int b = 0, r = q;
-        while (b < Lq && r >= Lq - b) r -= Lq - b++;
-        sm.qb[Lq - 1][q] = (unsigned char)min(b, kNPow - 1);
-    }
     for (int t = tid; t < kNPow * 2 * kCxyRow; t += NTHR) {
         const int Lq = t / (2 * kCxyRow) + 1, q = t % (2 * kCxyRow);
         int b = 0, r = q;
@@ -1025,7 +1032,7 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                         }
                     }
                 } else {
-                    recentre_x(pb, Q.tc, Q.sb, sm.rc, sm.bin, c_zs[lp], sm.qb, 64, NTHR - 64);
+                    recentre_x(pb, Q.tc, Q.sb, sm.rc, sm.bin, 64, NTHR - 64);
                 }
                 // stage 1 needs the z table and the re-expansion, not the x slices: warps 1-3
                 // go on to it while warp 0 still slices
@@ -1176,26 +1183,6 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
     }
     tc_teardown(cm, kCols, phase);
 }
-
-// The (g, b, a) of packed index t of degree lp as g | b << 4 | a << 8 | pair_index << 16,
-// for all lp: read through L1 (a search of the slab starts in shared memory took up to
-// lp dependent loads, on the path that ends every item).
-constexpr int d_decode_at(int lp) { return lp * (lp + 1) * (lp + 2) * (lp + 3) / 24; }
-struct Decode {
-    uint32_t e[d_decode_at(kMaxLp + 1)];
-};
-constexpr Decode make_decode() {
-    Decode d{};
-    for (int lp = 0; lp <= kMaxLp; lp++) {
-        int t = d_decode_at(lp);
-        for (int g = 0; g <= lp; g++)
-            for (int b = 0; b <= lp - g; b++)
-                for (int a = 0; a <= lp - g - b; a++)
-                    d.e[t++] = (uint32_t)(g | b << 4 | a << 8 | (b * (lp + 1) - (b * (b - 1)) / 2 + a) << 16);
-    }
-    return d;
-}
-__device__ const Decode d_decode = make_decode();
 
 // s += four products a b, the even and the odd ones in the two halves of s
 __device__ __forceinline__ void acc_four(ff2 &s, float4 ah, float4 al, float4 bh, float4 bnh, float4 bnl) {
