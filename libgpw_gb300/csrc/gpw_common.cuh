@@ -230,10 +230,6 @@ __device__ __forceinline__ bool general_row_fast32(const GeneralRow32 &G, float 
     }
     return true;
 }
-__device__ __noinline__ inline bool general_row_exact64(const double dh[3][3], const double gp[3], double dj, double dk,
-                                                        double radius, int &ismin, int &ismax) {
-    return general_row(dh, gp, dj, dk, radius, ismin, ismax);
-}
 #endif
 
 // ---------------------------------------------------------------------------

@@ -6,6 +6,8 @@
 
 #include <cuda_runtime.h>
 
+#include "gpw_common.cuh"
+
 namespace gpw {
 
 // 8-byte aligned, so that shared-memory arrays of ff load and store as one
@@ -225,7 +227,7 @@ __constant__ float2 c_exp2_32[32] = {
 // 2^-45 while the result is a normal float with a normal low part (a > -60);
 // below, the low part underflows gradually; a.hi < -103 returns 0.  Valid for
 // a.hi < 88.
-__device__ __forceinline__ ff ff_exp(ff a) {
+__device__ __forceinline__ ff ff_exp(ff a, const float2 *tab) {  // tab: c_exp2_32, or its copy in shared memory
     if (a.hi < -103.0f) return {0.0f, 0.0f};
     const float kf = rintf(__fmul_rn(a.hi, 46.16624069213867f));
     const int k = (int)kf;
@@ -236,13 +238,15 @@ __device__ __forceinline__ ff ff_exp(ff a) {
                                            0.1666666716337204f));
     const ff h = fast_two_sum(0.5f, t);
     ff p = ff_add(ff_add(ff{1.0f, 0.0f}, r), ff_mul(ff_mul(r, r), h));
-    const float2 tj = c_exp2_32[k & 31];
+    const float2 tj = tab[k & 31];
     p = ff_mul(p, ff{tj.x, tj.y});
     // 2^m in two normal-range factors (m >= -149 here)
     const int m = k >> 5, m1 = m >> 1, m2 = m - m1;
     const float s1 = __int_as_float((127 + m1) << 23), s2 = __int_as_float((127 + m2) << 23);
     return {__fmul_rn(__fmul_rn(p.hi, s1), s2), __fmul_rn(__fmul_rn(p.lo, s1), s2)};
 }
+
+__device__ __forceinline__ ff ff_exp(ff a) { return ff_exp(a, c_exp2_32); }
 
 // Two exponentials at once, ff_exp operation by operation.  tab: c_exp2_32 in shared
 // memory (the lanes' indices differ: a constant-bank read would be replayed per value).
@@ -269,5 +273,78 @@ __device__ __forceinline__ ff2 ff2_exp(ff2 a, const float2 *tab) {
     const float2 s2 = make_float2(pw(m0 - u0), pw(m1 - u1));
     return {f2_mul(f2_mul(p.hi, s1), s2), f2_mul(f2_mul(p.lo, s1), s2)};
 }
+
+// ---------------------------------------------------------------------------
+// Where general_row_fast32 is unsure (0.6 % of the rows near a sphere at steps of 0.12,
+// so one warp in six): the same quadratic in float-float with its error bound; only
+// where that is unsure too the FP64 rule, some 150 instructions of the FP64 pipe.  (9.3e7
+// random rows, exact ties among them: no row differs from the FP64 rule.  1500 pairs,
+// 128^3, float-float kernel: 7.86 -> 7.65 ms; 8000 pairs, tiled: 17.6 -> 16.9 ms.)
+struct GeneralRowFF {
+    ff dh[3][3];   // lattice steps
+    ff a4, inv2a;  // 4 |v0|^2 and 1 / (2 |v0|^2)
+    float hmax;    // largest |dh|
+};
+__host__ __device__ inline ff ff_split(double d) {
+    const float h = (float)d;
+    return {h, (float)(d - (double)h)};
+}
+__host__ __device__ inline void general_row_constants(const double dh[3][3], GeneralRow32 &r, GeneralRowFF &f) {
+    const double a = dh[0][0] * dh[0][0] + dh[0][1] * dh[0][1] + dh[0][2] * dh[0][2];
+    f.hmax = 0.0f;
+    for (int i = 0; i < 3; i++)
+        for (int k = 0; k < 3; k++) {
+            r.dh[i][k] = (float)dh[i][k];
+            f.dh[i][k] = ff_split(dh[i][k]);
+            f.hmax = fmaxf(f.hmax, fabsf((float)dh[i][k]));
+        }
+    r.a = (float)a;
+    r.inv2a = (float)(0.5 / a);
+    f.a4 = ff_split(4.0 * a);
+    f.inv2a = ff_split(0.5 / a);
+}
+#if defined(__CUDACC__)
+// The row (jj, kk) of a box at cc: its i-range, decided by float-float where the bound
+// allows, else by FP64.
+__device__ __noinline__ inline bool general_row_unsure(const GeneralRowFF *G, const double dh[3][3], const double gp[3],
+                                                       int cc0, int jj, int kk, double radius, int &ismin, int &ismax) {
+    const ff g0 = ff_from_double_bits(gp[0]), g1 = ff_from_double_bits(gp[1]), g2 = ff_from_double_bits(gp[2]);
+    const ff mgi = ff_add(ff{(float)cc0, 0.0f}, ff{-g0.hi, -g0.lo});  // -(gp_0 - cc_0): i' = i - cc_0
+    const ff dj = ff_add(ff{(float)jj, 0.0f}, ff{-g1.hi, -g1.lo}), dk = ff_add(ff{(float)kk, 0.0f}, ff{-g2.hi, -g2.lo});
+    const ff rad = ff_from_double_bits(radius), r2 = ff_mul(rad, rad);
+    ff hb = {0.0f, 0.0f}, c = {0.0f, 0.0f};  // b / 2 and c
+#pragma unroll 1
+    for (int i = 0; i < 3; i++) {
+        const ff v = ff_add(ff_add(ff_mul(G->dh[2][i], dk), ff_mul(G->dh[1][i], dj)), ff_mul(mgi, G->dh[0][i]));
+        hb = ff_add(hb, ff_mul(v, G->dh[0][i]));
+        c = ff_add(c, ff_mul(v, v));
+    }
+    const ff b = {2.0f * hb.hi, 2.0f * hb.lo};
+    const ff d = ff_add(ff_mul(b, b), ff_mul(ff{-G->a4.hi, -G->a4.lo}, ff_add(c, ff{-r2.hi, -r2.lo})));
+    // every operation to 2^-44 of its operands; the largest are bounded by V
+    const float eps = 2.3e-13f;  // 2^-42
+    const float V = 3.0f * G->hmax * (fabsf(mgi.hi) + fabsf(dj.hi) + fabsf(dk.hi) +
+                                      fabsf(g0.hi) + fabsf(g1.hi) + fabsf(g2.hi) + 3.0f);
+    const float eb = 6.0f * eps * V * G->hmax;
+    const float ed = 2.0f * fabsf(b.hi) * eb + eb * eb + eps * (b.hi * b.hi + G->a4.hi * (6.0f * V * V + r2.hi));
+    bool unsure = fabsf(d.hi) <= 4.0f * ed || fabsf((float)jj) > 4.0e6f || fabsf((float)kk) > 4.0e6f || fabsf((float)cc0) > 4.0e6f;
+    if (!unsure && d.hi < 0.0f) return false;
+    if (!unsure) {
+        const float s0 = sqrtf(d.hi);
+        const float res = __fadd_rn(__fmaf_rn(-s0, s0, d.hi), d.lo);
+        const ff sd = fast_two_sum(s0, res / (2.0f * s0));
+        const ff lo = ff_mul(ff_add(ff{-b.hi, -b.lo}, ff{-sd.hi, -sd.lo}), G->inv2a);
+        const ff hi = ff_mul(ff_add(ff{-b.hi, -b.lo}, sd), G->inv2a);
+        const float er = 2.0f * (eb + ed / s0 + eps * (fabsf(b.hi) + s0)) * G->inv2a.hi + 1e-10f;
+        const float l0 = rintf(lo.hi), h0 = rintf(hi.hi);
+        const float lf = __fadd_rn(__fsub_rn(lo.hi, l0), lo.lo), hf = __fadd_rn(__fsub_rn(hi.hi, h0), hi.lo);  // from the nearest integer
+        unsure = fabsf(lf) <= er || fabsf(hf) <= er;
+        ismin = cc0 + (int)l0 + (lf > 0.0f ? 1 : 0);
+        ismax = cc0 + (int)h0 - (hf < 0.0f ? 1 : 0);
+    }
+    if (unsure) return general_row(dh, gp, rsub((double)jj, gp[1]), rsub((double)kk, gp[2]), radius, ismin, ismax);
+    return true;
+}
+#endif
 
 }  // namespace gpw

@@ -675,11 +675,9 @@ k_general_ff(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
     auto met = [&](int a, int b) { return lv.dh[a][0] * lv.dh[b][0] + lv.dh[a][1] * lv.dh[b][1] + lv.dh[a][2] * lv.dh[b][2]; };
     const double G01 = met(0, 1), G02 = met(0, 2), G11 = met(1, 1), G12 = met(1, 2), G22 = met(2, 2);
     const ff g00 = ff_from_double(met(0, 0));
-    GeneralRow32 R32;
-    for (int a = 0; a < 3; a++)
-        for (int b = 0; b < 3; b++) R32.dh[a][b] = (float)lv.dh[a][b];
-    R32.a = (float)met(0, 0);
-    R32.inv2a = (float)(0.5 / met(0, 0));
+    __shared__ GeneralRow32 R32;
+    __shared__ GeneralRowFF Rff;
+    if (tid == 0) general_row_constants(lv.dh, R32, Rff);
     const float gi = (float)(g.off[0] - (double)cc0), gj = (float)(g.off[1] - (double)cc1), gk = (float)(g.off[2] - (double)cc2);
     const float r2f = (float)(g.radius * g.radius);
     const ff2n mz = ff2n_dup(ff_from_double(-g.zetp));
@@ -728,7 +726,7 @@ k_general_ff(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
                     bool some = general_row_fast32(R32, gi, gj, gk, (float)(r0 + r) - gj, dkc, r2f, cc0, ismin, ismax,
                                                    unsure);
                     if (unsure)
-                        some = general_row_exact64(lv.dh, g.off, rsub((double)jj, g.off[1]), dk, g.radius, ismin, ismax);
+                        some = general_row_unsure(&Rff, lv.dh, g.off, cc0, jj, kk, g.radius, ismin, ismax);
                     if (!some || ismin > ismax) {
                         ismin = 1;
                         ismax = 0;

@@ -109,6 +109,7 @@ struct TPair {
 // rule, and the cosines between the steps (cross terms of the Gaussian).
 struct GenLevel {
     GeneralRow32 row;
+    GeneralRowFF rowff;
     ff c01, c02, c12;   // cos(v0, v1), cos(v0, v2), cos(v1, v2)
 };
 // A pair's blob: the record padded to kHdr16 16-byte chunks, then its
@@ -215,7 +216,7 @@ __device__ __forceinline__ void row_range(const TPair &p, const ImgState &q, con
 
 // General cell: the row (jj, kk) of the index box holds the points i with
 // |i v0 + w|^2 <= r^2 (the reference's quadratic, grid_base_ref_c.cc:781-807; FP32 with
-// an error bound, general_row_fast32 in gpw_common.cuh).
+// an error bound, then float-float, then FP64).
 __device__ __forceinline__ bool general_row_fast(const LevelDev &lv, const GenLevel &G, const TPair &p, int jj,
                                                  int kk, int &ismin, int &ismax) {
     const float gi = (float)(p.gp[0] - (double)p.cc[0]);
@@ -224,7 +225,7 @@ __device__ __forceinline__ bool general_row_fast(const LevelDev &lv, const GenLe
     const bool some = general_row_fast32(G.row, gi, gj, gk, (float)(jj - p.cc[1]) - gj, (float)(kk - p.cc[2]) - gk,
                                          p.r2f, p.cc[0], ismin, ismax, unsure);
     if (!unsure) return some;
-    return general_row_exact64(lv.dh, p.gp, rsub((double)jj, p.gp[1]), rsub((double)kk, p.gp[2]), p.radius, ismin, ismax);
+    return general_row_unsure(&G.rowff, lv.dh, p.gp, p.cc[0], jj, kk, p.radius, ismin, ismax);
 }
 
 // Row (z, y) of the tile for a general-cell pair: tile-local x range [x0, x1].
@@ -314,6 +315,7 @@ struct TileCommon {
     // the z table for packed products of two or four z: high parts, and both parts negated
     alignas(16) float Zh[kNPow][kMaxTZ], Znh[kNPow][kMaxTZ], Znl[kNPow][kMaxTZ];
     int tile;
+    float2 exptab[32];  // c_exp2_32: the lanes' indices differ, a constant-bank read would be replayed per value
     uint64_t mbar;
     uint32_t tmem;
     int abort;
@@ -511,7 +513,7 @@ struct TabEntry {
     bool in;    // inside the cube box and the tile's valid extent
 };
 __device__ __forceinline__ TabEntry tab_entry(const TPair &p, const ImgState &q, const TileExt &ext,
-                                              const TileShape &sh, int warp, int ent) {
+                                              const TileShape &sh, const float2 *exptab, int warp, int ent) {
     TabEntry r;
     const bool isy = ent < sh.TY;
     r.d = warp == 0 ? 0 : (isy ? 1 : 2);
@@ -519,7 +521,7 @@ __device__ __forceinline__ TabEntry tab_entry(const TPair &p, const ImgState &q,
     const int g = q.o[r.d] + r.i;
     r.in = r.i < (warp == 0 ? ext.x : (isy ? ext.y : ext.z)) && g >= p.lb[r.d] && g <= p.hi[r.d];
     r.t = ff_add(ff_mul_f(p.h[r.d], (float)g), ff{-p.off[r.d].hi, -p.off[r.d].lo});
-    r.e = r.in ? ff_exp(ff_mul(ff_mul(r.t, r.t), ff{-p.zetp.hi, -p.zetp.lo})) : ff{0.0f, 0.0f};
+    r.e = r.in ? ff_exp(ff_mul(ff_mul(r.t, r.t), ff{-p.zetp.hi, -p.zetp.lo}), exptab) : ff{0.0f, 0.0f};
     return r;
 }
 // warp 1: one y or z entry's powers: Y as float-float entries (collocate) or, as Z, in
@@ -695,17 +697,21 @@ __device__ __forceinline__ void slice_row16(const ff2 *vin, float sc, int kw, in
 
 // General cell: the cross factor along row (z, y) of the current image, E(x) =
 // exp(alpha + beta t0(x)) with beta = -2 zetp (c01 t1 + c02 t2), alpha = -2 zetp
-// c12 t1 t2: returns E(x0) and q = E(x + 1) / E(x).
-__device__ __forceinline__ void cross_factor_row(const GenLevel &G, const TPair &P, const ImgState &Q, int z, int y,
-                                                 int x0, ff &e0, ff &q) {
+// c12 t1 t2: returns E(x0), E(x0 + 1) as a pair and the factor q^2, q = E(x + 1) / E(x),
+// from one pair of x to the next (twice).  x0 is the even x at or before the row's first
+// cube point: at most one step outside the cube.
+__device__ __forceinline__ void cross_factor_row(const GenLevel &G, const TPair &P, const ImgState &Q,
+                                                 const float2 *exptab, int z, int y, int x0, ff2 &e, ff2n &q2) {
     const ff t1 = ff_add(ff_mul_f(P.h[1], (float)(Q.o[1] + y)), ff{-P.off[1].hi, -P.off[1].lo});
     const ff t2 = ff_add(ff_mul_f(P.h[2], (float)(Q.o[2] + z)), ff{-P.off[2].hi, -P.off[2].lo});
     const ff t0 = ff_add(ff_mul_f(P.h[0], (float)(Q.o[0] + x0)), ff{-P.off[0].hi, -P.off[0].lo});
     const ff m2z = {-2.0f * P.zetp.hi, -2.0f * P.zetp.lo};
     const ff beta = ff_mul(m2z, ff_add(ff_mul(G.c01, t1), ff_mul(G.c02, t2)));
     const ff alpha = ff_mul(m2z, ff_mul(G.c12, ff_mul(t1, t2)));
-    e0 = ff_exp(ff_add(alpha, ff_mul(beta, t0)));
-    q = ff_exp(ff_mul(beta, P.h[0]));
+    const ff2 eq = ff2_exp(ff2_pair(ff_add(alpha, ff_mul(beta, t0)), ff_mul(beta, P.h[0])), exptab);
+    const ff e0 = {eq.hi.x, eq.lo.x}, q = {eq.hi.y, eq.lo.y};
+    e = ff2_pair(e0, ff_mul(e0, q));
+    q2 = ff2n_dup(ff_mul(q, q));
 }
 
 // General cell, integrate: the A operand row r = the slices of V(x) E(x) over the
@@ -714,36 +720,41 @@ template <class Smem>
 __device__ __forceinline__ int general_a_row(Smem &sm, const GenLevel &G, const TPair &P, const ImgState &Q,
                                              const TileShape &sh, int r, int x0, int x1) {
     if (x0 > x1) return kZeroExp;  // the row's products are not read
-    ff e0, q;
-    cross_factor_row(G, P, Q, r >> sh.ly, r & (sh.TY - 1), x0, e0, q);
-    // pass 1: the row maximum of |V E|
+    ff2 e0;
+    ff2n q2;
+    const int xs = x0 & ~1;  // two x per instruction
+    cross_factor_row(G, P, Q, sm.c.exptab, r >> sh.ly, r & (sh.TY - 1), xs, e0, q2);
+    // pass 1: the row maximum of |V E| (the leading products)
     float mx = 0.0f;
     {
-        ff e = e0;
-        for (int x = x0; x <= x1; x++) {
-            mx = fmaxf(mx, fabsf(ff_mul(sm.Vff[x][r], e).hi));
-            e = ff_mul(e, q);
+        ff2 e = e0;
+#pragma unroll 2
+        for (int x = xs; x <= x1; x += 2) {
+            const float2 v = f2_mul(make_float2(sm.Vff[x][r].hi, sm.Vff[x + 1][r].hi), e.hi);
+            if (x >= x0) mx = fmaxf(mx, fabsf(v.x));
+            if (x < x1) mx = fmaxf(mx, fabsf(v.y));
+            e = ff2_mul(e, q2);
         }
     }
     const int vmx = exp_of(mx);
     const float sc = vmx == kZeroExp ? 0.0f : pow2i(SLB - vmx);
     // pass 2: slices, 16-byte chunks of 8 x
-    ff e = e0;
+    ff2 e = e0;
 #pragma unroll 1
     for (int c = 0; c < TX / 8; c++) {
         uint32_t w[NSL][4];
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            ff v2[2];
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int x = 8 * c + 2 * i + h;
-                const bool in = x >= x0 && x <= x1;
-                v2[h] = in ? ff_mul(sm.Vff[x][r], e) : ff{0.0f, 0.0f};
-                if (in) e = ff_mul(e, q);
+            const int x = 8 * c + 2 * i;
+            ff2 v = {f2(0.0f), f2(0.0f)};
+            if (x >= xs && x <= x1) {
+                v = ff2_mul(ff2_pair(sm.Vff[x][r], sm.Vff[x + 1][r]), ff2n_of(e));
+                if (x < x0) v.hi.x = v.lo.x = 0.0f;
+                if (x == x1) v.hi.y = v.lo.y = 0.0f;
+                e = ff2_mul(e, q2);
             }
             float2 sl[NSL];
-            slice_scaled2(ff2_pair(v2[0], v2[1]), f2(sc), sl);
+            slice_scaled2(v, f2(sc), sl);
 #pragma unroll
             for (int qq = 0; qq < NSL; qq++) w[qq][i] = pack_halves(sl[qq]);
         }
@@ -818,6 +829,7 @@ __device__ __forceinline__ void tc_setup(TileCommon &c, uint32_t ncols) {
         c.kmax = KP;  // operand buffers start uninitialised: write every slot once
     }
     if (threadIdx.x < 32) {
+        c.exptab[threadIdx.x] = c_exp2_32[threadIdx.x];
         tc::tmem_alloc(&c.tmem, ncols);
         tc::tmem_relinquish();
     }
@@ -1014,7 +1026,7 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                 if (warp < 2) {
 #pragma unroll 1
                     for (int ent = tid & 31; ent < (warp == 0 ? TX : TY + TZ); ent += 32) {
-                        const TabEntry te = tab_entry(P, Q, ext, sh, warp, ent);
+                        const TabEntry te = tab_entry(P, Q, ext, sh, cm.exptab, warp, ent);
                         if (warp == 0) {
                             ff2 xv[kNPair];
                             x_powers(P, Q, te, ent, true, xv);
@@ -1068,10 +1080,11 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                 tc_wait(cm, phase, A.status);
                 phase ^= 1u;
                 if (tid == 0) cm.kmax = L;  // read again only after the next barrier
-                // cross factor of the general cell along this row: E0 at x0, ratio q
-                ff ecur = {1.0f, 0.0f}, eq = {1.0f, 0.0f};
+                // cross factor of the general cell along this row, two x at a time
+                ff2 ecur = {f2(1.0f), f2(0.0f)};
+                ff2n eq = {};
                 if constexpr (kGeneral) {
-                    if (x0 <= x1) cross_factor_row(A.glv[td.level], P, Q, z, y, x0, ecur, eq);
+                    if (x0 <= x1) cross_factor_row(A.glv[td.level], P, Q, cm.exptab, z, y, x0 & ~1, ecur, eq);
                 }
                 // tcgen05.ld is warp-collective: chunk decisions are made per warp
                 if (__any_sync(0xffffffffu, x0 <= x1)) {
@@ -1126,12 +1139,10 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                                     float2 rem = f2_sub(corr, f2_sub(h0, d2));  // lo = rem scl exactly
                                     if constexpr (kGeneral) {
                                         const int x = 8 * c + 2 * i;
-                                        if (x > x0) ecur = ff_mul(ecur, eq);  // E(x) on the row's cube points
-                                        const ff v = ff_mul(ff{hi.x, __fmul_rn(rem.x, scl.x)}, ecur);
-                                        if (x + 1 > x0) ecur = ff_mul(ecur, eq);
-                                        const ff w = ff_mul(ff{hi.y, __fmul_rn(rem.y, scl.y)}, ecur);
-                                        hi = make_float2(v.hi, w.hi);
-                                        rem = make_float2(v.lo, w.lo);
+                                        if (x > x0 && x <= x1) ecur = ff2_mul(ecur, eq);  // E on the row's cube points
+                                        const ff2 v = ff2_mul(ff2{hi, f2_mul(rem, scl)}, ff2n_of(ecur));
+                                        hi = v.hi;
+                                        rem = v.lo;
                                         scl = f2(1.0f);
                                     }
                                     float2 &ah = acc_hi[4 * hh + i];
@@ -1305,7 +1316,7 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                     // collocate, integrate is not limited by instruction fetch: warps 0 and 1
                     // keep separate table code.
                     ff2 xv[kNPair];
-                    x_powers(P, Q, tab_entry(P, Q, ext, sh, 0, tid), tid, false, xv);
+                    x_powers(P, Q, tab_entry(P, Q, ext, sh, cm.exptab, 0, tid), tid, false, xv);
 #pragma unroll
                     for (int a = 0; a < kNPow; a += 2) {  // in pairs; xv[a] = 0 for a >= L
                         if (a >= L) break;
@@ -1333,7 +1344,7 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                     }
                 } else if (warp == 1) {
 #pragma unroll 1
-                    for (int ent = tid - 32; ent < TY + TZ; ent += 32) yz_fill(sm, P, tab_entry(P, Q, ext, sh, 1, ent));
+                    for (int ent = tid - 32; ent < TY + TZ; ent += 32) yz_fill(sm, P, tab_entry(P, Q, ext, sh, cm.exptab, 1, ent));
                 } else if constexpr (!kGeneral) {
                     mask_a_row(sm, tid - 64, sm.mask[tid - 64], sm.todo[tid - 64]);
                     mask_a_row(sm, tid, sm.mask[tid], sm.todo[tid]);
@@ -1851,10 +1862,7 @@ int mixed_build(TaskSet &ts, std::string &err) {
                           C[0][2] * (C[1][0] * C[2][1] - C[1][1] * C[2][0]);
         if (!(m1 > 0.0 && m2 > 0.0 && m3 > 0.0)) gen_ok = false;
         GenLevel &q = glv[l];
-        for (int a = 0; a < 3; a++)
-            for (int b = 0; b < 3; b++) q.row.dh[a][b] = (float)lv.dh[a][b];
-        q.row.a = (float)G[0][0];
-        q.row.inv2a = (float)(0.5 / G[0][0]);
+        general_row_constants(lv.dh, q.row, q.rowff);
         auto sp = [](double d) {
             const float hi = (float)d;
             return ff{hi, (float)(d - (double)hi)};
