@@ -131,8 +131,8 @@ __global__ void k_backtransform(const PairGeom *__restrict__ geoms, const LevelD
 // A CTA (4 warps) takes one item: every nparts-th plane of a pair's cube.  The
 // three 1-D tables are built once per CTA; after that the warps work alone, one
 // plane at a time, with no CTA barrier:
-//   lane = x column (blocks of 32 columns; the last block of 32, 16 or 8, with the
-//   warp's other lanes on the following rows), so that
+//   lane = x column (blocks of 32 columns in integrate, of 16 in collocate; the last one
+//   of 32, 16 or 8; the warp's other lanes on the following rows), so that
 //   collocate  T[ly] = sum_lx Cxy[ly][lx] X[lx][x] once per column, in registers,
 //              then rho(y, x) = sum_ly T[ly] Y[ly][y] per point, Y broadcast from
 //              shared memory, one FP64 reduction into the grid;
@@ -257,8 +257,10 @@ k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
     const int gn0 = lv.ngrid[0], gn1 = lv.ngrid[1];
     __syncthreads();
     // integrate's CTAs end with a sum over the warps: planes taken as warps come free (485
-    // -> 455 us on the workload above; collocate, whose warps end alone, loses 1 %)
-    for (int pl = kAdj ? next_plane(&s_next) : warp; pl < np; pl = kAdj ? next_plane(&s_next) : pl + kOrthoWarps) {
+    // -> 458 us on the workload above; collocate, whose warps end alone, loses 1 %)
+    for (int turn = warp;; turn += kOrthoWarps) {
+        const int pl = kAdj ? next_plane(&s_next) : turn;
+        if (pl >= np) break;
         const int kg = kgmin + it.part + pl * it.nparts, kf = fold(kg);
         const int k = axis_index(lv.periodic[2], g.cc[2], kg, g.lb[2], lv.lb_grid[2], lv.npts[2], lv.ngrid[2]);
         if (k < 0) {
@@ -299,7 +301,10 @@ k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
         const int nrow = 2 - 2 * jgmin, xend = 1 - wide;
         for (int c0 = wide; c0 <= xend;) {
             const int left = xend - c0 + 1;
-            const int lw = left > 16 ? 5 : (left > 8 ? 4 : 3);  // log2 of the block's columns
+            const int lw = kAdj && left > 16 ? 5 : (left > 8 ? 4 : 3);  // log2 of the block's columns
+            // (blocks of at most 32, 16, 8 columns: collocate 461, 453, 540 us on the workload
+            // above, integrate, with its planes taken in turn, 485, 488, 536: fewer idle lanes
+            // at a row's ends, but T anew per block)
             const int grp = lane >> lw, ng = 32 >> lw;          // the lane's row group
             const int ig = c0 + (lane & ((1 << lw) - 1)), xc = min(ig - lb0, nx - 1);
             const bool in = ig <= xend;

@@ -602,27 +602,6 @@ __constant__ int c_zs[kNPow][kNPow + 1] = {GPW_ZS(0), GPW_ZS(1), GPW_ZS(2), GPW_
 #undef ZS_
 #undef GPW_ZS
 
-// The (g, b, a) of packed index t of degree lp as g | b << 4 | a << 8 | pair_index << 16,
-// for all lp: read through L1 (a search of the slab starts in shared memory took up to
-// lp dependent loads; integrate's last stage, which ends every item: 59.6 -> 56.5 ms
-// with the table and with the moments joined to doubles on the integer pipe).
-constexpr int d_decode_at(int lp) { return lp * (lp + 1) * (lp + 2) * (lp + 3) / 24; }
-struct Decode {
-    uint32_t e[d_decode_at(kMaxLp + 1)];
-};
-constexpr Decode make_decode() {
-    Decode d{};
-    for (int lp = 0; lp <= kMaxLp; lp++) {
-        int t = d_decode_at(lp);
-        for (int g = 0; g <= lp; g++)
-            for (int b = 0; b <= lp - g; b++)
-                for (int a = 0; a <= lp - g - b; a++)
-                    d.e[t++] = (uint32_t)(g | b << 4 | a << 8 | (b * (lp + 1) - (b * (b - 1)) / 2 + a) << 16);
-    }
-    return d;
-}
-__device__ const Decode d_decode = make_decode();
-
 // One item (g, b, a) per thread of [t0, t0 + nt): Horner in tc over a' = amax .. a
 // with the binomials from shared memory (bin[a'][a] = C(a', a)).  The row coefficients'
 // balancing factor 2^(a sb) is applied here, once per coefficient.
