@@ -319,7 +319,6 @@ struct TileCommon {
     uint64_t mbar;
     uint32_t tmem;
     int abort;
-    int kmax;  // collocate: K slots of A written by the previous pair (zeroed up to here)
 };
 
 // Cxy rows b (L - b values of a) padded to an even length: start of row b
@@ -340,7 +339,7 @@ struct alignas(128) SmemColl {
     ff Y[kNPow][kMaxTY + 1];  // rows padded: lanes reading different rows hit different banks
     alignas(16) float acc_lo[MROWS][TX + 4];  // low parts of the tile sums (row m belongs to thread m; padded rows)
     float bin[kNPow][kNPow];    // binomials C(a', a) of the re-expansion
-    alignas(16) float cs[TX];   // 2^fx per column (0 for an empty column)
+    alignas(16) float cs[2][TX];  // 2^fx per column (0 for an empty column), of this item and the next
     unsigned char qpad[kNPow][2 * kCxyRow];  // qpad[L-1][padded index of (b, a)] = b | a << 4
     TileCommon c;
 };
@@ -805,7 +804,6 @@ __device__ __forceinline__ void tc_setup(TileCommon &c, uint32_t ncols) {
         tc::mbar_init(&c.mbar, 1);
         tc::fence_mbar_init();
         c.abort = 0;
-        c.kmax = KP;  // operand buffers start uninitialised: write every slot once
     }
     if (threadIdx.x < 32) {
         c.exptab[threadIdx.x] = c_exp2_32[threadIdx.x];
@@ -958,6 +956,7 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
     tc_setup(cm, kCols);
     const uint32_t tbase = cm.tmem + ((uint32_t)(warp * 32) << 16);
     uint32_t phase = 0;
+    int kprev = KP;  // K slots of A and B that the previous pair wrote (uninitialised at first: all)
     for (int t = tid; t < kNPow * kNPow; t += NTHR) sm.bin[t / kNPow][t % kNPow] = c_binom[t / kNPow][t % kNPow];
     for (int t = tid; t < kNPow * 2 * kCxyRow; t += NTHR) {
         const int Lq = t / (2 * kCxyRow) + 1, q = t % (2 * kCxyRow);
@@ -993,8 +992,9 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
         const int64_t it0 = A.start[2 * tile], it1 = A.start[2 * tile + 1];
         uint64_t nxt = 0;
         first_pair(cm, sm.pb, A, it0, it1, nxt, true);
-        for (int64_t it = it0; it < it1 && !cm.abort; it++) {
-            const int cur = next_pair(cm, sm.pb, A, it, it0, it1, nxt, true);
+        for (int64_t it = it0; it < it1; it++) {
+            const int cur = (int)((it - it0) & 1);
+            if constexpr (!kGeneral) next_pair(cm, sm.pb, A, it, it0, it1, nxt, true);
             const PairBuf &pb = sm.pb[cur];
             const TPair &P = pb.p;
             const int L = P.L, lp = P.lp;
@@ -1014,10 +1014,10 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                             for (int i = 0; i < kNPair; i++)
                                 mx = fmaxf(mx, fmaxf(fabsf(xv[i].hi.x), fabsf(xv[i].hi.y)));
                             const int e = exp_of(mx);
-                            sm.cs[tid] = e == kZeroExp ? 0.0f : pow2i(e);
+                            sm.cs[cur][tid] = e == kZeroExp ? 0.0f : pow2i(e);
                             const float sc = e == kZeroExp ? 0.0f : pow2i(SLB - e);
                             // K slots beyond L may hold an earlier pair's slices: rewritten as zeros
-                            slice_row16(xv, sc, max(L, cm.kmax), L, sm.B[0], TX * KP, tid);
+                            slice_row16(xv, sc, max(L, kprev), L, sm.B[0], TX * KP, tid);
                         } else {
                             yz_fill(sm, P, te);
                         }
@@ -1032,6 +1032,9 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                     stage1_cxy(sm, L, lp, sh);
                 }
                 __syncthreads();
+                if (cm.abort) break;  // uniform: set before this barrier or after the next one
+                // (general cell: every warp is done with the previous item's record here)
+                if constexpr (kGeneral) next_pair(cm, sm.pb, A, it, it0, it1, nxt, true);
                 // stage 2 (this thread's row, all a at once) + culling + A slices
                 int x0, x1;
                 if constexpr (kGeneral)
@@ -1039,8 +1042,13 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                                       x1);
                 else
                     row_range(P, Q, A.table, Q.o[2] + z, Q.o[1] + y, row_ok, x0, x1);
-                const int em = stage2_row(sm, cm, L, lp, z, y, x0 <= x1, max(L, cm.kmax), m);
+                const int em = stage2_row(sm, cm, L, lp, z, y, x0 <= x1, max(L, kprev), m);
                 // stage 3 on the tensor cores: D_s = sum_{i+j=s} A_i B_j^T
+                // What follows reads none of the tables, and the record only on general cells:
+                // the next item's record, waited for here, and its tables may come in as the
+                // warps finish their readout, and no barrier ends the item (64.2 -> 62.4 ms,
+                // 100k pairs, 256^3).
+                cp_async_wait_all();
                 tc::fence_async_smem();
                 tc::fence_before_sync();
                 __syncthreads();
@@ -1058,7 +1066,7 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                 }
                 tc_wait(cm, phase, A.status);
                 phase ^= 1u;
-                if (tid == 0) cm.kmax = L;  // read again only after the next barrier
+                kprev = L;
                 // cross factor of the general cell along this row, two x at a time
                 ff2 ecur = {f2(1.0f), f2(0.0f)};
                 ff2n eq = {};
@@ -1087,8 +1095,8 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                             const uint32_t mc = rmask >> (8 * c);
                             if (__any_sync(0xffffffffu, (mc & 0xFFu) != 0u)) {
                                 uint32_t r2[8], r3[8], r4[8], r5[8];
-                                const float4 csa = reinterpret_cast<const float4 *>(sm.cs)[2 * c];
-                                const float4 csb = reinterpret_cast<const float4 *>(sm.cs)[2 * c + 1];
+                                const float4 csa = reinterpret_cast<const float4 *>(sm.cs[cur])[2 * c];
+                                const float4 csb = reinterpret_cast<const float4 *>(sm.cs[cur])[2 * c + 1];
                                 const float2 csv[4] = {{csa.x, csa.y}, {csa.z, csa.w}, {csb.x, csb.y}, {csb.z, csb.w}};
                                 tc::tmem_ld8(tbase + 8 * c, r2);
                                 tc::tmem_ld8(tbase + 32 + 8 * c, r3);
@@ -1145,9 +1153,9 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                         for (int i = 0; i < 4 * kCh; i++) acc_hi[TX / 2 - 4 * kCh + i] = tr[i];
                     }
                 }
-                end_item();
             }
         }
+        __syncthreads();
         if (cm.abort) break;
         // flush: grid += tile sum (FP64)
         if (row_ok) {
