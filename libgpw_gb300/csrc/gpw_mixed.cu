@@ -312,8 +312,6 @@ struct alignas(16) PairHdr {
 // shared state of both tiled kernels
 struct TileCommon {
     ItemImg ii[2];  // the image of the current item and of the one being fetched
-    // the z table for packed products of two or four z: high parts, and both parts negated
-    alignas(16) float Zh[kNPow][kMaxTZ], Znh[kNPow][kMaxTZ], Znl[kNPow][kMaxTZ];
     int tile;
     float2 exptab[32];  // c_exp2_32: the lanes' indices differ, a constant-bank read would be replayed per value
     uint64_t mbar;
@@ -337,6 +335,8 @@ struct alignas(128) SmemColl {
     float4 Cxy[kMaxTZColl][kCxyRow];  // stage 1 output, pairs of a: {hi, hi, lo, lo}
     PairBuf pb[2];              // the current pair and the one being fetched
     ff Y[kNPow][kMaxTY + 1];  // rows padded: lanes reading different rows hit different banks
+    // the z table for packed products of two z: high parts, and both parts negated
+    alignas(16) float Zh[kNPow][kMaxTZ], Znh[kNPow][kMaxTZ], Znl[kNPow][kMaxTZ];
     alignas(16) float acc_lo[MROWS][TX + 4];  // low parts of the tile sums (row m belongs to thread m; padded rows)
     float bin[kNPow][kNPow];    // binomials C(a', a) of the re-expansion
     alignas(16) float cs[2][TX];  // 2^fx per column (0 for an empty column), of this item and the next
@@ -383,21 +383,18 @@ static_assert(kBPlane == 2 * kBSbo, "the planes follow one another along N");
 struct IntCommon {
     alignas(16) float Yh[kNPow][kYRow], Ynl[kNPow][kYRow];
     alignas(8) float gsc[KP];                // 2^(g - SLB), g the alpha row's exponent (0: an empty row)
-    unsigned char qb[kNPow][NPAIR_MAX + 2];  // qb[L-1][pair_index(L, b, a)] = b
     PairHdr pb[2];                           // the current pair's record and the one being fetched
     TileCommon c;
 };
 template <bool kGeneral>
 struct alignas(128) SmemInt : IntCommon {
     alignas(16) float Ynh[kNPow][kYRow];
+    alignas(16) float Zh[2][kNPow][kMaxTZ], Znl[2][kNPow][kMaxTZ];  // of this item and the next
     uint32_t mask[MROWS];          // each row's points inside the item's range
     uint8_t todo[MROWS];           // the chunks of its A row to be masked to them
     __half A[2][NSL][MROWS * KP];  // masked V slices, K halves x in [0,16) and [16,32)
-    IntSums st;
-    union {
-        alignas(16) unsigned char B[2 * kBHalf];  // X' slices: plane (h, q) at h kBHalf + q kBPlane
-        IntTsum tt;                               // after the MMAs have read B
-    };
+    IntSums st;                    // S, then T in the columns of S that a warp is done with
+    alignas(16) unsigned char B[2 * kBHalf];  // X' slices: plane (h, q) at h kBHalf + q kBPlane
 };
 template <>  // (without the plane of -Y: three CTAs per SM)
 struct alignas(128) SmemInt<true> : IntCommon {
@@ -409,6 +406,7 @@ struct alignas(128) SmemInt<true> : IntCommon {
         alignas(16) unsigned char B[2 * kBHalf];
         IntTsum tt;
     };
+    alignas(16) float Zh[1][kNPow][kMaxTZ], Znl[1][kNPow][kMaxTZ];
     ff Vff[TX][MROWS];  // this tile's V (x-major: lanes read consecutive rows)
 };
 static_assert(sizeof(IntTsum) <= 2 * kBHalf, "T fits in B");
@@ -526,15 +524,15 @@ __device__ __forceinline__ TabEntry tab_entry(const TPair &p, const ImgState &q,
 // warp 1: one y or z entry's powers: Y as float-float entries (collocate) or, as Z, in
 // three planes (high parts, both parts negated) for packed products
 template <class Smem>
-__device__ __forceinline__ void yz_fill(Smem &sm, const TPair &p, const TabEntry &te) {
+__device__ __forceinline__ void yz_fill(Smem &sm, const TPair &p, const TabEntry &te, int zbuf) {
     constexpr int kY = kYPlanes<Smem>;
     const bool isy = te.d == 1;
     const int L = te.in ? p.L : 0;
     ff e = te.e;
     if constexpr (kY == 0) {
-        float *hi = isy ? &sm.Y[0][te.i].hi : &sm.c.Zh[0][te.i], *lo = isy ? hi + 1 : &sm.c.Znl[0][te.i];
+        float *hi = isy ? &sm.Y[0][te.i].hi : &sm.Zh[0][te.i], *lo = isy ? hi + 1 : &sm.Znl[0][te.i];
         const int stride = isy ? 2 * (kMaxTY + 1) : kMaxTZ;
-        float *nhi = &sm.c.Znh[0][te.i];
+        float *nhi = &sm.Znh[0][te.i];
         const float sg = isy ? 1.0f : -1.0f;
 #pragma unroll 1
         for (int k = 0; k < kNPow; k++) {
@@ -544,14 +542,14 @@ __device__ __forceinline__ void yz_fill(Smem &sm, const TPair &p, const TabEntry
             e = ff_mul(e, te.t);
         }
     } else {
-        float *hi = isy ? &sm.Yh[0][te.i] : &sm.c.Zh[0][te.i];
-        float *nlo = isy ? &sm.Ynl[0][te.i] : &sm.c.Znl[0][te.i], *nhi = &sm.c.Znh[0][te.i];
-        if constexpr (kY == 3) nhi = isy ? &sm.Ynh[0][te.i] : nhi;
+        float *hi = isy ? &sm.Yh[0][te.i] : &sm.Zh[zbuf][0][te.i];
+        float *nlo = isy ? &sm.Ynl[0][te.i] : &sm.Znl[zbuf][0][te.i], *nhi = hi;
+        if constexpr (kY == 3) nhi = &sm.Ynh[0][te.i];
         const int stride = isy ? kYRow : kMaxTZ;
 #pragma unroll 1
         for (int k = 0; k < p.L; k++) {
             hi[k * stride] = k < L ? e.hi : 0.0f;
-            if (kY == 3 || !isy) nhi[k * stride] = k < L ? -e.hi : 0.0f;
+            if (kY == 3 && isy) nhi[k * stride] = k < L ? -e.hi : 0.0f;
             nlo[k * stride] = k < L ? -e.lo : 0.0f;
             e = ff_mul(e, te.t);
         }
@@ -870,7 +868,6 @@ __device__ __forceinline__ void first_pair(TileCommon &cm, Buf *pb, const MixedA
 // number of a (the padding gets zeros), so that stage 2 reads its pairs of a as
 // 16-byte entries {hi(a), hi(a+1), lo(a), lo(a+1)}.
 __device__ __forceinline__ void stage1_cxy(SmemColl &sm, int L, int lp, const TileShape &sh) {
-    const TileCommon &cm = sm.c;
     const int *zs = c_zs[lp];
     const int npad = 2 * (L >> 1) * ((L >> 1) + 1) + (L & 1) * (L + 1);  // cxy_pad_row(L, L)
     const unsigned char *qp = sm.qpad[L - 1];
@@ -880,8 +877,8 @@ __device__ __forceinline__ void stage1_cxy(SmemColl &sm, int L, int lp, const Ti
         const ff *c = sm.rc + (b * (lp + 1) - (b * (b - 1)) / 2 + a);
         ff2 s0 = {f2(0.0f), f2(0.0f)}, s1 = s0;
         auto zpair = [&](int g) {
-            return ff2n{*reinterpret_cast<const float2 *>(&cm.Zh[g][zz]), *reinterpret_cast<const float2 *>(&cm.Znh[g][zz]),
-                        *reinterpret_cast<const float2 *>(&cm.Znl[g][zz])};
+            return ff2n{*reinterpret_cast<const float2 *>(&sm.Zh[g][zz]), *reinterpret_cast<const float2 *>(&sm.Znh[g][zz]),
+                        *reinterpret_cast<const float2 *>(&sm.Znl[g][zz])};
         };
         int g = 0, bg = 0;
 #pragma unroll 1
@@ -1019,7 +1016,7 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                             // K slots beyond L may hold an earlier pair's slices: rewritten as zeros
                             slice_row16(xv, sc, max(L, kprev), L, sm.B[0], TX * KP, tid);
                         } else {
-                            yz_fill(sm, P, te);
+                            yz_fill(sm, P, te, 0);
                         }
                     }
                 } else {
@@ -1190,6 +1187,41 @@ __device__ __forceinline__ void acc_four(ff2 &s, float4 ah, float4 al, float4 bh
                  ff2n{make_float2(bh.z, bh.w), make_float2(bnh.z, bnh.w), make_float2(bnl.z, bnl.w)});
 }
 
+// Stage 1 transposed, orthorhombic: the moments W[g][b][a] += sum_z T[z][(b,a)] Z[g][z]
+// of an item of degree lp, by 96 threads (t0 of 96).  T lies in the columns of S that a
+// warp was done with: pass p of its (b,a) in row lp - p (see stage 2 transposed).  It is
+// a serial chain of loads and sums; run between barriers of its own it took 3.5 of 56 ms
+// of 100k pairs on 256^3, beside the next item's tables it takes none of the item's path.
+template <class Smem>
+__device__ __forceinline__ void add_moments(const Smem &sm, double *mom, int lp, int zbuf, const TileShape &sh, int t0) {
+    const int nc = ncoef(lp), lzw = 5 - sh.ly;
+    for (int t = t0; t < nc; t += 96) {
+        const uint32_t de = __ldg(&d_decode.e[d_decode_at(lp) + t]);  // (g, b, a) of packed index t
+        const int g = de & 15, pi = de >> 16;
+        const int p = pi >> (5 - lzw), col = (pi << lzw) & 31;
+        const float *th = sm.st.Sh[lp - p] + col, *tl = sm.st.Sl[lp - p] + col;
+        ff2 s2 = {f2(0.0f), f2(0.0f)};
+#pragma unroll 1
+        for (int z4 = 0; z4 < sh.TZ; z4 += 4) {
+            float4 h, l;
+            if (lzw) {  // two z per warp: (z, z + 1) in one column pair of warp z / 2
+                const float2 h0 = *reinterpret_cast<const float2 *>(th + 16 * z4), h1 = *reinterpret_cast<const float2 *>(th + 16 * z4 + 32);
+                const float2 l0 = *reinterpret_cast<const float2 *>(tl + 16 * z4), l1 = *reinterpret_cast<const float2 *>(tl + 16 * z4 + 32);
+                h = make_float4(h0.x, h0.y, h1.x, h1.y);
+                l = make_float4(l0.x, l0.y, l1.x, l1.y);
+            } else {  // one z per warp
+                h = make_float4(th[32 * z4], th[32 * z4 + 32], th[32 * z4 + 64], th[32 * z4 + 96]);
+                l = make_float4(tl[32 * z4], tl[32 * z4 + 32], tl[32 * z4 + 64], tl[32 * z4 + 96]);
+            }
+            const float4 zh = *reinterpret_cast<const float4 *>(&sm.Zh[zbuf][g][z4]);
+            acc_four(s2, h, l, zh, make_float4(-zh.x, -zh.y, -zh.z, -zh.w),
+                     *reinterpret_cast<const float4 *>(&sm.Znl[zbuf][g][z4]));
+        }
+        const ff s = ff_add(ff{s2.hi.x, s2.lo.x}, ff{s2.hi.y, s2.lo.y});
+        if (s.hi != 0.0f) atomicAdd(mom + t, ff_to_double_bits(s));
+    }
+}
+
 // kGeneral: tiles of general-cell levels; the A operand holds the slices of
 // V(x) E(x) (E the cross factor of the Gaussian along the row), one row per
 // thread, with its own exponent per row and image.
@@ -1205,12 +1237,6 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
     tc_setup(cm, kCols);
     const uint32_t tbase = cm.tmem + ((uint32_t)(warp * 32) << 16);
     uint32_t phase = 0;
-    for (int t = tid; t < kNPow * (NPAIR_MAX + 2); t += NTHR) {
-        const int Lq = t / (NPAIR_MAX + 2) + 1, q = t % (NPAIR_MAX + 2);
-        int b = 0, r = q;
-        while (b < Lq && r >= Lq - b) r -= Lq - b++;
-        sm.qb[Lq - 1][q] = (unsigned char)min(b, kNPow - 1);
-    }
     // B rows alpha >= L are never written: start them finite (zero)
     for (int t = tid; t < (int)(sizeof(sm.B) / sizeof(uint4)); t += NTHR)
         reinterpret_cast<uint4 *>(sm.B)[t] = make_uint4(0u, 0u, 0u, 0u);
@@ -1283,7 +1309,11 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
             sm.todo[m] = chunks_to_mask(M, have);
             __syncthreads();
         }
-        for (int64_t it = it0; it < it1 && !cm.abort; it++) {
+        // orthorhombic: the item whose moments are still to be added (by warps 1-3, while
+        // warp 0 makes the next item's B): its degree and moments
+        int lp_done = -1;
+        double *mom_done = nullptr;
+        for (int64_t it = it0; it < it1; it++) {
             const int cur = next_pair(cm, sm.pb, A, it, it0, it1, nxt, false);
             const TPair &P = sm.pb[cur].p;
             const int L = P.L, lp = P.lp;
@@ -1331,8 +1361,12 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                     }
                 } else if (warp == 1) {
 #pragma unroll 1
-                    for (int ent = tid - 32; ent < TY + TZ; ent += 32) yz_fill(sm, P, tab_entry(P, Q, ext, sh, cm.exptab, 1, ent));
+                    for (int ent = tid - 32; ent < TY + TZ; ent += 32)
+                        yz_fill(sm, P, tab_entry(P, Q, ext, sh, cm.exptab, 1, ent), kGeneral ? 0 : cur);
+                    if constexpr (!kGeneral)
+                        if (lp_done >= 0) add_moments(sm, mom_done, lp_done, cur ^ 1, sh, tid + 32);
                 } else if constexpr (!kGeneral) {
+                    if (lp_done >= 0) add_moments(sm, mom_done, lp_done, cur ^ 1, sh, tid - 64);
                     mask_a_row(sm, tid - 64, sm.mask[tid - 64], sm.todo[tid - 64]);
                     mask_a_row(sm, tid, sm.mask[tid], sm.todo[tid]);
                 }
@@ -1417,11 +1451,17 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                 // sums, over even and odd y, as one packed sum
                 const int lzw = 5 - sh.ly;  // log2 of the z values per warp
                 const int zbase = (warp * 32) >> sh.ly;
-                const unsigned char *qbL = sm.qb[L - 1];
-                for (int t = tid & 31; t < (npair << lzw); t += 32) {
+                // T: general cell in [q][z]; orthorhombic, pass p of a warp's (q, z) in its 32
+                // columns of S's row lp - p, which its later (b, a) don't read: the pairs with
+                // b <= p, the only ones with a = lp - p, are among the first 16 (p + 1)
+                int row = lp;
+                const int nt = npair << lzw;
+                for (int tt = tid & 31; tt < (kGeneral ? nt : nt + (tid & 31)); tt += 32, row--) {
+                    const int t = kGeneral ? tt : min(tt, nt - 1);  // (all lanes come to the warp barrier)
                     const int zz = zbase + (t & ((1 << lzw) - 1));
-                    const int q = t >> lzw, b = qbL[q];  // q = pair_index(L, b, a)
-                    const int a = q - (b * L - (b * (b - 1)) / 2);
+                    const int q = t >> lzw;  // pair_index(L, b, a)
+                    const uint32_t de = __ldg(&d_decode.e[d_decode_at(lp) + q]);  // (0, b, a)
+                    const int b = (de >> 4) & 15, a = (de >> 8) & 15;
                     const float4 *ph = reinterpret_cast<const float4 *>(&sm.st.Sh[a][zz * TY]);
                     const float4 *pl = reinterpret_cast<const float4 *>(&sm.st.Sl[a][zz * TY]);
                     const float4 *yh = reinterpret_cast<const float4 *>(sm.Yh[b]);
@@ -1436,33 +1476,46 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                         acc_four(s, ph[y4], pl[y4], yh[y4], nh, ynl[y4]);
                     }
                     const ff r = ff_add(ff{s.hi.x, s.lo.x}, ff{s.hi.y, s.lo.y});
-                    sm.tt.Th[q][zz] = r.hi;
-                    sm.tt.Tl[q][zz] = r.lo;
+                    if constexpr (kGeneral) {
+                        sm.tt.Th[q][zz] = r.hi;
+                        sm.tt.Tl[q][zz] = r.lo;
+                    } else {
+                        __syncwarp();  // the pass's reads of S come first
+                        sm.st.Sh[row][m] = r.hi;
+                        sm.st.Sl[row][m] = r.lo;
+                    }
                 }
+                if constexpr (!kGeneral) cp_async_wait_all();  // A rows restored for the next item, masked after this
                 __syncthreads();
+                if (cm.abort) break;  // uniform: set before this barrier or after the next one
+                if constexpr (!kGeneral) {
+                    lp_done = lp;
+                    mom_done = A.mom + moff;
+                    continue;
+                }
                 // stage 1 transposed: W[g][b][a] += sum_z T[z][(b,a)] Z[g][z]
                 const int nc = ncoef(lp);
-                for (int t = tid; t < nc; t += NTHR) {
+                for (int t = tid; t < nc && kGeneral; t += NTHR) {
                     const uint32_t de = __ldg(&d_decode.e[d_decode_at(lp) + t]);  // (g, b, a) of packed index t
-                    const int g = de & 15, pi = de >> 16;
-                    [[maybe_unused]] const int b = (de >> 4) & 15, a = (de >> 8) & 15;
+                    const int g = de & 15, b = (de >> 4) & 15, a = (de >> 8) & 15, pi = de >> 16;
                     ff2 s2 = {f2(0.0f), f2(0.0f)};
+                    if constexpr (kGeneral) {
 #pragma unroll 1
-                    for (int z4 = 0; z4 < TZ; z4 += 4)
-                        acc_four(s2, *reinterpret_cast<const float4 *>(&sm.tt.Th[pi][z4]),
-                                 *reinterpret_cast<const float4 *>(&sm.tt.Tl[pi][z4]),
-                                 *reinterpret_cast<const float4 *>(&cm.Zh[g][z4]),
-                                 *reinterpret_cast<const float4 *>(&cm.Znh[g][z4]),
-                                 *reinterpret_cast<const float4 *>(&cm.Znl[g][z4]));
+                        for (int z4 = 0; z4 < TZ; z4 += 4) {
+                            const float4 zh = *reinterpret_cast<const float4 *>(&sm.Zh[0][g][z4]);
+                            acc_four(s2, *reinterpret_cast<const float4 *>(&sm.tt.Th[pi][z4]),
+                                     *reinterpret_cast<const float4 *>(&sm.tt.Tl[pi][z4]), zh,
+                                     make_float4(-zh.x, -zh.y, -zh.z, -zh.w),
+                                     *reinterpret_cast<const float4 *>(&sm.Znl[0][g][z4]));
+                        }
+                    }
                     const ff s = ff_add(ff{s2.hi.x, s2.lo.x}, ff{s2.hi.y, s2.lo.y});
                     if (s.hi != 0.0f) {
                         double val = ff_to_double_bits(s);
-                        if constexpr (kGeneral) {
-                            // moments in powers of t_d = d_d |v_d| -> lattice-index powers d_d
-                            for (int e = 0; e < a; e++) val *= P.hx;
-                            for (int e = 0; e < b; e++) val *= P.hy;
-                            for (int e = 0; e < g; e++) val *= P.hz;
-                        }
+                        // moments in powers of t_d = d_d |v_d| -> lattice-index powers d_d
+                        for (int e = 0; e < a; e++) val *= P.hx;
+                        for (int e = 0; e < b; e++) val *= P.hy;
+                        for (int e = 0; e < g; e++) val *= P.hz;
                         atomicAdd(A.mom + moff + t, val);
                     }
                 }
@@ -1470,6 +1523,8 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
             }
         }
         if (cm.abort) break;
+        if constexpr (!kGeneral)  // the last item's (the next tile starts with a barrier)
+            if (warp >= 1 && lp_done >= 0) add_moments(sm, mom_done, lp_done, (int)((it1 - 1 - it0) & 1), sh, warp == 1 ? tid + 32 : tid - 64);
     }
     tc_teardown(cm, kCols, phase);
 }

@@ -54,3 +54,16 @@ def test_too_many_images():
     with pytest.raises(capi.GpwError) as e:
         run_collocate(wl, "mixed")
     assert e.value.status == 4  # GPW_ERR_UNSUPPORTED
+
+
+# every degree of the summed moments, both tile shapes
+@pytest.mark.parametrize("l", range(5))
+@pytest.mark.parametrize("tz", [4, 8])
+def test_integrate_degrees(l, tz, oracle_lib):
+    wl = T.synthetic("degrees", 10, l, (0.4, 2.0), 9.0, [(35, 40, 27)], 50 + l, lmin=max(l - 1, 0))
+    plan = capi.Plan(wl.levels)
+    ts = capi.TaskSet.from_workload(plan, wl)
+    ts.set_tiles([tz])
+    V = wl.potentials(seed=3)
+    hab = oracle_lib.batch(wl, V=V)
+    assert np.abs(run_integrate(wl, V, "mixed", ts=ts, plan=plan) - hab).max() <= TOL * np.abs(hab).max()
