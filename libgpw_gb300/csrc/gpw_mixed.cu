@@ -100,7 +100,8 @@ struct TPair {
     ff h[3];
     int lb[3], hi[3], cc[3];
     int kgmin, lp, L;
-    int general, pad_;  // general cell: box-relative cube (lb = 0), lattice-step lengths in h
+    float gpf[3];       // general: gp - cc as FP32 (once per pair: FP64 conversions per row are slow)
+    int general;        // general cell: box-relative cube (lb = 0), lattice-step lengths in h
     int64_t coef_off, table_off;
     double gp[3];       // general: the product centre in lattice coordinates (dh_inv^T rp)
     double radius;      // general: the cube radius (the row rule squares it itself)
@@ -219,11 +220,9 @@ __device__ __forceinline__ void row_range(const TPair &p, const ImgState &q, con
 // an error bound, then float-float, then FP64).
 __device__ __forceinline__ bool general_row_fast(const LevelDev &lv, const GenLevel &G, const TPair &p, int jj,
                                                  int kk, int &ismin, int &ismax) {
-    const float gi = (float)(p.gp[0] - (double)p.cc[0]);
-    const float gj = (float)(p.gp[1] - (double)p.cc[1]), gk = (float)(p.gp[2] - (double)p.cc[2]);
     bool unsure;
-    const bool some = general_row_fast32(G.row, gi, gj, gk, (float)(jj - p.cc[1]) - gj, (float)(kk - p.cc[2]) - gk,
-                                         p.r2f, p.cc[0], ismin, ismax, unsure);
+    const bool some = general_row_fast32(G.row, p.gpf[0], p.gpf[1], p.gpf[2], (float)(jj - p.cc[1]) - p.gpf[1],
+                                         (float)(kk - p.cc[2]) - p.gpf[2], p.r2f, p.cc[0], ismin, ismax, unsure);
     if (!unsure) return some;
     return general_row_unsure(&G.rowff, lv.dh, p.gp, p.cc[0], jj, kk, p.radius, ismin, ismax);
 }
@@ -1497,7 +1496,7 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                 const int nc = ncoef(lp);
                 for (int t = tid; t < nc && kGeneral; t += NTHR) {
                     const uint32_t de = __ldg(&d_decode.e[d_decode_at(lp) + t]);  // (g, b, a) of packed index t
-                    const int g = de & 15, b = (de >> 4) & 15, a = (de >> 8) & 15, pi = de >> 16;
+                    const int g = de & 15, pi = de >> 16;
                     ff2 s2 = {f2(0.0f), f2(0.0f)};
                     if constexpr (kGeneral) {
 #pragma unroll 1
@@ -1510,14 +1509,7 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                         }
                     }
                     const ff s = ff_add(ff{s2.hi.x, s2.lo.x}, ff{s2.hi.y, s2.lo.y});
-                    if (s.hi != 0.0f) {
-                        double val = ff_to_double_bits(s);
-                        // moments in powers of t_d = d_d |v_d| -> lattice-index powers d_d
-                        for (int e = 0; e < a; e++) val *= P.hx;
-                        for (int e = 0; e < b; e++) val *= P.hy;
-                        for (int e = 0; e < g; e++) val *= P.hz;
-                        atomicAdd(A.mom + moff + t, val);
-                    }
+                    if (s.hi != 0.0f) atomicAdd(A.mom + moff + t, ff_to_double_bits(s));
                 }
                 end_item();
             }
@@ -1563,6 +1555,29 @@ __global__ void k_coef_to_blob(const double *__restrict__ c, uint4 *blob, const 
             }
             const float h = __double2float_rn(d);
             dst[t] = make_float2(h, __double2float_rn(d - (double)h));
+        }
+    }
+}
+
+// General-cell pairs [k0, k1) of an integrate call: the summed moments, in powers of
+// t_d = d_d |v_d|, to powers of the lattice indices d_d; one warp per pair.  (As FP64
+// products of every item's sums, up to 3 lp of them in line at 17 cycles a warp, they
+// were a fifth of the integrate kernel.)
+__global__ void k_scale_moments(double *mom, const uint4 *__restrict__ blob, const int64_t *__restrict__ off16,
+                                int64_t k0, int64_t k1) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t k = k0 + blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); k < k1; k += nw) {
+        const TPair *p = reinterpret_cast<const TPair *>(blob + off16[k]);
+        double *w = mom + p->coef_off;
+        const int lp = p->lp, nc = ncoef(lp);
+        for (int t = lane; t < nc; t += 32) {
+            const uint32_t de = __ldg(&d_decode.e[d_decode_at(lp) + t]);  // (g, b, a) of packed index t
+            double v = w[t];
+            for (int e = de >> 8 & 15; e > 0; e--) v *= p->hx;
+            for (int e = de >> 4 & 15; e > 0; e--) v *= p->hy;
+            for (int e = de & 15; e > 0; e--) v *= p->hz;
+            w[t] = v;
         }
     }
 }
@@ -1841,6 +1856,7 @@ __global__ void k_make_records(const PairGeom *__restrict__ geoms, int64_t nbin,
                 p.hi[d] = g.hi[d] - g.cc[d];
                 p.cc[d] = g.cc[d];
                 p.gp[d] = g.off[d];
+                p.gpf[d] = (float)(g.off[d] - (double)p.cc[d]);
             }
             p.table_off = -1;
         } else {
@@ -2258,6 +2274,10 @@ cudaError_t launch_integrate_mixed(const TaskSet &ts, const GridPtrs &g, cudaStr
             ProfScope prof(ts, s);
             k_integrate_tiled<true><<<std::min(ntg, M.sms * M.per_sm_ig), NTHR, sizeof(SmemInt<true>), s>>>(
                 make_args(ts, g, 1, true));
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            ts.n_kernels++;
+            k_scale_moments<<<(unsigned)std::min<int64_t>((M.nbin - M.northo + 7) / 8, 8192), 256, 0, s>>>(
+                ts.d_mom, M.d_blob, M.d_blob_off, M.northo, M.nbin);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
     }
