@@ -158,7 +158,7 @@ struct MixedState {
     int grid_ctas_i = 0;  // integrate
     int sms = 0;
     int per_sm = 0, per_sm_i = 0, per_sm_ig = 0;  // resident CTAs: collocate, integrate (ortho, general)
-    uint4 *d_vslot = nullptr;  // orthorhombic integrate: per-CTA V slots
+    uint4 *d_vslot = nullptr;  // integrate: per-CTA V slots
     // binning state kept for re-binning on the device (gpw_taskset_update_geometry)
     std::vector<TileDesc> h_tiles;  // every tile of the binned levels, in tile-index order
     struct BinLevel *d_bl = nullptr;  // per level: first tile index, tiles per axis, tile shape
@@ -244,9 +244,6 @@ __device__ __forceinline__ void general_row_range(const LevelDev &lv, const GenL
 // (8 halves of K).  Element (row r, k) of an operand with R rows, K = 16:
 //   byte offset = (r / 8) * SBO + (k / 8) * LBO + (r % 8) * 16 + (k % 8) * 2,
 // LBO = 128 (next 8 K-elements), SBO = 256 (next 8 rows).
-__device__ __forceinline__ int umma_off(int r, int k) {
-    return (r >> 3) * 256 + (k >> 3) * 128 + (r & 7) * 16 + (k & 7) * 2;
-}
 
 constexpr int kZeroExp = -1000;
 // 2^k as a float, -126 <= k <= 127
@@ -284,7 +281,7 @@ struct MixedArgs {
     const int *table;
     const GenLevel *glv;  // general levels: FP32 steps, cosines
     double *mom;  // integrate: per-pair moments
-    uint4 *vslot;  // orthorhombic integrate: one slot of kVSlot16 chunks per CTA (the tile's V slices)
+    uint4 *vslot;  // integrate: one slot of kVSlot16 chunks per CTA (the tile's V)
     GridPtrs grids;
     int *queue;
     int *status;
@@ -345,12 +342,13 @@ struct alignas(128) SmemColl {
 
 static_assert(4 * (sizeof(SmemColl) + 1024) <= 228 * 1024, "4 collocate CTAs per SM");
 
-// The V slices of the tile an orthorhombic integrate CTA works on stand in its A
-// operand; each pair zeroes what lies outside its rows' ranges, and restores it
-// afterwards from a copy of the slices (the A operand's layout, both K halves) in a
-// 32 KB per-CTA global slot that stays in L2.  General cells keep V as float-float in
-// shared memory (the rows are rescaled per image) and build A anew each time, so their
-// S and T may lie in A once the MMAs have read it.
+// Integrate keeps the tile's V in a 32 KB per-CTA global slot that stays in L2.
+// Orthorhombic: V's slices stand in the A operand; each pair zeroes what lies outside its
+// rows' ranges, and restores it afterwards from the slot, a copy of the slices in the A
+// operand's layout (both K halves).  General cells rescale the rows per image: A is built
+// anew from V as float-float in the slot, [x pair][row], read one 16-byte chunk group
+// ahead.  (With V in shared memory three CTAs fitted an SM, and S and T had to share the
+// operands' memory: 7.47 ms for 8000 pairs on 128^3, 7.13 with four.)
 constexpr int kVSlot16 = 2 * NSL * MROWS * KP / 8;
 
 // Integrate's tables and sums for packed products of four y or z (16-byte loads):
@@ -361,10 +359,6 @@ constexpr int kSRow = MROWS + 4;
 struct IntSums {
     alignas(16) float Sh[kNPow][kSRow], Sl[kNPow][kSRow];
 };
-struct IntTsum {
-    alignas(16) float Th[NPAIR_MAX][kMaxTZ], Tl[NPAIR_MAX][kMaxTZ];
-};
-
 // Integrate's B operand (N = 16 alpha x K = 16 x per half, per slice): core
 // matrices 160 bytes apart along K and 288 along N, the second K half 64 bytes
 // further on.  Warp 0 stores one alpha row at a time, lane (h, k) the 2-byte
@@ -379,59 +373,28 @@ __host__ __device__ constexpr int b_off(int row, int k) {    // bytes within a p
 static_assert(b_off(15, 15) + 2 <= kBPlane && kBPlane % 16 == 0 && kBHalf % 16 == 0, "B planes");
 static_assert(kBPlane == 2 * kBSbo, "the planes follow one another along N");
 
-struct IntCommon {
+struct alignas(128) SmemInt {
     alignas(16) float Yh[kNPow][kYRow], Ynl[kNPow][kYRow];
     alignas(8) float gsc[KP];                // 2^(g - SLB), g the alpha row's exponent (0: an empty row)
     PairHdr pb[2];                           // the current pair's record and the one being fetched
     TileCommon c;
-};
-template <bool kGeneral>
-struct alignas(128) SmemInt : IntCommon {
     alignas(16) float Ynh[kNPow][kYRow];
     alignas(16) float Zh[2][kNPow][kMaxTZ], Znl[2][kNPow][kMaxTZ];  // of this item and the next
-    uint32_t mask[MROWS];          // each row's points inside the item's range
+    uint32_t mask[MROWS];          // orthorhombic: each row's points inside the item's range
     uint8_t todo[MROWS];           // the chunks of its A row to be masked to them
-    __half A[2][NSL][MROWS * KP];  // masked V slices, K halves x in [0,16) and [16,32)
+    __half A[2][NSL][MROWS * KP];  // slices of V (times the cross factor), K halves x in [0,16) and [16,32)
     IntSums st;                    // S, then T in the columns of S that a warp is done with
     alignas(16) unsigned char B[2 * kBHalf];  // X' slices: plane (h, q) at h kBHalf + q kBPlane
 };
-template <>  // (without the plane of -Y: three CTAs per SM)
-struct alignas(128) SmemInt<true> : IntCommon {
-    union {
-        __half A[2][NSL][MROWS * KP];
-        IntSums st;  // after the MMAs have read A
-    };
-    union {
-        alignas(16) unsigned char B[2 * kBHalf];
-        IntTsum tt;
-    };
-    alignas(16) float Zh[1][kNPow][kMaxTZ], Znl[1][kNPow][kMaxTZ];
-    ff Vff[TX][MROWS];  // this tile's V (x-major: lanes read consecutive rows)
-};
-static_assert(sizeof(IntTsum) <= 2 * kBHalf, "T fits in B");
-static_assert(3 * (sizeof(SmemInt<true>) + 1024) <= 228 * 1024, "3 general-cell integrate CTAs per SM");
 // planes of the y table: none (collocate: float-float entries), high and negated low, and -Y.hi
 template <class Smem>
 constexpr int kYPlanes = 3;
 template <>
 constexpr int kYPlanes<SmemColl> = 0;
-template <>
-constexpr int kYPlanes<SmemInt<true>> = 2;
-// dynamic shared memory of the orthorhombic integrate CTAs: at least 46 KB, so
-// that no fifth CTA (for which TMEM has no columns left) is placed on an SM
-constexpr size_t kSmemIntOrtho = sizeof(SmemInt<false>) > 46 * 1024 ? sizeof(SmemInt<false>) : 46 * 1024;
-static_assert(kSmemIntOrtho + 1024 <= 228 * 1024 / 4, "4 orthorhombic integrate CTAs per SM");
-static_assert(5 * (kSmemIntOrtho + 1024) > 228 * 1024, "at most 4 orthorhombic integrate CTAs per SM");
-
-// pair index of (b, a), b + a <= lp, rows of constant b
-__device__ __forceinline__ int pair_index(int L, int b, int a) { return b * L - (b * (b - 1)) / 2 + a; }
-
-// packed index of (g, b, 0) in closed form: sum_{z<g} (lp-z+1)(lp-z+2)/2 + sum_{y<b} (lp-g-y+1)
-__device__ __forceinline__ int row_start(int lp, int g, int b) {
-    const int n1 = lp + 1, n2 = lp + 1 - g;
-    const int q = lp - g;
-    return (n1 * (n1 + 1) * (n1 + 2) - n2 * (n2 + 1) * (n2 + 2)) / 6 + b * (q + 1) - (b * (b - 1)) / 2;
-}
+// dynamic shared memory of integrate: more than 46 KB, so that no fifth CTA (for which
+// TMEM has no columns left) is placed on an SM
+static_assert(4 * (sizeof(SmemInt) + 1024) <= 228 * 1024, "4 integrate CTAs per SM");
+static_assert(5 * (sizeof(SmemInt) + 1024) > 228 * 1024, "at most 4 integrate CTAs per SM");
 
 // ---- asynchronous record copies (cp.async, 16-byte chunks, L2 only)
 __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
@@ -542,26 +505,24 @@ __device__ __forceinline__ void yz_fill(Smem &sm, const TPair &p, const TabEntry
         }
     } else {
         float *hi = isy ? &sm.Yh[0][te.i] : &sm.Zh[zbuf][0][te.i];
-        float *nlo = isy ? &sm.Ynl[0][te.i] : &sm.Znl[zbuf][0][te.i], *nhi = hi;
-        if constexpr (kY == 3) nhi = &sm.Ynh[0][te.i];
+        float *nlo = isy ? &sm.Ynl[0][te.i] : &sm.Znl[zbuf][0][te.i], *nhi = &sm.Ynh[0][te.i];
         const int stride = isy ? kYRow : kMaxTZ;
 #pragma unroll 1
         for (int k = 0; k < p.L; k++) {
             hi[k * stride] = k < L ? e.hi : 0.0f;
-            if (kY == 3 && isy) nhi[k * stride] = k < L ? -e.hi : 0.0f;
+            if (isy) nhi[k * stride] = k < L ? -e.hi : 0.0f;
             nlo[k * stride] = k < L ? -e.lo : 0.0f;
             e = ff_mul(e, te.t);
         }
     }
 }
-// warp 0: the x column of entry x in registers, xv[i] the powers 2 i and 2 i + 1: of u
-// (collocate: recentre) or of t (integrate); each step multiplies a pair by u^2.
-__device__ __forceinline__ void x_powers(const TPair &p, const ImgState &q, const TabEntry &te, int x, bool recentre,
-                                         ff2 *xv) {
+// collocate, warp 0: the x column of entry x in registers, xv[i] the powers 2 i and 2 i + 1
+// of u; each step multiplies a pair by u^2.
+__device__ __forceinline__ void x_powers(const TPair &p, const ImgState &q, const TabEntry &te, int x, ff2 *xv) {
 #pragma unroll
     for (int i = 0; i < kNPair; i++) xv[i] = ff2{f2(0.0f), f2(0.0f)};
     if (!te.in) return;
-    const ff u = recentre ? ff_mul_f(p.h[0], ldexpf((float)(x - q.ic), -q.sb)) : te.t;
+    const ff u = ff_mul_f(p.h[0], ldexpf((float)(x - q.ic), -q.sb));
     const ff2n u2 = ff2n_dup(ff_mul(u, u));
     ff2 e = ff2_pair(te.e, ff_mul(te.e, u));
 #pragma unroll
@@ -648,7 +609,7 @@ __device__ __forceinline__ void slice_row16(const ff2 *vin, float sc, int kw, in
 #pragma unroll 1
     for (int kg = 0; kg < KP / 8; kg++) {
         if (8 * kg >= kw) break;
-        const int o16 = (row >> 3) * 16 + kg * 8 + (row & 7);  // umma_off(row, 8 kg) / 16
+        const int o16 = (row >> 3) * 16 + kg * 8 + (row & 7);  // offset of (row, 8 kg) / 16
         if (8 * kg >= nval) {  // only zeros left: rewrite the stale slots without slicing
 #pragma unroll
             for (int q = 0; q < NSL; q++) reinterpret_cast<uint4 *>(plane0 + q * plane_halves)[o16] = make_uint4(0, 0, 0, 0);
@@ -691,24 +652,41 @@ __device__ __forceinline__ void cross_factor_row(const GenLevel &G, const TPair 
 
 // General cell, integrate: the A operand row r = the slices of V(x) E(x) over the
 // row's cube points [x0, x1] (zero elsewhere), with the row's own exponent (returned).
+// V (float-float, two x per 16 bytes) comes from the CTA's slot, 8 x ahead of their use.
 template <class Smem>
-__device__ __forceinline__ int general_a_row(Smem &sm, const GenLevel &G, const TPair &P, const ImgState &Q,
-                                             const TileShape &sh, int r, int x0, int x1) {
+__device__ __forceinline__ int general_a_row(Smem &sm, const uint4 *vslot, const GenLevel &G, const TPair &P,
+                                             const ImgState &Q, const TileShape &sh, int r, int x0, int x1) {
     if (x0 > x1) return kZeroExp;  // the row's products are not read
+    const float4 *const vrow = reinterpret_cast<const float4 *>(vslot) + r;
     ff2 e0;
     ff2n q2;
     const int xs = x0 & ~1;  // two x per instruction
+    float4 nx[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) nx[i] = vrow[(4 * (xs >> 3) + i) * MROWS];
     cross_factor_row(G, P, Q, sm.c.exptab, r >> sh.ly, r & (sh.TY - 1), xs, e0, q2);
     // pass 1: the row maximum of |V E| (the leading products)
     float mx = 0.0f;
     {
         ff2 e = e0;
-#pragma unroll 2
-        for (int x = xs; x <= x1; x += 2) {
-            const float2 v = f2_mul(make_float2(sm.Vff[x][r].hi, sm.Vff[x + 1][r].hi), e.hi);
-            if (x >= x0) mx = fmaxf(mx, fabsf(v.x));
-            if (x < x1) mx = fmaxf(mx, fabsf(v.y));
-            e = ff2_mul(e, q2);
+#pragma unroll 1
+        for (int c = xs >> 3; 8 * c <= x1; c++) {
+            float4 v4[4];
+            const int cn = 8 * (c + 1) <= x1 ? c + 1 : 0;
+#pragma unroll
+            for (int i = 0; i < 4; i++) v4[i] = nx[i];
+#pragma unroll
+            for (int i = 0; i < 4; i++) nx[i] = vrow[(4 * cn + i) * MROWS];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int x = 8 * c + 2 * i;
+                if (x >= xs && x <= x1) {
+                    const float2 v = f2_mul(make_float2(v4[i].x, v4[i].z), e.hi);
+                    if (x >= x0) mx = fmaxf(mx, fabsf(v.x));
+                    if (x < x1) mx = fmaxf(mx, fabsf(v.y));
+                    e = ff2_mul(e, q2);
+                }
+            }
         }
     }
     const int vmx = exp_of(mx);
@@ -718,12 +696,19 @@ __device__ __forceinline__ int general_a_row(Smem &sm, const GenLevel &G, const 
 #pragma unroll 1
     for (int c = 0; c < TX / 8; c++) {
         uint32_t w[NSL][4];
+        float4 v4[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) v4[i] = nx[i];
+        if (c < TX / 8 - 1) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) nx[i] = vrow[(4 * c + 4 + i) * MROWS];
+        }
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             const int x = 8 * c + 2 * i;
             ff2 v = {f2(0.0f), f2(0.0f)};
             if (x >= xs && x <= x1) {
-                v = ff2_mul(ff2_pair(sm.Vff[x][r], sm.Vff[x + 1][r]), ff2n_of(e));
+                v = ff2_mul(ff2{make_float2(v4[i].x, v4[i].z), make_float2(v4[i].y, v4[i].w)}, ff2n_of(e));
                 if (x < x0) v.hi.x = v.lo.x = 0.0f;
                 if (x == x1) v.hi.y = v.lo.y = 0.0f;
                 e = ff2_mul(e, q2);
@@ -833,7 +818,7 @@ __device__ __forceinline__ void tc_wait(TileCommon &c, uint32_t phase, int *stat
 
 // The pair loop of a tile: item it + 1 is copied while item it is processed.  Item
 // it is visible to all threads and every thread is done with the other slot:
-// first_pair and end_item end with a barrier.
+// first_pair ends with a barrier.
 template <class Buf>
 __device__ __forceinline__ int next_pair(TileCommon &cm, Buf *pb, const MixedArgs &A, int64_t it, int64_t it0,
                                          int64_t it1, uint64_t &nxt, bool with_coef) {
@@ -844,14 +829,6 @@ __device__ __forceinline__ int next_pair(TileCommon &cm, Buf *pb, const MixedArg
     }
     return cur;
 }
-// the last barrier of an item: its TMEM columns and shared memory may be reused, the
-// next item's copies are visible
-__device__ __forceinline__ void end_item() {
-    cp_async_wait_all();
-    tc::fence_before_sync();
-    __syncthreads();
-}
-
 template <class Buf>
 __device__ __forceinline__ void first_pair(TileCommon &cm, Buf *pb, const MixedArgs &A, int64_t it0, int64_t it1,
                                            uint64_t &nxt, bool with_coef) {
@@ -1004,7 +981,7 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                         const TabEntry te = tab_entry(P, Q, ext, sh, cm.exptab, warp, ent);
                         if (warp == 0) {
                             ff2 xv[kNPair];
-                            x_powers(P, Q, te, ent, true, xv);
+                            x_powers(P, Q, te, ent, xv);
                             float mx = 0.0f;
 #pragma unroll
                             for (int i = 0; i < kNPair; i++)
@@ -1186,7 +1163,7 @@ __device__ __forceinline__ void acc_four(ff2 &s, float4 ah, float4 al, float4 bh
                  ff2n{make_float2(bh.z, bh.w), make_float2(bnh.z, bnh.w), make_float2(bnl.z, bnl.w)});
 }
 
-// Stage 1 transposed, orthorhombic: the moments W[g][b][a] += sum_z T[z][(b,a)] Z[g][z]
+// Stage 1 transposed: the moments W[g][b][a] += sum_z T[z][(b,a)] Z[g][z]
 // of an item of degree lp, by 96 threads (t0 of 96).  T lies in the columns of S that a
 // warp was done with: pass p of its (b,a) in row lp - p (see stage 2 transposed).  It is
 // a serial chain of loads and sums; run between barriers of its own it took 3.5 of 56 ms
@@ -1204,8 +1181,10 @@ __device__ __forceinline__ void add_moments(const Smem &sm, double *mom, int lp,
         for (int z4 = 0; z4 < sh.TZ; z4 += 4) {
             float4 h, l;
             if (lzw) {  // two z per warp: (z, z + 1) in one column pair of warp z / 2
-                const float2 h0 = *reinterpret_cast<const float2 *>(th + 16 * z4), h1 = *reinterpret_cast<const float2 *>(th + 16 * z4 + 32);
-                const float2 l0 = *reinterpret_cast<const float2 *>(tl + 16 * z4), l1 = *reinterpret_cast<const float2 *>(tl + 16 * z4 + 32);
+                const float2 h0 = *reinterpret_cast<const float2 *>(th + 16 * z4),
+                             h1 = *reinterpret_cast<const float2 *>(th + 16 * z4 + 32);
+                const float2 l0 = *reinterpret_cast<const float2 *>(tl + 16 * z4),
+                             l1 = *reinterpret_cast<const float2 *>(tl + 16 * z4 + 32);
                 h = make_float4(h0.x, h0.y, h1.x, h1.y);
                 l = make_float4(l0.x, l0.y, l1.x, l1.y);
             } else {  // one z per warp
@@ -1225,10 +1204,10 @@ __device__ __forceinline__ void add_moments(const Smem &sm, double *mom, int lp,
 // V(x) E(x) (E the cross factor of the Gaussian along the row), one row per
 // thread, with its own exponent per row and image.
 template <bool kGeneral>
-__global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(MixedArgs A) {
+__global__ void __launch_bounds__(NTHR, 4) k_integrate_tiled(MixedArgs A) {
     extern __shared__ __align__(128) unsigned char smraw[];
-    SmemInt<kGeneral> &sm = *reinterpret_cast<SmemInt<kGeneral> *>(smraw);
-    uint4 *const vslot = kGeneral ? nullptr : A.vslot + (size_t)blockIdx.x * kVSlot16;
+    SmemInt &sm = *reinterpret_cast<SmemInt *>(smraw);
+    uint4 *const vslot = A.vslot + (size_t)blockIdx.x * kVSlot16;
     TileCommon &cm = sm.c;
     const int tid = threadIdx.x, warp = tid >> 5;
     const int m = tid;
@@ -1267,10 +1246,12 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
 #pragma unroll
                 for (int i = 0; i < 8; i++) v8[i] = (row_ok && x8 + i < ext.x) ? grid[row + x8 + i] : 0.0;
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const ff v = ff_from_double(v8[i]);
-                    if constexpr (kGeneral) sm.Vff[x8 + i][m] = v;
-                    mx = fmaxf(mx, fabsf(v.hi));
+                for (int i = 0; i < 8; i += 2) {
+                    const ff v0 = ff_from_double(v8[i]), v1 = ff_from_double(v8[i + 1]);
+                    if constexpr (kGeneral)
+                        reinterpret_cast<float4 *>(vslot)[((x8 + i) / 2) * MROWS + m] =
+                            make_float4(v0.hi, v0.lo, v1.hi, v1.lo);
+                    mx = fmaxf(mx, fmaxf(fabsf(v0.hi), fabsf(v1.hi)));
                 }
             }
             vm = exp_of(mx);
@@ -1288,7 +1269,7 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
 #pragma unroll
                     for (int q = 0; q < NSL; q++) w[q][i] = pack_halves(sl[q]);
                 }
-                const int o16 = (m >> 3) * 16 + (c & 1) * 8 + (m & 7);  // umma_off / 16
+                const int o16 = (m >> 3) * 16 + (c & 1) * 8 + (m & 7);  // offset of (m, 8 c) / 16
 #pragma unroll
                 for (int q = 0; q < NSL; q++) {
                     const uint4 val = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
@@ -1308,8 +1289,8 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
             sm.todo[m] = chunks_to_mask(M, have);
             __syncthreads();
         }
-        // orthorhombic: the item whose moments are still to be added (by warps 1-3, while
-        // warp 0 makes the next item's B): its degree and moments
+        // the item whose moments are still to be added (by warps 1-3, while warp 0 makes the
+        // next item's B): its degree and moments
         int lp_done = -1;
         double *mom_done = nullptr;
         for (int64_t it = it0; it < it1; it++) {
@@ -1323,19 +1304,37 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                 int x0 = 1, x1 = 0, vrow = vm;
                 if constexpr (kGeneral) {  // every thread: its row's cube x range and its A row
                     general_row_range(lv, A.glv[td.level], P, Q, Q.o[2] + z, Q.o[1] + y, row_ok, x0, x1);
-                    vrow = general_a_row(sm, A.glv[td.level], P, Q, sh, m, x0, x1);
+                    vrow = general_a_row(sm, vslot, A.glv[td.level], P, Q, sh, m, x0, x1);
+                }
+                // Code size counts: four CTAs per SM at different points of the loop share the
+                // instruction caches, and the general-cell kernel, which has the row rule
+                // and the cross factor as well, lost a fifth of its issue slots to fetches.
+                // It has one copy of the table code (7.13 ms with the compact B loop below,
+                // 7.93 without either, 6.86 with stage 2 transposed rolled as well); the
+                // orthorhombic one is faster with a copy per warp (53.0 against 53.7 ms,
+                // 100k pairs, 256^3), with stage 2 unrolled by 4 (53.0 against 53.4).
+                TabEntry te0;
+                if constexpr (kGeneral) {
+                    if (warp < 2) {
+#pragma unroll 1
+                        for (int ent = tid & 31; ent < (warp == 0 ? TX : TY + TZ); ent += 32) {
+                            te0 = tab_entry(P, Q, ext, sh, cm.exptab, warp, ent);
+                            if (warp == 1) yz_fill(sm, P, te0, cur);
+                        }
+                    }
                 }
                 if (warp == 0) {
-                    // X column (lane x) in registers, then B: row alpha = X[alpha][x] over x,
-                    // scaled by 2^(SLB - g[alpha]) (maximum over the warp); rows alpha >= L
-                    // are left as they are (their output columns are not read).  Unlike
-                    // collocate, integrate is not limited by instruction fetch: warps 0 and 1
-                    // keep separate table code.
-                    ff2 xv[kNPair];
-                    x_powers(P, Q, tab_entry(P, Q, ext, sh, cm.exptab, 0, tid), tid, false, xv);
-#pragma unroll
-                    for (int a = 0; a < kNPow; a += 2) {  // in pairs; xv[a] = 0 for a >= L
-                        if (a >= L) break;
+                    // B: row alpha = X[alpha][x] over x (lane x), two alpha at a time, scaled by
+                    // 2^(SLB - g[alpha]) (maximum over the warp); rows alpha >= L are left as
+                    // they are (their output columns are not read).  The powers are formed as
+                    // the loop goes (unrolled over a table in registers: 53.5 against 53.0 ms).
+                    if constexpr (!kGeneral) te0 = tab_entry(P, Q, ext, sh, cm.exptab, 0, tid);
+                    if (!te0.in) te0.e = te0.t = ff{0.0f, 0.0f};
+                    ff2 xa = ff2_pair(te0.e, ff_mul(te0.e, te0.t));  // alpha, alpha + 1
+                    const ff2n u2 = ff2n_dup(ff_mul(te0.t, te0.t));
+#pragma unroll 1
+                    for (int a = 0; a < L; a += 2) {
+                        if (a + 1 >= L) xa.hi.y = xa.lo.y = 0.0f;
                         // per-alpha maximum over x: one warp reduction (the bit patterns of
                         // non-negative floats order as their values)
                         float sc[2];
@@ -1343,13 +1342,13 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                         for (int h = 0; h < 2; h++) {
                             const float mxb =
                                 __uint_as_float(__reduce_max_sync(
-                                    0xffffffffu, __float_as_uint(fabsf(h ? xv[a / 2].hi.y : xv[a / 2].hi.x))));
+                                    0xffffffffu, __float_as_uint(fabsf(h ? xa.hi.y : xa.hi.x))));
                             const int e = exp_of(mxb);
                             if (tid == a + h) sm.gsc[a + h] = e == kZeroExp ? 0.0f : pow2i(e - SLB);
                             sc[h] = e == kZeroExp ? 0.0f : pow2i(SLB - e);
                         }
                         float2 sl[NSL];
-                        slice_scaled2(xv[a / 2], make_float2(sc[0], sc[1]), sl);
+                        slice_scaled2(xa, make_float2(sc[0], sc[1]), sl);
                         unsigned char *const bp = sm.B + (tid >> 4) * kBHalf + b_off(a, tid & 15);
 #pragma unroll
                         for (int q = 0; q < NSL; q++) {
@@ -1357,17 +1356,21 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                             *reinterpret_cast<uint16_t *>(bp + q * kBPlane) = (uint16_t)w;
                             *reinterpret_cast<uint16_t *>(bp + q * kBPlane + 16) = (uint16_t)(w >> 16);
                         }
+                        xa = ff2_mul(xa, u2);
                     }
-                } else if (warp == 1) {
+                } else if (!kGeneral && warp == 1) {
 #pragma unroll 1
                     for (int ent = tid - 32; ent < TY + TZ; ent += 32)
-                        yz_fill(sm, P, tab_entry(P, Q, ext, sh, cm.exptab, 1, ent), kGeneral ? 0 : cur);
-                    if constexpr (!kGeneral)
-                        if (lp_done >= 0) add_moments(sm, mom_done, lp_done, cur ^ 1, sh, tid + 32);
+                        yz_fill(sm, P, tab_entry(P, Q, ext, sh, cm.exptab, 1, ent), cur);
+                    if (lp_done >= 0) add_moments(sm, mom_done, lp_done, cur ^ 1, sh, tid + 32);
                 } else if constexpr (!kGeneral) {
                     if (lp_done >= 0) add_moments(sm, mom_done, lp_done, cur ^ 1, sh, tid - 64);
                     mask_a_row(sm, tid - 64, sm.mask[tid - 64], sm.todo[tid - 64]);
                     mask_a_row(sm, tid, sm.mask[tid], sm.todo[tid]);
+                }
+                if constexpr (kGeneral) {
+                    if (warp >= 1 && lp_done >= 0)
+                        add_moments(sm, mom_done, lp_done, cur ^ 1, sh, warp == 1 ? tid + 32 : tid - 64);
                 }
                 cp_async_wait_all();  // the next item's record, read after this barrier
                 tc::fence_async_smem();
@@ -1450,73 +1453,41 @@ __global__ void __launch_bounds__(NTHR, kGeneral ? 3 : 4) k_integrate_tiled(Mixe
                 // sums, over even and odd y, as one packed sum
                 const int lzw = 5 - sh.ly;  // log2 of the z values per warp
                 const int zbase = (warp * 32) >> sh.ly;
-                // T: general cell in [q][z]; orthorhombic, pass p of a warp's (q, z) in its 32
-                // columns of S's row lp - p, which its later (b, a) don't read: the pairs with
-                // b <= p, the only ones with a = lp - p, are among the first 16 (p + 1)
+                // T: pass p of a warp's (q, z) in its 32 columns of S's row lp - p, which its later
+                // (b, a) don't read: the pairs with b <= p, the only ones with a = lp - p, are
+                // among the first 16 (p + 1)
                 int row = lp;
                 const int nt = npair << lzw;
-                for (int tt = tid & 31; tt < (kGeneral ? nt : nt + (tid & 31)); tt += 32, row--) {
-                    const int t = kGeneral ? tt : min(tt, nt - 1);  // (all lanes come to the warp barrier)
+                for (int t0 = 0; t0 < nt; t0 += 32, row--) {
+                    const int t = min(t0 + (tid & 31), nt - 1);  // (all lanes come to the warp barrier)
                     const int zz = zbase + (t & ((1 << lzw) - 1));
-                    const int q = t >> lzw;  // pair_index(L, b, a)
+                    const int q = t >> lzw;  // index of (b, a), rows of constant b
                     const uint32_t de = __ldg(&d_decode.e[d_decode_at(lp) + q]);  // (0, b, a)
                     const int b = (de >> 4) & 15, a = (de >> 8) & 15;
                     const float4 *ph = reinterpret_cast<const float4 *>(&sm.st.Sh[a][zz * TY]);
                     const float4 *pl = reinterpret_cast<const float4 *>(&sm.st.Sl[a][zz * TY]);
                     const float4 *yh = reinterpret_cast<const float4 *>(sm.Yh[b]);
-                    const float4 *ynh = yh;
-                    if constexpr (!kGeneral) ynh = reinterpret_cast<const float4 *>(sm.Ynh[b]);
+                    const float4 *ynh = reinterpret_cast<const float4 *>(sm.Ynh[b]);
                     const float4 *ynl = reinterpret_cast<const float4 *>(sm.Ynl[b]);
                     ff2 s = {f2(0.0f), f2(0.0f)};
-#pragma unroll 4
-                    for (int y4 = 0; y4 < TY / 4; y4++) {
-                        float4 nh = ynh[y4];
-                        if constexpr (kGeneral) nh = make_float4(-nh.x, -nh.y, -nh.z, -nh.w);
-                        acc_four(s, ph[y4], pl[y4], yh[y4], nh, ynl[y4]);
-                    }
+#pragma unroll kGeneral ? 1 : 4
+                    for (int y4 = 0; y4 < TY / 4; y4++) acc_four(s, ph[y4], pl[y4], yh[y4], ynh[y4], ynl[y4]);
                     const ff r = ff_add(ff{s.hi.x, s.lo.x}, ff{s.hi.y, s.lo.y});
-                    if constexpr (kGeneral) {
-                        sm.tt.Th[q][zz] = r.hi;
-                        sm.tt.Tl[q][zz] = r.lo;
-                    } else {
-                        __syncwarp();  // the pass's reads of S come first
-                        sm.st.Sh[row][m] = r.hi;
-                        sm.st.Sl[row][m] = r.lo;
-                    }
+                    __syncwarp();  // the pass's reads of S come first
+                    sm.st.Sh[row][m] = r.hi;
+                    sm.st.Sl[row][m] = r.lo;
                 }
                 if constexpr (!kGeneral) cp_async_wait_all();  // A rows restored for the next item, masked after this
                 __syncthreads();
                 if (cm.abort) break;  // uniform: set before this barrier or after the next one
-                if constexpr (!kGeneral) {
-                    lp_done = lp;
-                    mom_done = A.mom + moff;
-                    continue;
-                }
-                // stage 1 transposed: W[g][b][a] += sum_z T[z][(b,a)] Z[g][z]
-                const int nc = ncoef(lp);
-                for (int t = tid; t < nc && kGeneral; t += NTHR) {
-                    const uint32_t de = __ldg(&d_decode.e[d_decode_at(lp) + t]);  // (g, b, a) of packed index t
-                    const int g = de & 15, pi = de >> 16;
-                    ff2 s2 = {f2(0.0f), f2(0.0f)};
-                    if constexpr (kGeneral) {
-#pragma unroll 1
-                        for (int z4 = 0; z4 < TZ; z4 += 4) {
-                            const float4 zh = *reinterpret_cast<const float4 *>(&sm.Zh[0][g][z4]);
-                            acc_four(s2, *reinterpret_cast<const float4 *>(&sm.tt.Th[pi][z4]),
-                                     *reinterpret_cast<const float4 *>(&sm.tt.Tl[pi][z4]), zh,
-                                     make_float4(-zh.x, -zh.y, -zh.z, -zh.w),
-                                     *reinterpret_cast<const float4 *>(&sm.Znl[0][g][z4]));
-                        }
-                    }
-                    const ff s = ff_add(ff{s2.hi.x, s2.lo.x}, ff{s2.hi.y, s2.lo.y});
-                    if (s.hi != 0.0f) atomicAdd(A.mom + moff + t, ff_to_double_bits(s));
-                }
-                end_item();
+                lp_done = lp;
+                mom_done = A.mom + moff;
             }
         }
         if (cm.abort) break;
-        if constexpr (!kGeneral)  // the last item's (the next tile starts with a barrier)
-            if (warp >= 1 && lp_done >= 0) add_moments(sm, mom_done, lp_done, (int)((it1 - 1 - it0) & 1), sh, warp == 1 ? tid + 32 : tid - 64);
+        // the last item's (the next tile starts with a barrier)
+        if (warp >= 1 && lp_done >= 0)
+            add_moments(sm, mom_done, lp_done, (int)((it1 - 1 - it0) & 1), sh, warp == 1 ? tid + 32 : tid - 64);
     }
     tc_teardown(cm, kCols, phase);
 }
@@ -2028,7 +1999,7 @@ int mixed_build(TaskSet &ts, std::string &err) {
         e = cudaFuncSetAttribute(kc[v], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemColl));
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(ki[v], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)(v ? sizeof(SmemInt<true>) : kSmemIntOrtho));
+                                     (int)sizeof(SmemInt));
     }
     if (e != cudaSuccess) {
         err = std::string("mixed_build: ") + cudaGetErrorString(e);
@@ -2047,14 +2018,14 @@ int mixed_build(TaskSet &ts, std::string &err) {
         return std::max(1, std::min({by_regs, by_smem, 4}));
     };
     per_sm = std::min(resident(kc[0], sizeof(SmemColl)), resident(kc[1], sizeof(SmemColl)));
-    const int per_sm_i = resident(ki[0], kSmemIntOrtho);
+    const int per_sm_i = resident(ki[0], sizeof(SmemInt));
     M->per_sm = per_sm;
     M->per_sm_i = per_sm_i;
-    M->per_sm_ig = resident(ki[1], sizeof(SmemInt<true>));
+    M->per_sm_ig = resident(ki[1], sizeof(SmemInt));
     M->sms = sms;
-    // one V slot per resident orthorhombic integrate CTA
-    if (northo > 0) {
-        e = cudaMalloc(&M->d_vslot, sizeof(uint4) * kVSlot16 * (size_t)sms * per_sm_i);
+    // one V slot per resident integrate CTA
+    if (nbin > 0) {
+        e = cudaMalloc(&M->d_vslot, sizeof(uint4) * kVSlot16 * (size_t)sms * std::max(per_sm_i, M->per_sm_ig));
         if (e != cudaSuccess) {
             err = std::string("mixed_build: ") + cudaGetErrorString(e);
             return GPW_ERR_CUDA;
@@ -2265,14 +2236,14 @@ cudaError_t launch_integrate_mixed(const TaskSet &ts, const GridPtrs &g, cudaStr
         if (nto > 0) {
             if ((e = cudaMemsetAsync(M.d_queue + 1, 0, sizeof(int), s)) != cudaSuccess) return e;
             ProfScope prof(ts, s);
-            k_integrate_tiled<false><<<std::min(nto, M.sms * M.per_sm_i), NTHR, kSmemIntOrtho, s>>>(
+            k_integrate_tiled<false><<<std::min(nto, M.sms * M.per_sm_i), NTHR, sizeof(SmemInt), s>>>(
                 make_args(ts, g, 1, false));
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
         if (ntg > 0) {
             if ((e = cudaMemsetAsync(M.d_queue + 3, 0, sizeof(int), s)) != cudaSuccess) return e;
             ProfScope prof(ts, s);
-            k_integrate_tiled<true><<<std::min(ntg, M.sms * M.per_sm_ig), NTHR, sizeof(SmemInt<true>), s>>>(
+            k_integrate_tiled<true><<<std::min(ntg, M.sms * M.per_sm_ig), NTHR, sizeof(SmemInt), s>>>(
                 make_args(ts, g, 1, true));
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
             ts.n_kernels++;

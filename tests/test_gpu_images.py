@@ -59,8 +59,10 @@ def test_too_many_images():
 # every degree of the summed moments, both tile shapes
 @pytest.mark.parametrize("l", range(5))
 @pytest.mark.parametrize("tz", [4, 8])
-def test_integrate_degrees(l, tz, oracle_lib):
-    wl = T.synthetic("degrees", 10, l, (0.4, 2.0), 9.0, [(35, 40, 27)], 50 + l, lmin=max(l - 1, 0))
+@pytest.mark.parametrize("ortho", [True, False])
+def test_integrate_degrees(l, tz, ortho, oracle_lib):
+    cell = 9.0 if ortho else T.lattice_15(length=9.0)
+    wl = T.synthetic("degrees", 10, l, (0.4, 2.0), cell, [(35, 40, 27)], 50 + l, lmin=max(l - 1, 0), ortho=ortho)
     plan = capi.Plan(wl.levels)
     ts = capi.TaskSet.from_workload(plan, wl)
     ts.set_tiles([tz])
