@@ -516,24 +516,6 @@ __device__ __forceinline__ void yz_fill(Smem &sm, const TPair &p, const TabEntry
         }
     }
 }
-// collocate, warp 0: the x column of entry x in registers, xv[i] the powers 2 i and 2 i + 1
-// of u; each step multiplies a pair by u^2.
-__device__ __forceinline__ void x_powers(const TPair &p, const ImgState &q, const TabEntry &te, int x, ff2 *xv) {
-#pragma unroll
-    for (int i = 0; i < kNPair; i++) xv[i] = ff2{f2(0.0f), f2(0.0f)};
-    if (!te.in) return;
-    const ff u = ff_mul_f(p.h[0], ldexpf((float)(x - q.ic), -q.sb));
-    const ff2n u2 = ff2n_dup(ff_mul(u, u));
-    ff2 e = ff2_pair(te.e, ff_mul(te.e, u));
-#pragma unroll
-    for (int i = 0; i < kNPair; i++) {
-        if (2 * i >= p.L) break;
-        xv[i] = e;
-        if (2 * i + 1 >= p.L) xv[i].hi.y = xv[i].lo.y = 0.0f;
-        e = ff2_mul(e, u2);
-    }
-}
-
 // Binomials C(a', a) of the re-expansion c'[g][b][a] = sum_{a' >= a} C(a', a)
 // tc^(a' - a) c[g][b][a'] around column ic of the tile: powers of the small
 // offsets u = x - x_ic keep the stage-3 operands well conditioned for the
@@ -980,17 +962,35 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                     for (int ent = tid & 31; ent < (warp == 0 ? TX : TY + TZ); ent += 32) {
                         const TabEntry te = tab_entry(P, Q, ext, sh, cm.exptab, warp, ent);
                         if (warp == 0) {
-                            ff2 xv[kNPair];
-                            x_powers(P, Q, te, ent, xv);
+                            // the powers of u, two per step, in rolled loops: once for their
+                            // maximum, once to be sliced (K slots beyond L may hold an earlier
+                            // pair's slices: rewritten as zeros)
+                            const ff u = ff_mul_f(P.h[0], ldexpf((float)(ent - Q.ic), -Q.sb));
+                            const ff2n u2 = ff2n_dup(ff_mul(u, u));
+                            ff2 xa = te.in ? ff2_pair(te.e, ff_mul(te.e, u)) : ff2{f2(0.0f), f2(0.0f)};
                             float mx = 0.0f;
-#pragma unroll
-                            for (int i = 0; i < kNPair; i++)
-                                mx = fmaxf(mx, fmaxf(fabsf(xv[i].hi.x), fabsf(xv[i].hi.y)));
+                            ff2 xb = xa;
+#pragma unroll 1
+                            for (int a = 0; a < L; a += 2) {
+                                mx = fmaxf(mx, a + 1 < L ? fmaxf(fabsf(xb.hi.x), fabsf(xb.hi.y)) : fabsf(xb.hi.x));
+                                xb = ff2_mul(xb, u2);
+                            }
                             const int e = exp_of(mx);
                             sm.cs[cur][tid] = e == kZeroExp ? 0.0f : pow2i(e);
                             const float sc = e == kZeroExp ? 0.0f : pow2i(SLB - e);
-                            // K slots beyond L may hold an earlier pair's slices: rewritten as zeros
-                            slice_row16(xv, sc, max(L, kprev), L, sm.B[0], TX * KP, tid);
+                            uint32_t *bp = reinterpret_cast<uint32_t *>(sm.B[0]) + (tid >> 3) * 64 + (tid & 7) * 4;
+                            const int kw = (max(L, kprev) + 7) & ~7;
+#pragma unroll 1
+                            for (int a = 0; a < kw; a += 2) {
+                                if (a >= L) xa = ff2{f2(0.0f), f2(0.0f)};
+                                if (a + 1 >= L) xa.hi.y = xa.lo.y = 0.0f;
+                                float2 sl[NSL];
+                                slice_scaled2(xa, f2(sc), sl);
+#pragma unroll
+                                for (int q = 0; q < NSL; q++)
+                                    bp[q * (TX * KP / 2) + (a >> 3) * 32 + ((a & 7) >> 1)] = pack_halves(sl[q]);
+                                xa = ff2_mul(xa, u2);
+                            }
                         } else {
                             yz_fill(sm, P, te, 0);
                         }
