@@ -1409,10 +1409,13 @@ __global__ void __launch_bounds__(NTHR, 4) k_integrate_tiled(MixedArgs A) {
                         sm.todo[m] = chunks_to_mask(M, have);
                     }
                 }
+                // A warp whose rows all lie outside has only zeros to hand on (3.95 -> 3.86 ms on
+                // the three-level workload, 53.0 -> 52.7 ms for 100k pairs on 256^3).
+                const bool wlive = __any_sync(0xffffffffu, live);
                 const float2 rsc = f2(vrow != kZeroExp ? pow2i(vrow - SLB) : 0.0f);  // 2^(row exponent - SLB)
 #pragma unroll 1
                 for (int c = 0; c < KP / 8; c++) {
-                    if (8 * c >= L) break;  // uniform: S columns alpha >= L are not read
+                    if (8 * c >= L || !wlive) break;  // uniform: S columns alpha >= L are not read
                     uint32_t ra[8], rb[8], r3[8], r4[8], r5[8];
                     tc::tmem_ld8(tbase + 8 * c, ra);
                     tc::tmem_ld8(tbase + 16 + 8 * c, rb);
@@ -1459,6 +1462,10 @@ __global__ void __launch_bounds__(NTHR, 4) k_integrate_tiled(MixedArgs A) {
                 int row = lp;
                 const int nt = npair << lzw;
                 for (int t0 = 0; t0 < nt; t0 += 32, row--) {
+                    if (!wlive) {
+                        sm.st.Sh[row][m] = sm.st.Sl[row][m] = 0.0f;
+                        continue;
+                    }
                     const int t = min(t0 + (tid & 31), nt - 1);  // (all lanes come to the warp barrier)
                     const int zz = zbase + (t & ((1 << lzw) - 1));
                     const int q = t >> lzw;  // index of (b, a), rows of constant b
