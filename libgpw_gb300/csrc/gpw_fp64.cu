@@ -301,24 +301,37 @@ k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
         const int nrow = 2 - 2 * jgmin, xend = 1 - wide;
         for (int c0 = wide; c0 <= xend;) {
             const int left = xend - c0 + 1;
-            const int lw = kAdj && left > 16 ? 5 : (left > 8 ? 4 : 3);  // log2 of the block's columns
+            const int lw = kAdj && left > 24 ? 5 : (left > 8 ? 4 : 3);  // log2 of the block's columns
             // (blocks of at most 32, 16, 8 columns: collocate 461, 453, 540 us on the workload
-            // above, integrate, with its planes taken in turn, 485, 488, 536: fewer idle lanes
-            // at a row's ends, but T anew per block)
+            // above, integrate 485, 488, 536: fewer idle lanes at a row's ends, but T, or the sums
+            // over the columns, anew per block.  Done for 32 columns at a time: collocate with
+            // blocks of 16 453 -> 421 us, integrate with blocks of 32 only where more than 24
+            // columns are left 456 -> 451; 592 -> 574 with two more powers)
             const int grp = lane >> lw, ng = 32 >> lw;          // the lane's row group
             const int ig = c0 + (lane & ((1 << lw) - 1)), xc = min(ig - lb0, nx - 1);
             const bool in = ig <= xend;
             const int igf = fold(ig), xi = xidx[xc];
             double T[kAcc];
             if (!kAdj) {
-                const double *c = sC;
+                // T of 32 columns at a time, a lane each (an FP64 operation costs a warp the same
+                // with half its lanes idle): two blocks of 16 share them
+                const int off = (c0 - wide) & 31;
+                if (off == 0) {
+                    const int xt = min(c0 + lane - lb0, nx - 1);
+                    const double *c = sC;
+                    __syncwarp();
+                    for (int ly = 0; ly < L; ly++) {
+                        double s = 0.0;
+                        for (int lx = 0; lx < L - ly; lx++) s += c[lx] * Xt[lx * nx + xt];
+                        c += L - ly;
+                        sT[ly * 33 + lane] = s;
+                    }
+                    __syncwarp();
+                }
 #pragma unroll
                 for (int ly = 0; ly < kAcc; ly++) {
                     if (ly >= L) break;
-                    double s = 0.0;
-                    for (int lx = 0; lx < L - ly; lx++) s += c[lx] * Xt[lx * nx + xc];
-                    c += L - ly;
-                    T[ly] = s;
+                    T[ly] = sT[ly * 33 + off + (lane & ((1 << lw) - 1))];
                 }
             } else {
 #pragma unroll
@@ -363,22 +376,29 @@ k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
                         if (act[u]) atomicAdd(grid + at[u], v[u]);
                 }
             }
-            if (kAdj) {
+            if (kAdj) {  // the row groups' sums, then cxy over the columns of (up to) two blocks
+                const int off = (c0 - wide) & 31;
 #pragma unroll
-                for (int ly = 0; ly < kAcc; ly++)
-                    if (ly < L) sT[ly * 33 + lane] = T[ly];
-                __syncwarp();
-                const int wm = (1 << lw) - 1, cx = c0 - lb0;
-#pragma unroll
-                for (int m = 0; m < kM2; m++) {
-                    if (oly[m] < 0) continue;
-                    const double *t = sT + oly[m] * 33, *x = Xt + olx[m] * nx;
-                    double s = cxy[m];
-                    for (int i = lane & ((1 << lg) - 1); i < 32; i += 1 << lg)
-                        s = fma(t[i], x[min(cx + (i & wm), nx - 1)], s);
-                    cxy[m] = s;
+                for (int ly = 0; ly < kAcc; ly++) {
+                    if (ly >= L) break;
+                    double v = T[ly];
+                    for (int o = 1 << lw; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                    if (grp == 0) sT[ly * 33 + off + lane] = v;
                 }
-                __syncwarp();
+                if (off + (1 << lw) == 32 || left <= 1 << lw) {
+                    __syncwarp();
+                    const int n = off + min(left, 1 << lw);
+                    const double *xw = Xt + (c0 - off - lb0);
+#pragma unroll
+                    for (int m = 0; m < kM2; m++) {
+                        if (oly[m] < 0) continue;
+                        const double *t = sT + oly[m] * 33, *x = xw + olx[m] * nx;
+                        double s = cxy[m];
+                        for (int i = lane & ((1 << lg) - 1); i < n; i += 1 << lg) s = fma(t[i], x[i], s);
+                        cxy[m] = s;
+                    }
+                    __syncwarp();
+                }
             }
             c0 += 1 << lw;
         }
