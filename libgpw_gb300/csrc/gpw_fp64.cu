@@ -258,7 +258,11 @@ k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
     __syncthreads();
     // integrate's CTAs end with a sum over the warps: planes taken as warps come free (485
     // -> 458 us on the workload above; collocate, whose warps end alone, loses 1 %)
-    for (int turn = warp;; turn += kOrthoWarps) {
+    // Collocate with fewer planes than warps (a call with one pair): 2^lsub warps share a
+    // plane's rows, T computed by each (36 planes of 36 x 36, one pair, L = 2: 9 CTAs of four
+    // planes 14.3 us, 36 CTAs of one 9.0 us).
+    const int lsub = kAdj || np > 2 ? 0 : 3 - np, sub = warp & ((1 << lsub) - 1);
+    for (int turn = warp >> lsub;; turn += kOrthoWarps >> lsub) {
         const int pl = kAdj ? next_plane(&s_next) : turn;
         if (pl >= np) break;
         const int kg = kgmin + it.part + pl * it.nparts, kf = fold(kg);
@@ -338,7 +342,7 @@ k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
                 for (int ly = 0; ly < kAcc; ly++) T[ly] = 0.0;
             }
             constexpr int kU = kAdj ? 4 : 2;  // rows in flight per lane
-            for (int r0 = grp; r0 - grp < nrow; r0 += kU * ng) {
+            for (int r0 = grp + sub * kU * ng; r0 - grp < nrow; r0 += (kU * ng) << lsub) {
                 bool act[kU];
                 int jy[kU];
                 int64_t at[kU];
@@ -1065,10 +1069,9 @@ cudaError_t launch_pairs_fp64(const PairGeom *d_geoms, const LevelDev *d_levels,
     return cudaGetLastError();
 }
 
-// one plane per warp (orthorhombic), four planes per CTA (general cell)
+// one plane per CTA (orthorhombic), four planes per CTA (general cell)
 int fp64_single_parts(const PairGeom &g) {
-    const int planes = g.ortho ? 2 - 2 * g.kgmin : g.ext0[2];
-    return std::max(1, (planes + kOrthoWarps - 1) / kOrthoWarps);
+    return std::max(1, g.ortho ? 2 - 2 * g.kgmin : (g.ext0[2] + kOrthoWarps - 1) / kOrthoWarps);
 }
 
 // One pair from raw device pointers, orthorhombic (with its cube list in d_table

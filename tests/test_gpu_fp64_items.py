@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from gpu_util import run_collocate, run_integrate
-from libgpw_gb300 import tasks as T
+from libgpw_gb300 import capi, tasks as T
 
 pytestmark = pytest.mark.gpu
 
@@ -41,3 +41,18 @@ def test_general_items(half, precision, tol, oracle_lib):
     got = run_collocate(wl, precision)[0]
     assert np.linalg.norm(got - want) <= tol * np.linalg.norm(want)
     assert np.abs(run_integrate(wl, V, precision) - hab).max() <= tol * np.abs(hab).max()
+
+
+@pytest.mark.parametrize("n", [1, 60, 64])
+def test_few_planes_per_cta(n, oracle_lib):
+    """20 planes of a pair in CTAs of one, two, and two or three (152 SMs): warps share a plane's rows."""
+    import torch
+
+    wl = _pairs(9, 2, 0, True, n=n)
+    level, tasks = np.array([wl.levels[0]], dtype=T.GRID_DTYPE), np.ascontiguousarray(wl.tasks)
+    pab = torch.from_numpy(wl.pab).cuda()
+    grid = torch.zeros(T.grid_shape(wl.levels[0]), dtype=torch.float64, device="cuda")
+    capi.check(capi.lib().gpw_collocate_noalloc(level.ctypes.data, tasks.ctypes.data, n, 0, pab.data_ptr(),
+                                                grid.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    want = oracle_lib.batch(wl)[0]
+    assert np.linalg.norm(grid.cpu().numpy() - want) <= 1e-12 * np.linalg.norm(want)
