@@ -497,7 +497,7 @@ __device__ __forceinline__ void yz_fill(Smem &sm, const TPair &p, const TabEntry
         float *nhi = &sm.Znh[0][te.i];
         const float sg = isy ? 1.0f : -1.0f;
 #pragma unroll 1
-        for (int k = 0; k < kNPow; k++) {
+        for (int k = 0; k < p.L; k++) {  // (to kNPow: 61.0 -> 62.2 ms, 100k pairs, 256^3)
             hi[k * stride] = k < L ? e.hi : 0.0f;
             lo[k * stride] = k < L ? sg * e.lo : 0.0f;
             if (!isy) nhi[k * stride] = k < L ? -e.hi : 0.0f;
