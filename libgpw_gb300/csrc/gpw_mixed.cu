@@ -324,6 +324,36 @@ __host__ __device__ constexpr int cxy_pad_row(int L, int b) {
 constexpr int kNPair = (kNPow + 1) / 2;                     // pairs of a
 constexpr int kCxyRow = cxy_pad_row(kNPow, kNPow) / 2;      // 16-byte entries of one z
 
+// Collocate's re-expansion and stage 1 have one output per thread and turn, each the end
+// of a chain of up to lp + 1 steps: the outputs in order of falling chain length, so that
+// the lanes of a warp have chains of about one length (in packed order a warp's longest
+// was two to three times its mean: XX).
+struct Order {
+    uint32_t rec[d_decode_at(kNPow)];       // per lp: g | b << 4 | a << 8 | packed index << 16
+    unsigned char st1[kNPow][2 * kCxyRow];  // [L - 1]: b | a << 4, the padding of rows as well
+};
+constexpr Order make_order() {
+    Order o{};
+    for (int lp = 0; lp < kNPow; lp++) {
+        int at = d_decode_at(lp);
+        for (int d = 0; d <= lp; d++) {  // chain length lp + 1 - d
+            int t = 0;
+            for (int g = 0; g <= lp; g++)
+                for (int b = 0; b <= lp - g; b++)
+                    for (int a = 0; a <= lp - g - b; a++, t++)
+                        if (g + b + a == d) o.rec[at++] = (uint32_t)(g | b << 4 | a << 8 | t << 16);
+        }
+        at = 0;
+        for (int d = 0; d <= lp + 1; d++) {  // d = lp + 1: the padding, no terms
+            for (int b = 0; b <= lp; b++)
+                for (int a = 0; a < ((lp - b + 2) & ~1); a++)
+                    if (a + b == d) o.st1[lp][at++] = (unsigned char)(b | a << 4);
+        }
+    }
+    return o;
+}
+static __device__ const Order d_order = make_order();
+
 struct alignas(128) SmemColl {
     __half A[NSL][MROWS * KP];  // Cx slices, M=128 x K=16
     __half B[NSL][TX * KP];     // X slices, N=32 x K=16
@@ -335,8 +365,8 @@ struct alignas(128) SmemColl {
     alignas(16) float Zh[kNPow][kMaxTZ], Znh[kNPow][kMaxTZ], Znl[kNPow][kMaxTZ];
     alignas(16) float acc_lo[MROWS][TX + 4];  // low parts of the tile sums (row m belongs to thread m; padded rows)
     float bin[kNPow][kNPow];    // binomials C(a', a) of the re-expansion
+    unsigned char st1[kNPow][2 * kCxyRow];  // d_order.st1
     alignas(16) float cs[2][TX];  // 2^fx per column (0 for an empty column), of this item and the next
-    unsigned char qpad[kNPow][2 * kCxyRow];  // qpad[L-1][padded index of (b, a)] = b | a << 4
     TileCommon c;
 };
 
@@ -547,9 +577,9 @@ __constant__ int c_zs[kNPow][kNPow + 1] = {GPW_ZS(0), GPW_ZS(1), GPW_ZS(2), GPW_
 __device__ void recentre_x(const PairBuf &pb, ff tc, int sb, ff *out, const float (*bin)[kNPow], int t0, int nt) {
     const int lp = pb.p.lp;
     const int nc = ncoef(lp);
-    for (int t = (int)threadIdx.x - t0; t < nc; t += nt) {
-        const uint32_t de = __ldg(&d_decode.e[d_decode_at(lp) + t]);
-        const int g = de & 15, b = (de >> 4) & 15, a = (de >> 8) & 15, amax = lp - g - b;
+    for (int i = (int)threadIdx.x - t0; i < nc; i += nt) {
+        const uint32_t de = __ldg(&d_order.rec[d_decode_at(lp) + i]);
+        const int g = de & 15, b = (de >> 4) & 15, a = (de >> 8) & 15, t = de >> 16, amax = lp - g - b;
         const int base = t - a;  // packed index of (g, b, 0)
         ff s = {0.0f, 0.0f};
 #pragma unroll 1
@@ -828,10 +858,11 @@ __device__ __forceinline__ void first_pair(TileCommon &cm, Buf *pb, const MixedA
 __device__ __forceinline__ void stage1_cxy(SmemColl &sm, int L, int lp, const TileShape &sh) {
     const int *zs = c_zs[lp];
     const int npad = 2 * (L >> 1) * ((L >> 1) + 1) + (L & 1) * (L + 1);  // cxy_pad_row(L, L)
-    const unsigned char *qp = sm.qpad[L - 1];
     for (int t = (int)threadIdx.x - 32; t < (npad << (sh.lz - 1)); t += NTHR - 32) {
-        const int zz = 2 * (t & ((sh.TZ >> 1) - 1)), q = t >> (sh.lz - 1);
-        const int b = qp[q] & 15, a = qp[q] >> 4, n = lp - a - b;
+        const int zz = 2 * (t & ((sh.TZ >> 1) - 1));
+        const uint32_t de = sm.st1[lp][t >> (sh.lz - 1)];
+        const int b = de & 15, a = de >> 4, n = lp - a - b;
+        const int q = b * L - (b * (b - 1)) / 2 + ((b + (L & 1)) >> 1) + a;  // cxy_pad_row(L, b) + a
         const ff *c = sm.rc + (b * (lp + 1) - (b * (b - 1)) / 2 + a);
         ff2 s0 = {f2(0.0f), f2(0.0f)}, s1 = s0;
         auto zpair = [&](int g) {
@@ -912,13 +943,8 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
     const uint32_t tbase = cm.tmem + ((uint32_t)(warp * 32) << 16);
     uint32_t phase = 0;
     int kprev = KP;  // K slots of A and B that the previous pair wrote (uninitialised at first: all)
+    for (int t = tid; t < kNPow * 2 * kCxyRow; t += NTHR) (&sm.st1[0][0])[t] = (&d_order.st1[0][0])[t];
     for (int t = tid; t < kNPow * kNPow; t += NTHR) sm.bin[t / kNPow][t % kNPow] = c_binom[t / kNPow][t % kNPow];
-    for (int t = tid; t < kNPow * 2 * kCxyRow; t += NTHR) {
-        const int Lq = t / (2 * kCxyRow) + 1, q = t % (2 * kCxyRow);
-        int b = 0, r = q;
-        while (b < Lq && r >= ((Lq - b + 1) & ~1)) r -= (Lq - b++ + 1) & ~1;
-        sm.qpad[Lq - 1][q] = (unsigned char)(min(b, kNPow - 1) | (r & 15) << 4);
-    }
     for (;;) {
         if (tid == 0) cm.tile = atomicAdd(A.queue, 1);
         __syncthreads();
