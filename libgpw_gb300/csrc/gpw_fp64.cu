@@ -945,17 +945,23 @@ cudaError_t launch_prep(const TaskSet &ts, const double *d_pab, cudaStream_t s) 
 
 // The items of the FP64 launches and of the float-float general-cell kernel (1500
 // pairs of a general cell, 128^3, collocate + integrate: one CTA per pair 38.1 ms, most
-// of it the tail of the largest boxes; with items and the same kernel 10.7 ms).  A pair is divided into parts (interleaved planes, so
-// that parts cost alike) where it holds more than 1/kWaves of an even per-CTA share
-// of all cube points, down to one plane per warp; the largest pairs come first
-// (the sorted order).  The number of planes is not needed exactly: a geometry
-// update may move a general box's extent by one.
+// of it the tail of the largest boxes; with items and the same kernel 10.7 ms).  A pair
+// is divided into parts (interleaved planes, so that parts cost alike) where it holds
+// more than a given part of an even per-CTA share of all cube points, down to one plane
+// per warp.  The number of planes is not needed exactly: a geometry update may move a
+// general box's extent by one.
 void fp64_items(TaskSet &ts, int sms, int smem_limit, std::vector<Fp64Item> &items) {
-    constexpr int kWaves = 8, kCtas = 4;
+    // Parts of at most 1/kWaves of a CTA's share.  Orthorhombic: a part costs a CTA's tables and
+    // (integrate) the sum over its warps, and the largest parts run first (integrate and
+    // collocate of 1000 pairs, 64^3: 443 and 418 us; 8 waves in the pairs' order 450 and 423;
+    // two more powers 569 and 543 against 571 and 549; 16 waves 462 and 421).  General cells,
+    // whose CTAs set little up: 4.04 and 3.28 ms for 1500 pairs on 128^3, mixed, with 16 waves in
+    // the pairs' order, 4.15 and 3.32 sorted, 4.15 and 3.49 with 8 waves.
+    constexpr int kWavesOrtho = 7, kWavesGeneral = 16, kCtas = 4;
     constexpr double kLeast = 16384.0;  // points x powers: below this a part is mostly tables and set-up
     double total = 0.0;
     for (const PairGeom &g : ts.h_geom) total += (double)g.cost * (g.lp + 1);
-    const double target = std::max(kLeast, total / ((double)sms * kCtas * kWaves));
+    const double share = total / ((double)sms * kCtas);
     ts.fp64_ortho = ts.fp64_general = 0;
     ts.fp64_smem = ts.fp64_smem_ext = ts.fp64_smem_gen = ts.fp64_smem_gen_ext = 0;
     ts.fp64_split = false;
@@ -963,6 +969,7 @@ void fp64_items(TaskSet &ts, int sms, int smem_limit, std::vector<Fp64Item> &ite
         const PairGeom &g = ts.h_geom[k];
         const int planes = g.ortho ? 2 - 2 * g.kgmin : g.ext0[2];
         const int most = std::max(1, (planes + kOrthoWarps - 1) / kOrthoWarps);
+        const double target = std::max(kLeast, share / (g.ortho ? kWavesOrtho : kWavesGeneral));
         int parts = (int)std::min<double>(most, std::ceil((double)g.cost * (g.lp + 1) / target));
         parts = std::max(parts, 1);
         if (g.ortho) {
@@ -978,6 +985,12 @@ void fp64_items(TaskSet &ts, int sms, int smem_limit, std::vector<Fp64Item> &ite
         ts.fp64_split = ts.fp64_split || parts > 1;
         for (int p = 0; p < parts; p++) items.push_back(Fp64Item{(int)k, p, parts});
     }
+    auto cost = [&](const Fp64Item &i) {
+        const PairGeom &g = ts.h_geom[i.pair];
+        return (float)((double)g.cost * (g.lp + 1) / i.nparts);
+    };
+    std::stable_sort(items.begin(), items.begin() + ts.fp64_ortho,
+                     [&](const Fp64Item &x, const Fp64Item &y) { return cost(x) > cost(y); });
 }
 
 static cudaError_t launch_fp64_impl(const TaskSet &ts, const GridPtrs &g, bool adj, int extra, double *mom,
