@@ -872,11 +872,11 @@ __device__ __forceinline__ void stage1_cxy(SmemColl &sm, int L, int lp, const Ti
         int g = 0, bg = 0;
 #pragma unroll 1
         for (; g + 1 <= n; g += 2, bg += 2 * b) {
-            ff2_acc_lazy(s0, ff2_dup(c[zs[g] - bg]), zpair(g));
-            ff2_acc_lazy(s1, ff2_dup(c[zs[g + 1] - bg - b]), zpair(g + 1));
+            s0 = ff2_fma(ff2_dup(c[zs[g] - bg]), zpair(g), s0);
+            s1 = ff2_fma(ff2_dup(c[zs[g + 1] - bg - b]), zpair(g + 1), s1);
         }
-        if (g <= n) ff2_acc_lazy(s0, ff2_dup(c[zs[g] - bg]), zpair(g));
-        s0 = ff2_add(s0, s1);  // (renormalises)
+        if (g <= n) s0 = ff2_fma(ff2_dup(c[zs[g] - bg]), zpair(g), s0);
+        s0 = ff2_add(s0, s1);
         float *o = reinterpret_cast<float *>(&sm.Cxy[zz][q >> 1]) + (q & 1);
         o[0] = s0.hi.x;
         o[2] = s0.lo.x;
