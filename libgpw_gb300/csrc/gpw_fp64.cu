@@ -7,6 +7,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 
 #include "gpw_coef.cuh"
 #include "gpw_ff.cuh"
@@ -965,6 +966,10 @@ void fp64_items(TaskSet &ts, int sms, int smem_limit, std::vector<Fp64Item> &ite
     ts.fp64_ortho = ts.fp64_general = 0;
     ts.fp64_smem = ts.fp64_smem_ext = ts.fp64_smem_gen = ts.fp64_smem_gen_ext = 0;
     ts.fp64_split = false;
+    constexpr int kClasses = 1024;  // sign, exponent and two mantissa bits
+    std::vector<unsigned short> cls(ts.h_geom.size());
+    std::vector<int> nparts(ts.h_geom.size());
+    std::vector<int64_t> first(kClasses + 1, 0);
     for (int64_t k = 0; k < (int64_t)ts.h_geom.size(); k++) {
         const PairGeom &g = ts.h_geom[k];
         const int planes = g.ortho ? 2 - 2 * g.kgmin : g.ext0[2];
@@ -983,14 +988,22 @@ void fp64_items(TaskSet &ts, int sms, int smem_limit, std::vector<Fp64Item> &ite
             ts.fp64_general += parts;
         }
         ts.fp64_split = ts.fp64_split || parts > 1;
-        for (int p = 0; p < parts; p++) items.push_back(Fp64Item{(int)k, p, parts});
+        // class of the items' cost: a factor 2^(1/4) or so, from the float's leading bits
+        const float c = (float)((double)g.cost * (g.lp + 1) / parts);
+        unsigned bits;
+        memcpy(&bits, &c, sizeof bits);
+        cls[(size_t)k] = (unsigned short)(kClasses - 1 - std::min(bits >> 21, (unsigned)kClasses - 1));
+        nparts[(size_t)k] = parts;
+        if (g.ortho) first[cls[(size_t)k] + 1] += parts;
     }
-    auto cost = [&](const Fp64Item &i) {
-        const PairGeom &g = ts.h_geom[i.pair];
-        return (float)((double)g.cost * (g.lp + 1) / i.nparts);
-    };
-    std::stable_sort(items.begin(), items.begin() + ts.fp64_ortho,
-                     [&](const Fp64Item &x, const Fp64Item &y) { return cost(x) > cost(y); });
+    // orthorhombic items by falling class (a counting sort), then the general cells' in order
+    for (int c = 0; c < kClasses; c++) first[c + 1] += first[c];
+    items.resize((size_t)(ts.fp64_ortho + ts.fp64_general));
+    int64_t at_gen = ts.fp64_ortho;
+    for (size_t k = 0; k < ts.h_geom.size(); k++) {
+        int64_t &at = ts.h_geom[k].ortho ? first[cls[k]] : at_gen;
+        for (int p = 0; p < nparts[k]; p++) items[(size_t)at++] = Fp64Item{(int)k, p, nparts[k]};
+    }
 }
 
 static cudaError_t launch_fp64_impl(const TaskSet &ts, const GridPtrs &g, bool adj, int extra, double *mom,
