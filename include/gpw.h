@@ -60,7 +60,7 @@ enum gpw_function {
 
 /* Arithmetic of the cube contraction. */
 enum gpw_precision {
-    GPW_PREC_FP64 = 0,   /* plain FP64 kernels, one CTA per pair, FP64 atomics   */
+    GPW_PREC_FP64 = 0,   /* plain FP64 kernels, FP64 atomics into the grid       */
     GPW_PREC_MIXED = 1   /* tiled kernels: FP64 pair set-up, split-FP32 tables,   */
                          /* tensor-core cube contraction, compensated            */
                          /* accumulation, one FP64 write per grid point          */
@@ -224,7 +224,7 @@ int gpw_taskset_stats(gpw_taskset *ts, double *contraction_ms,
  * of 32 x (128 / tz) x tz grid points (x, y, z), tz = 4 or 8; the shape sets
  * how many tiles a cube touches and how much per-tile work a pair costs.  A
  * general-cell level may also take tz = 0 (its default): no tiles, its pairs
- * run on the float-float kernel, one CTA per pair.  No reference counterpart:
+ * run on the float-float kernel of untiled general cells.  No reference counterpart:
  * the reference has no tiled path; the shapes change the speed, not the
  * results beyond rounding.
  *

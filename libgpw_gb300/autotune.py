@@ -3,7 +3,7 @@
 The tiled kernels cut every orthorhombic grid level into tiles of 32 x (128/tz)
 x tz points; tz (4 or 8) trades the number of tiles a cube touches against
 the per-tile work of a pair.  On general-cell levels tz = 0 (no tiles: the
-float-float kernel, one CTA per pair) is a third candidate.  ``gpw_taskset_autotune`` times one collocate +
+untiled float-float kernel) is a third candidate.  ``gpw_taskset_autotune`` times one collocate +
 integrate per candidate and level on the device.  This module keys the result
 by a workload signature (grid levels and the task set's size, angular momentum
 and exponent spread) and keeps it in a JSON table, so a task set of the same

@@ -2,10 +2,10 @@
 //
 // Persistent CTAs take work units from an atomic queue.  A unit is one tile of
 // one grid level (TX x TY x TZ points, x fastest; TX = 32, TY x TZ = 128 rows with
-// TZ = 4 or 8 per level, chosen by the tile autotuner) with the pairs whose cube
-// touches it, or a part of that list for the busiest tiles (those units flush
-// with atomics).  The pair records, coefficients and per-tile images are copied
-// one item ahead with cp.async.  Per pair and tile:
+// TZ = 4 or 8 per level, chosen by the tile autotuner) with its items, the periodic
+// images of pairs whose sphere reaches it, or a part of that list for the busiest
+// tiles and at the queue's end (those units flush with atomics).  The pair records,
+// coefficients and images are copied one item ahead with cp.async.  Per item:
 //   1-D tables t^k exp(-zetp t^2) over the tile's three ranges   (float-float)
 //   stage 1  Cxy[z][b][a] = sum_g c[g][b][a] Z[g][z]              (float-float)
 //   stage 2  Cx[(z,y)][a] = sum_b Cxy[z][b][a] Y[b][y]            (float-float)
@@ -20,8 +20,8 @@
 // operand to ~2^-35 of its row's scale (its low part enters through one float32
 // remainder).  Every slice product is an integer of at most 2^20, so the
 // anti-diagonal sums D_s = sum over i+j=s of A_i B_j are exact in FP32 for the
-// leading two (16 and 32 products, at most 2^24); the next two (3 and 4 MMAs
-// into one accumulator) can pass 2^24 only in the worst case, where their
+// leading two (16 and 32 products, at most 2^24); the next two (48 and 64 products)
+// can pass 2^24 only in the worst case, where their
 // rounding stays below 2^-40 of the scales.  (Integrate contracts 32 x: D2 is
 // kept as two K halves of 16 products; its D3 sums 64 and can round in the worst
 // case, by less than 2^-35 of the scales.)  The diagonals are recombined in
@@ -30,8 +30,8 @@
 // memory), added to the FP64 grid once per tile.
 //
 // Integrate is the transpose: S[(z,y)][a] = sum_x V[(z,y)][x] X[a][x] by the same
-// slices (V sliced once per tile into a per-CTA global slot that stays in L1/L2,
-// copied per pair into the operand with the pair's row masks), then the adjoint
+// slices (V sliced once per unit into the A operand, each item masking its rows there
+// and restoring them from a per-CTA global slot that stays in L2), then the adjoint
 // stages, and the per-pair moments are added to FP64 scratch with atomics.
 //
 // General (non-orthorhombic) cells use the same kernels instantiated with
