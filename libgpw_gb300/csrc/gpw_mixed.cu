@@ -1263,20 +1263,33 @@ __global__ void __launch_bounds__(NTHR, 4) k_integrate_tiled(MixedArgs A) {
             const double *grid = A.grids.p[td.level];
             const int64_t row = ((int64_t)(td.t[2] * TZ + z) * lv.ngrid[1] + (td.t[1] * TY + y)) * lv.ngrid[0] +
                                 td.t[0] * TX;
-            // compact loops (once per unit): the row maximum, then 16-byte chunks of 8 x; 8
-            // loads in flight (one at a time, their latency was a tenth of a 16-item unit)
+            // compact loops (once per unit): the row as float-float and its maximum, then
+            // 16-byte chunks of 8 x; 8 loads in flight (one at a time, their latency was a
+            // tenth of a 16-item unit).  Between the two the row lies where its slices will
+            // (as many bytes), and the split is done on the integer pipe (read twice and split
+            // by conversions, 17 cycles a warp each: 1000 pairs on 64^3, units of 31 items, 261
+            // against 240 us; three levels, units of 60, 3.86 against 3.80 ms).
             float mx = 0.0f;
 #pragma unroll 1
-            for (int x8 = 0; x8 < TX; x8 += 8) {
+            for (int c = 0; c < TX / 8; c++) {
+                const int o16 = (m >> 3) * 16 + (c & 1) * 8 + (m & 7);  // offset of (m, 8 c) / 16
                 double v8[8];
 #pragma unroll
-                for (int i = 0; i < 8; i++) v8[i] = (row_ok && x8 + i < ext.x) ? grid[row + x8 + i] : 0.0;
+                for (int i = 0; i < 8; i++) v8[i] = (row_ok && 8 * c + i < ext.x) ? grid[row + 8 * c + i] : 0.0;
 #pragma unroll
-                for (int i = 0; i < 8; i += 2) {
-                    const ff v0 = ff_from_double(v8[i]), v1 = ff_from_double(v8[i + 1]);
-                    if constexpr (kGeneral)
-                        reinterpret_cast<float4 *>(vslot)[((x8 + i) / 2) * MROWS + m] =
-                            make_float4(v0.hi, v0.lo, v1.hi, v1.lo);
+                for (int i = 0; i < 4; i++) {
+                    ff v0, v1;
+                    if constexpr (kGeneral) {  // (shorter code counts for more: 6.76 against 6.83 ms)
+                        v0 = ff_from_double(v8[2 * i]);
+                        v1 = ff_from_double(v8[2 * i + 1]);
+                    } else {
+                        const bool in0 = row_ok && 8 * c + 2 * i < ext.x, in1 = row_ok && 8 * c + 2 * i + 1 < ext.x;
+                        v0 = in0 ? ff_from_double_bits(v8[2 * i]) : ff{0.0f, 0.0f};
+                        v1 = in1 ? ff_from_double_bits(v8[2 * i + 1]) : ff{0.0f, 0.0f};
+                    }
+                    const float4 v = make_float4(v0.hi, v0.lo, v1.hi, v1.lo);
+                    if constexpr (kGeneral) reinterpret_cast<float4 *>(vslot)[(4 * c + i) * MROWS + m] = v;
+                    else reinterpret_cast<float4 *>(sm.A[c >> 1][i])[o16] = v;
                     mx = fmaxf(mx, fmaxf(fabsf(v0.hi), fabsf(v1.hi)));
                 }
             }
@@ -1284,18 +1297,17 @@ __global__ void __launch_bounds__(NTHR, 4) k_integrate_tiled(MixedArgs A) {
             const float sc = vm == kZeroExp ? 0.0f : pow2i(SLB - vm);
 #pragma unroll 1
             for (int c = 0; c < TX / 8 && !kGeneral; c++) {  // 8 x per 16-byte chunk of the UMMA layout
+                const int o16 = (m >> 3) * 16 + (c & 1) * 8 + (m & 7);
                 uint32_t w[NSL][4];
+                static_assert(NSL == 4, "8 float-float values fill the chunks of their slices");
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
-                    const int x = 8 * c + 2 * i;
-                    const ff v0 = (row_ok && x < ext.x) ? ff_from_double(grid[row + x]) : ff{0.0f, 0.0f};
-                    const ff v1 = (row_ok && x + 1 < ext.x) ? ff_from_double(grid[row + x + 1]) : ff{0.0f, 0.0f};
+                    const float4 v = reinterpret_cast<const float4 *>(sm.A[c >> 1][i])[o16];
                     float2 sl[NSL];
-                    slice_scaled2(ff2_pair(v0, v1), f2(sc), sl);
+                    slice_scaled2(ff2{make_float2(v.x, v.z), make_float2(v.y, v.w)}, f2(sc), sl);
 #pragma unroll
                     for (int q = 0; q < NSL; q++) w[q][i] = pack_halves(sl[q]);
                 }
-                const int o16 = (m >> 3) * 16 + (c & 1) * 8 + (m & 7);  // offset of (m, 8 c) / 16
 #pragma unroll
                 for (int q = 0; q < NSL; q++) {
                     const uint4 val = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
