@@ -16,7 +16,6 @@ struct alignas(8) ff {
     float hi, lo;
 };
 
-__device__ __forceinline__ ff ff_make(float a) { return {a, 0.0f}; }
 
 // The same split on the integer pipe (a conversion costs as much as an FP64 multiply-add
 // here, 17 cycles a warp and SM): the 23 leading mantissa bits rounded to nearest, then
@@ -53,7 +52,6 @@ __device__ __forceinline__ ff ff_from_double(double d) {
     return {h, __double2float_rn(d - (double)h)};
 }
 
-__device__ __forceinline__ double ff_to_double(ff a) { return (double)a.hi + (double)a.lo; }
 
 // s + e == a + b exactly (Knuth)
 __device__ __forceinline__ ff two_sum(float a, float b) {
@@ -99,20 +97,6 @@ __device__ __forceinline__ ff ff_fma(ff a, ff b, ff c) {
     const ff s = two_sum(p, c.hi);
     const float t = __fadd_rn(s.lo, __fadd_rn(e, c.lo));
     return fast_two_sum(s.hi, t);
-}
-
-// s += a*b with the sum kept unnormalised: s.hi takes the rounded sum of the
-// leading products (exact error by two-sum), s.lo gathers the errors and the
-// cross terms.  |s.lo| stays a few ulps of s.hi over short sums; normalise with
-// ff_add / fast_two_sum before the value is used elsewhere.
-__device__ __forceinline__ void ff_acc_lazy(ff &s, ff a, ff b) {
-    const float p = __fmul_rn(a.hi, b.hi);
-    float e = __fmaf_rn(a.hi, b.hi, -p);
-    e = __fmaf_rn(a.hi, b.lo, e);
-    e = __fmaf_rn(a.lo, b.hi, e);
-    const ff t = two_sum(s.hi, p);
-    s.hi = t.hi;
-    s.lo = __fadd_rn(s.lo, __fadd_rn(t.lo, e));
 }
 
 // Two independent floats per instruction (FFMA2 / FADD2 / FMUL2): the same
@@ -173,6 +157,9 @@ __device__ __forceinline__ ff2 ff2_fma(ff2 a, ff2n b, ff2 c) {
     const ff2 q = ff2_prodn(a, b), s = two_sum2(q.hi, c.hi);
     return fast_two_sum2(s.hi, f2_add(s.lo, f2_sub(c.lo, q.lo)));
 }
+// s += a b with the sums kept unnormalised: s.hi takes the rounded sum of the leading
+// products (exact error by two-sum), s.lo gathers the errors and the cross terms.
+// |s.lo| stays a few ulps of s.hi over short sums; normalise before other use.
 __device__ __forceinline__ void ff2_acc_lazy(ff2 &s, ff2 a, ff2n b) {
     const ff2 q = ff2_prodn(a, b), t = two_sum2(s.hi, q.hi);
     s.hi = t.hi;

@@ -154,8 +154,6 @@ struct MixedState {
     int64_t nbin = 0;            // tasks [0, nbin) are binned (the ortho ones, then general ones if tiled)
     bool gen_tiled = false;      // general-cell pairs run on the tiled kernels
     int ntiles_ortho = 0;        // tiles [0, ntiles_ortho) are orthorhombic, the rest general
-    int grid_ctas = 0;    // collocate
-    int grid_ctas_i = 0;  // integrate
     int sms = 0;
     int per_sm = 0, per_sm_i = 0, per_sm_ig = 0;  // resident CTAs: collocate, integrate (ortho, general)
     uint4 *d_vslot = nullptr;  // integrate: per-CTA V slots
@@ -2212,8 +2210,6 @@ int mixed_rebin(TaskSet &ts, std::string &err) {
     M->ntiles_ortho = nuo;
     M->ntiles = nunits;
     M->nitems = nitems;
-    M->grid_ctas_i = std::max(1, std::min(nunits, M->sms * M->per_sm_i));
-    M->grid_ctas = std::max(1, std::min(nunits, M->sms * M->per_sm));
     return GPW_SUCCESS;
 }
 

@@ -107,13 +107,6 @@ __device__ __forceinline__ void tmem_wait_ld8(uint32_t *r) {
                  : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
                  :: "memory");
 }
-__device__ __forceinline__ void tmem_wait_ld24(uint32_t *a, uint32_t *b, uint32_t *c) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
-                   "+r"(b[0]), "+r"(b[1]), "+r"(b[2]), "+r"(b[3]), "+r"(b[4]), "+r"(b[5]), "+r"(b[6]), "+r"(b[7]),
-                   "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]), "+r"(c[4]), "+r"(c[5]), "+r"(c[6]), "+r"(c[7])
-                 :: "memory");
-}
 __device__ __forceinline__ void tmem_wait_ld32(uint32_t *a, uint32_t *b, uint32_t *c, uint32_t *d) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
                  : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
