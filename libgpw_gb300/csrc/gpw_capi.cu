@@ -531,6 +531,7 @@ int gpw_taskset_create(gpw_plan *plan, const gpw_task *tasks, int64_t ntasks, in
         coef += ncoef(g.lp);
         g.mom_ext_off = mom_ext;
         mom_ext += ncoef(g.lp + 2);
+        T->level_mask |= 1u << g.level;
         T->max_lp = std::max(T->max_lp, g.lp);
         T->max_A = std::max(T->max_A, g.la_max);
         T->max_B = std::max(T->max_B, g.lb_max);
@@ -671,6 +672,10 @@ int gpw_backward(gpw_taskset *ts, const double *d_pab, double *const *d_grids, d
     cudaStream_t s = (cudaStream_t)stream;
     GridPtrs g = grid_ptrs(*ts->plan, d_grids);
     const bool grads = d_dra || d_drb || d_dzeta || d_dzetb;
+    // every grid for the matrix elements (as gpw_integrate), those with pairs for the gradients
+    for (int l = 0; l < ts->plan->nlevels; l++)
+        if (!d_grids[l] && (d_hab || (grads && (ts->level_mask >> l & 1u))))
+            return fail(GPW_ERR_INVALID_ARG, "gpw_backward: null grid");
     if (d_hab && !(grads && backward_supported(*ts))) {
         int st = gpw_integrate(ts, GPW_PREC_FP64, d_grids, d_hab, stream);
         if (st) return st;

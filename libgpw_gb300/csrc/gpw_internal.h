@@ -34,6 +34,7 @@ struct TaskSet {
     int64_t pab_extent = 0;
     int max_lp = 0;
     int max_A = 0, max_B = 0;
+    unsigned level_mask = 0;       // bit l: some pair lies on level l
     std::vector<PairGeom> h_geom;  // sorted (stale after a device geometry update until refreshed)
     bool h_geom_stale = false;
     PairGeom *d_geom = nullptr;
