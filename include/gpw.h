@@ -60,7 +60,9 @@ enum gpw_function {
 
 /* Arithmetic of the cube contraction. */
 enum gpw_precision {
-    GPW_PREC_FP64 = 0,   /* plain FP64 kernels, FP64 atomics into the grid       */
+    GPW_PREC_FP64 = 0,   /* plain FP64 kernels, FP64 atomics into the grid;      */
+                         /* integrate and backward repeat bit for bit where no   */
+                         /* two pairs share an element of the block buffer       */
     GPW_PREC_MIXED = 1   /* tiled kernels: FP64 pair set-up, split-FP32 tables,   */
                          /* tensor-core cube contraction, compensated            */
                          /* accumulation, one FP64 write per grid point          */

@@ -554,10 +554,7 @@ int gpw_taskset_create(gpw_plan *plan, const gpw_task *tasks, int64_t ntasks, in
     int gen_limit = 0;
     for (int64_t m = 0; m < ntasks; m++) {
         if (T->h_geom[m].ortho) continue;
-        if (T->gen_count == 0) {
-            T->gen_first = (int)m;
-            T->gen_coef_first = T->h_geom[m].coef_off;
-        }
+        if (T->gen_count == 0) T->gen_first = (int)m;
         T->gen_count++;
         T->gen_smem = std::max(T->gen_smem, smem_general_ff(T->h_geom[m]));
         gen_limit = std::max(gen_limit, smem_general_ff_limit(T->h_geom[m]));
@@ -579,7 +576,13 @@ int gpw_taskset_create(gpw_plan *plan, const gpw_task *tasks, int64_t ntasks, in
     alloc((void **)&T->d_coef, sizeof(double) * (size_t)coef);
     alloc((void **)&T->d_mom, sizeof(double) * (size_t)coef);
     alloc((void **)&T->d_status, sizeof(int));
-    alloc((void **)&T->d_fp64_items, sizeof(Fp64Item) * items.size());
+    // the FP64 items, and the divided pairs' slots and tickets, in one block
+    const size_t slots = (size_t)T->fp64_slots, items_len = sizeof(Fp64Item) * items.size(),
+                 parts_len = sizeof(double) * slots * ncoef(T->max_lp);
+    alloc((void **)&T->d_fp64_items, items_len + parts_len + sizeof(int) * slots);
+    T->d_parts = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(T->d_fp64_items) + items_len);
+    T->d_ticket = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(T->d_parts) + parts_len);
+    if (e == cudaSuccess && slots > 0) e = cudaMemset(T->d_ticket, 0, sizeof(int) * slots);
     if (e == cudaSuccess && !items.empty())
         e = cudaMemcpy(T->d_fp64_items, items.data(), sizeof(Fp64Item) * items.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && ntasks > 0)

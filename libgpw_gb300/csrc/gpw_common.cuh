@@ -279,9 +279,10 @@ struct PairGeom {
     int pad_;
 };
 
-// One CTA's work in the FP64 launches: planes part, part + nparts, ... of a pair.
+// One CTA's work in the FP64 launches: planes part, part + nparts, ... of a pair.  The
+// items of divided pairs are counted through, a pair's in a row: slot (-1: undivided).
 struct Fp64Item {
-    int pair, part, nparts;
+    int pair, part, nparts, slot;
 };
 
 // Device status bits (OR-ed by kernels, read by gpw_taskset_check).

@@ -148,7 +148,7 @@ __global__ void k_backtransform(const PairGeom *__restrict__ geoms, const LevelD
 // other) took 21.1 ms to integrate and 6.1 ms to collocate 1000 pairs (l <= 2,
 // 64^3); this one takes 0.46 and 0.46 ms, 62 % of the FP64 rate (1.10 TFLOP/s in a
 // GEMM) counting L multiply-adds per cube point.
-constexpr int kOrthoWarps = 4;
+constexpr int kOrthoWarps = 4;  // (a power of two)
 
 // the shared memory of orthorhombic item (pair g, 1 of nparts), in bytes
 int smem_ortho_item(const PairGeom &g, int extra, int nparts) {
@@ -167,12 +167,49 @@ int smem_ortho_fp64(const PairGeom &g) {
     return 8 * (L * L * L + L * (nx + ny + nz) + L * L + ny * L) + 8 * ny;
 }
 
-// the item's next plane, taken warp by warp (planes differ in size: the middle ones hold
-// most of a sphere's points)
-__device__ __forceinline__ int next_plane(int *counter) {
-    int p = 0;
-    if ((threadIdx.x & 31) == 0) p = atomicAdd(counter, 1);
-    return __shfl_sync(0xffffffffu, p, 0);
+// Integrate's results are the same bits from call to call: every sum has a fixed order.
+// Where a warp's planes are added up they are dealt out beforehand, turn t (warp w has
+// t = w, w + 4, ...) of an item of np planes, the largest (the middle ones) first and the
+// warps in alternating order, so that their shares are about equal; -1: none in this turn.
+// (Planes taken from a counter as warps come free, and parts added by atomics: 860 us for
+// both directions of 1000 pairs on 64^3, 6.82 ms for 1500 general pairs on 128^3, mixed;
+// this order 863 us and 6.72 ms.)
+__device__ __forceinline__ int plane_of_turn(int t, int np) {
+    const int j = np - 1 - ((t / kOrthoWarps) & 1 ? t ^ (kOrthoWarps - 1) : t);
+    return j < 0 ? -1 : (j & 1 ? np - 1 - (j >> 1) : j >> 1);
+}
+
+// Moments of divided pairs: a slot per item, stride moments each.
+struct PartSums {
+    double *sum;
+    int *ticket;
+    int stride;
+};
+// An item's moments value(t), t < nc, to its pair's.  Those of a divided pair go to the
+// item's slot, and the CTA that comes last adds up the parts, in order.
+template <class F>
+__device__ __forceinline__ void put_moments(const Fp64Item &it, int nc, const PartSums &ps, double *out, F value) {
+    if (it.nparts == 1) {
+        for (int t = threadIdx.x; t < nc; t += blockDim.x) out[t] = value(t);
+        return;
+    }
+    __shared__ bool last;
+    double *first = ps.sum + (int64_t)(it.slot - it.part) * ps.stride;
+    for (int t = threadIdx.x; t < nc; t += blockDim.x) __stcg(first + (int64_t)it.part * ps.stride + t, value(t));
+    __threadfence();
+    __syncthreads();
+    int *ticket = ps.ticket + (it.slot - it.part);
+    if (threadIdx.x == 0) last = atomicAdd(ticket, 1) == it.nparts - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int t = threadIdx.x; t < nc; t += blockDim.x) {
+        double s = 0.0;
+#pragma unroll 8
+        for (int p = 0; p < it.nparts; p++) s += __ldcg(first + (int64_t)p * ps.stride + t);
+        out[t] = s;
+    }
+    if (threadIdx.x == 0) *ticket = 0;  // for the next launch
 }
 
 // kAcc: the registers of T, L <= kAcc (kNPow, or kNPowB for the backward pass's
@@ -181,12 +218,12 @@ template <bool kAdj, int kAcc>
 __global__ void __launch_bounds__(32 * kOrthoWarps)
 k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ items, int uparts,
              const LevelDev *__restrict__ levels, const int *__restrict__ table, const double *__restrict__ coef,
-             double *__restrict__ mom, GridPtrs grids, int *status, int extra) {
+             double *__restrict__ mom, PartSums ps, GridPtrs grids, int *status, int extra) {
     extern __shared__ double sm[];
     constexpr int kN2 = (kAcc * (kAcc + 1)) / 2, kM2 = (kN2 + 31) / 32;        // (ly, lx) sums per lane
     constexpr int kNC = (kAcc * (kAcc + 1) * (kAcc + 2)) / 6, kMC = (kNC + 31) / 32;  // moments per lane
     const int bid = blockIdx.x;
-    const Fp64Item it = items ? items[bid] : Fp64Item{bid / uparts, bid % uparts, uparts};
+    const Fp64Item it = items ? items[bid] : Fp64Item{bid / uparts, bid % uparts, uparts, -1};
     const PairGeom &g = geoms[it.pair];
     const LevelDev &lv = levels[g.level];
     double *__restrict__ grid = grids.p[g.level];
@@ -252,20 +289,16 @@ k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
 #pragma unroll
     for (int m = 0; m < (kAdj ? kMC : 1); m++) W[m] = 0.0;
     const SphereRule rule(g.radius, lv.dh[0][0], lv.dh[1][1], lv.dh[2][2]);
-    __shared__ int s_next;
-    if (tid == 0) s_next = 0;
     const int *T0 = g.table_off >= 0 ? table + g.table_off : nullptr;
     const int gn0 = lv.ngrid[0], gn1 = lv.ngrid[1];
     __syncthreads();
-    // integrate's CTAs end with a sum over the warps: planes taken as warps come free (485
-    // -> 458 us on the workload above; collocate, whose warps end alone, loses 1 %)
     // Collocate with fewer planes than warps (a call with one pair): 2^lsub warps share a
     // plane's rows, T computed by each (36 planes of 36 x 36, one pair, L = 2: 9 CTAs of four
     // planes 14.3 us, 36 CTAs of one 9.0 us).
     const int lsub = kAdj || np > 2 ? 0 : 3 - np, sub = warp & ((1 << lsub) - 1);
-    for (int turn = warp >> lsub;; turn += kOrthoWarps >> lsub) {
-        const int pl = kAdj ? next_plane(&s_next) : turn;
-        if (pl >= np) break;
+    for (int turn = warp >> lsub; (kAdj ? turn - warp : turn) < np; turn += kOrthoWarps >> lsub) {
+        const int pl = kAdj ? plane_of_turn(turn, np) : turn;
+        if (kAdj && pl < 0) continue;
         const int kg = kgmin + it.part + pl * it.nparts, kf = fold(kg);
         const int k = axis_index(lv.periodic[2], g.cc[2], kg, g.lb[2], lv.lb_grid[2], lv.npts[2], lv.ngrid[2]);
         if (k < 0) {
@@ -429,11 +462,7 @@ k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
             }
             __syncthreads();
         }
-        double *out = mom + (extra ? g.mom_ext_off : g.coef_off);
-        for (int t = tid; t < nc; t += 32 * kOrthoWarps) {
-            if (it.nparts == 1) out[t] = C[t];
-            else atomicAdd(out + t, C[t]);  // several items of one pair (zeroed before the launch)
-        }
+        put_moments(it, nc, ps, mom + (extra ? g.mom_ext_off : g.coef_off), [&](int t) { return C[t]; });
     }
 }
 
@@ -451,10 +480,10 @@ template <bool kAdj>
 __global__ void __launch_bounds__(256)
 k_general_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ items, int uparts,
              const LevelDev *__restrict__ levels,
-               const double *__restrict__ coef, double *__restrict__ mom, GridPtrs grids,
+               const double *__restrict__ coef, double *__restrict__ mom, PartSums ps, GridPtrs grids,
                int *status, int extra) {
     extern __shared__ double sm[];
-    const Fp64Item it = items ? items[blockIdx.x] : Fp64Item{(int)blockIdx.x / uparts, (int)blockIdx.x % uparts, uparts};
+    const Fp64Item it = items ? items[blockIdx.x] : Fp64Item{(int)blockIdx.x / uparts, (int)blockIdx.x % uparts, uparts, -1};
     const PairGeom g = geoms[it.pair];
     const LevelDev &lv = levels[g.level];
     double *__restrict__ grid = grids.p[g.level];
@@ -591,13 +620,11 @@ k_general_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ 
         }
     }
     if (kAdj) {
-        for (int t = tid; t < L * L * L; t += nthr) {
-            const int i = t % L, j = (t / L) % L, k = t / (L * L);
-            if (i + j + k > lp) continue;
-            double *out = mom + mom_off + pidx(lp, k, j, i);
-            if (it.nparts == 1) *out = Q[t];
-            else atomicAdd(out, Q[t]);
-        }
+        const uint32_t *dec = d_decode.e + d_decode_at(lp);
+        put_moments(it, ncoef(lp), ps, mom + mom_off, [&](int t) {
+            const uint32_t de = __ldg(dec + t);  // (k, j, i)
+            return Q[((de & 15) * L + (de >> 4 & 15)) * L + (de >> 8 & 15)];
+        });
     }
 }
 
@@ -642,10 +669,10 @@ template <bool kAdj>
 __global__ void __launch_bounds__(32 * kOrthoWarps, 4)
 k_general_ff(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ items, int uparts,
              const LevelDev *__restrict__ levels, const double *__restrict__ coef, double *__restrict__ mom,
-             GridPtrs grids, int *status) {
+             PartSums ps, GridPtrs grids, int *status) {
     extern __shared__ double smd[];
     constexpr int kM2 = (kNPow * (kNPow + 1) / 2 + 31) / 32, kMC = ((kMaxLp + 1) * (kMaxLp + 2) * (kMaxLp + 3) / 6 + 31) / 32;
-    const Fp64Item it = items ? items[blockIdx.x] : Fp64Item{(int)blockIdx.x / uparts, (int)blockIdx.x % uparts, uparts};
+    const Fp64Item it = items ? items[blockIdx.x] : Fp64Item{(int)blockIdx.x / uparts, (int)blockIdx.x % uparts, uparts, -1};
     const PairGeom &g = geoms[it.pair];
     const LevelDev &lv = levels[g.level];
     double *__restrict__ grid = grids.p[g.level];
@@ -665,8 +692,6 @@ k_general_ff(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
     int *i0 = reinterpret_cast<int *>(a0l + kGenRows), *i1 = i0 + kGenRows;
     ff *sC = reinterpret_cast<ff *>(i1 + 2 * kGenRows);  // Qjk, packed (j, i)
     ff *sT = sC + n2;                                    // [j][lane], rows of 33
-    __shared__ int s_next;
-    if (tid == 0) s_next = 0;
     if (tid < 32) exptab[tid] = c_exp2_32[tid];
     int off[3];
     for (int d = 0; d < 3; d++) off[d] = imod(g.cc[d] + lv.lb_grid[d], lv.npts[d]);
@@ -713,9 +738,11 @@ k_general_ff(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
     const ff2n mz = ff2n_dup(ff_from_double(-g.zetp));
     const int gn0 = lv.ngrid[0], gn1 = lv.ngrid[1], np0 = lv.npts[0], per0 = lv.periodic[0];
     __syncthreads();
-    for (;;) {
-        const int kk = cc2 + it.part + next_plane(&s_next) * it.nparts;
-        if (kk > g.hi[2]) break;
+    const int np = (g.hi[2] - cc2 + it.nparts - it.part) / it.nparts;  // this item's planes
+    for (int turn = warp; turn - warp < np; turn += kOrthoWarps) {
+        const int pl = plane_of_turn(turn, np);
+        if (pl < 0) continue;
+        const int kk = cc2 + it.part + pl * it.nparts;
         const double dk = rsub((double)kk, g.off[2]);
         const int kidx = lv.periodic[2] ? imod(kk, lv.npts[2]) : kk - cc2 + off[2];
         if (kidx < 0 || kidx >= lv.ngrid[2]) {
@@ -902,12 +929,7 @@ k_general_ff(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
             }
             __syncthreads();
         }
-        double *out = mom + g.coef_off;
-        for (int t = tid; t < nc; t += 32 * kOrthoWarps) {
-            const double v = (double)Q[t].hi + (double)Q[t].lo;
-            if (it.nparts == 1) out[t] = v;
-            else atomicAdd(out + t, v);
-        }
+        put_moments(it, nc, ps, mom + g.coef_off, [&](int t) { return (double)Q[t].hi + (double)Q[t].lo; });
     }
 }
 
@@ -965,7 +987,7 @@ void fp64_items(TaskSet &ts, int sms, int smem_limit, std::vector<Fp64Item> &ite
     const double share = total / ((double)sms * kCtas);
     ts.fp64_ortho = ts.fp64_general = 0;
     ts.fp64_smem = ts.fp64_smem_ext = ts.fp64_smem_gen = ts.fp64_smem_gen_ext = 0;
-    ts.fp64_split = false;
+    ts.fp64_slots = 0;
     constexpr int kClasses = 1024;  // sign, exponent and two mantissa bits
     std::vector<unsigned short> cls(ts.h_geom.size());
     std::vector<int> nparts(ts.h_geom.size());
@@ -987,7 +1009,6 @@ void fp64_items(TaskSet &ts, int sms, int smem_limit, std::vector<Fp64Item> &ite
             ts.fp64_smem_gen_ext = std::max(ts.fp64_smem_gen_ext, std::min(smem_general_fp64(g, 2), smem_limit));
             ts.fp64_general += parts;
         }
-        ts.fp64_split = ts.fp64_split || parts > 1;
         // class of the items' cost: a factor 2^(1/4) or so, from the float's leading bits
         const float c = (float)((double)g.cost * (g.lp + 1) / parts);
         unsigned bits;
@@ -1002,29 +1023,28 @@ void fp64_items(TaskSet &ts, int sms, int smem_limit, std::vector<Fp64Item> &ite
     int64_t at_gen = ts.fp64_ortho;
     for (size_t k = 0; k < ts.h_geom.size(); k++) {
         int64_t &at = ts.h_geom[k].ortho ? first[cls[k]] : at_gen;
-        for (int p = 0; p < nparts[k]; p++) items[(size_t)at++] = Fp64Item{(int)k, p, nparts[k]};
+        const bool split = nparts[k] > 1;
+        for (int p = 0; p < nparts[k]; p++)
+            items[(size_t)at++] = Fp64Item{(int)k, p, nparts[k], split ? ts.fp64_slots++ : -1};
     }
 }
 
 static cudaError_t launch_fp64_impl(const TaskSet &ts, const GridPtrs &g, bool adj, int extra, double *mom,
                                     cudaStream_t s) {
     const Plan &P = *ts.plan;
-    if (adj && ts.fp64_split) {  // several items add to one pair's moments
-        const cudaError_t e = cudaMemsetAsync(mom, 0, sizeof(double) * (extra ? ts.mom_ext_len : ts.coef_len), s);
-        if (e != cudaSuccess) return e;
-    }
+    const PartSums ps = {extra ? ts.d_parts_ext : ts.d_parts, ts.d_ticket, ncoef(ts.max_lp + extra)};
     if (ts.fp64_ortho > 0) {
         ProfScope prof(ts, s);
         const unsigned n = (unsigned)ts.fp64_ortho;
         if (adj && extra)
             k_ortho_fp64<true, kNPowB><<<n, 32 * kOrthoWarps, ts.fp64_smem_ext, s>>>(
-                ts.d_geom, ts.d_fp64_items, 1, P.d_levels, ts.d_table, ts.d_coef, mom, g, ts.d_status, extra);
+                ts.d_geom, ts.d_fp64_items, 1, P.d_levels, ts.d_table, ts.d_coef, mom, ps, g, ts.d_status, extra);
         else if (adj)
             k_ortho_fp64<true, kNPow><<<n, 32 * kOrthoWarps, ts.fp64_smem, s>>>(
-                ts.d_geom, ts.d_fp64_items, 1, P.d_levels, ts.d_table, ts.d_coef, mom, g, ts.d_status, 0);
+                ts.d_geom, ts.d_fp64_items, 1, P.d_levels, ts.d_table, ts.d_coef, mom, ps, g, ts.d_status, 0);
         else
             k_ortho_fp64<false, kNPow><<<n, 32 * kOrthoWarps, ts.fp64_smem, s>>>(
-                ts.d_geom, ts.d_fp64_items, 1, P.d_levels, ts.d_table, ts.d_coef, mom, g, ts.d_status, 0);
+                ts.d_geom, ts.d_fp64_items, 1, P.d_levels, ts.d_table, ts.d_coef, mom, ps, g, ts.d_status, 0);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
@@ -1034,9 +1054,9 @@ static cudaError_t launch_fp64_impl(const TaskSet &ts, const GridPtrs &g, bool a
         const Fp64Item *items = ts.d_fp64_items + ts.fp64_ortho;
         if (adj)
             k_general_fp64<true><<<n, 256, extra ? ts.fp64_smem_gen_ext : ts.fp64_smem_gen, s>>>(
-                ts.d_geom, items, 1, P.d_levels, ts.d_coef, mom, g, ts.d_status, extra);
+                ts.d_geom, items, 1, P.d_levels, ts.d_coef, mom, ps, g, ts.d_status, extra);
         else
-            k_general_fp64<false><<<n, 256, ts.fp64_smem_gen, s>>>(ts.d_geom, items, 1, P.d_levels, ts.d_coef, mom, g,
+            k_general_fp64<false><<<n, 256, ts.fp64_smem_gen, s>>>(ts.d_geom, items, 1, P.d_levels, ts.d_coef, mom, ps, g,
                                                                   ts.d_status, 0);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
@@ -1059,19 +1079,15 @@ int smem_general_ff_limit(const PairGeom &g) {
 // one launch over the items of all general-cell pairs
 cudaError_t launch_general_ff(const TaskSet &ts, const GridPtrs &g, bool adj, cudaStream_t s) {
     if (ts.gen_count == 0) return cudaSuccess;
-    if (adj && ts.fp64_split) {  // several items add to one pair's moments
-        const int64_t c0 = ts.gen_coef_first;
-        const cudaError_t e = cudaMemsetAsync(ts.d_mom + c0, 0, sizeof(double) * (ts.coef_len - c0), s);
-        if (e != cudaSuccess) return e;
-    }
+    const PartSums ps = {ts.d_parts, ts.d_ticket, ncoef(ts.max_lp)};
     ProfScope prof(ts, s);
     const unsigned n = (unsigned)ts.fp64_general;
     const Fp64Item *items = ts.d_fp64_items + ts.fp64_ortho;
     if (adj)
-        k_general_ff<true><<<n, 32 * kOrthoWarps, ts.gen_smem, s>>>(ts.d_geom, items, 1, ts.plan->d_levels, ts.d_coef, ts.d_mom, g,
+        k_general_ff<true><<<n, 32 * kOrthoWarps, ts.gen_smem, s>>>(ts.d_geom, items, 1, ts.plan->d_levels, ts.d_coef, ts.d_mom, ps, g,
                                                       ts.d_status);
     else
-        k_general_ff<false><<<n, 32 * kOrthoWarps, ts.gen_smem, s>>>(ts.d_geom, items, 1, ts.plan->d_levels, ts.d_coef, ts.d_mom, g,
+        k_general_ff<false><<<n, 32 * kOrthoWarps, ts.gen_smem, s>>>(ts.d_geom, items, 1, ts.plan->d_levels, ts.d_coef, ts.d_mom, ps, g,
                                                        ts.d_status);
     return cudaGetLastError();
 }
@@ -1091,7 +1107,7 @@ cudaError_t launch_pairs_fp64(const PairGeom *d_geoms, const LevelDev *d_levels,
     GridPtrs g;
     for (int l = 0; l < GPW_MAX_LEVELS; l++) g.p[l] = d_grid;
     k_ortho_fp64<false, kNPow><<<(unsigned)(n * uparts), 32 * kOrthoWarps, smem_coll, s>>>(
-        d_geoms, nullptr, uparts, d_levels, nullptr, d_coef, nullptr, g, d_status, 0);
+        d_geoms, nullptr, uparts, d_levels, nullptr, d_coef, nullptr, PartSums{}, g, d_status, 0);
     return cudaGetLastError();
 }
 
@@ -1113,10 +1129,10 @@ cudaError_t launch_one_fp64(const PairGeom &g, const PairGeom *d_geom, const Lev
     const int parts = fp64_single_parts(g);
     if (g.ortho)
         k_ortho_fp64<false, kNPow><<<(unsigned)parts, 32 * kOrthoWarps, smem_ortho_item(g, 0, parts), s>>>(
-            d_geom, nullptr, parts, d_levels, d_table, d_coef, nullptr, gp, d_status, 0);
+            d_geom, nullptr, parts, d_levels, d_table, d_coef, nullptr, PartSums{}, gp, d_status, 0);
     else
         k_general_fp64<false><<<(unsigned)parts, 256, smem_general_fp64(g), s>>>(d_geom, nullptr, parts, d_levels,
-                                                                               d_coef, nullptr, gp, d_status, 0);
+                                                                               d_coef, nullptr, PartSums{}, gp, d_status, 0);
     return cudaGetLastError();
 }
 

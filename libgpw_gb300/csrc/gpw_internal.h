@@ -51,8 +51,12 @@ struct TaskSet {
     int64_t fp64_ortho = 0, fp64_general = 0;
     int fp64_smem = 0, fp64_smem_ext = 0;          // shared memory (ext: with two extra powers)
     int fp64_smem_gen = 0, fp64_smem_gen_ext = 0;
-    bool fp64_split = false;       // some pair is divided into several items
-    int64_t gen_coef_first = 0;    // general-cell pairs: first coefficient
+    // divided pairs: per slot the part's moments (ext: to degree lp + 2), and at a pair's
+    // first slot the count of its parts that are done.  d_parts and d_ticket lie behind
+    // the items, d_parts_ext behind d_mom_ext.
+    int fp64_slots = 0;
+    double *d_parts = nullptr, *d_parts_ext = nullptr;
+    int *d_ticket = nullptr;
     MixedState *mixed = nullptr;
     int tile_lz[GPW_MAX_LEVELS];   // tiled path: log2 of the tile's z extent per level
     int gen_first = 0, gen_count = 0, gen_smem = 0;  // general-cell pairs (float-float kernel)
