@@ -174,11 +174,11 @@ k_backward_epilogue(const PairGeom *__restrict__ geoms, const LevelDev *__restri
 }
 
 // orthorhombic moments go to degree lp + 2 <= kMaxLpB; general cells map them through
-// the lattice transform, which is built to degree kMaxLp
+// the lattice transform, which is built to degree kMaxLp; their tables must fit a CTA
 bool backward_supported(const TaskSet &ts) {
     for (int64_t k = ts.gen_first; k < ts.gen_first + ts.gen_count; k++)
         if (ts.h_geom[k].lp + 2 > kMaxLp) return false;
-    return ts.max_lp + 2 <= kMaxLpB;
+    return ts.fp64_ext_fits && ts.max_lp + 2 <= kMaxLpB;
 }
 
 cudaError_t launch_backward(const TaskSet &ts, const double *d_pab, const GridPtrs &g, double *d_hab,

@@ -577,7 +577,7 @@ int gpw_taskset_create(gpw_plan *plan, const gpw_task *tasks, int64_t ntasks, in
     alloc((void **)&T->d_mom, sizeof(double) * (size_t)coef);
     alloc((void **)&T->d_status, sizeof(int));
     // the FP64 items, and the divided pairs' slots and tickets, in one block
-    const size_t slots = (size_t)T->fp64_slots, items_len = sizeof(Fp64Item) * items.size(),
+    const size_t slots = (size_t)T->fp64_slots, items_len = (sizeof(Fp64Item) * items.size() + 15) / 16 * 16,
                  parts_len = sizeof(double) * slots * ncoef(T->max_lp);
     alloc((void **)&T->d_fp64_items, items_len + parts_len + sizeof(int) * slots);
     T->d_parts = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(T->d_fp64_items) + items_len);
@@ -1050,7 +1050,7 @@ int gpw_collocate_pgf_product_rspace(int compute_tau, int use_ortho, int la_max,
     double *d_grid = reinterpret_cast<double *>(C.d_buf + o_grid);
     GPW_CUDA(launch_one_fp64(g, reinterpret_cast<PairGeom *>(C.d_buf), C.plan->d_levels, C.plan->d_tmat,
                              reinterpret_cast<int *>(C.d_buf + o_table), C.d_coef, d_status, func,
-                             reinterpret_cast<double *>(C.d_buf + o_pab), d_grid, s));
+                             reinterpret_cast<double *>(C.d_buf + o_pab), d_grid, smem_limit, s));
     GPW_CUDA(cudaMemcpyAsync(C.h_buf + o_stat, C.d_buf + o_stat, total - o_stat, cudaMemcpyDeviceToHost, s));
     GPW_CUDA(cudaStreamSynchronize(s));
     int h = 0;

@@ -279,10 +279,12 @@ struct PairGeom {
     int pad_;
 };
 
-// One CTA's work in the FP64 launches: planes part, part + nparts, ... of a pair.  The
-// items of divided pairs are counted through, a pair's in a row: slot (-1: undivided).
+// One CTA's work in the FP64 launches: planes part, part + nparts, ... of a pair, or,
+// where an orthorhombic cube's x table would not fit a CTA, part is (planes' part) xparts +
+// (x part) and nparts the product of both.  The items of divided pairs are counted
+// through, a pair's in a row: slot (-1: undivided).
 struct Fp64Item {
-    int pair, part, nparts, slot;
+    int pair, part, nparts, xparts, slot;
 };
 
 // Device status bits (OR-ed by kernels, read by gpw_taskset_check).

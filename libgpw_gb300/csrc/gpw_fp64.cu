@@ -150,13 +150,27 @@ __global__ void k_backtransform(const PairGeom *__restrict__ geoms, const LevelD
 // GEMM) counting L multiply-adds per cube point.
 constexpr int kOrthoWarps = 4;  // (a power of two)
 
-// the shared memory of orthorhombic item (pair g, 1 of nparts), in bytes
-int smem_ortho_item(const PairGeom &g, int extra, int nparts) {
+// the rows jf <= 0 that a cube can have: those whose mirror 1 - jf lies inside as well
+GPW_HD int folded_rows(const PairGeom &g) { return 1 - (g.lb[1] > 1 - g.hi[1] ? g.lb[1] : 1 - g.hi[1]); }
+
+// the shared memory of one of the items of pair g (planes in zparts, columns in xparts), in
+// bytes; kOrthoStatic of it are the kernel's static shared variables
+constexpr int kOrthoStatic = 16;
+int smem_ortho_item(const PairGeom &g, int extra, int zparts, int xparts) {
     const int L = g.lp + 1 + extra;
-    const int nx = g.hi[0] - g.lb[0] + 1, ny = g.hi[1] - g.lb[1] + 1, nz = g.hi[2] - g.lb[2] + 1;
-    const int np = (nz + nparts - 1) / nparts, nc = ncoef(L - 1);
+    const int nx = (g.hi[0] - g.lb[0] + xparts) / xparts, ny = g.hi[1] - g.lb[1] + 1, nz = g.hi[2] - g.lb[2] + 1;
+    const int np = (nz + zparts - 1) / zparts, nc = ncoef(L - 1);
     return 8 * (nc + L * (nx + ny + np) + kOrthoWarps * (33 * L + nshell(L - 1))) +
-           4 * (nx + ny + nc + kOrthoWarps * (1 - g.lb[1]));
+           4 * (nx + ny + nc + kOrthoWarps * folded_rows(g)) + kOrthoStatic;
+}
+// Parts such that an item fits a CTA: planes first, then columns.  extra = 0: one plane
+// and a few columns always fit where smem_ortho_fp64 does, since the tables of y then take
+// 8 L + 12 bytes a row, less than its 16 L + 8.  (Matters for thousands of columns only.)
+bool fit_ortho_item(const PairGeom &g, int extra, int smem_limit, int &zparts, int &xparts) {
+    const int planes = 2 - 2 * g.kgmin, nx = g.hi[0] - g.lb[0] + 1;
+    while (zparts < planes && smem_ortho_item(g, extra, zparts, xparts) > smem_limit) zparts++;
+    while (xparts < nx && smem_ortho_item(g, extra, zparts, xparts) > smem_limit) xparts *= 2;
+    return smem_ortho_item(g, extra, zparts, xparts) <= smem_limit;
 }
 
 // The cube sizes that the FP64 path accepts: what one CTA held when it kept a
@@ -216,22 +230,30 @@ __device__ __forceinline__ void put_moments(const Fp64Item &it, int nc, const Pa
 // moments to degree lp + 2)
 template <bool kAdj, int kAcc>
 __global__ void __launch_bounds__(32 * kOrthoWarps)
-k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ items, int uparts,
+k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ items, int uparts, int uxparts,
              const LevelDev *__restrict__ levels, const int *__restrict__ table, const double *__restrict__ coef,
              double *__restrict__ mom, PartSums ps, GridPtrs grids, int *status, int extra) {
     extern __shared__ double sm[];
     constexpr int kN2 = (kAcc * (kAcc + 1)) / 2, kM2 = (kN2 + 31) / 32;        // (ly, lx) sums per lane
     constexpr int kNC = (kAcc * (kAcc + 1) * (kAcc + 2)) / 6, kMC = (kNC + 31) / 32;  // moments per lane
     const int bid = blockIdx.x;
-    const Fp64Item it = items ? items[bid] : Fp64Item{bid / uparts, bid % uparts, uparts, -1};
+    const Fp64Item it = items ? items[bid] : Fp64Item{bid / uparts, bid % uparts, uparts, uxparts, -1};
     const PairGeom &g = geoms[it.pair];
     const LevelDev &lv = levels[g.level];
     double *__restrict__ grid = grids.p[g.level];
     const int lp = g.lp + extra, L = lp + 1, nc = ncoef(lp), n2 = nshell(lp);
-    const int lb0 = g.lb[0], lb1 = g.lb[1], kgmin = g.kgmin;
-    const int nx = g.hi[0] - lb0 + 1, ny = g.hi[1] - lb1 + 1;
+    int lb0 = g.lb[0], nx = g.hi[0] - lb0 + 1, zpart = it.part, zparts = it.nparts;
+    if (it.xparts > 1) {  // a part of the columns only
+        const int w = (nx + it.xparts - 1) / it.xparts, xpart = it.part % it.xparts;
+        zpart = it.part / it.xparts;
+        zparts = it.nparts / it.xparts;
+        lb0 += xpart * w;
+        nx = max(0, min(w, nx - xpart * w));
+    }
+    const int lb1 = g.lb[1], kgmin = g.kgmin, ny = g.hi[1] - lb1 + 1, rlb = 1 - folded_rows(g);
     const int tot = 2 - 2 * kgmin;  // planes kgmin .. 1 - kgmin
-    const int np = it.part < tot ? (tot - it.part + it.nparts - 1) / it.nparts : 0;
+    const int np = zpart < tot ? (tot - zpart + zparts - 1) / zparts : 0;
+    const int kg0 = kgmin + zpart;
     double *C = sm;            // packed coefficients, or the CTA's moments
     double *Xt = C + nc;       // [lx][x]
     double *Yt = Xt + L * nx;  // [ly][y]
@@ -244,11 +266,11 @@ k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     double *sT = wsp + warp * (33 * L + n2);  // [ly][lane], rows of 33
     double *sC = sT + 33 * L;                 // Cxy, packed (ly, lx)
-    int *rows = rows_all + warp * (1 - lb1);  // igmin of the folded rows jf = lb1 .. 0
+    int *rows = rows_all + warp * (1 - rlb) - rlb;  // igmin of the folded rows jf = rlb .. 0
     for (int t = tid; t < nx + ny + np; t += 32 * kOrthoWarps) {
         const int d = t < nx ? 0 : (t < nx + ny ? 1 : 2);
         const int gi = d == 0 ? t : (d == 1 ? t - nx : t - nx - ny);
-        const int gg = d == 0 ? lb0 + gi : (d == 1 ? lb1 + gi : kgmin + it.part + gi * it.nparts);
+        const int gg = d == 0 ? lb0 + gi : (d == 1 ? lb1 + gi : kg0 + gi * zparts);
         const int n = d == 0 ? nx : (d == 1 ? ny : np);
         double *tab = (d == 0 ? Xt : (d == 1 ? Yt : Zt)) + gi;
         const double u = (double)gg * lv.dh[d][d] - g.off[d];
@@ -289,6 +311,9 @@ k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
 #pragma unroll
     for (int m = 0; m < (kAdj ? kMC : 1); m++) W[m] = 0.0;
     const SphereRule rule(g.radius, lv.dh[0][0], lv.dh[1][1], lv.dh[2][2]);
+    const double *Xt0 = Xt - lb0;  // by cube offset
+    const int *xidx0 = xidx - lb0;
+    const int xlast = lb0 + nx - 1;
     const int *T0 = g.table_off >= 0 ? table + g.table_off : nullptr;
     const int gn0 = lv.ngrid[0], gn1 = lv.ngrid[1];
     __syncthreads();
@@ -299,7 +324,7 @@ k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
     for (int turn = warp >> lsub; (kAdj ? turn - warp : turn) < np; turn += kOrthoWarps >> lsub) {
         const int pl = kAdj ? plane_of_turn(turn, np) : turn;
         if (kAdj && pl < 0) continue;
-        const int kg = kgmin + it.part + pl * it.nparts, kf = fold(kg);
+        const int kg = kg0 + pl * zparts, kf = fold(kg);
         const int k = axis_index(lv.periodic[2], g.cc[2], kg, g.lb[2], lv.lb_grid[2], lv.npts[2], lv.ngrid[2]);
         if (k < 0) {
             if (lane == 0) atomicOr(status, kStatOutOfWindow);
@@ -312,7 +337,7 @@ k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
         __syncwarp();
         for (int jf = jgmin + lane; jf <= 0; jf += 32) {
             const int ig = Tr ? Tr[jf - jgmin] : -sphere_imax_fast(rule, kf, jf);
-            rows[jf - lb1] = ig;
+            rows[jf] = ig;
             wide = min(wide, ig);
         }
         wide = __reduce_min_sync(0xffffffffu, wide);
@@ -336,8 +361,8 @@ k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
         double cxy[kAdj ? kM2 : 1];
 #pragma unroll
         for (int m = 0; m < (kAdj ? kM2 : 1); m++) cxy[m] = 0.0;
-        const int nrow = 2 - 2 * jgmin, xend = 1 - wide;
-        for (int c0 = wide; c0 <= xend;) {
+        const int nrow = 2 - 2 * jgmin, xbeg = max(wide, lb0), xend = min(1 - wide, xlast);
+        for (int c0 = xbeg; c0 <= xend;) {
             const int left = xend - c0 + 1;
             const int lw = kAdj && left > 24 ? 5 : (left > 8 ? 4 : 3);  // log2 of the block's columns
             // (blocks of at most 32, 16, 8 columns: collocate 461, 453, 540 us on the workload
@@ -346,21 +371,21 @@ k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
             // blocks of 16 453 -> 421 us, integrate with blocks of 32 only where more than 24
             // columns are left 456 -> 451; 592 -> 574 with two more powers)
             const int grp = lane >> lw, ng = 32 >> lw;          // the lane's row group
-            const int ig = c0 + (lane & ((1 << lw) - 1)), xc = min(ig - lb0, nx - 1);
+            const int ig = c0 + (lane & ((1 << lw) - 1));
             const bool in = ig <= xend;
-            const int igf = fold(ig), xi = xidx[xc];
+            const int igf = fold(ig), xi = xidx0[min(ig, xlast)];
             double T[kAcc];
             if (!kAdj) {
                 // T of 32 columns at a time, a lane each (an FP64 operation costs a warp the same
                 // with half its lanes idle): two blocks of 16 share them
-                const int off = (c0 - wide) & 31;
+                const int off = (c0 - xbeg) & 31;
                 if (off == 0) {
-                    const int xt = min(c0 + lane - lb0, nx - 1);
+                    const double *xt = Xt0 + min(c0 + lane, xlast);
                     const double *c = sC;
                     __syncwarp();
                     for (int ly = 0; ly < L; ly++) {
                         double s = 0.0;
-                        for (int lx = 0; lx < L - ly; lx++) s += c[lx] * Xt[lx * nx + xt];
+                        for (int lx = 0; lx < L - ly; lx++) s += c[lx] * xt[lx * nx];
                         c += L - ly;
                         sT[ly * 33 + lane] = s;
                     }
@@ -385,7 +410,7 @@ k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
                 for (int u = 0; u < kU; u++) {
                     const int r = r0 + u * ng, jg = jgmin + min(r, nrow - 1);
                     jy[u] = jg - lb1;
-                    act[u] = in && r < nrow && igf >= rows[fold(jg) - lb1];
+                    act[u] = in && r < nrow && igf >= rows[fold(jg)];
                     const int yi = yidx[jy[u]];
                     if (act[u] && (xi < 0 || yi < 0)) {
                         atomicOr(status, kStatOutOfWindow);
@@ -415,7 +440,7 @@ k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
                 }
             }
             if (kAdj) {  // the row groups' sums, then cxy over the columns of (up to) two blocks
-                const int off = (c0 - wide) & 31;
+                const int off = (c0 - xbeg) & 31;
 #pragma unroll
                 for (int ly = 0; ly < kAcc; ly++) {
                     if (ly >= L) break;
@@ -426,7 +451,7 @@ k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
                 if (off + (1 << lw) == 32 || left <= 1 << lw) {
                     __syncwarp();
                     const int n = off + min(left, 1 << lw);
-                    const double *xw = Xt + (c0 - off - lb0);
+                    const double *xw = Xt0 + (c0 - off);
 #pragma unroll
                     for (int m = 0; m < kM2; m++) {
                         if (oly[m] < 0) continue;
@@ -462,7 +487,7 @@ k_ortho_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
             }
             __syncthreads();
         }
-        put_moments(it, nc, ps, mom + (extra ? g.mom_ext_off : g.coef_off), [&](int t) { return C[t]; });
+        put_moments(items[blockIdx.x], nc, ps, mom + (extra ? g.mom_ext_off : g.coef_off), [&](int t) { return C[t]; });
     }
 }
 
@@ -483,7 +508,7 @@ k_general_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ 
                const double *__restrict__ coef, double *__restrict__ mom, PartSums ps, GridPtrs grids,
                int *status, int extra) {
     extern __shared__ double sm[];
-    const Fp64Item it = items ? items[blockIdx.x] : Fp64Item{(int)blockIdx.x / uparts, (int)blockIdx.x % uparts, uparts, -1};
+    const Fp64Item it = items ? items[blockIdx.x] : Fp64Item{(int)blockIdx.x / uparts, (int)blockIdx.x % uparts, uparts, 1, -1};
     const PairGeom g = geoms[it.pair];
     const LevelDev &lv = levels[g.level];
     double *__restrict__ grid = grids.p[g.level];
@@ -672,7 +697,7 @@ k_general_ff(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ it
              PartSums ps, GridPtrs grids, int *status) {
     extern __shared__ double smd[];
     constexpr int kM2 = (kNPow * (kNPow + 1) / 2 + 31) / 32, kMC = ((kMaxLp + 1) * (kMaxLp + 2) * (kMaxLp + 3) / 6 + 31) / 32;
-    const Fp64Item it = items ? items[blockIdx.x] : Fp64Item{(int)blockIdx.x / uparts, (int)blockIdx.x % uparts, uparts, -1};
+    const Fp64Item it = items ? items[blockIdx.x] : Fp64Item{(int)blockIdx.x / uparts, (int)blockIdx.x % uparts, uparts, 1, -1};
     const PairGeom &g = geoms[it.pair];
     const LevelDev &lv = levels[g.level];
     double *__restrict__ grid = grids.p[g.level];
@@ -988,9 +1013,10 @@ void fp64_items(TaskSet &ts, int sms, int smem_limit, std::vector<Fp64Item> &ite
     ts.fp64_ortho = ts.fp64_general = 0;
     ts.fp64_smem = ts.fp64_smem_ext = ts.fp64_smem_gen = ts.fp64_smem_gen_ext = 0;
     ts.fp64_slots = 0;
+    ts.fp64_ext_fits = true;
     constexpr int kClasses = 1024;  // sign, exponent and two mantissa bits
     std::vector<unsigned short> cls(ts.h_geom.size());
-    std::vector<int> nparts(ts.h_geom.size());
+    std::vector<int> nparts(ts.h_geom.size()), xparts(ts.h_geom.size(), 1);
     std::vector<int64_t> first(kClasses + 1, 0);
     for (int64_t k = 0; k < (int64_t)ts.h_geom.size(); k++) {
         const PairGeom &g = ts.h_geom[k];
@@ -1000,13 +1026,23 @@ void fp64_items(TaskSet &ts, int sms, int smem_limit, std::vector<Fp64Item> &ite
         int parts = (int)std::min<double>(most, std::ceil((double)g.cost * (g.lp + 1) / target));
         parts = std::max(parts, 1);
         if (g.ortho) {
-            while (parts < planes && smem_ortho_item(g, 2, parts) > smem_limit) parts++;
-            ts.fp64_smem = std::max(ts.fp64_smem, smem_ortho_item(g, 0, parts));
-            ts.fp64_smem_ext = std::max(ts.fp64_smem_ext, smem_ortho_item(g, 2, parts));
+            int &xp = xparts[(size_t)k];
+            int zp = parts;
+            if (fit_ortho_item(g, 2, smem_limit, zp, xp)) {
+                parts = zp;
+            } else {  // thousands of rows: no gradients
+                xp = 1;
+                fit_ortho_item(g, 0, smem_limit, parts, xp);
+                ts.fp64_ext_fits = false;
+            }
+            ts.fp64_smem = std::max(ts.fp64_smem, smem_ortho_item(g, 0, parts, xp) - kOrthoStatic);
+            ts.fp64_smem_ext = std::max(ts.fp64_smem_ext, smem_ortho_item(g, 2, parts, xp) - kOrthoStatic);
+            parts *= xp;
             ts.fp64_ortho += parts;
         } else {
             ts.fp64_smem_gen = std::max(ts.fp64_smem_gen, smem_general_fp64(g));
-            ts.fp64_smem_gen_ext = std::max(ts.fp64_smem_gen_ext, std::min(smem_general_fp64(g, 2), smem_limit));
+            // (fits: the test of smem_general_ff_limit, 16 L + 36 bytes a row, is the narrower one)
+            ts.fp64_smem_gen_ext = std::max(ts.fp64_smem_gen_ext, smem_general_fp64(g, 2));
             ts.fp64_general += parts;
         }
         // class of the items' cost: a factor 2^(1/4) or so, from the float's leading bits
@@ -1025,7 +1061,7 @@ void fp64_items(TaskSet &ts, int sms, int smem_limit, std::vector<Fp64Item> &ite
         int64_t &at = ts.h_geom[k].ortho ? first[cls[k]] : at_gen;
         const bool split = nparts[k] > 1;
         for (int p = 0; p < nparts[k]; p++)
-            items[(size_t)at++] = Fp64Item{(int)k, p, nparts[k], split ? ts.fp64_slots++ : -1};
+            items[(size_t)at++] = Fp64Item{(int)k, p, nparts[k], xparts[k], split ? ts.fp64_slots++ : -1};
     }
 }
 
@@ -1038,13 +1074,13 @@ static cudaError_t launch_fp64_impl(const TaskSet &ts, const GridPtrs &g, bool a
         const unsigned n = (unsigned)ts.fp64_ortho;
         if (adj && extra)
             k_ortho_fp64<true, kNPowB><<<n, 32 * kOrthoWarps, ts.fp64_smem_ext, s>>>(
-                ts.d_geom, ts.d_fp64_items, 1, P.d_levels, ts.d_table, ts.d_coef, mom, ps, g, ts.d_status, extra);
+                ts.d_geom, ts.d_fp64_items, 1, 1, P.d_levels, ts.d_table, ts.d_coef, mom, ps, g, ts.d_status, extra);
         else if (adj)
             k_ortho_fp64<true, kNPow><<<n, 32 * kOrthoWarps, ts.fp64_smem, s>>>(
-                ts.d_geom, ts.d_fp64_items, 1, P.d_levels, ts.d_table, ts.d_coef, mom, ps, g, ts.d_status, 0);
+                ts.d_geom, ts.d_fp64_items, 1, 1, P.d_levels, ts.d_table, ts.d_coef, mom, ps, g, ts.d_status, 0);
         else
             k_ortho_fp64<false, kNPow><<<n, 32 * kOrthoWarps, ts.fp64_smem, s>>>(
-                ts.d_geom, ts.d_fp64_items, 1, P.d_levels, ts.d_table, ts.d_coef, mom, ps, g, ts.d_status, 0);
+                ts.d_geom, ts.d_fp64_items, 1, 1, P.d_levels, ts.d_table, ts.d_coef, mom, ps, g, ts.d_status, 0);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
@@ -1096,9 +1132,9 @@ cudaError_t launch_moments_fp64(const TaskSet &ts, const GridPtrs &g, int extra,
     return launch_fp64_impl(ts, g, true, extra, out, s);
 }
 
-// n pairs without a task set: every pair in uparts parts
+// n pairs without a task set: every pair in zparts xparts parts
 cudaError_t launch_pairs_fp64(const PairGeom *d_geoms, const LevelDev *d_levels, const double *d_tmat,
-                              double *d_coef, int *d_status, int n, int uparts, int tau, int max_A, int max_B,
+                              double *d_coef, int *d_status, int n, int zparts, int xparts, int tau, int max_A, int max_B,
                               int smem_coll, const double *d_pab, double *d_grid, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     k_prep<<<(unsigned)n, 128, smem_prep(max_A, max_B), s>>>(d_geoms, d_levels, d_tmat, tau, d_pab, d_coef);
@@ -1106,8 +1142,9 @@ cudaError_t launch_pairs_fp64(const PairGeom *d_geoms, const LevelDev *d_levels,
     if (e != cudaSuccess) return e;
     GridPtrs g;
     for (int l = 0; l < GPW_MAX_LEVELS; l++) g.p[l] = d_grid;
-    k_ortho_fp64<false, kNPow><<<(unsigned)(n * uparts), 32 * kOrthoWarps, smem_coll, s>>>(
-        d_geoms, nullptr, uparts, d_levels, nullptr, d_coef, nullptr, PartSums{}, g, d_status, 0);
+    const int parts = zparts * xparts;
+    k_ortho_fp64<false, kNPow><<<(unsigned)(n * parts), 32 * kOrthoWarps, smem_coll - kOrthoStatic, s>>>(
+        d_geoms, nullptr, parts, xparts, d_levels, nullptr, d_coef, nullptr, PartSums{}, g, d_status, 0);
     return cudaGetLastError();
 }
 
@@ -1120,16 +1157,18 @@ int fp64_single_parts(const PairGeom &g) {
 // when the pair has one) or general cell: set-up, then the FP64 collocation.
 cudaError_t launch_one_fp64(const PairGeom &g, const PairGeom *d_geom, const LevelDev *d_levels, const double *d_tmat,
                             const int *d_table, double *d_coef, int *d_status, int func, const double *d_pab,
-                            double *d_grid, cudaStream_t s) {
+                            double *d_grid, int smem_limit, cudaStream_t s) {
     k_prep<<<1, 128, smem_prep(g.la_max, g.lb_max), s>>>(d_geom, d_levels, d_tmat, func, d_pab, d_coef);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     GridPtrs gp;
     for (int l = 0; l < GPW_MAX_LEVELS; l++) gp.p[l] = d_grid;
-    const int parts = fp64_single_parts(g);
+    int parts = fp64_single_parts(g), xparts = 1;
+    if (g.ortho) fit_ortho_item(g, 0, smem_limit, parts, xparts);
     if (g.ortho)
-        k_ortho_fp64<false, kNPow><<<(unsigned)parts, 32 * kOrthoWarps, smem_ortho_item(g, 0, parts), s>>>(
-            d_geom, nullptr, parts, d_levels, d_table, d_coef, nullptr, PartSums{}, gp, d_status, 0);
+        k_ortho_fp64<false, kNPow><<<(unsigned)(parts * xparts), 32 * kOrthoWarps,
+                                     smem_ortho_item(g, 0, parts, xparts) - kOrthoStatic, s>>>(
+            d_geom, nullptr, parts * xparts, xparts, d_levels, d_table, d_coef, nullptr, PartSums{}, gp, d_status, 0);
     else
         k_general_fp64<false><<<(unsigned)parts, 256, smem_general_fp64(g), s>>>(d_geom, nullptr, parts, d_levels,
                                                                                d_coef, nullptr, PartSums{}, gp, d_status, 0);

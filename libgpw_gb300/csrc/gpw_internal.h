@@ -51,6 +51,7 @@ struct TaskSet {
     int64_t fp64_ortho = 0, fp64_general = 0;
     int fp64_smem = 0, fp64_smem_ext = 0;          // shared memory (ext: with two extra powers)
     int fp64_smem_gen = 0, fp64_smem_gen_ext = 0;
+    bool fp64_ext_fits = true;
     // divided pairs: per slot the part's moments (ext: to degree lp + 2), and at a pair's
     // first slot the count of its parts that are done.  d_parts and d_ticket lie behind
     // the items, d_parts_ext behind d_mom_ext.
@@ -98,7 +99,8 @@ cudaError_t launch_backtransform(const TaskSet &ts, const double *d_mom, int ext
                                  cudaStream_t s);
 void fp64_items(TaskSet &ts, int sms, int smem_limit, std::vector<Fp64Item> &items);
 int smem_ortho_fp64(const PairGeom &g);
-int smem_ortho_item(const PairGeom &g, int extra, int nparts);
+int smem_ortho_item(const PairGeom &g, int extra, int zparts, int xparts);
+bool fit_ortho_item(const PairGeom &g, int extra, int smem_limit, int &zparts, int &xparts);
 int fp64_single_parts(const PairGeom &g);
 int smem_general_fp64(const PairGeom &g, int extra = 0);
 // moments <V | t^k...> up to degree lp + extra into out (offsets coef_off, or mom_ext_off when extra > 0)
@@ -131,13 +133,13 @@ void set_last_error(const std::string &msg);
 
 // gpw_fp64.cu: set-up + orthorhombic collocate of n pairs from raw device pointers
 cudaError_t launch_pairs_fp64(const PairGeom *d_geoms, const LevelDev *d_levels, const double *d_tmat,
-                              double *d_coef, int *d_status, int n, int uparts, int tau, int max_A, int max_B,
+                              double *d_coef, int *d_status, int n, int zparts, int xparts, int tau, int max_A, int max_B,
                               int smem_coll, const double *d_pab, double *d_grid, cudaStream_t s);
 
 // gpw_fp64.cu: one pair (the drop-in entry): set-up + collocation from raw device pointers
 cudaError_t launch_one_fp64(const PairGeom &g, const PairGeom *d_geom, const LevelDev *d_levels, const double *d_tmat,
                             const int *d_table, double *d_coef, int *d_status, int func, const double *d_pab,
-                            double *d_grid, cudaStream_t s);
+                            double *d_grid, int smem_limit, cudaStream_t s);
 
 // gpw_selftest.cu
 int tc_selftest(int64_t *mismatches, std::string &err);

@@ -112,10 +112,11 @@ extern "C" int gpw_collocate_noalloc(const gpw_grid_desc *level, const gpw_task 
         return GPW_ERR_UNSUPPORTED;
     }
     // few pairs: divide each one so that the launch has about four CTAs per SM
-    int sms = 1, smem_coll = 0;
+    int sms = 1, smem_coll = 0, xparts = 1;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     parts = std::max(1, std::min(parts, 4 * sms / ntasks));
-    for (int i = 0; i < ntasks; i++) smem_coll = std::max(smem_coll, smem_ortho_item(geo[i], 0, parts));
+    for (int i = 0; i < ntasks; i++) fit_ortho_item(geo[i], 0, smem_limit, parts, xparts);
+    for (int i = 0; i < ntasks; i++) smem_coll = std::max(smem_coll, smem_ortho_item(geo[i], 0, parts, xparts));
     unsigned char *base = nullptr;
     st = scratch_address(dev, &base);
     if (st) return st;
@@ -135,7 +136,7 @@ extern "C" int gpw_collocate_noalloc(const gpw_grid_desc *level, const gpw_task 
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(d_geom, geo.data(), sizeof(PairGeom) * ntasks, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
-        e = launch_pairs_fp64(d_geom, d_level, nullptr, d_coef, d_status, ntasks, parts, compute_tau ? 1 : 0, max_A, max_B,
+        e = launch_pairs_fp64(d_geom, d_level, nullptr, d_coef, d_status, ntasks, parts, xparts, compute_tau ? 1 : 0, max_A, max_B,
                               smem_coll, d_pab, d_grid, s);
     // the kernels' error bits, read into a stack variable (a copy, no allocation)
     int flags = 0;
