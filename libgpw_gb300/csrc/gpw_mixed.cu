@@ -66,21 +66,21 @@ constexpr int KP = 16;          // padded contraction length (alpha)
 constexpr int NPAIR_MAX = (kNPow * (kNPow + 1)) / 2;  // (b, a) with b + a <= lp
 constexpr int NCOEF_MAX = ((kMaxLp + 1) * (kMaxLp + 2) * (kMaxLp + 3)) / 6;
 
-constexpr int kMaxImages = 4;  // periodic images of one cube axis over one tile
+// Periodic images of one axis of a cube over one tile.  Every image is an item of its
+// own, so the limit only bounds their number: a cube far larger than its cell has some
+// k^3 images over each tile (500 pairs with cubes of 10 cells a side on a 16^3 grid:
+// 678,000 items, 42 MB).  The binning leaves such a pair out, and tiled calls report it.
+constexpr int kMaxImages = 4;
 
 struct TileDesc {
     int level;
     int t[3];  // tile indices
     int lz;    // log2 TZ (TY = MROWS >> lz)
-    int flags; // kUnitSplit, kUnitOver
+    int flags; // kUnitSplit
 };
 
 // the tile's pairs are divided among several work units: flush with atomics
 constexpr int kUnitSplit = 1;
-// some cube has more than kMaxImages images over a tile axis: reported when the unit
-// runs (once per unit: a check per item, an atomic in the item loop, cost collocate
-// 7 % more instructions, since no level data then stays in registers across it)
-constexpr int kUnitOver = 2;
 
 // tile extents of a tile descriptor
 struct TileShape {
@@ -161,7 +161,8 @@ struct MixedState {
     std::vector<TileDesc> h_tiles;  // every tile of the binned levels, in tile-index order
     struct BinLevel *d_bl = nullptr;  // per level: first tile index, tiles per axis, tile shape
     int *d_blob_len = nullptr;      // per binned pair: chunks of its blob
-    int *d_count = nullptr;         // per tile: items
+    int *d_count = nullptr;         // per tile: items; then whether pairs were left out (kMaxImages)
+    bool over = false;              // the last binning's
     unsigned long long *d_cursor = nullptr;  // per tile: next item slot (fill pass)
     unsigned char *d_units = nullptr;        // d_cursor, d_start and d_tiles, one after the other
     int64_t cap_items = 0, cap_units = 0;    // capacities of d_items / d_iimg, and of d_units in bytes
@@ -446,14 +447,6 @@ __device__ __forceinline__ void fetch_pair(uint4 *dst, ItemImg &ii, const MixedA
         else cp_async16(idst + (t - n), isrc + (t - n));
     }
     cp_async_commit();
-}
-
-// the number of images of one axis: cube offsets o such that the tile [o, o + ext) meets [lb, hi]
-__device__ int axis_image_count(const LevelDev &lv, int d, int tt, int T, const TPair &p) {
-    if (!lv.periodic[d]) return 1;
-    const int N = lv.npts[d], ext = min(T, lv.ngrid[d] - tt * T), base = tt * T - p.cc[d];
-    auto floor_div = [](int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); };
-    return floor_div(p.hi[d] - base, N) - floor_div(p.lb[d] - base - ext, N);
 }
 
 __device__ __forceinline__ void set_image_x(const TPair &p, ImgState &q, int ox, int ext_x) {
@@ -949,7 +942,6 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
         const int tile = cm.tile;
         if (tile >= A.ntiles || cm.abort) break;
         const TileDesc td = A.tiles[tile];
-        if (tid == 0 && (td.flags & kUnitOver)) atomicOr(A.status, kStatTooManyImages);
         const LevelDev &lv = A.levels[td.level];
         const TileShape sh(td.lz);
         const int TY = sh.TY, TZ = sh.TZ;
@@ -1248,7 +1240,6 @@ __global__ void __launch_bounds__(NTHR, 4) k_integrate_tiled(MixedArgs A) {
         const int tile = cm.tile;
         if (tile >= A.ntiles || cm.abort) break;
         const TileDesc td = A.tiles[tile];
-        if (tid == 0 && (td.flags & kUnitOver)) atomicOr(A.status, kStatTooManyImages);
         const LevelDev &lv = A.levels[td.level];
         const TileShape sh(td.lz);
         const int TY = sh.TY, TZ = sh.TZ, z = m >> sh.ly, y = m & (TY - 1);
@@ -1603,26 +1594,23 @@ __global__ void k_scale_moments(double *mom, const uint4 *__restrict__ blob, con
 
 // the image state of every item from its offsets (left in im.o by the binning),
 // once per task set; one block per work unit
-__global__ void k_item_images(TileDesc *tiles, const int64_t *__restrict__ start,
+__global__ void k_item_images(const TileDesc *__restrict__ tiles, const int64_t *__restrict__ start,
                               const uint64_t *__restrict__ items, const uint4 *__restrict__ blob,
                               const LevelDev *__restrict__ levels, ItemImg *out, int ntiles) {
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const TileDesc td = tiles[tile];
-        const LevelDev &lv = levels[td.level];
-        const TileShape sh(td.lz);
-        const int ext_x = min(TX, lv.ngrid[0] - td.t[0] * TX);
+        const int ext_x = min(TX, levels[td.level].ngrid[0] - td.t[0] * TX);
         for (int64_t it = start[2 * tile] + threadIdx.x; it < start[2 * tile + 1]; it += blockDim.x) {
             const TPair &p = *reinterpret_cast<const TPair *>(blob + (items[it] >> 16));
             ItemImg r = out[it];
             set_image_x(p, r.im, r.im.o[0], ext_x);
             out[it] = r;
-            if (axis_image_count(lv, 0, td.t[0], TX, p) > kMaxImages ||
-                axis_image_count(lv, 1, td.t[1], sh.TY, p) > kMaxImages ||
-                axis_image_count(lv, 2, td.t[2], sh.TZ, p) > kMaxImages)
-                atomicOr(&tiles[tile].flags, kUnitOver);
         }
     }
 }
+
+// tiled calls on a task set with pairs that the binning left out
+__global__ void k_report(int *status, int bits) { atomicOr(status, bits); }
 
 // ---------------------------------------------------------------------------
 // Binning on the device: the (tile, pair) items of every binned pair.
@@ -1722,7 +1710,8 @@ __device__ __forceinline__ int run_fold(int a, int b) { return (a <= 1 && b >= 0
 // the image in the tile can be inside its sphere (with a margin): orthorhombic, the
 // folded distance of the runs' nearest offsets <= radius; general cell, the least
 // |r - rp|^2 over the lattice-index box of the runs (box_min_q) <= radius^2, tested
-// per axis, then per item.  Explicit cube lists are not culled.
+// per axis, then per item.  Explicit cube lists are not culled.  A pair of which some tile
+// sees more than kMaxImages images along an axis gets no items: *over is set.
 // kGen: the general-cell pairs [k0, k1) (the culling's box minimum needs registers
 // and stack that would slow the orthorhombic launch, kGen = false).
 // 2^lper threads share a pair, each on its own (z, y) runs: the largest cubes have
@@ -1732,7 +1721,7 @@ template <bool kGen>
 __global__ void k_bin_pairs(const PairGeom *__restrict__ geoms, int64_t k0, int64_t k1, int lper,
                             const LevelDev *__restrict__ levels, const BinLevel *__restrict__ bl,
                             const int64_t *__restrict__ off16, const int *__restrict__ len16, int pass, int *count,
-                            unsigned long long *cursor, uint64_t *items, ItemImg *iimg) {
+                            int *over, unsigned long long *cursor, uint64_t *items, ItemImg *iimg) {
     const int mask = (1 << lper) - 1;
     for (int64_t k = k0 + ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> lper); k < k1;
          k += ((int64_t)gridDim.x * blockDim.x) >> lper) {
@@ -1749,6 +1738,10 @@ __global__ void k_bin_pairs(const PairGeom *__restrict__ geoms, int64_t k0, int6
         ax.init(lv, 0, g.cc[0], lb[0], hi[0], TX, B.nt[0]);
         ay.init(lv, 1, g.cc[1], lb[1], hi[1], sh.TY, B.nt[1]);
         az.init(lv, 2, g.cc[2], lb[2], hi[2], sh.TZ, B.nt[2]);
+        if (ax.n > kMaxImages * B.nt[0] || ay.n > kMaxImages * B.nt[1] || az.n > kMaxImages * B.nt[2]) {
+            *over = 1;
+            continue;
+        }
         int tx, ty, tz, x0, x1, y0, y1, z0, z1, ox, oy, oz;
         const double r2 = g.radius * g.radius * (1.0 + 1e-9) + 1e-12;
         const double hx = lv.dh[0][0], hy = lv.dh[1][1], hz = lv.dh[2][2];
@@ -1812,7 +1805,7 @@ __global__ void k_bin_pairs(const PairGeom *__restrict__ geoms, int64_t k0, int6
 }
 
 // both kinds of pairs of a task set (orthorhombic first in the sorted order)
-static cudaError_t bin_pairs(const TaskSet &ts, const MixedState &M, int pass, int *count,
+static cudaError_t bin_pairs(const TaskSet &ts, const MixedState &M, int pass, int *count, int *over,
                              unsigned long long *cursor, uint64_t *items, ItemImg *iimg) {
     const Plan &P = *ts.plan;
     auto blocks = [](int64_t threads) {
@@ -1827,13 +1820,13 @@ static cudaError_t bin_pairs(const TaskSet &ts, const MixedState &M, int pass, i
     if (M.northo > 0) {
         const int l = share(M.northo);
         k_bin_pairs<false><<<blocks((int64_t)M.northo << l), 128>>>(ts.d_geom, 0, M.northo, l, P.d_levels, M.d_bl,
-                                                                  M.d_blob_off, M.d_blob_len, pass, count, cursor,
+                                                                  M.d_blob_off, M.d_blob_len, pass, count, over, cursor,
                                                                   items, iimg);
     }
     if (M.nbin > M.northo) {
         const int l = share(M.nbin - M.northo);
         k_bin_pairs<true><<<blocks((M.nbin - M.northo) << l), 128>>>(ts.d_geom, M.northo, M.nbin, l, P.d_levels,
-                                                                   M.d_bl, M.d_blob_off, M.d_blob_len, pass, count,
+                                                                   M.d_bl, M.d_blob_off, M.d_blob_len, pass, count, over,
                                                                    cursor, items, iimg);
     }
     return cudaGetLastError();
@@ -1952,8 +1945,8 @@ int mixed_build(TaskSet &ts, std::string &err) {
     // ... when every general level has a tile shape (not kUntiled) ...
     for (int l = 0; l < P.nlevels; l++)
         if (!P.lv[l].ortho && ts.tile_lz[l] == kUntiled) gen_ok = false;
-    // ... and when no general box spans more periodic images of one tile axis
-    // than the kernels hold (kMaxImages): count <= (extent + T - 1) / N + 1
+    // ... and when no general box has more than kMaxImages periodic images over one tile
+    // axis: count <= (extent + T - 1) / N + 1
     for (int64_t k = northo; k < ts.ntasks && gen_ok; k++) {
         const PairGeom &g = ts.h_geom[k];
         const LevelDev &lv = P.lv[g.level];
@@ -2023,7 +2016,7 @@ int mixed_build(TaskSet &ts, std::string &err) {
     alloc((void **)&M->d_blob_off, sizeof(int64_t) * off16.size());
     alloc((void **)&M->d_blob_len, sizeof(int) * len16.size());
     alloc((void **)&M->d_bl, sizeof(BinLevel) * blv.size());
-    alloc((void **)&M->d_count, sizeof(int) * (size_t)std::max(ntiles, 1));
+    alloc((void **)&M->d_count, sizeof(int) * ((size_t)ntiles + 1));
     alloc((void **)&M->d_queue, sizeof(int) * 4);
     alloc((void **)&M->d_glv, sizeof(GenLevel) * glv.size());
     if (e == cudaSuccess) e = cudaMemset(M->d_blob, 0, sizeof(uint4) * (size_t)std::max<int64_t>(nchunks, 1));
@@ -2100,11 +2093,13 @@ int mixed_rebin(TaskSet &ts, std::string &err) {
         k_make_records<<<nblk, 128>>>(ts.d_geom, nbin, P.d_levels, M->d_blob_off, M->d_blob);
         if ((e = cudaGetLastError()) != cudaSuccess) return fail(e);
     }
-    if ((e = cudaMemset(M->d_count, 0, sizeof(int) * (size_t)std::max(ntiles, 1))) != cudaSuccess) return fail(e);
-    if (nbin > 0 && (e = bin_pairs(ts, *M, 0, M->d_count, nullptr, nullptr, nullptr)) != cudaSuccess) return fail(e);
-    std::vector<int> count((size_t)std::max(ntiles, 1), 0);
+    if ((e = cudaMemset(M->d_count, 0, sizeof(int) * ((size_t)ntiles + 1))) != cudaSuccess) return fail(e);
+    int *over = M->d_count + ntiles;
+    if (nbin > 0 && (e = bin_pairs(ts, *M, 0, M->d_count, over, nullptr, nullptr, nullptr)) != cudaSuccess) return fail(e);
+    std::vector<int> count((size_t)ntiles + 1, 0);
     if ((e = cudaMemcpy(count.data(), M->d_count, sizeof(int) * count.size(), cudaMemcpyDeviceToHost)) != cudaSuccess)
         return fail(e);
+    M->over = count[(size_t)ntiles] != 0;
     // items grouped by tile
     std::vector<int64_t> start(ntiles + 1, 0);
     for (int i = 0; i < ntiles; i++) start[i + 1] = start[i] + count[i];
@@ -2203,10 +2198,8 @@ int mixed_rebin(TaskSet &ts, std::string &err) {
     M->d_start = reinterpret_cast<int64_t *>(M->d_units) + nslot;
     M->d_tiles = reinterpret_cast<TileDesc *>(M->d_start + 2 * nun);
     if ((e = cudaMemcpy(M->d_units, image.data(), image.size(), cudaMemcpyHostToDevice)) != cudaSuccess) return fail(e);
-    if (nbin > 0 && (e = bin_pairs(ts, *M, 1, nullptr, M->d_cursor, M->d_items, M->d_iimg)) != cudaSuccess) return fail(e);
+    if (nbin > 0 && (e = bin_pairs(ts, *M, 1, nullptr, over, M->d_cursor, M->d_items, M->d_iimg)) != cudaSuccess) return fail(e);
     if (nitems) {
-        // (image overflows are reported by the tiled kernels when they run: a plain
-        // FP64 call on this task set must not see them)
         k_item_images<<<std::max(1, std::min(nunits, 8192)), 128>>>(M->d_tiles, M->d_start, M->d_items, M->d_blob,
                                                                     P.d_levels, M->d_iimg, nunits);
         if ((e = cudaGetLastError()) != cudaSuccess) return fail(e);
@@ -2266,10 +2259,18 @@ static cudaError_t general_ff(const TaskSet &ts, const GridPtrs &g, bool adj, cu
     return launch_general_ff(ts, g, adj, s);
 }
 
+// a tiled call that lacks pairs: an error status (a plain FP64 call must not see it)
+static cudaError_t report_over(const TaskSet &ts, cudaStream_t s) {
+    ts.n_kernels++;
+    k_report<<<1, 1, 0, s>>>(ts.d_status, kStatTooManyImages);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_collocate_mixed(const TaskSet &ts, const GridPtrs &g, cudaStream_t s) {
     if (!ts.mixed) return cudaErrorNotSupported;
     const MixedState &M = *ts.mixed;
     cudaError_t e = cudaSuccess;
+    if (M.over && (e = report_over(ts, s)) != cudaSuccess) return e;
     if (M.nbin > 0 && M.ntiles > 0) {
         ts.n_kernels++;
         k_coef_to_blob<<<(unsigned)std::min<int64_t>((M.nbin + 7) / 8, 8192), 256, 0, s>>>(ts.d_coef, M.d_blob,
@@ -2297,7 +2298,8 @@ cudaError_t launch_integrate_mixed(const TaskSet &ts, const GridPtrs &g, cudaStr
     if (!ts.mixed) return cudaErrorNotSupported;
     const MixedState &M = *ts.mixed;
     cudaError_t e = cudaSuccess;
-    if (M.nbin > 0 && M.ntiles > 0) {
+    if (M.over && (e = report_over(ts, s)) != cudaSuccess) return e;
+    if (M.nbin > 0) {
         if ((e = cudaMemsetAsync(ts.d_mom, 0, sizeof(double) * ts.coef_len, s)) != cudaSuccess) return e;
         const int nto = M.ntiles_ortho, ntg = M.ntiles - M.ntiles_ortho;
         if (nto > 0) {

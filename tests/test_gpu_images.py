@@ -69,3 +69,22 @@ def test_integrate_degrees(l, tz, ortho, oracle_lib):
     V = wl.potentials(seed=3)
     hab = oracle_lib.batch(wl, V=V)
     assert np.abs(run_integrate(wl, V, "mixed", ts=ts, plan=plan) - hab).max() <= TOL * np.abs(hab).max()
+
+
+def test_too_many_images_bounded(oracle_lib):
+    """Cubes of about ten cells a side beside ordinary ones: no items for them (they would have
+    hundreds per tile), the same status from tiled calls, and plain FP64 calls are not affected."""
+    wl = T.synthetic("some", 40, 0, (0.05, 0.06), 3.0, [(16, 16, 16)], 5)
+    wl.tasks["radius"][::2] = 1.4
+    plan = capi.Plan(wl.levels)
+    ts = capi.TaskSet.from_workload(plan, wl)
+    items = ts.bins()[0]
+    assert 20 <= items <= 20 * 2 * 8  # 20 pairs, 2 tiles, at most two images of an axis
+    V = wl.potentials(seed=3)
+    for run in (lambda: run_collocate(wl, "mixed", ts=ts, plan=plan), lambda: run_integrate(wl, V, "mixed", ts=ts, plan=plan)):
+        with pytest.raises(capi.GpwError) as e:
+            run()
+        assert e.value.status == 4  # GPW_ERR_UNSUPPORTED
+    want, hab = oracle_lib.batch(wl)[0], oracle_lib.batch(wl, V=V)
+    assert np.linalg.norm(run_collocate(wl, "fp64", ts=ts, plan=plan)[0] - want) <= 1e-12 * np.linalg.norm(want)
+    assert np.abs(run_integrate(wl, V, "fp64", ts=ts, plan=plan) - hab).max() <= 1e-12 * np.abs(hab).max()
