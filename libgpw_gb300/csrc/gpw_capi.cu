@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <numeric>
 #include <string>
@@ -494,6 +495,7 @@ int gpw_taskset_create(gpw_plan *plan, const gpw_task *tasks, int64_t ntasks, in
     std::vector<PairGeom> geo((size_t)ntasks);
     std::vector<int> table;
     int64_t extent = 0;
+    double work = 0.0;  // points x powers
     for (int64_t i = 0; i < ntasks; i++) {
         int st = make_geom(tasks[i], (int)i, *plan, func, sphere_table, sphere_table_len,
                            geo[i], table);
@@ -507,6 +509,7 @@ int gpw_taskset_create(gpw_plan *plan, const gpw_task *tasks, int64_t ntasks, in
             return fail(GPW_ERR_INVALID_ARG, buf);
         }
         extent = std::max(extent, hi + 1);
+        work += (double)geo[i].cost * (geo[i].lp + 1);
     }
     // sort: kind (ortho first), then the largest cubes first
     std::vector<int> order((size_t)ntasks);
@@ -523,10 +526,21 @@ int gpw_taskset_create(gpw_plan *plan, const gpw_task *tasks, int64_t ntasks, in
     T->ntasks = ntasks;
     T->pab_extent = extent;
     T->h_geom.resize((size_t)ntasks);
+    int smem_limit = 0, sms = 1;  // what one CTA holds
+    cudaDeviceGetAttribute(&smem_limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, plan->device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, plan->device);
+    Fp64Planner planner(*T, work, sms, smem_limit);
     int64_t coef = 0;
     int64_t mom_ext = 0;
+    // the sorted order jumps about in geo: fetched ahead (1M pairs, the planner's work
+    // included: 246 -> 96 ms)
+    constexpr int64_t kAhead = 12;
     for (int64_t k = 0; k < ntasks; k++) {
-        PairGeom g = geo[order[k]];
+        if (k + kAhead < ntasks)
+            for (size_t b = 0; b < sizeof(PairGeom); b += 64)
+                __builtin_prefetch(reinterpret_cast<const char *>(&geo[order[k + kAhead]]) + b);
+        PairGeom &g = T->h_geom[k];
+        g = geo[order[k]];
         g.coef_off = coef;
         coef += ncoef(g.lp);
         g.mom_ext_off = mom_ext;
@@ -535,34 +549,21 @@ int gpw_taskset_create(gpw_plan *plan, const gpw_task *tasks, int64_t ntasks, in
         T->max_lp = std::max(T->max_lp, g.lp);
         T->max_A = std::max(T->max_A, g.la_max);
         T->max_B = std::max(T->max_B, g.lb_max);
-        T->h_geom[k] = g;
-    }
-    T->coef_len = coef;
-    T->mom_ext_len = mom_ext;
-    // what one CTA holds
-    int smem_limit = 0, sms = 1;
-    cudaDeviceGetAttribute(&smem_limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, plan->device);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, plan->device);
-    for (const PairGeom &g : T->h_geom)
-        if ((g.ortho ? smem_ortho_fp64(g) : smem_general_fp64(g)) > smem_limit) {
+        int need = g.ortho ? smem_ortho_fp64(g) : smem_general_fp64(g);
+        if (!g.ortho) {  // sorted after the orthorhombic pairs; the float-float kernel
+            if (T->gen_count == 0) T->gen_first = (int)k;
+            T->gen_count++;
+            T->gen_smem = std::max(T->gen_smem, smem_general_ff(g));
+            need = std::max({need, T->gen_smem, smem_general_ff_limit(g)});
+        }
+        if (need > smem_limit) {
             delete T;
             return fail(GPW_ERR_UNSUPPORTED, "gpw_taskset_create: a cube is too large for one CTA");
         }
-    std::vector<Fp64Item> items;
-    fp64_items(*T, sms, smem_limit, items);
-    // general-cell pairs (sorted after the orthorhombic ones) for the float-float kernel
-    int gen_limit = 0;
-    for (int64_t m = 0; m < ntasks; m++) {
-        if (T->h_geom[m].ortho) continue;
-        if (T->gen_count == 0) T->gen_first = (int)m;
-        T->gen_count++;
-        T->gen_smem = std::max(T->gen_smem, smem_general_ff(T->h_geom[m]));
-        gen_limit = std::max(gen_limit, smem_general_ff_limit(T->h_geom[m]));
+        planner.add(g);
     }
-    if (std::max(T->gen_smem, gen_limit) > smem_limit) {
-        delete T;
-        return fail(GPW_ERR_UNSUPPORTED, "gpw_taskset_create: a general-cell cube is too large for one CTA");
-    }
+    T->coef_len = coef;
+    T->mom_ext_len = mom_ext;
     if (smem_prep(T->max_A, T->max_B) > smem_limit) {
         delete T;
         return fail(GPW_ERR_UNSUPPORTED, "gpw_taskset_create: angular momenta too high for the set-up kernel");
@@ -577,14 +578,18 @@ int gpw_taskset_create(gpw_plan *plan, const gpw_task *tasks, int64_t ntasks, in
     alloc((void **)&T->d_mom, sizeof(double) * (size_t)coef);
     alloc((void **)&T->d_status, sizeof(int));
     // the FP64 items, and the divided pairs' slots and tickets, in one block
-    const size_t slots = (size_t)T->fp64_slots, items_len = (sizeof(Fp64Item) * items.size() + 15) / 16 * 16,
+    const size_t nitems = (size_t)(T->fp64_ortho + T->fp64_general), slots = (size_t)T->fp64_slots,
+                 items_len = (sizeof(Fp64Item) * nitems + 15) / 16 * 16,
                  parts_len = sizeof(double) * slots * ncoef(T->max_lp);
     alloc((void **)&T->d_fp64_items, items_len + parts_len + sizeof(int) * slots);
     T->d_parts = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(T->d_fp64_items) + items_len);
     T->d_ticket = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(T->d_parts) + parts_len);
     if (e == cudaSuccess && slots > 0) e = cudaMemset(T->d_ticket, 0, sizeof(int) * slots);
-    if (e == cudaSuccess && !items.empty())
-        e = cudaMemcpy(T->d_fp64_items, items.data(), sizeof(Fp64Item) * items.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && nitems > 0) {
+        std::unique_ptr<Fp64Item[]> items(new Fp64Item[nitems]);
+        planner.write(items.get());
+        e = cudaMemcpy(T->d_fp64_items, items.get(), sizeof(Fp64Item) * nitems, cudaMemcpyHostToDevice);
+    }
     if (e == cudaSuccess && ntasks > 0)
         e = cudaMemcpy(T->d_geom, T->h_geom.data(), sizeof(PairGeom) * (size_t)ntasks, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !table.empty())

@@ -998,70 +998,68 @@ cudaError_t launch_prep(const TaskSet &ts, const double *d_pab, cudaStream_t s) 
 // more than a given part of an even per-CTA share of all cube points, down to one plane
 // per warp.  The number of planes is not needed exactly: a geometry update may move a
 // general box's extent by one.
-void fp64_items(TaskSet &ts, int sms, int smem_limit, std::vector<Fp64Item> &items) {
-    // Parts of at most 1/kWaves of a CTA's share.  Orthorhombic: a part costs a CTA's tables and
-    // (integrate) the sum over its warps, and the largest parts run first (integrate and
-    // collocate of 1000 pairs, 64^3: 443 and 418 us; 8 waves in the pairs' order 450 and 423;
-    // two more powers 569 and 543 against 571 and 549; 16 waves 462 and 421).  General cells,
-    // whose CTAs set little up: 4.04 and 3.28 ms for 1500 pairs on 128^3, mixed, with 16 waves in
-    // the pairs' order, 4.15 and 3.32 sorted, 4.15 and 3.49 with 8 waves.
-    constexpr int kWavesOrtho = 7, kWavesGeneral = 16, kCtas = 4;
-    constexpr double kLeast = 16384.0;  // points x powers: below this a part is mostly tables and set-up
-    double total = 0.0;
-    for (const PairGeom &g : ts.h_geom) total += (double)g.cost * (g.lp + 1);
-    const double share = total / ((double)sms * kCtas);
-    ts.fp64_ortho = ts.fp64_general = 0;
-    ts.fp64_smem = ts.fp64_smem_ext = ts.fp64_smem_gen = ts.fp64_smem_gen_ext = 0;
-    ts.fp64_slots = 0;
-    ts.fp64_ext_fits = true;
-    constexpr int kClasses = 1024;  // sign, exponent and two mantissa bits
-    std::vector<unsigned short> cls(ts.h_geom.size());
-    std::vector<int> nparts(ts.h_geom.size()), xparts(ts.h_geom.size(), 1);
-    std::vector<int64_t> first(kClasses + 1, 0);
-    for (int64_t k = 0; k < (int64_t)ts.h_geom.size(); k++) {
-        const PairGeom &g = ts.h_geom[k];
-        const int planes = g.ortho ? 2 - 2 * g.kgmin : g.ext0[2];
-        const int most = std::max(1, (planes + kOrthoWarps - 1) / kOrthoWarps);
-        const double target = std::max(kLeast, share / (g.ortho ? kWavesOrtho : kWavesGeneral));
-        int parts = (int)std::min<double>(most, std::ceil((double)g.cost * (g.lp + 1) / target));
-        parts = std::max(parts, 1);
-        if (g.ortho) {
-            int &xp = xparts[(size_t)k];
-            int zp = parts;
-            if (fit_ortho_item(g, 2, smem_limit, zp, xp)) {
-                parts = zp;
-            } else {  // thousands of rows: no gradients
-                xp = 1;
-                fit_ortho_item(g, 0, smem_limit, parts, xp);
-                ts.fp64_ext_fits = false;
-            }
-            ts.fp64_smem = std::max(ts.fp64_smem, smem_ortho_item(g, 0, parts, xp) - kOrthoStatic);
-            ts.fp64_smem_ext = std::max(ts.fp64_smem_ext, smem_ortho_item(g, 2, parts, xp) - kOrthoStatic);
-            parts *= xp;
-            ts.fp64_ortho += parts;
-        } else {
-            ts.fp64_smem_gen = std::max(ts.fp64_smem_gen, smem_general_fp64(g));
-            // (fits: the test of smem_general_ff_limit, 16 L + 36 bytes a row, is the narrower one)
-            ts.fp64_smem_gen_ext = std::max(ts.fp64_smem_gen_ext, smem_general_fp64(g, 2));
-            ts.fp64_general += parts;
+//
+// Parts of at most 1/kWaves of a CTA's share.  Orthorhombic: a part costs a CTA's tables and
+// (integrate) the sum over its warps, and the largest parts run first (integrate and
+// collocate of 1000 pairs, 64^3: 443 and 418 us; 8 waves in the pairs' order 450 and 423;
+// two more powers 569 and 543 against 571 and 549; 16 waves 462 and 421).  General cells,
+// whose CTAs set little up: 4.04 and 3.28 ms for 1500 pairs on 128^3, mixed, with 16 waves in
+// the pairs' order, 4.15 and 3.32 sorted, 4.15 and 3.49 with 8 waves.
+constexpr int kWavesOrtho = 7, kWavesGeneral = 16, kCtas = 4;
+constexpr double kLeast = 16384.0;  // points x powers: below this a part is mostly tables and set-up
+
+Fp64Planner::Fp64Planner(TaskSet &t, double total, int sms, int smem_limit_)
+    : ts(t), smem_limit(smem_limit_),
+      target{std::max(kLeast, total / ((double)sms * kCtas) / kWavesGeneral),
+             std::max(kLeast, total / ((double)sms * kCtas) / kWavesOrtho)},
+      first(kClasses + 1, 0) {
+    pairs.reserve((size_t)ts.ntasks);
+}
+
+void Fp64Planner::add(const PairGeom &g) {
+    const int planes = g.ortho ? 2 - 2 * g.kgmin : g.ext0[2];
+    const int most = std::max(1, (planes + kOrthoWarps - 1) / kOrthoWarps);
+    const double cost = (double)g.cost * (g.lp + 1);
+    int parts = std::max(1, (int)std::min<double>(most, std::ceil(cost / target[g.ortho ? 1 : 0])));
+    int xp = 1;
+    if (g.ortho) {
+        int zp = parts;
+        if (fit_ortho_item(g, 2, smem_limit, zp, xp)) {
+            parts = zp;
+        } else {  // thousands of rows: no gradients
+            xp = 1;
+            fit_ortho_item(g, 0, smem_limit, parts, xp);
+            ts.fp64_ext_fits = false;
         }
-        // class of the items' cost: a factor 2^(1/4) or so, from the float's leading bits
-        const float c = (float)((double)g.cost * (g.lp + 1) / parts);
-        unsigned bits;
-        memcpy(&bits, &c, sizeof bits);
-        cls[(size_t)k] = (unsigned short)(kClasses - 1 - std::min(bits >> 21, (unsigned)kClasses - 1));
-        nparts[(size_t)k] = parts;
-        if (g.ortho) first[cls[(size_t)k] + 1] += parts;
+        ts.fp64_smem = std::max(ts.fp64_smem, smem_ortho_item(g, 0, parts, xp) - kOrthoStatic);
+        ts.fp64_smem_ext = std::max(ts.fp64_smem_ext, smem_ortho_item(g, 2, parts, xp) - kOrthoStatic);
+        parts *= xp;
+        ts.fp64_ortho += parts;
+    } else {
+        ts.fp64_smem_gen = std::max(ts.fp64_smem_gen, smem_general_fp64(g));
+        // (fits: the test of smem_general_ff_limit, 16 L + 36 bytes a row, is the narrower one)
+        ts.fp64_smem_gen_ext = std::max(ts.fp64_smem_gen_ext, smem_general_fp64(g, 2));
+        ts.fp64_general += parts;
     }
-    // orthorhombic items by falling class (a counting sort), then the general cells' in order
+    if (parts > 1) ts.fp64_slots += parts;
+    // class of the items' cost: a factor 2^(1/4) or so, from the float's leading bits
+    const float c = (float)(cost / parts);
+    unsigned bits;
+    memcpy(&bits, &c, sizeof bits);
+    const int cls = kClasses - 1 - (int)std::min(bits >> 21, (unsigned)kClasses - 1);
+    if (g.ortho) first[cls + 1] += parts;
+    pairs.push_back(Pair{parts, xp, g.ortho ? cls : -1});
+}
+
+void Fp64Planner::write(Fp64Item *items) {
     for (int c = 0; c < kClasses; c++) first[c + 1] += first[c];
-    items.resize((size_t)(ts.fp64_ortho + ts.fp64_general));
     int64_t at_gen = ts.fp64_ortho;
-    for (size_t k = 0; k < ts.h_geom.size(); k++) {
-        int64_t &at = ts.h_geom[k].ortho ? first[cls[k]] : at_gen;
-        const bool split = nparts[k] > 1;
-        for (int p = 0; p < nparts[k]; p++)
-            items[(size_t)at++] = Fp64Item{(int)k, p, nparts[k], xparts[k], split ? ts.fp64_slots++ : -1};
+    int slot = 0;
+    for (size_t k = 0; k < pairs.size(); k++) {
+        const Pair &p = pairs[k];
+        int64_t &at = p.cls >= 0 ? first[p.cls] : at_gen;
+        for (int i = 0; i < p.parts; i++)
+            items[at++] = Fp64Item{(int)k, i, p.parts, p.xparts, p.parts > 1 ? slot++ : -1};
     }
 }
 
