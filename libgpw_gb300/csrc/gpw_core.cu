@@ -141,9 +141,10 @@ k_integrate_core(int nz, int ny, int nx, int L, const double *__restrict__ pol, 
 
 cudaError_t launch_collocate_core(const int length[3], int L, const double *co, const double *pol, int ld,
                                   double *out, cudaStream_t s) {
+    // The sizes accepted are those of the form that kept a plane's rows in shared memory.
+    const int64_t rows = 8 * ((int64_t)L * L + (int64_t)length[1] * L);
+    if (rows < 0 || rows > 227 * 1024) return cudaErrorInvalidValue;
     if (length[0] > 0 && length[1] <= 0) return cudaSuccess;  // no points
-    // the largest ny L accepted is that of the form that kept a plane's rows in shared memory
-    if (8 * ((int64_t)L * L + (int64_t)length[1] * L) > 227 * 1024) return cudaErrorInvalidValue;
     const dim3 grid((unsigned)length[0], (unsigned)((length[1] + kCoreRows - 1) / kCoreRows));
     k_collocate_core<<<grid, 32 * kCoreRows, 0, s>>>(length[0], length[1], length[2], L, co, pol, ld, out);
     return cudaGetLastError();

@@ -34,3 +34,17 @@ def test_core_shapes(shape):
     assert np.abs(out.cpu().numpy() - want).max() <= 4 * eps * L**3 * (3 * L + 3)
     want = np.einsum("zyx,gz,by,ax->gba", V, Z, Y, X, optimize=True)
     assert np.abs(back.cpu().numpy() - want).max() <= 4 * eps * nz * ny * nx * 8
+
+
+@pytest.mark.parametrize("nz,ny,L,ok", [(3, 0, 2, True), (3, -1, 2, True), (3, -5, 1, False), (0, 4, 2, False)])
+def test_core_no_points(nz, ny, L, ok):
+    """Calls without points: nothing is written; a negative need of shared memory (8 L (L + ny)
+    bytes for a plane's rows) and an empty grid of planes are errors."""
+    torch, dev = torch_dev()
+    pol, co = torch.ones(3 * L * 8, dtype=torch.float64, device=dev), torch.ones(L**3, dtype=torch.float64, device=dev)
+    out = torch.full((64,), 9.0, dtype=torch.float64, device=dev)
+    s = torch.cuda.current_stream().cuda_stream
+    st = capi.lib().gpw_collocate_core((C.c_int * 3)(nz, ny, 3), L, co.data_ptr(), pol.data_ptr(), 8, out.data_ptr(), s)
+    assert (st == 0) == ok
+    torch.cuda.synchronize()
+    assert bool((out == 9.0).all())
