@@ -113,6 +113,15 @@ struct GenLevel {
     GeneralRowFF rowff;
     ff c01, c02, c12;   // cos(v0, v1), cos(v0, v2), cos(v1, v2)
 };
+// The sphere of a general-cell pair in the tiled path.  On tiled levels sum t_d^2 <=
+// 2.5 r^2 (mixed_build), so the cross factor at a point is at most exp(1.5 zetp r^2): it
+// must not leave float's range, nor dwarf the row's other points, whose slices share one
+// scale.  Points beyond zetp r^2 = 46, below 1e-20 of the Gaussian's peak, are left out (radii
+// from eps = 1e-10 give 23).
+constexpr double kMaxExponent = 46.0;
+__device__ __forceinline__ double tiled_radius(const PairGeom &g) {
+    return fmin(g.radius, sqrt(kMaxExponent / g.zetp));
+}
 // A pair's blob: the record padded to kHdr16 16-byte chunks, then its
 // coefficients as float-float (written by every collocate call), padded to 16 bytes.
 constexpr int kHdr16 = (int)((sizeof(TPair) + 15) / 16);
@@ -636,11 +645,11 @@ __device__ __forceinline__ void slice_row16(const ff2 *vin, float sc, int kw, in
 
 // General cell: the cross factor along row (z, y) of the current image, E(x) =
 // exp(alpha + beta t0(x)) with beta = -2 zetp (c01 t1 + c02 t2), alpha = -2 zetp
-// c12 t1 t2: returns E(x0), E(x0 + 1) as a pair and the factor q^2, q = E(x + 1) / E(x),
-// from one pair of x to the next (twice).  x0 is the even x at or before the row's first
-// cube point: at most one step outside the cube.
+// c12 t1 t2: returns E of the pair of x (even, odd) that holds the row's first cube point
+// x0, and what next_cross needs.  Outside the cube's points E may leave float's range, so
+// no value comes from outside: where x0 is the odd one the even one is not used.
 __device__ __forceinline__ void cross_factor_row(const GenLevel &G, const TPair &P, const ImgState &Q,
-                                                 const float2 *exptab, int z, int y, int x0, ff2 &e, ff2n &q2) {
+                                                 const float2 *exptab, int z, int y, int x0, ff2 &e, ff2n &qn) {
     const ff t1 = ff_add(ff_mul_f(P.h[1], (float)(Q.o[1] + y)), ff{-P.off[1].hi, -P.off[1].lo});
     const ff t2 = ff_add(ff_mul_f(P.h[2], (float)(Q.o[2] + z)), ff{-P.off[2].hi, -P.off[2].lo});
     const ff t0 = ff_add(ff_mul_f(P.h[0], (float)(Q.o[0] + x0)), ff{-P.off[0].hi, -P.off[0].lo});
@@ -649,9 +658,11 @@ __device__ __forceinline__ void cross_factor_row(const GenLevel &G, const TPair 
     const ff alpha = ff_mul(m2z, ff_mul(G.c12, ff_mul(t1, t2)));
     const ff2 eq = ff2_exp(ff2_pair(ff_add(alpha, ff_mul(beta, t0)), ff_mul(beta, P.h[0])), exptab);
     const ff e0 = {eq.hi.x, eq.lo.x}, q = {eq.hi.y, eq.lo.y};
-    e = ff2_pair(e0, ff_mul(e0, q));
-    q2 = ff2n_dup(ff_mul(q, q));
+    e = ff2_pair(e0, x0 & 1 ? e0 : ff_mul(e0, q));
+    qn = ff2n_of(ff2_pair(q, ff_mul(q, q)));
 }
+// the next pair's, from the odd one: E q, E q^2
+__device__ __forceinline__ ff2 next_cross(ff2 e, ff2n q) { return ff2_mul(ff2_dup(ff{e.hi.y, e.lo.y}), q); }
 
 // General cell, integrate: the A operand row r = the slices of V(x) E(x) over the
 // row's cube points [x0, x1] (zero elsewhere), with the row's own exponent (returned).
@@ -662,16 +673,17 @@ __device__ __forceinline__ int general_a_row(Smem &sm, const uint4 *vslot, const
     if (x0 > x1) return kZeroExp;  // the row's products are not read
     const float4 *const vrow = reinterpret_cast<const float4 *>(vslot) + r;
     ff2 e0;
-    ff2n q2;
+    ff2n q;
     const int xs = x0 & ~1;  // two x per instruction
     float4 nx[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) nx[i] = vrow[(4 * (xs >> 3) + i) * MROWS];
-    cross_factor_row(G, P, Q, sm.c.exptab, r >> sh.ly, r & (sh.TY - 1), xs, e0, q2);
-    // pass 1: the row maximum of |V E| (the leading products)
+    cross_factor_row(G, P, Q, sm.c.exptab, r >> sh.ly, r & (sh.TY - 1), x0, e0, q);
+    // pass 1: the row maximum of |V E|, of which only the exponent counts: leading parts alone
+    // (a value may exceed the scale by 2^-19 of it, which the first slice absorbs)
     float mx = 0.0f;
     {
-        ff2 e = e0;
+        float2 e = e0.hi;
 #pragma unroll 1
         for (int c = xs >> 3; 8 * c <= x1; c++) {
             float4 v4[4];
@@ -684,10 +696,10 @@ __device__ __forceinline__ int general_a_row(Smem &sm, const uint4 *vslot, const
             for (int i = 0; i < 4; i++) {
                 const int x = 8 * c + 2 * i;
                 if (x >= xs && x <= x1) {
-                    const float2 v = f2_mul(make_float2(v4[i].x, v4[i].z), e.hi);
+                    const float2 v = f2_mul(make_float2(v4[i].x, v4[i].z), e);
                     if (x >= x0) mx = fmaxf(mx, fabsf(v.x));
                     if (x < x1) mx = fmaxf(mx, fabsf(v.y));
-                    e = ff2_mul(e, q2);
+                    e = f2_mul(f2(e.y), q.hi);
                 }
             }
         }
@@ -714,7 +726,7 @@ __device__ __forceinline__ int general_a_row(Smem &sm, const uint4 *vslot, const
                 v = ff2_mul(ff2{make_float2(v4[i].x, v4[i].z), make_float2(v4[i].y, v4[i].w)}, ff2n_of(e));
                 if (x < x0) v.hi.x = v.lo.x = 0.0f;
                 if (x == x1) v.hi.y = v.lo.y = 0.0f;
-                e = ff2_mul(e, q2);
+                e = next_cross(e, q);
             }
             float2 sl[NSL];
             slice_scaled2(v, f2(sc), sl);
@@ -1060,7 +1072,7 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                 ff2 ecur = {f2(1.0f), f2(0.0f)};
                 ff2n eq = {};
                 if constexpr (kGeneral) {
-                    if (x0 <= x1) cross_factor_row(A.glv[td.level], P, Q, cm.exptab, z, y, x0 & ~1, ecur, eq);
+                    if (x0 <= x1) cross_factor_row(A.glv[td.level], P, Q, cm.exptab, z, y, x0, ecur, eq);
                 }
                 // tcgen05.ld is warp-collective: chunk decisions are made per warp
                 if (__any_sync(0xffffffffu, x0 <= x1)) {
@@ -1115,7 +1127,7 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                                     float2 rem = f2_sub(corr, f2_sub(h0, d2));  // lo = rem scl exactly
                                     if constexpr (kGeneral) {
                                         const int x = 8 * c + 2 * i;
-                                        if (x > x0 && x <= x1) ecur = ff2_mul(ecur, eq);  // E on the row's cube points
+                                        if (x > x0 && x <= x1) ecur = next_cross(ecur, eq);  // E on the row's cube points
                                         const ff2 v = ff2_mul(ff2{hi, f2_mul(rem, scl)}, ff2n_of(ecur));
                                         hi = v.hi;
                                         rem = v.lo;
@@ -1762,7 +1774,7 @@ __global__ void k_bin_pairs(const PairGeom *__restrict__ geoms, int64_t k0, int6
         if constexpr (kGen) {
             // lattice-index offsets from the product centre: d_a = cc_a + gg - gp_a
             const double c[3] = {g.off[0] - g.cc[0], g.off[1] - g.cc[1], g.off[2] - g.cc[2]};
-            const double rg = g.radius * g.radius * (1.0 + 1e-6) + 1e-12;
+            const double rt = tiled_radius(g), rg = rt * rt * (1.0 + 1e-6) + 1e-12;
             double lo[3], up[3];
             auto set = [&](int a, int g0, int g1) {  // false: the run's slab lies outside the sphere
                 lo[a] = g0 - c[a];
@@ -1844,7 +1856,8 @@ __global__ void k_make_records(const PairGeom *__restrict__ geoms, int64_t nbin,
         const LevelDev &lv = levels[g.level];
         TPair p;
         memset(&p, 0, sizeof p);
-        p.r2 = rmul(g.radius, g.radius);
+        const double radius = g.ortho ? g.radius : tiled_radius(g);
+        p.r2 = rmul(radius, radius);
         p.r2f = __double2float_rn(p.r2);
         p.zetp = split(g.zetp);
         p.lp = g.lp;
@@ -1860,7 +1873,7 @@ __global__ void k_make_records(const PairGeom *__restrict__ geoms, int64_t nbin,
             p.hx = rdiv(1.0, len[0]);
             p.hy = rdiv(1.0, len[1]);
             p.hz = rdiv(1.0, len[2]);
-            p.radius = g.radius;
+            p.radius = radius;
             for (int d = 0; d < 3; d++) {
                 p.h[d] = split(len[d]);
                 p.off[d] = split(rmul(rsub(g.off[d], (double)g.cc[d]), len[d]));
