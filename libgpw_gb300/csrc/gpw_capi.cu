@@ -705,7 +705,6 @@ int gpw_taskset_check(gpw_taskset *ts, void *stream) {
     if (h & kStatOutOfWindow) return fail(GPW_ERR_OUT_OF_WINDOW, "a cube left the local grid window");
     if (h & kStatTimeout) return fail(GPW_ERR_TIMEOUT, "a bounded device wait gave up");
     if (h & kStatBadTable) return fail(GPW_ERR_INVALID_ARG, "a cube list was inconsistent on the device");
-    if (h & kStatBadTile) return fail(GPW_ERR_INVALID_ARG, "a tile shape the collocate kernel does not hold");
     if (h & kStatTooManyImages)
         return fail(GPW_ERR_UNSUPPORTED, "a cube spans more periodic images than the tiled path handles");
     return GPW_SUCCESS;

@@ -293,7 +293,6 @@ enum : int {
     kStatTimeout = 2,
     kStatBadTable = 4,
     kStatTooManyImages = 8,
-    kStatBadTile = 16,
     kStatBadGeom = 32,      // a geometry update that the task set cannot take
 };
 

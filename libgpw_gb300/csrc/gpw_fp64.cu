@@ -142,7 +142,7 @@ __global__ void k_backtransform(const PairGeom *__restrict__ geoms, const LevelD
 //              lanes, T through shared memory), then W[lz][ly][lx] += Cxy Z[lz], the
 //              packed moments spread over the lanes' registers.
 // A row's range comes from the FP32 sphere rule where its error bound allows
-// (sphere_row_fast), one folded row per lane.
+// (sphere_jmax_fast, sphere_imax_fast), one folded row per lane.
 // The form before it (one CTA per pair, three barriers per plane, a shuffle
 // reduction of 11 accumulators per row, launches of similar pairs one after the
 // other) took 21.1 ms to integrate and 6.1 ms to collocate 1000 pairs (l <= 2,
@@ -658,7 +658,7 @@ k_general_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ 
 // General cell in float-float (the mixed path).  The value at a point of the index
 // box is P(di, dj, dk) exp(-zetp r^2), r^2 = G00 di^2 + A1 di + A0 along a row (metric
 // G = dh dh^T; A1, A0 per row in FP64, split to float-float); the row's i-range is the
-// reference's quadratic (general_row_checked), so the point set is the reference's.
+// reference's quadratic (general_row_fast32, general_row_unsure), so the point set is the reference's.
 //
 // As k_ortho_fp64: a CTA (4 warps) takes an item, a warp a plane, 64 rows at a time, a
 // lane a column i (blocks of 32, 16 or 8 columns):

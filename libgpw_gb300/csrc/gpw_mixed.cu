@@ -59,11 +59,11 @@ constexpr int TX = 32;
 constexpr int MROWS = 128;       // TY * TZ rows per tile, one per thread
 constexpr int kMaxTY = 32, kMaxTZ = 8;  // tiles of 32 x 16 x 8 or 32 x 32 x 4
 constexpr int kMaxTZColl = 8;  // collocate keeps its stage-1 output for at most 8 z (tiles with TZ <= 8)
+static_assert(kMaxTZ <= kMaxTZColl, "tile shapes that collocate holds");
 constexpr int NTHR = MROWS;
 constexpr int NSL = 4;          // slices per operand
 constexpr int SLB = 10;         // bits per slice
 constexpr int KP = 16;          // padded contraction length (alpha)
-constexpr int NPAIR_MAX = (kNPow * (kNPow + 1)) / 2;  // (b, a) with b + a <= lp
 constexpr int NCOEF_MAX = ((kMaxLp + 1) * (kMaxLp + 2) * (kMaxLp + 3)) / 6;
 
 // Periodic images of one axis of a cube over one tile.  Every image is an item of its
@@ -280,7 +280,6 @@ __device__ __forceinline__ uint32_t pack_halves(float2 s) {
 
 struct MixedArgs {
     const uint4 *blob;        // per pair: record (kHdr16 chunks) then float-float coefficients
-    const PairGeom *geoms;
     const LevelDev *levels;
     const TileDesc *tiles;
     const int64_t *start;
@@ -334,8 +333,8 @@ constexpr int kCxyRow = cxy_pad_row(kNPow, kNPow) / 2;      // 16-byte entries o
 
 // Collocate's re-expansion and stage 1 have one output per thread and turn, each the end
 // of a chain of up to lp + 1 steps: the outputs in order of falling chain length, so that
-// the lanes of a warp have chains of about one length (in packed order a warp's longest
-// was two to three times its mean: XX).
+// the lanes of a warp have chains of about one length (re-expansion at lp = 8: in packed
+// order a warp's longest chain was 2.4 times the mean of all, in this order 1.4 times).
 struct Order {
     uint32_t rec[d_decode_at(kNPow)];       // per lp: g | b << 4 | a << 8 | packed index << 16
     unsigned char st1[kNPow][2 * kCxyRow];  // [L - 1]: b | a << 4, the padding of rows as well
@@ -893,7 +892,7 @@ __device__ __forceinline__ void stage1_cxy(SmemColl &sm, int L, int lp, const Ti
 // two a per instruction, then the row's A slices (K slots below kw rewritten);
 // returns the row exponent.  b outer, the pairs of a unrolled inside (uniform exit at
 // the row's end), so that Y is read once per b; each sum renormalised once at the end.
-__device__ __forceinline__ int stage2_row(SmemColl &sm, const TileCommon &cm, int L, int lp, int z, int y, bool live,
+__device__ __forceinline__ int stage2_row(SmemColl &sm, int L, int lp, int z, int y, bool live,
                                           int kw, int m) {
     ff2 cx[kNPair];
 #pragma unroll
@@ -959,10 +958,6 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
         const int TY = sh.TY, TZ = sh.TZ;
         // a warp's 32 rows: 8 y x 4 z, so that more warps (and chunks) lie wholly outside a sphere
         const int wy = TY >> 3, y = (warp & (wy - 1)) * 8 + (m & 7), z = (warp / wy) * 4 + ((m >> 3) & 3);
-        if (TZ > kMaxTZColl) {  // shapes are validated on the host; never taken
-            if (tid == 0) atomicOr(A.status, kStatBadTile);
-            continue;
-        }
         float2 acc_hi[TX / 2];  // pairs of x; the low parts live in shared memory (registers for 4 CTAs per SM)
         float *acc_lo = sm.acc_lo[m];
 #pragma unroll
@@ -1043,7 +1038,7 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
                                       x1);
                 else
                     row_range(P, Q, A.table, Q.o[2] + z, Q.o[1] + y, row_ok, x0, x1);
-                const int em = stage2_row(sm, cm, L, lp, z, y, x0 <= x1, max(L, kprev), m);
+                const int em = stage2_row(sm, L, lp, z, y, x0 <= x1, max(L, kprev), m);
                 // stage 3 on the tensor cores: D_s = sum_{i+j=s} A_i B_j^T
                 // What follows reads none of the tables, and the record only on general cells:
                 // the next item's record, waited for here, and its tables may come in as the
@@ -1923,8 +1918,8 @@ int mixed_build(TaskSet &ts, std::string &err) {
     M->northo = (int)northo;
     // General-cell levels go on the tiled kernels when the cosine matrix C of the
     // lattice steps satisfies C >= 0.4 I: then sum t_d^2 <= 2.5 r^2, so inside the
-    // cube the cross factor exp(-2 zetp sum c_de t_d t_e) of the Gaussian stays
-    // within exp(+-58) (float range).  Otherwise they stay on the float-float
+    // cube the cross factor exp(-2 zetp sum c_de t_d t_e) = exp(zetp (sum t_d^2 -
+    // r^2)) of the Gaussian stays within exp(69) (tiled_radius).  Otherwise they stay on the float-float
     // general kernel.
     std::vector<GenLevel> glv(P.nlevels);
     bool gen_ok = true;
@@ -2250,7 +2245,6 @@ static MixedArgs make_args(const TaskSet &ts, const GridPtrs &g, int which, bool
     const int t0 = general ? M.ntiles_ortho : 0;
     MixedArgs a;
     a.blob = M.d_blob;
-    a.geoms = ts.d_geom;
     a.levels = ts.plan->d_levels;
     a.tiles = M.d_tiles + t0;
     a.start = M.d_start + 2 * t0;
@@ -2265,11 +2259,6 @@ static MixedArgs make_args(const TaskSet &ts, const GridPtrs &g, int which, bool
     a.status = ts.d_status;
     a.ntiles = general ? M.ntiles - M.ntiles_ortho : M.ntiles_ortho;
     return a;
-}
-
-// general-cell pairs of a mixed call run on the float-float general kernel
-static cudaError_t general_ff(const TaskSet &ts, const GridPtrs &g, bool adj, cudaStream_t s) {
-    return launch_general_ff(ts, g, adj, s);
 }
 
 // a tiled call that lacks pairs: an error status (a plain FP64 call must not see it)
@@ -2304,7 +2293,7 @@ cudaError_t launch_collocate_mixed(const TaskSet &ts, const GridPtrs &g, cudaStr
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
     }
-    return M.gen_tiled ? cudaSuccess : general_ff(ts, g, false, s);
+    return M.gen_tiled ? cudaSuccess : launch_general_ff(ts, g, false, s);
 }
 
 cudaError_t launch_integrate_mixed(const TaskSet &ts, const GridPtrs &g, cudaStream_t s) {
@@ -2334,7 +2323,7 @@ cudaError_t launch_integrate_mixed(const TaskSet &ts, const GridPtrs &g, cudaStr
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
     }
-    return M.gen_tiled ? cudaSuccess : general_ff(ts, g, true, s);
+    return M.gen_tiled ? cudaSuccess : launch_general_ff(ts, g, true, s);
 }
 
 }  // namespace gpw
