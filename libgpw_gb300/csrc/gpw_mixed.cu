@@ -1158,16 +1158,22 @@ __global__ void __launch_bounds__(NTHR, 4) k_collocate_tiled(MixedArgs A) {
             double *grid = A.grids.p[td.level];
             const int64_t row = ((int64_t)(td.t[2] * TZ + z) * lv.ngrid[1] + (td.t[1] * TY + y)) * lv.ngrid[0] +
                                 td.t[0] * TX;
-            // 8 points per iteration, acc_hi rotated by 8 after each (compact code)
+            // 8 points per iteration, acc_hi rotated by 8 after each (compact code); all eight
+            // loads first (left to the compiler, one build loaded, added and stored point by
+            // point: 1000 pairs on 256^3, 20 items a unit, 1.56 against 0.69 ms)
+            const bool split = td.flags & kUnitSplit;  // other work units add to the same tile
 #pragma unroll 1
             for (int c = 0; c < TX / 8; c++) {
+                double g8[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) g8[i] = split || 8 * c + i >= ext.x ? 0.0 : grid[row + 8 * c + i];
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
                     const int x = 8 * c + i;
                     if (x >= ext.x) continue;
                     const double v = (double)(i & 1 ? acc_hi[i / 2].y : acc_hi[i / 2].x) + (double)acc_lo[x];
-                    if (td.flags & kUnitSplit) atomicAdd(grid + row + x, v);  // other work units add to the same tile
-                    else grid[row + x] += v;
+                    if (split) atomicAdd(grid + row + x, v);
+                    else grid[row + x] = g8[i] + v;
                 }
 #pragma unroll
                 for (int i = 0; i < TX / 2 - 4; i++) acc_hi[i] = acc_hi[i + 4];
