@@ -186,11 +186,11 @@ cudaError_t launch_backward(const TaskSet &ts, const double *d_pab, const GridPt
     if (ts.ntasks == 0) return cudaSuccess;
     if (!backward_supported(ts)) return cudaErrorNotSupported;
     TaskSet &mts = const_cast<TaskSet &>(ts);
-    if (!mts.d_mom_ext) {  // the moments, then the divided pairs' slots
-        const int64_t parts = (int64_t)ts.fp64_slots * ncoef(ts.max_lp + 2);
-        cudaError_t e = cudaMalloc(&mts.d_mom_ext, sizeof(double) * std::max<int64_t>(ts.mom_ext_len + parts, 1));
+    if (!mts.d_mom_ext) {  // the moments, and the divided pairs' slots where the scratch memory is too small
+        const size_t parts = sizeof(double) * (size_t)ts.fp64_slots * ncoef(ts.max_lp + 2), own = parts > ts.scratch_bytes ? parts : 0;
+        cudaError_t e = cudaMalloc(&mts.d_mom_ext, std::max<size_t>(sizeof(double) * (size_t)ts.mom_ext_len + own, 8));
         if (e != cudaSuccess) return e;
-        mts.d_parts_ext = mts.d_mom_ext + ts.mom_ext_len;
+        mts.d_parts_ext = own ? mts.d_mom_ext + ts.mom_ext_len : static_cast<double *>(ts.d_scratch);
     }
     cudaError_t e = launch_moments_fp64(ts, g, 2, mts.d_mom_ext, s);
     if (e != cudaSuccess) return e;

@@ -577,13 +577,10 @@ int gpw_taskset_create(gpw_plan *plan, const gpw_task *tasks, int64_t ntasks, in
     alloc((void **)&T->d_coef, sizeof(double) * (size_t)coef);
     alloc((void **)&T->d_mom, sizeof(double) * (size_t)coef);
     alloc((void **)&T->d_status, sizeof(int));
-    // the FP64 items, and the divided pairs' slots and tickets, in one block
-    const size_t nitems = (size_t)(T->fp64_ortho + T->fp64_general), slots = (size_t)T->fp64_slots,
-                 items_len = (sizeof(Fp64Item) * nitems + 15) / 16 * 16,
-                 parts_len = sizeof(double) * slots * ncoef(T->max_lp);
-    alloc((void **)&T->d_fp64_items, items_len + parts_len + sizeof(int) * slots);
-    T->d_parts = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(T->d_fp64_items) + items_len);
-    T->d_ticket = reinterpret_cast<int *>(reinterpret_cast<unsigned char *>(T->d_parts) + parts_len);
+    // the FP64 items, then the divided pairs' tickets
+    const size_t nitems = (size_t)(T->fp64_ortho + T->fp64_general), slots = (size_t)T->fp64_slots;
+    alloc((void **)&T->d_fp64_items, sizeof(Fp64Item) * nitems + sizeof(int) * slots);
+    T->d_ticket = reinterpret_cast<int *>(T->d_fp64_items + nitems);
     if (e == cudaSuccess && slots > 0) e = cudaMemset(T->d_ticket, 0, sizeof(int) * slots);
     if (e == cudaSuccess && nitems > 0) {
         std::unique_ptr<Fp64Item[]> items(new Fp64Item[nitems]);
@@ -626,6 +623,7 @@ int gpw_taskset_destroy(gpw_taskset *ts) {
     cudaFree(ts->d_geom_next);
     cudaFree(ts->d_table);
     cudaFree(ts->d_fp64_items);
+    cudaFree(ts->d_scratch);
     cudaFree(ts->d_coef);
     cudaFree(ts->d_mom);
     cudaFree(ts->d_mom_ext);

@@ -1066,7 +1066,8 @@ void Fp64Planner::write(Fp64Item *items) {
 static cudaError_t launch_fp64_impl(const TaskSet &ts, const GridPtrs &g, bool adj, int extra, double *mom,
                                     cudaStream_t s) {
     const Plan &P = *ts.plan;
-    const PartSums ps = {extra ? ts.d_parts_ext : ts.d_parts, ts.d_ticket, ncoef(ts.max_lp + extra)};
+    const PartSums ps = {extra ? ts.d_parts_ext : static_cast<double *>(ts.d_scratch), ts.d_ticket,
+                         ncoef(ts.max_lp + extra)};
     if (ts.fp64_ortho > 0) {
         ProfScope prof(ts, s);
         const unsigned n = (unsigned)ts.fp64_ortho;
@@ -1113,7 +1114,7 @@ int smem_general_ff_limit(const PairGeom &g) {
 // one launch over the items of all general-cell pairs
 cudaError_t launch_general_ff(const TaskSet &ts, const GridPtrs &g, bool adj, cudaStream_t s) {
     if (ts.gen_count == 0) return cudaSuccess;
-    const PartSums ps = {ts.d_parts, ts.d_ticket, ncoef(ts.max_lp)};
+    const PartSums ps = {static_cast<double *>(ts.d_scratch), ts.d_ticket, ncoef(ts.max_lp)};
     ProfScope prof(ts, s);
     const unsigned n = (unsigned)ts.fp64_general;
     const Fp64Item *items = ts.d_fp64_items + ts.fp64_ortho;

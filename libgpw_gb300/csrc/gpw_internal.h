@@ -53,11 +53,15 @@ struct TaskSet {
     int fp64_smem_gen = 0, fp64_smem_gen_ext = 0;
     bool fp64_ext_fits = true;
     // divided pairs: per slot the part's moments (ext: to degree lp + 2), and at a pair's
-    // first slot the count of its parts that are done.  d_parts and d_ticket lie behind
-    // the items, d_parts_ext behind d_mom_ext.
+    // first slot the count of its parts that are done (behind the items)
     int fp64_slots = 0;
-    double *d_parts = nullptr, *d_parts_ext = nullptr;
+    double *d_parts_ext = nullptr;
     int *d_ticket = nullptr;
+    // Memory that only one launch at a time uses, allocated at creation and kept to the end
+    // (captured graphs hold its address): the parts' moments, or the tiled integrate
+    // kernel's V slots where they fit.
+    void *d_scratch = nullptr;
+    size_t scratch_bytes = 0;
     MixedState *mixed = nullptr;
     int tile_lz[GPW_MAX_LEVELS];   // tiled path: log2 of the tile's z extent per level
     int gen_first = 0, gen_count = 0, gen_smem = 0;  // general-cell pairs (float-float kernel)

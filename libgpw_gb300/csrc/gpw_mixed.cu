@@ -165,7 +165,7 @@ struct MixedState {
     int ntiles_ortho = 0;        // tiles [0, ntiles_ortho) are orthorhombic, the rest general
     int sms = 0;
     int per_sm = 0, per_sm_i = 0, per_sm_ig = 0;  // resident CTAs: collocate, integrate (ortho, general)
-    uint4 *d_vslot = nullptr;  // integrate: per-CTA V slots
+    uint4 *d_vslot = nullptr, *own_vslot = nullptr;  // integrate: per-CTA V slots, in the scratch memory or their own
     // binning state kept for re-binning on the device (gpw_taskset_update_geometry)
     std::vector<TileDesc> h_tiles;  // every tile of the binned levels, in tile-index order
     struct BinLevel *d_bl = nullptr;  // per level: first tile index, tiles per axis, tile shape
@@ -2079,12 +2079,19 @@ int mixed_build(TaskSet &ts, std::string &err) {
     M->per_sm_ig = resident(ki[1], sizeof(SmemInt));
     M->sms = sms;
     // one V slot per resident integrate CTA
-    if (nbin > 0) {
-        e = cudaMalloc(&M->d_vslot, sizeof(uint4) * kVSlot16 * (size_t)sms * std::max(per_sm_i, M->per_sm_ig));
-        if (e != cudaSuccess) {
-            err = std::string("mixed_build: ") + cudaGetErrorString(e);
-            return GPW_ERR_CUDA;
-        }
+    const size_t vbytes = nbin > 0 ? sizeof(uint4) * kVSlot16 * (size_t)sms * std::max(per_sm_i, M->per_sm_ig) : 0;
+    if (!ts.d_scratch) {
+        ts.scratch_bytes = std::max(vbytes, sizeof(double) * (size_t)ts.fp64_slots * ncoef(ts.max_lp));
+        if (ts.scratch_bytes > 0) e = cudaMalloc(&ts.d_scratch, ts.scratch_bytes);
+    }
+    M->d_vslot = static_cast<uint4 *>(ts.d_scratch);
+    if (e == cudaSuccess && vbytes > ts.scratch_bytes) {
+        e = cudaMalloc(&M->own_vslot, vbytes);
+        M->d_vslot = M->own_vslot;
+    }
+    if (e != cudaSuccess) {
+        err = std::string("mixed_build: ") + cudaGetErrorString(e);
+        return GPW_ERR_CUDA;
     }
     return mixed_rebin(ts, err);
 }
@@ -2238,7 +2245,7 @@ void mixed_free(TaskSet &ts) {
     cudaFree(M->d_iimg);
     cudaFree(M->d_queue);
     cudaFree(M->d_glv);
-    cudaFree(M->d_vslot);
+    cudaFree(M->own_vslot);
     cudaFree(M->d_bl);
     cudaFree(M->d_blob_len);
     cudaFree(M->d_count);

@@ -140,3 +140,29 @@ def test_long_cubes_backward(axis, n, oracle_lib):
     assert np.abs(dra.cpu().numpy()[0] - want).max() <= 1e-12 * 3.0 * size
     assert abs(float(dza) + (w * (X * X + Y * Y + Z * Z)).sum()) <= 1e-12 * 9.0 * size
     assert np.abs(hab.cpu().numpy() - oracle_lib.batch(wl, V=V)).max() <= 1e-12 * np.abs(w).sum() / abs(wl.pab[0])
+
+
+@pytest.mark.parametrize("ortho", [True, False])
+def test_captured_integrate_between_mixed_calls(ortho):
+    """The parts' moments share their memory with the tiled integrate kernel's V slots: a captured FP64
+    call gives the same bits after mixed calls, new tiles (general cells: the slots' first use) and a backward pass."""
+    import torch
+
+    cell = 10.0 if ortho else T.lattice_15(length=10.0)
+    wl = T.synthetic("captured", 6, 2, (0.2, 0.4), cell, [(64,) * 3], 9, ortho=ortho)
+    ts = capi.TaskSet.from_workload(capi.Plan(wl.levels), wl)
+    V, pab, hab, other = [_dev(v) for v in wl.potentials(seed=3)], _dev(wl.pab), _zeros(wl.pab.size), _zeros(wl.pab.size)
+    ts.integrate(V, hab)
+    torch.cuda.synchronize()
+    want = hab.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ts.integrate(V, hab)
+    for tz in (8, 4):
+        ts.set_tiles([tz])
+        ts.integrate(V, other, "mixed")
+        ts.backward(pab, V, other, dra := _zeros(6, 3))
+        hab.zero_()
+        graph.replay()
+        ts.check()
+        assert torch.equal(hab, want) and bool(dra.any())
