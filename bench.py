@@ -190,13 +190,13 @@ class Clocks:
 
 # ----------------------------------------------------------------------------
 # DRAM bytes (read + write) of one launch of each tiled kernel on the 1M-pair
-# workload (256^3, tile 32 x 16 x 8, 79,272,268 (tile, pair) items), from a
-# single-pass ncu capture of dram__bytes_read.sum + dram__bytes_write.sum with
-# gpu__time_duration.sum.  Other workloads scale it by their item count (an
+# workload (256^3, tile 32 x 16 x 8, 79,305,840 items, one per tile and pair image),
+# from a single-pass ncu capture of dram__bytes_read.sum + dram__bytes_write.sum
+# with gpu__time_duration.sum.  Other workloads scale it by their item count (an
 # estimate: the share of a pair's record and coefficients served by L2 depends
 # on the workload).
-TRAFFIC_1M = {"k_collocate_tiled": (9.028e9 + 0.193e9, 79_272_268),
-              "k_integrate_tiled": (9.510e9 + 2.966e9, 79_272_268)}
+TRAFFIC_1M = {"k_collocate_tiled": (9.095e9 + 0.177e9, 79_305_840),
+              "k_integrate_tiled": (9.558e9 + 2.888e9, 79_305_840)}
 
 
 def algorithmic_flops(wl) -> tuple:
@@ -544,11 +544,11 @@ def main():
                 "frac": achieved_tf / peak,
                 "traffic": TRAFFIC_1M[kname][0] * items / TRAFFIC_1M[kname][1],
                 "traffic_basis": "measured on the 1M-pair workload (one-pass ncu capture), scaled by this "
-                                 "launch's (tile, pair) items",
+                                 "launch's items (tile, pair image)",
                 "items_per_launch": items,
                 "peak_source": "bf16 sustained, MEASURED_PEAKS.json (of measured)",
                 "limiter": "FP32/integer instruction issue of the float-float stages, not the tensor pipe "
-                           "(tensor pipe active ~5%, issue slots busy 55% collocate / 49% integrate in the ncu captures)"}
+                           "(tensor pipe active ~5%, issue slots busy 56% collocate / 51% integrate in the ncu captures)"}
     else:
         hbm = peaks.get("hbm_gbs") or 6800.0
         gbytes_alg = 16.0 * points  # FP64 read+write per cube point (no reuse)

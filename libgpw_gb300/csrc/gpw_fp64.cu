@@ -146,7 +146,7 @@ __global__ void k_backtransform(const PairGeom *__restrict__ geoms, const LevelD
 // The form before it (one CTA per pair, three barriers per plane, a shuffle
 // reduction of 11 accumulators per row, launches of similar pairs one after the
 // other) took 21.1 ms to integrate and 6.1 ms to collocate 1000 pairs (l <= 2,
-// 64^3); this one takes 0.46 and 0.46 ms, 62 % of the FP64 rate (1.10 TFLOP/s in a
+// 64^3); this one takes 0.45 and 0.42 ms, 65 % of the FP64 rate (1.10 TFLOP/s in a
 // GEMM) counting L multiply-adds per cube point.
 constexpr int kOrthoWarps = 4;  // (a power of two)
 
@@ -669,8 +669,8 @@ k_general_fp64(const PairGeom *__restrict__ geoms, const Fp64Item *__restrict__ 
 // values) is converted on the integer pipe: the FP64 pipe takes 17 cycles per
 // instruction, conversions included.  (One warp per row, points one at a time, shuffle
 // reductions per row and conversions on the FP64 pipe: 6.84 ms to integrate and 3.86 ms
-// to collocate 1500 pairs, l <= 4, 128^3; this form 4.20 and 3.66 ms.)  128 registers
-// for four CTAs per SM: with 232 (two CTAs) 5.52 and 4.53 ms, the chains being long.
+// to collocate 1500 pairs, l <= 4, 128^3; this form 3.98 and 3.21 ms.)  128 registers
+// for four CTAs per SM: with 232 (two CTAs) 5.52 and 4.53 against 4.42 and 3.68 ms, the chains being long.
 constexpr int kGenRows = 64;  // rows of a plane in hand
 
 // a warp's working set (floats): row data, Qjk; integrate: T of the block's columns
